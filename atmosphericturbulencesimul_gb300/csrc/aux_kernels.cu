@@ -382,33 +382,54 @@ __device__ __forceinline__ void philox4x32_10(uint32_t c[4], uint32_t k0, uint32
 
 // ---------------------------------------------------------------------------
 // Frame copy-out into the caller's sink (pinned host or device memory).
-// The host link, not the issuer, bounds a device-to-host copy (about 190
-// GB/s here for the copy engine and for SM stores alike), and 8 CTAs of
+//
+// Pinned host memory: the host link, not the issuer, bounds the copy (about
+// 190 GB/s here for the copy engine and for SM stores alike), and 8 CTAs of
 // plain 16-byte stores reach 185 GB/s while holding 8 of the 152 SMs; the
 // copy engine reading the frames meanwhile slows the passes more (measured
 // on the batched series: 29,291 frames/s end to end with 8 copy CTAs, 29,153
 // with 16, 27,811 with 32, 26,280 with the copy engine).
+//
+// Device memory: HBM bounds the copy, and the same 8 CTAs (185 GB/s) would
+// take longer than the step itself (a 512^2 phase-only fan of 16 directions:
+// 181 of 307 us per step), so the grid covers the GPU, four CTAs per SM with
+// four 16-byte loads in flight per thread.
 // ---------------------------------------------------------------------------
+__device__ __forceinline__ void copy_f4(const float4* __restrict__ s, float4* __restrict__ d, long n)
+{
+    const long stride = (long)gridDim.x * blockDim.x;
+    long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
+    for (; i + 3 * stride < n; i += 4 * stride) {
+        const float4 a = s[i], b = s[i + stride], c = s[i + 2 * stride], e = s[i + 3 * stride];
+        d[i] = a;
+        d[i + stride] = b;
+        d[i + 2 * stride] = c;
+        d[i + 3 * stride] = e;
+    }
+    for (; i < n; i += stride) d[i] = s[i];
+}
+
 __global__ void k_copy_out(const float4* __restrict__ s0, float4* __restrict__ d0, long n0,
                            const float4* __restrict__ s1, float4* __restrict__ d1, long n1)
 {
-    const long stride = (long)gridDim.x * blockDim.x;
-    for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n0; i += stride) d0[i] = s0[i];
-    for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n1; i += stride) d1[i] = s1[i];
+    copy_f4(s0, d0, n0);
+    copy_f4(s1, d1, n1);
 }
 
 cudaError_t copy_out(const float4* src0, float4* dst0, long n0, const float4* src1, float4* dst1, long n1,
-                     cudaStream_t st)
+                     bool device_sink, cudaStream_t st)
 {
     if (!dst0) n0 = 0;
     if (!dst1) n1 = 0;
     if (n0 + n1 == 0) return cudaSuccess;
-    // CTAs of the copy (ATMWFS_COPY_CTAS overrides the measured default)
-    static const int ctas = [] {
+    // CTAs of a copy to host memory (ATMWFS_COPY_CTAS overrides the measured default)
+    static const int host_ctas = [] {
         const char* e = getenv("ATMWFS_COPY_CTAS");
         const int v = e ? atoi(e) : 0;
         return v >= 1 && v <= 152 ? v : 8;
     }();
+    const long need = (std::max(n0, n1) + 255) / 256;
+    const int ctas = device_sink ? (int)std::min<long>(need, 4 * 152) : host_ctas;
     k_copy_out<<<ctas, 256, 0, st>>>(src0, dst0, n0, src1, dst1, n1);
     return cudaGetLastError();
 }

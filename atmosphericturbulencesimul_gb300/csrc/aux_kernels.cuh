@@ -18,7 +18,7 @@ cudaError_t group_sums(const GroupSumJob* jobs, int njobs, int L, int maxside, c
 // Frame copy-out by a small grid of copy CTAs (16-byte aligned pointers,
 // counts in float4): dst0 = src0, dst1 = src1 (either pair may be absent).
 cudaError_t copy_out(const float4* src0, float4* dst0, long n0, const float4* src1, float4* dst1, long n1,
-                     cudaStream_t st);
+                     bool device_sink, cudaStream_t st);
 cudaError_t screen_spectrum(uint64_t seed, uint32_t stream, int M, double fo, double fi, float2* C, cudaStream_t st);
 cudaError_t strf_lags(const float2* F, int M, double* acc, cudaStream_t st);
 cudaError_t split_scale(const float2* F, long n, double s1, double s2, float* o1, float* o2, cudaStream_t st);

@@ -1293,6 +1293,7 @@ atmwfs_status atmwfs_run(atmwfs_ctx* c, long nsteps, const atmwfs_sink* sink)
     // copy kernel when the sink is pinned host or device memory on 16-byte
     // boundaries (frames are a multiple of four floats); else the copy engine
     bool by_kernel = copies && c->frame_floats % 4 == 0;
+    bool device_sink = true;                  // every sink buffer is device memory
     float* dev_sink[2] = {nullptr, nullptr};  // the sink as the device addresses it
     for (int o = 0; o < 2 && by_kernel; o++) {
         float* p = o == 0 ? sink->pha : sink->amp;
@@ -1305,6 +1306,7 @@ atmwfs_status atmwfs_run(atmwfs_ctx* c, long nsteps, const atmwfs_sink* sink)
         }
         const bool reachable = pa.type == cudaMemoryTypeDevice || pa.type == cudaMemoryTypeHost ||
                                pa.type == cudaMemoryTypeManaged;
+        device_sink = device_sink && pa.type == cudaMemoryTypeDevice;
         dev_sink[o] = static_cast<float*>(pa.devicePointer);
         if (!reachable || !dev_sink[o] || (reinterpret_cast<uintptr_t>(dev_sink[o]) & 15) != 0) by_kernel = false;
     }
@@ -1348,7 +1350,7 @@ atmwfs_status atmwfs_run(atmwfs_ctx* c, long nsteps, const atmwfs_sink* sink)
                     auto f4 = [](const float* q) { return reinterpret_cast<const float4*>(q); };
                     auto h4 = [&](float* q) { return q ? reinterpret_cast<float4*>(q + (size_t)hs * ff) : nullptr; };
                     AW_CUDA(copy_out(f4(c->d_out_pha + slot * ff), h4(dev_sink[0]), (long)(ff / 4),
-                                     f4(c->d_out_amp + slot * ff), h4(dev_sink[1]), (long)(ff / 4), c->out_st));
+                                     f4(c->d_out_amp + slot * ff), h4(dev_sink[1]), (long)(ff / 4), device_sink, c->out_st));
                 } else {
                     if (sink->pha)
                         AW_CUDA(cudaMemcpyAsync(sink->pha + (size_t)hs * ff, c->d_out_pha + slot * ff, sizeof(float) * ff,
