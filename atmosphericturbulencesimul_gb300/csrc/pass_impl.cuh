@@ -233,7 +233,9 @@ __device__ __forceinline__ void fft_rt(float2* v, float2* xrow, int t, const flo
                                        const float2* twr = nullptr)
 {
     if (ds > 0.0f) conj_all<E>(v);     // inverse = conj(forward(conj))
-    if constexpr (V != 0 && Stages<N, V>::S == 3) {
+    // (the whole-row transforms above 2048 keep the stage loop: 8192^2 882 us
+    // against 933 with this form)
+    if constexpr (Stages<N, V>::S == 3 && N <= 2048) {
         constexpr int R0 = Stages<N, V>::R0, R1 = Stages<N, V>::R1, R2 = Stages<N, V>::R2;
         if (rev) fft3_ct<N, T, E, R2, R1, R0>(v, xrow, t, tw + tw_offset<N, V>(1, 1), tw + tw_offset<N, V>(1, 2));
         else fft3_ct<N, T, E, R0, R1, R2>(v, xrow, t, tw + tw_offset<N, V>(0, 1), tw + tw_offset<N, V>(0, 2));
