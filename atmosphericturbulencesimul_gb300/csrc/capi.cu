@@ -1570,7 +1570,7 @@ static atmwfs_status two_pass(const void* in, void* out, long n, int var, const 
     if (!tw) return fail(ATMWFS_ERR_NOMEM, "twiddle allocation failed");
     float2* tmp = nullptr;
     AW_CUDA(cudaMallocAsync((void**)&tmp, sizeof(float2) * n * n, st));
-    const int RR = rows_per_cta((int)n);
+    const int RR = unit_rows((int)n);
     PassArgs a;
     memset(&a, 0, sizeof a);
     a.H1 = H;

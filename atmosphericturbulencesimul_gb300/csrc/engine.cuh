@@ -61,10 +61,11 @@ inline int& pdl_hold()
 }
 
 // Launch k<<<grid, block, sm, st>>>(args...), with programmatic stream
-// serialization when the grid is small (above); k must open with
+// serialization when the grid has at most max_ctas CTAs; k must open with
 // pdl_gate().
 template <typename... P, typename... A>
-cudaError_t launch_gated(void (*k)(P...), dim3 grid, dim3 block, size_t sm, cudaStream_t st, A&&... args)
+cudaError_t launch_gated_up_to(long max_ctas, void (*k)(P...), dim3 grid, dim3 block, size_t sm, cudaStream_t st,
+                               A&&... args)
 {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
@@ -75,8 +76,13 @@ cudaError_t launch_gated(void (*k)(P...), dim3 grid, dim3 block, size_t sm, cuda
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
-    cfg.numAttrs = pdl_hold() == 0 && (long)grid.x * grid.y * grid.z <= pdl_max_ctas() ? 1 : 0;
+    cfg.numAttrs = pdl_hold() == 0 && (long)grid.x * grid.y * grid.z <= max_ctas ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, k, std::forward<A>(args)...);
+}
+template <typename... P, typename... A>
+cudaError_t launch_gated(void (*k)(P...), dim3 grid, dim3 block, size_t sm, cudaStream_t st, A&&... args)
+{
+    return launch_gated_up_to(pdl_max_ctas(), k, grid, block, sm, st, std::forward<A>(args)...);
 }
 
 constexpr int kMaxLayers = 16;
@@ -262,8 +268,21 @@ inline int phasum_blocks(int Nout)
     return (int)(n < 1024 ? n : 1024);
 }
 
-// Rows per CTA of configuration 0 (unit operators).
-inline int rows_per_cta(int N) { return tile_cfg(N, 0).rr; }
+// Unit operators (one 2-D transform or hop: two row passes of one image).
+// One image has N rows, so the shape decides how many SMs work on it, and the
+// transposed store writes runs of 8 unit_rows bytes.  Measured as pairs of
+// passes (us, transform / hop):
+//   256: 16 rows 5.4 / 7.6, 8 rows 4.4 / 5.6, 4 rows 4.3 / 5.4, 2 rows 4.4 / 5.4
+//   512: 16 rows 8.5 / 12.8, 8 rows 6.3 / 8.9, 4 rows 6.3 / 8.4, 2 rows 6.7 / 8.5
+//   1024: 8 rows 9.3 / 12.8, 4 rows 12.2 / 16.3 (more CTAs than SMs, 32-byte runs)
+//   2048: 4 rows 47 / 68, 2 rows 48 / 66 (16-byte runs)
+// 64 and 128 lie within 0.3 us of each other below 32 rows.
+constexpr int unit_rows(int N) { return N <= 64 ? 16 : N <= 128 ? 8 : N <= 512 ? 4 : N <= 1024 ? 8 : 4; }
+// The two passes of a unit operator run alone on their stream, so they take
+// programmatic dependent launch up to this many CTAs per SM, not one: there is
+// no branch of a step whose SM slots the waiting CTAs would hold (2048
+// transform pair: 51 -> 47 us).
+constexpr int kUnitPdlWaves = 8;
 
 PassLauncher pass_launcher(int N);
 PassLauncherCfg pass_launcher_cfg(int N);

@@ -26,7 +26,6 @@ using namespace atmwfs;
 constexpr long kMaxN = ATMWFS_NOALLOC_MAX_N;
 constexpr long kMaxTw = 2 * kMaxN;  // stage twiddle tables of the largest grid
 constexpr int kMaxDevices = 64;
-constexpr double kPi = 3.14159265358979323846264338328;
 
 // Scratch shared by every call on a device: the field after the first
 // (transposed) pass, the 1-D transfer table and the twiddles of the call's
@@ -73,19 +72,25 @@ atmwfs_status scratch_for_current_device(Scratch** out)
 // One thread per entry of the call's tables, evaluated in double like the
 // host tables of the allocating path:
 //   table[k] = exp(-i c f_k^2) / n, f_k the centred frequency of unshifted
-//   index k, the angle reduced to [-pi, pi] in double before the cosine and
-//   sine (Fresnel_propagate_wavefront, WFpropagate.c:68-152);
+//   index k, c f^2 = pi t f^2 with t = z lambda / (dx n)^2, so that sincospi
+//   reduces the angle in double (Fresnel_propagate_wavefront,
+//   WFpropagate.c:68-152);
 //   twiddles: for each order (o = 0, 1) and stage st >= 1 of the size's plan,
 //   tab[r * ns + k] = exp(-2 pi i k r / (ns R)) at offset tw_offset(o, st).
+// FP64 bounds it: an SM of this part does about two double FMAs a cycle, so
+// the 3 n entries go one warp to a CTA, over as many SMs as there are warps
+// (256-thread CTAs put 256^2's tables on three SMs: 6.6 us).
+constexpr int kTableThreads = 32;
 template <int N>
-__global__ void k_noalloc_tables(double coeff)
+__global__ void __launch_bounds__(kTableThreads) k_noalloc_tables(double t)
 {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
+    pdl_gate();
+    const int j = blockIdx.x * kTableThreads + threadIdx.x;
+    double s, c;
     if (j < N) {
         const long f = j < N / 2 ? j : j - N;
-        double ang = -coeff * (double)(f * f);
-        ang -= 2.0 * kPi * nearbyint(ang / (2.0 * kPi));
-        g_table[j] = make_float2((float)(cos(ang) / N), (float)(sin(ang) / N));
+        sincospi(-t * (double)(f * f), &s, &c);
+        g_table[j] = make_float2((float)(c / N), (float)(s / N));
         return;
     }
     const int i = j - N;
@@ -96,28 +101,28 @@ __global__ void k_noalloc_tables(double coeff)
             const int R = stage_radix<N>(st, o), ns = stage_ns<N>(st, o);
             if (i < base || i >= base + R * ns) continue;
             const int r = (i - base) / ns, k = (i - base) % ns;
-            const double a = -2.0 * kPi * (double)(k * r) / (double)(ns * R);
-            g_twiddle[i] = make_float2((float)cos(a), (float)sin(a));
+            sincospi(-2.0 * (double)(k * r) / (double)(ns * R), &s, &c);
+            g_twiddle[i] = make_float2((float)c, (float)s);
             return;
         }
 }
 
 template <int N>
-cudaError_t launch_tables_n(double coeff, cudaStream_t cs)
+cudaError_t launch_tables_n(double t, cudaStream_t cs)
 {
     if (tw_total<N>() > kMaxTw) return cudaErrorInvalidValue;  // the static twiddle array is too small
     const int total = N + tw_total<N>();
-    k_noalloc_tables<N><<<(total + 255) / 256, 256, 0, cs>>>(coeff);
-    return cudaGetLastError();
+    return launch_gated(k_noalloc_tables<N>, dim3((total + kTableThreads - 1) / kTableThreads), dim3(kTableThreads), 0, cs,
+                        t);
 }
 
-cudaError_t launch_tables(long n, double coeff, cudaStream_t cs)
+cudaError_t launch_tables(long n, double t, cudaStream_t cs)
 {
     switch (n) {
-        case 64: return launch_tables_n<64>(coeff, cs);
-        case 128: return launch_tables_n<128>(coeff, cs);
-        case 256: return launch_tables_n<256>(coeff, cs);
-        case 512: return launch_tables_n<512>(coeff, cs);
+        case 64: return launch_tables_n<64>(t, cs);
+        case 128: return launch_tables_n<128>(t, cs);
+        case 256: return launch_tables_n<256>(t, cs);
+        case 512: return launch_tables_n<512>(t, cs);
         default: return cudaErrorInvalidValue;
     }
 }
@@ -141,8 +146,8 @@ extern "C" atmwfs_status atmwfs_fresnel_noalloc(const void* in, void* out, long 
     // transfer table and twiddles of this size, written into the static
     // arrays by a kernel on the caller's stream: nothing is copied from host
     // memory, so the call does not wait for the stream to drain
-    const double coeff = kPi * z * lambda / (dx * (double)n) / (dx * (double)n);
-    cudaError_t e = launch_tables(n, coeff, cs);
+    const double t = z * lambda / (dx * (double)n) / (dx * (double)n);
+    cudaError_t e = launch_tables(n, t, cs);
     if (e != cudaSuccess) return err(ATMWFS_ERR_CUDA, cudaGetErrorString(e));
     const PassLauncher fn = pass_launcher((int)n);
     PassArgs a;
@@ -151,7 +156,7 @@ extern "C" atmwfs_status atmwfs_fresnel_noalloc(const void* in, void* out, long 
     a.H2 = s->table;
     a.ext_in = (const float2*)in;
     a.ext_out = s->field;
-    const dim3 grid((unsigned)(n / rows_per_cta((int)n)), 1);
+    const dim3 grid((unsigned)(n / unit_rows((int)n)), 1);
     e = fn(kVarUnitProp, grid, a, nullptr, s->twiddle, cs);
     if (e == cudaSuccess) {
         a.ext_in = s->field;

@@ -751,8 +751,9 @@ __global__ void __launch_bounds__(kPhasumThreads, 4) k_phasum(const __grid_const
 }
 
 // host launcher for one (N, configuration); SO: the series passes only (the
-// unit operators, phase sums and windows launch in configuration 0)
-template <int N, int RR, int MINB, bool ALIAS, bool HP = false, int V = 0, bool SO = false, bool HS = false>
+// phase sums and windows launch in configuration 0); UNIT: the unit operators
+template <int N, int RR, int MINB, bool ALIAS, bool HP = false, int V = 0, bool SO = false, bool HS = false,
+          bool UNIT = false>
 cudaError_t launch_pass_t(int var, dim3 grid, const PassArgs& a, const TmaSet* maps, const float2* tw, cudaStream_t st)
 {
     using G = PassGeom<N, RR, V>;
@@ -768,9 +769,16 @@ cudaError_t launch_pass_t(int var, dim3 grid, const PassArgs& a, const TmaSet* m
             if (e != cudaSuccess) return e;                                                            \
             attr = true;                                                                               \
         }                                                                                              \
-        return launch_gated(k_pass<N, RR, MINB, VAR, ALIAS, HP, V, HS>, grid, block, sm, st, a, m, tw); \
+        return launch_gated_up_to(I_SERIES(VAR) ? pdl_max_ctas() : kUnitPdlWaves * pdl_max_ctas(), k_pass<N, RR, MINB, VAR, ALIAS, HP, V, HS>, grid, block, sm, st, a, m, tw); \
     }
-    if constexpr (HP || V != 0 || SO || HS) {
+    if constexpr (UNIT) {
+        switch (var) {
+            AW_CASE(kVarUnitProp)
+            AW_CASE(kVarUnitFwd)
+            AW_CASE(kVarUnitInv)
+            default: return cudaErrorInvalidValue;
+        }
+    } else if constexpr (HP || V != 0 || SO || HS) {
         // FP16 transforms, the alternative radix plans and configurations
         // other than 0: the series passes only
         switch (var) {
@@ -786,9 +794,6 @@ cudaError_t launch_pass_t(int var, dim3 grid, const PassArgs& a, const TmaSet* m
         AW_CASE(kVarMid)
         AW_CASE(kVarLast)
         AW_CASE(kVarSingle)
-        AW_CASE(kVarUnitProp)
-        AW_CASE(kVarUnitFwd)
-        AW_CASE(kVarUnitInv)
         case kVarPhasum: {
             return launch_gated(k_phasum<N>, grid, dim3(kPhasumThreads), 0, st, a);
         }
@@ -811,8 +816,7 @@ cudaError_t launch_pass_t(int var, dim3 grid, const PassArgs& a, const TmaSet* m
 template <int N>
 cudaError_t launch_pass_n(int var, dim3 grid, const PassArgs& a, const TmaSet* maps, const float2* tw, cudaStream_t st)
 {
-    constexpr TileCfg c0 = tile_cfg(N, 0);
-    return launch_pass_t<N, c0.rr, c0.minb, c0.alias>(var, grid, a, maps, tw, st);
+    return launch_pass_t<N, unit_rows(N), 1, false, false, 0, false, false, true>(var, grid, a, maps, tw, st);
 }
 
 // FP16-transform passes: tile configuration 2, tw = the FP16 twiddle table
