@@ -30,6 +30,7 @@ bool fft2d_large_supported(long M);
 // Concatenated stage twiddle tables of the in-CTA transform of size N
 // (64..2048), device memory owned by the library.
 const float2* stage_twiddles(int N);
+const float2* circle_table(int M);
 
 // PSF consumers (psf.cu): row and column passes of zero-padded fields and
 // the chromatic zoom sum.

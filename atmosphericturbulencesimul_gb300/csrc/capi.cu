@@ -108,6 +108,14 @@ static std::vector<float2> host_twiddles(int N, int V = 0)
         build_twiddles<1024, 1>(h.data());
         return h;
     }
+    if (V == 2) {  // the whole circle (circle_table)
+        h.resize(N);
+        for (int k = 0; k < N; k++) {
+            const double a = -2.0 * kPi * (double)k / (double)N;
+            h[k] = make_float2((float)cos(a), (float)sin(a));
+        }
+        return h;
+    }
     if (V != 0) return h;
     switch (N) {
         case 64: h.resize(tw_total<64>()); build_twiddles<64>(h.data()); break;
@@ -173,6 +181,9 @@ static const float2* twiddles(int N, int V = 0)
 }
 
 const float2* stage_twiddles(int N) { return twiddles(N); }
+
+// exp(-2 pi i k / M), k = 0 .. M - 1, kept like the stage tables.
+const float2* circle_table(int M) { return twiddles(M, 2); }
 
 // The same tables rounded to FP16 for the FP16-transform passes.
 static const __half2* twiddles_half(int N)

@@ -32,16 +32,18 @@ void set_error_message(const char* msg);
 // rows per CTA: 128 threads per CTA at every size
 template <int N> struct PsfRows { static constexpr int RR = N <= 128 ? 16 : N <= 512 ? 8 : N == 1024 ? 4 : 2; };
 
-// Row pass.  Field b: rows [off, off + W) hold amp * exp(i c_b pha) at
-// columns [off, off + W); zero elsewhere.  Writes G[b][kx][y] for the band
-// rows y (the other entries of G are never read).
-template <int N>
+// Row pass.  Field b: rows and columns [0, W) hold amp * exp(i c_b pha), the
+// rest is zero (PAD: W = N / 2, else W = N).  The reference places an exposure
+// frame at offset W / 2; the origin only turns the phase of the transform, of
+// which |F|^2 is kept, and at offset 0 a thread's values are all frame or all
+// padding.  Writes G[b][kx][y], y < W.
+template <int N, bool PAD>
 __global__ void __launch_bounds__(Plan<N>::T * PsfRows<N>::RR)
 k_psf_rows(const float* __restrict__ amp, long amp_fstride, const float* __restrict__ pha, long pha_fstride,
-           const float* __restrict__ cscale, int W, int off, float2* __restrict__ G, const float2* __restrict__ tw)
+           const float* __restrict__ cscale, float2* __restrict__ G, const float2* __restrict__ tw)
 {
     constexpr int RR = PsfRows<N>::RR, T = Plan<N>::T, E = Plan<N>::E, NT = T * RR, RS = row_stride<N>();
-    constexpr int RL = last_radix<N>();
+    constexpr int RL = last_radix<N>(), W = PAD ? N / 2 : N;
     __shared__ __align__(16) float2 xb[RR * RS];
     const int tid = threadIdx.x, t = tid % T, rr = tid / T;
     const int b = blockIdx.y;
@@ -53,10 +55,9 @@ k_psf_rows(const float* __restrict__ amp, long amp_fstride, const float* __restr
     float2 v[E];
 #pragma unroll
     for (int e = 0; e < E; e++) {
-        const int xi = t + e * T - off;
-        if (xi >= 0 && xi < W) {
-            const float a = A[xi];
-            const float2 z = phasor(__fmul_rn(c, P[xi]));     // c * pha: float, as the reference's image product
+        if (e * T < W) {
+            const float a = A[t + e * T];
+            const float2 z = phasor(__fmul_rn(c, P[t + e * T]));     // c * pha: float, as the reference's image product
             v[e] = make_float2(a * z.x, a * z.y);
         } else {
             v[e] = make_float2(0.0f, 0.0f);
@@ -67,12 +68,12 @@ k_psf_rows(const float* __restrict__ amp, long amp_fstride, const float* __restr
 #pragma unroll
     for (int s = 0; s < E; s++) xrow[padi(last_index<N, T, RL>(t, s))] = v[s];
     __syncthreads();
-    float2* dst = G + (size_t)b * N * N + off + blockIdx.x * RR;
+    float2* dst = G + (size_t)b * N * W + blockIdx.x * RR;
 #pragma unroll 4
     for (int k = 0; k < E; k++) {
         const int idx = tid + NT * k;
         const int r2 = idx % RR, x = idx / RR;
-        dst[(size_t)x * N + r2] = xb[r2 * RS + padi(x)];
+        dst[(size_t)x * W + r2] = xb[r2 * RS + padi(x)];
     }
 }
 
@@ -80,20 +81,19 @@ k_psf_rows(const float* __restrict__ amp, long amp_fstride, const float* __restr
 // over F frame lanes of the CTA (lane f takes fields f, f + F, ...), so that
 // a batch of fields keeps F transforms of the column in flight per CTA (a
 // column per CTA with the fields in sequence left a 1024-column transform
-// with 1.7 CTAs of four warps per SM).  mode 0 (exposure): acc[kx][ky] +=
+// with 1.7 CTAs of four warps per SM).  PAD (exposure): acc[kx][ky] +=
 // |F_b[ky][kx]|^2 for b = 0..B-1: each lane sums its fields in order, then
 // the lanes' partial sums are added to the accumulator in lane order (the
 // accumulator is kept transposed and uncentred so that these updates are
-// coalesced).  mode 1 (chromatic): I[b][kx][ky] = |F_b[ky][kx]|^2.
+// coalesced).  Else (chromatic): I[b][kx][ky] = |F_b[ky][kx]|^2.
 template <int N> struct PsfLanes { static constexpr int F = Plan<N>::T >= 64 ? 2 : 4; };
 
-template <int N>
+template <int N, bool PAD>
 __global__ void __launch_bounds__(Plan<N>::T * PsfLanes<N>::F, 4)
-k_psf_cols(const float2* __restrict__ G, int B, int W, int off, int mode, float* __restrict__ out,
-           const float2* __restrict__ tw)
+k_psf_cols(const float2* __restrict__ G, int B, float* __restrict__ out, const float2* __restrict__ tw)
 {
     constexpr int F = PsfLanes<N>::F, T = Plan<N>::T, E = Plan<N>::E, RS = row_stride<N>();
-    constexpr int RL = last_radix<N>();
+    constexpr int RL = last_radix<N>(), W = PAD ? N / 2 : N;
     static_assert(F * RS * 2 >= F * N, "the lane sums fit the exchange rows");
     __shared__ __align__(16) float2 xb[F * RS];
     const int tid = threadIdx.x, t = tid % T, f = tid / T;
@@ -107,15 +107,12 @@ k_psf_cols(const float2* __restrict__ G, int B, int W, int off, int mode, float*
     for (int b0 = 0; b0 < B; b0 += F) {
         const int b = b0 + f;
         const bool have = b < B;
-        const float2* src = G + (size_t)(have ? b : 0) * N * N + (size_t)kx * N;
+        const float2* src = G + (size_t)(have ? b : 0) * N * W + (size_t)kx * W;
         float2 v[E];
 #pragma unroll
-        for (int e = 0; e < E; e++) {
-            const int yi = t + e * T - off;
-            v[e] = (have && yi >= 0 && yi < W) ? src[t + e * T] : make_float2(0.0f, 0.0f);
-        }
+        for (int e = 0; e < E; e++) v[e] = (have && e * T < W) ? src[t + e * T] : make_float2(0.0f, 0.0f);
         fft_rt<N, T, E>(v, xrow, t, tw, -1.0f, 0);
-        if (mode == 0) {
+        if constexpr (PAD) {
 #pragma unroll
             for (int s = 0; s < E; s++)
                 s2[s] = __fadd_rn(s2[s], __fadd_rn(__fmul_rn(v[s].x, v[s].x), __fmul_rn(v[s].y, v[s].y)));
@@ -126,7 +123,7 @@ k_psf_cols(const float2* __restrict__ G, int B, int W, int off, int mode, float*
                 I[last_index<N, T, RL>(t, s)] = __fadd_rn(__fmul_rn(v[s].x, v[s].x), __fmul_rn(v[s].y, v[s].y));
         }
     }
-    if (mode == 0) {
+    if constexpr (PAD) {
         __syncthreads();  // every lane's last transform is done with its exchange row
         float* red = reinterpret_cast<float*>(xb);  // [F][N]
 #pragma unroll
@@ -196,48 +193,48 @@ __global__ void k_chromat_sum(const float* __restrict__ I, int S, int n, const f
     }
 }
 
-template <int N>
-static cudaError_t psf_rows_n(const float* amp, long as, const float* pha, long ps, const float* cs, int W, int off,
-                              int B, float2* G, const float2* tw, cudaStream_t st)
+template <int N, bool PAD>
+static cudaError_t psf_rows_n(const float* amp, long as, const float* pha, long ps, const float* cs, int B, float2* G,
+                              const float2* tw, cudaStream_t st)
 {
-    constexpr int RR = PsfRows<N>::RR;
-    if (W % RR != 0 || W > N || off + W > N) return cudaErrorInvalidValue;
-    k_psf_rows<N><<<dim3((unsigned)(W / RR), (unsigned)B), Plan<N>::T * RR, 0, st>>>(amp, as, pha, ps, cs, W, off, G, tw);
+    constexpr int RR = PsfRows<N>::RR, W = PAD ? N / 2 : N;
+    static_assert(W % RR == 0, "whole CTAs of rows");
+    k_psf_rows<N, PAD><<<dim3((unsigned)(W / RR), (unsigned)B), Plan<N>::T * RR, 0, st>>>(amp, as, pha, ps, cs, G, tw);
     return cudaGetLastError();
 }
 
-template <int N>
-static cudaError_t psf_cols_n(const float2* G, int B, int W, int off, int mode, float* out, const float2* tw,
-                              cudaStream_t st)
+template <int N, bool PAD>
+static cudaError_t psf_cols_n(const float2* G, int B, float* out, const float2* tw, cudaStream_t st)
 {
-    k_psf_cols<N><<<N, Plan<N>::T * PsfLanes<N>::F, 0, st>>>(G, B, W, off, mode, out, tw);
+    k_psf_cols<N, PAD><<<N, Plan<N>::T * PsfLanes<N>::F, 0, st>>>(G, B, out, tw);
     return cudaGetLastError();
 }
 
-cudaError_t psf_rows(int N, const float* amp, long as, const float* pha, long ps, const float* cs, int W, int off,
-                     int B, float2* G, const float2* tw, cudaStream_t st)
+template <bool PAD>
+cudaError_t psf_rows(int N, const float* amp, long as, const float* pha, long ps, const float* cs, int B, float2* G,
+                     const float2* tw, cudaStream_t st)
 {
     switch (N) {
-        case 64: return psf_rows_n<64>(amp, as, pha, ps, cs, W, off, B, G, tw, st);
-        case 128: return psf_rows_n<128>(amp, as, pha, ps, cs, W, off, B, G, tw, st);
-        case 256: return psf_rows_n<256>(amp, as, pha, ps, cs, W, off, B, G, tw, st);
-        case 512: return psf_rows_n<512>(amp, as, pha, ps, cs, W, off, B, G, tw, st);
-        case 1024: return psf_rows_n<1024>(amp, as, pha, ps, cs, W, off, B, G, tw, st);
-        case 2048: return psf_rows_n<2048>(amp, as, pha, ps, cs, W, off, B, G, tw, st);
+        case 64: return psf_rows_n<64, PAD>(amp, as, pha, ps, cs, B, G, tw, st);
+        case 128: return psf_rows_n<128, PAD>(amp, as, pha, ps, cs, B, G, tw, st);
+        case 256: return psf_rows_n<256, PAD>(amp, as, pha, ps, cs, B, G, tw, st);
+        case 512: return psf_rows_n<512, PAD>(amp, as, pha, ps, cs, B, G, tw, st);
+        case 1024: return psf_rows_n<1024, PAD>(amp, as, pha, ps, cs, B, G, tw, st);
+        case 2048: return psf_rows_n<2048, PAD>(amp, as, pha, ps, cs, B, G, tw, st);
         default: return cudaErrorInvalidValue;
     }
 }
 
-cudaError_t psf_cols(int N, const float2* G, int B, int W, int off, int mode, float* out, const float2* tw,
-                     cudaStream_t st)
+template <bool PAD>
+cudaError_t psf_cols(int N, const float2* G, int B, float* out, const float2* tw, cudaStream_t st)
 {
     switch (N) {
-        case 64: return psf_cols_n<64>(G, B, W, off, mode, out, tw, st);
-        case 128: return psf_cols_n<128>(G, B, W, off, mode, out, tw, st);
-        case 256: return psf_cols_n<256>(G, B, W, off, mode, out, tw, st);
-        case 512: return psf_cols_n<512>(G, B, W, off, mode, out, tw, st);
-        case 1024: return psf_cols_n<1024>(G, B, W, off, mode, out, tw, st);
-        case 2048: return psf_cols_n<2048>(G, B, W, off, mode, out, tw, st);
+        case 64: return psf_cols_n<64, PAD>(G, B, out, tw, st);
+        case 128: return psf_cols_n<128, PAD>(G, B, out, tw, st);
+        case 256: return psf_cols_n<256, PAD>(G, B, out, tw, st);
+        case 512: return psf_cols_n<512, PAD>(G, B, out, tw, st);
+        case 1024: return psf_cols_n<1024, PAD>(G, B, out, tw, st);
+        case 2048: return psf_cols_n<2048, PAD>(G, B, out, tw, st);
         default: return cudaErrorInvalidValue;
     }
 }
@@ -275,8 +272,10 @@ atmwfs_status psf_cuda(cudaError_t e, const char* what)
 
 bool pow2_between(long n, long lo, long hi) { return n >= lo && n <= hi && (n & (n - 1)) == 0; }
 
-// Fields per launch: about 256 MB of intermediate, 1..64 fields.
-long psf_batch(long N) { return std::max(1L, std::min(64L, (256L << 20) / (N * N * 8))); }
+// Fields per launch, 1..64: a batch's intermediate (N x W complex values per
+// field) is written by the row pass and read by the column pass.
+long psf_mb() { const char* e = getenv("PSF_MB"); return e ? atol(e) : 64; }
+long psf_batch(long N, long W) { return std::max(1L, std::min(64L, (psf_mb() << 20) / (N * W * 8))); }
 
 // Step coefficients and weights with the reference's types (psf.c:86-99):
 // float coeff, x and mcoeff from double expressions.
@@ -315,15 +314,15 @@ atmwfs_status atmwfs_psf_expo_accumulate_dev(const float* amp, long amp_fstride,
     const long N = 2 * W;
     const float2* tw = stage_twiddles((int)N);
     if (!tw) return psf_fail(ATMWFS_ERR_NOMEM, "twiddle allocation failed");
-    const long B = std::min(psf_batch(N), nframes);
+    const long B = std::min(psf_batch(N, W), nframes);
     float2* G = nullptr;
-    atmwfs_status s = psf_cuda(cudaMallocAsync((void**)&G, sizeof(float2) * B * N * N, st), "intermediate allocation");
+    atmwfs_status s = psf_cuda(cudaMallocAsync((void**)&G, sizeof(float2) * B * N * W, st), "intermediate allocation");
     if (s != ATMWFS_OK) return s;
     for (long f0 = 0; f0 < nframes && s == ATMWFS_OK; f0 += B) {
         const long b = std::min(B, nframes - f0);
-        s = psf_cuda(psf_rows((int)N, amp + f0 * amp_fstride, amp_fstride, pha + f0 * W * W, W * W, nullptr, (int)W,
-                              (int)(W / 2), (int)b, G, tw, st), "row pass");
-        if (s == ATMWFS_OK) s = psf_cuda(psf_cols((int)N, G, (int)b, (int)W, (int)(W / 2), 0, acc, tw, st), "column pass");
+        s = psf_cuda(psf_rows<true>((int)N, amp + f0 * amp_fstride, amp_fstride, pha + f0 * W * W, W * W, nullptr, (int)b, G,
+                                    tw, st), "row pass");
+        if (s == ATMWFS_OK) s = psf_cuda(psf_cols<true>((int)N, G, (int)b, acc, tw, st), "column pass");
     }
     cudaFreeAsync(G, st);
     return s;
@@ -381,7 +380,7 @@ atmwfs_status atmwfs_chromat_psf(const float* amp, const float* pha, long n, flo
     chromat_weights(coeff1, coeff2, nbstep, apo_coeff, c, m);
     const float2* tw = stage_twiddles((int)n);
     if (!tw) return psf_fail(ATMWFS_ERR_NOMEM, "twiddle allocation failed");
-    const long B = std::min(psf_batch(n), nbstep);
+    const long B = std::min(psf_batch(n, n), nbstep);
     float *da = nullptr, *dp = nullptr, *dI = nullptr, *dout = nullptr, *dc = nullptr, *dm = nullptr;
     float2* G = nullptr;
     atmwfs_status s = psf_cuda(cudaMalloc(&da, sizeof(float) * n * n), "allocation");
@@ -398,8 +397,8 @@ atmwfs_status atmwfs_chromat_psf(const float* amp, const float* pha, long n, flo
     if (s == ATMWFS_OK) s = psf_cuda(cudaMemset(dout, 0, sizeof(float) * n * n), "memset");
     for (long s0 = 0; s0 < nbstep && s == ATMWFS_OK; s0 += B) {
         const long b = std::min(B, nbstep - s0);
-        s = psf_cuda(psf_rows((int)n, da, 0, dp, 0, dc + s0, (int)n, 0, (int)b, G, tw, nullptr), "row pass");
-        if (s == ATMWFS_OK) s = psf_cuda(psf_cols((int)n, G, (int)b, (int)n, 0, 1, dI, tw, nullptr), "column pass");
+        s = psf_cuda(psf_rows<false>((int)n, da, 0, dp, 0, dc + s0, (int)b, G, tw, nullptr), "row pass");
+        if (s == ATMWFS_OK) s = psf_cuda(psf_cols<false>((int)n, G, (int)b, dI, tw, nullptr), "column pass");
         if (s == ATMWFS_OK) s = psf_cuda(chromat_sum(dI, (int)b, (int)n, dc + s0, dm + s0, dout, nullptr), "zoom sum");
     }
     if (s == ATMWFS_OK) s = psf_cuda(cudaMemcpy(out, dout, sizeof(float) * n * n, cudaMemcpyDeviceToHost), "copy");
