@@ -309,6 +309,11 @@ struct Class {
     std::vector<GroupSumJob> gjobs;
     GroupSumJob* d_gjobs = nullptr;
     bool need_phasum = true;
+    // phase-only context: the frames of the groups whose side is N
+    std::vector<PhaseJob> pjobs;
+    std::vector<int> pslots;
+    PhaseJob* d_pjobs = nullptr;
+    int* d_pslots = nullptr;
 };
 
 }  // namespace atmwfs
@@ -525,12 +530,44 @@ atmwfs_status launch_windows(atmwfs_ctx* c, Class& cl, int j0, int j1, double* b
     return ATMWFS_OK;
 }
 
+// The phase-only frames of the groups cl computes; optionally their
+// algorithmic bytes (the screens under the rows, the frames out).
+atmwfs_status launch_phases(atmwfs_ctx* c, Class& cl, double* bytes, cudaStream_t st)
+{
+    if (bytes) *bytes = 0;
+    if (cl.pjobs.empty()) return ATMWFS_OK;
+    PassArgs a;
+    memset(&a, 0, sizeof a);
+    a.inst = c->d_inst;
+    a.pos = c->d_pos;
+    a.d_step = c->d_step;
+    a.d_status = c->d_status;
+    a.L = c->L;
+    a.ninst_total = c->ninst;
+    a.poscap = c->poscap;
+    a.pjobs = cl.d_pjobs;
+    a.pslots = cl.d_pslots;
+    const int RR = phase_rows(cl.N);
+    if (bytes) {
+        *bytes = 4.0 * (RR + 3) / RR * c->L * (double)cl.N * cl.N * cl.pjobs.size();
+        for (int q : cl.pslots) *bytes += 8.0 * c->hinst[q].Nout * c->hinst[q].Nout;
+    }
+    AW_CUDA(pass_launcher_cfg(cl.N)(0, kVarPhases, dim3(cl.N / RR, (unsigned)cl.pjobs.size()), a, &cl.maps[0], nullptr, st));
+    return ATMWFS_OK;
+}
+
 // Launch pass k (1-based) for grid class cl; optionally report the
 // algorithmic bytes of the launch.
 atmwfs_status launch_pass(atmwfs_ctx* c, int k, Class& cl, double* bytes, cudaStream_t st)
 {
     const int Q = (int)c->plane_lo.size();
     const int P = Q - 1;
+    if (!c->amplitude) {
+        // phase-only frames are one kernel: pass 1
+        if (k == 1) return launch_phases(c, cl, bytes, st);
+        if (bytes) *bytes = 0;
+        return ATMWFS_OK;
+    }
     if (k == 0) {
         // geometric phase sums: the layer sums of the window groups this class
         // computes (instances whose Scoeff factors out), then the per-instance
@@ -639,6 +676,11 @@ atmwfs_status launch_step(atmwfs_ctx* c)
     const int Q = (int)c->plane_lo.size();
     const int nc = (int)c->classes.size();
     cudaEvent_t fork = c->gev[0], sums = c->gev[1];
+    if (!c->amplitude) {
+        for (Class& cl : c->classes) AW_TRY(launch_phases(c, cl, nullptr, c->st));
+        AW_CUDA(step_advance(c->d_step, c->st));
+        return ATMWFS_OK;
+    }
     // the step's screen windows, read by the phase sums and by every pass
     // (launching those of the later passes beside the first pass measured no
     // faster: the transforms keep every SM's registers busy)
@@ -717,7 +759,9 @@ atmwfs_status autotune(atmwfs_ctx* c)
     AW_CUDA(cudaEventCreate(&e1));
     atmwfs_status s = ATMWFS_OK;
     for (Class& cl : c->classes) {
-        if (c->fp16) {
+        if (!c->amplitude) {
+            cl.cfg = 0;  // phase-only frames have one configuration
+        } else if (c->fp16) {
             cl.cfg = 2;  // the FP16-transform passes are compiled for configuration 2
         } else if (forced_cfg(force, cl.N) >= 0) {
             const int g = forced_cfg(force, cl.N);
@@ -759,6 +803,47 @@ atmwfs_status autotune(atmwfs_ctx* c)
     return check_status(c);
 }
 
+// Whether the phase sums of window group g factor (ATMWFS_GROUP_PHASE_SUM=0:
+// never): every member's Scoeff equal on all layers, bit for bit.
+bool group_factors(const atmwfs_ctx* c, int g)
+{
+    const char* gps = getenv("ATMWFS_GROUP_PHASE_SUM");
+    if (gps && atoi(gps) == 0) return false;
+    for (int i = 0; i < c->ninst; i++)
+        if (c->group_of[i] == g)
+            for (int l = 1; l < c->L; l++)
+                if (c->scoeff[i][l] != c->scoeff[i][0]) return false;
+    return true;
+}
+
+// Jobs of the phase-only frames for the groups of side cl.N: one per group
+// whose Scoeff factors, one per member otherwise (the interpolation repeated
+// per member costs less than storing the windows for it).
+atmwfs_status phase_jobs(atmwfs_ctx* c, Class& cl)
+{
+    cl.pjobs.clear();
+    cl.pslots.clear();
+    for (size_t g = 0; g < c->group_leader.size(); g++) {
+        if (c->wg[g] != cl.N) continue;
+        const bool f = group_factors(c, (int)g);
+        const int first = (int)cl.pslots.size();
+        for (int i = 0; i < c->ninst; i++) {
+            if (c->group_of[i] != (int)g) continue;
+            if (!f) cl.pjobs.push_back(PhaseJob{c->group_leader[g], (int)cl.pslots.size(), 1, 0});
+            cl.pslots.push_back(c->slot_of[i]);
+        }
+        if (f) cl.pjobs.push_back(PhaseJob{c->group_leader[g], first, (int)cl.pslots.size() - first, 1});
+    }
+    if (cl.pjobs.empty()) return ATMWFS_OK;
+    if (!cl.d_pjobs) {
+        AW_TRY(dalloc(c, (void**)&cl.d_pjobs, sizeof(PhaseJob) * cl.pslots.size()));  // at most one job per member
+        AW_TRY(dalloc(c, (void**)&cl.d_pslots, sizeof(int) * cl.pslots.size()));
+    }
+    AW_CUDA(cudaMemcpyAsync(cl.d_pjobs, cl.pjobs.data(), sizeof(PhaseJob) * cl.pjobs.size(), cudaMemcpyHostToDevice, c->st));
+    AW_CUDA(cudaMemcpyAsync(cl.d_pslots, cl.pslots.data(), sizeof(int) * cl.pslots.size(), cudaMemcpyHostToDevice, c->st));
+    return ATMWFS_OK;
+}
+
 atmwfs_status commit(atmwfs_ctx* c)
 {
     if (c->committed) return ATMWFS_OK;
@@ -784,7 +869,7 @@ atmwfs_status commit(atmwfs_ctx* c)
     // transposed passes
     const int G = (int)c->group_leader.size();
     for (int o = 0; o < 2; o++) c->d_win[o].resize((size_t)G * c->L, nullptr);
-    for (int g = 0; g < G; g++)
+    for (int g = 0; g < G && c->amplitude; g++)  // phase-only frames store no windows
         for (int o = 0; o < 2; o++)
             for (int l = 0; l < c->L; l++) {
                 if (o == 1 && !need1[l]) continue;
@@ -803,6 +888,10 @@ atmwfs_status commit(atmwfs_ctx* c)
             if (other.N == cl.N) owner = false;
         }
         if (!owner) continue;
+        if (!c->amplitude) {
+            AW_TRY(phase_jobs(c, cl));
+            continue;
+        }
         for (int g = 0; g < G; g++) {
             if (c->wg[g] != cl.N) continue;
             for (int o = 0; o < 2; o++)
@@ -816,15 +905,9 @@ atmwfs_status commit(atmwfs_ctx* c)
     }
     // Phase-sum factoring per group (ATMWFS_GROUP_PHASE_SUM=0 turns it off):
     // every member's Scoeff equal on all layers (bit for bit)
-    const char* gps = getenv("ATMWFS_GROUP_PHASE_SUM");
-    const bool factor = !(gps && atoi(gps) == 0);
     c->d_gsum.resize(G, nullptr);
-    for (int g = 0; g < G; g++) {
-        bool ok = factor && c->L <= kMaxLayers;
-        for (int i = 0; i < c->ninst && ok; i++)
-            if (c->group_of[i] == g)
-                for (int l = 1; l < c->L && ok; l++) ok = c->scoeff[i][l] == c->scoeff[i][0];
-        if (ok && !c->d_gsum[g]) AW_TRY(dalloc(c, (void**)&c->d_gsum[g], sizeof(float2) * (size_t)c->wg[g] * c->wg[g]));
+    for (int g = 0; g < G && c->amplitude; g++) {
+        if (group_factors(c, g) && !c->d_gsum[g]) AW_TRY(dalloc(c, (void**)&c->d_gsum[g], sizeof(float2) * (size_t)c->wg[g] * c->wg[g]));
     }
     for (Class& cl : c->classes) {
         cl.gjobs.clear();
@@ -859,7 +942,8 @@ atmwfs_status commit(atmwfs_ctx* c)
             for (int o = 0; o < 2; o++)
                 for (int l = 0; l < c->L; l++)
                     if (c->d_pad[o][l] && tile_cfg(cl.N, g).rr > 0)
-                        AW_TRY(make_tma_map(&cl.maps[g].m[o][l], c->d_pad[o][l], c->Wp, c->Hp, tile_cfg(cl.N, g).rr + 3));
+                        AW_TRY(make_tma_map(&cl.maps[g].m[o][l], c->d_pad[o][l], c->Wp, c->Hp,
+                                            (c->amplitude ? tile_cfg(cl.N, g).rr : phase_rows(cl.N)) + 3));
     }
     AW_CUDA(cudaStreamSynchronize(c->st));
     AW_TRY(autotune(c));

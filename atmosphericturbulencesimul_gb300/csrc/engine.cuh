@@ -152,6 +152,14 @@ struct WinJob {
     int gidx, layer, orient, stride;
 };
 
+// One job of the phase-only frames (k_phase_frames): the instances
+// [first, first + count) of the job list's slots, which share the windows of
+// group leader `gidx`.  factored: every one of them has one Scoeff for all its
+// layers; else the job holds a single instance.
+struct PhaseJob {
+    int gidx, first, count, factored;
+};
+
 enum : int { kModeRef = 0, kModeSci = 1, kModePhase = 2 };
 
 // Operation flags of a row pass.
@@ -166,6 +174,7 @@ enum : int {
     OP_FFT_INV = 128,  // unit: inverse 1-D FFT only
     OP_PHASUM = 256,   // geometric phase sum of all layers (k_phasum)
     OP_WINDOWS = 512,  // per-step bicubic windows of the window groups (k_layer_windows)
+    OP_PHASES = 1024,  // phase-only frames (k_phase_frames)
 };
 
 constexpr int kVarFirst = OP_GATHER | OP_PROP2 | OP_STORE_T;
@@ -177,6 +186,7 @@ constexpr int kVarUnitFwd = OP_LOAD | OP_FFT_FWD | OP_STORE_T;
 constexpr int kVarUnitInv = OP_LOAD | OP_FFT_INV | OP_STORE_T;
 constexpr int kVarPhasum = OP_PHASUM;
 constexpr int kVarWindows = OP_WINDOWS;
+constexpr int kVarPhases = OP_PHASES;
 
 // Status bits written by kernels.
 enum : unsigned {
@@ -203,6 +213,9 @@ struct PassArgs {
     const float2* H2;
     // window kernel: its jobs (blockIdx.y)
     const WinJob* jobs;
+    // phase-only frames: their jobs (blockIdx.y) and the jobs' instance slots
+    const PhaseJob* pjobs;
+    const int* pslots;
 };
 
 // Tensor maps of the halo-padded screens: [orientation][layer].
@@ -258,6 +271,12 @@ constexpr TileCfg tile_cfg(int N, int c)
          : N == 2048  ? (c == 0 ? TileCfg{4, 1, false, 0, false} : c == 1 ? TileCfg{2, 3, false, 0, false} : TileCfg{2, 3, true, 0, false})
                       : TileCfg{0, 0, false, 0, false};
 }
+
+// Phase-only frames: rows per CTA and threads.  Eight rows cost 11 / 8 of the
+// horizontal sums and leave four CTAs per SM at 512; 2048 takes four so that
+// two tiles fit the shared memory.
+constexpr int phase_rows(int N) { return N <= 1024 ? 8 : 4; }
+constexpr int phase_threads(int N) { return N < 256 ? N : 256; }
 
 // Threads of a phase-sum CTA and CTAs per instance of its launch.
 constexpr int kPhasumThreads = 256;

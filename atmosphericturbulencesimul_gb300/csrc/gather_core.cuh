@@ -40,31 +40,34 @@ AW_HD TileGeom tile_geom(LayerPos p, int orient, int y0)
 template <int TROWS>
 AW_HD int tile_index(int r, int c) { return ((c >> 5) * TROWS + r) * kBoxW + (c & (kBoxW - 1)); }
 
-// Interpolate one layer for the CTA's RR rows.  Thread tid walks columns
-// x = tid, tid + NT, ...; for each it forms the RR + 3 horizontal cubic
-// sums of the tile rows and slides the vertical cubic down the column.
-// Calls emit(r, x, value) for every pixel.
+// Interpolate column x of one layer for the CTA's RR rows: the RR + 3
+// horizontal cubic sums of the tile rows, then the vertical cubic slides down
+// the column.  Calls emit(r, value) for every row.
+template <int RR, typename F>
+AW_HD void gather_column(const float* tile, const TileGeom& g, const float wx[4], const float wy[4], int x, F emit)
+{
+    constexpr int TROWS = RR + 3;
+    const int c = g.d + x;
+    float h[TROWS];
+    AW_UNROLL
+    for (int b = 0; b < TROWS; b++) {
+        h[b] = wx[0] * tile[tile_index<TROWS>(b, c)] + wx[1] * tile[tile_index<TROWS>(b, c + 1)] +
+               wx[2] * tile[tile_index<TROWS>(b, c + 2)] + wx[3] * tile[tile_index<TROWS>(b, c + 3)];
+    }
+    AW_UNROLL
+    for (int r = 0; r < RR; r++) emit(r, wy[0] * h[r] + wy[1] * h[r + 1] + wy[2] * h[r + 2] + wy[3] * h[r + 3]);
+}
+
+// Interpolate one layer for the CTA's RR rows; thread tid walks columns
+// x = tid, tid + NT, ...  Calls emit(r, x, value) for every pixel.
 template <int N, int RR, int NT, typename F>
 AW_HD void gather_tile(const float* tile, const TileGeom& g, float sc, int tid, F emit)
 {
-    constexpr int TROWS = RR + 3;
     float wx[4], wy[4];
     keys_weights(g.fx, wx);
     keys_weights(g.fy, wy);
-    for (int x = tid; x < N; x += NT) {
-        const int c = g.d + x;
-        float h[TROWS];
-        AW_UNROLL
-        for (int b = 0; b < TROWS; b++) {
-            h[b] = wx[0] * tile[tile_index<TROWS>(b, c)] + wx[1] * tile[tile_index<TROWS>(b, c + 1)] +
-                   wx[2] * tile[tile_index<TROWS>(b, c + 2)] + wx[3] * tile[tile_index<TROWS>(b, c + 3)];
-        }
-        AW_UNROLL
-        for (int r = 0; r < RR; r++) {
-            const float val = (wy[0] * h[r] + wy[1] * h[r + 1] + wy[2] * h[r + 2] + wy[3] * h[r + 3]) * sc;
-            emit(r, x, val);
-        }
-    }
+    for (int x = tid; x < N; x += NT)
+        gather_column<RR>(tile, g, wx, wy, x, [&](int r, float val) { emit(r, x, val * sc); });
 }
 
 }  // namespace atmwfs

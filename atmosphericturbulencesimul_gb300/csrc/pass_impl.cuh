@@ -545,26 +545,14 @@ __global__ void __launch_bounds__(Plan<N, V>::T* RR, MINB)
         }
         // [NJ][N]: per bin row, per column; clear of the staged rows in xb
         float2* colsum = reinterpret_cast<float2*>(wrows);
-        // One loop per output mode with a branch-free body: every pixel of the
+        // A branch-free body: every pixel of the
         // thread's columns is computed (rows and columns outside the crop read
         // a valid staged value) and only the stores and bin sums are
         // predicated, so the compiler can interleave the pixels.
         bool rin[RR];
 #pragma unroll
         for (int r = 0; r < RR; r++) rin[r] = y0 + r >= ya && y0 + r < yb;
-        if (mode == kModePhase) {
-#pragma unroll
-            for (int c = 0; c < CPT; c++) {
-                const int x = off + tid + c * NT;
-#pragma unroll
-                for (int r = 0; r < RR; r++) {
-                    if (!(rin[r] && x < off + Nout)) continue;
-                    const size_t o = (size_t)(y0 + r - off) * Nout + (x - off);
-                    opha[o] = ps[r][c];
-                    oamp[o] = 1.0f;
-                }
-            }
-        } else {
+        {
             const bool ref = mode == kModeRef;
 #pragma unroll
             for (int c = 0; c < CPT; c++) {
@@ -688,6 +676,97 @@ __global__ void __launch_bounds__(PassGeom<N, RR>::NT)
 }
 
 // ---------------------------------------------------------------------------
+// Phase-only frames (WAVEFRONT_AMPLITUDE 0): pha = the geometric phase sum,
+// amp = 1 (AtmosphericTurbulence.c:2909-2916, 3237-3245 without the field).
+// There is no field to propagate, so the windows are not stored: a CTA takes
+// RR rows of a window group, walks the layers from the top down with the next
+// layer's tile in flight (two buffers, TMA), interpolates in registers, keeps
+// the two-sum of every pixel there and writes the frames of the group's
+// instances.  The same samples and sums as k_layer_windows + k_group_sum (or
+// k_phasum where Scoeff depends on the layer) and an output pass, bit for bit.
+// Issue bounds it: about 18 instructions per pixel and layer.  16 directions
+// of 512^2 through 10 layers: windows 60 + sums 45 + output pass 46 us before.
+// ---------------------------------------------------------------------------
+template <int N, int RR, int NT>
+__global__ void __launch_bounds__(NT) k_phase_frames(const __grid_constant__ PassArgs a, const __grid_constant__ TmaSet maps)
+{
+    using G = PassGeom<N, RR>;
+    constexpr int CPT = N / NT;  // columns per thread
+    static_assert(N % NT == 0, "whole columns");
+    extern __shared__ __align__(1024) unsigned char sm[];
+    float* tiles = reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(sm) + 127) & ~uintptr_t(127));
+    constexpr int TILE = (int)(G::TILE_BYTES / 4);
+    __shared__ __align__(8) uint64_t bar[2];
+    pdl_gate();
+    const PhaseJob J = a.pjobs[blockIdx.y];
+    const int tid = threadIdx.x, y0 = blockIdx.x * RR, L = a.L;
+    const int step = *a.d_step;
+    const LayerPos* pos = a.pos + ((size_t)(step % a.poscap) * a.ninst_total + J.gidx) * L;
+    if (tid == 0) {
+        mbar_init(&bar[0], 1);
+        mbar_init(&bar[1], 1);
+    }
+    __syncthreads();
+    auto issue = [&](int i) {
+        const TileGeom g = tile_geom(pos[L - 1 - i], 0, y0);
+        tma_issue_layer<N, RR>(maps, 0, L - 1 - i, g, tiles + (i & 1) * TILE, &bar[i & 1], tid, NT);
+    };
+    issue(0);
+    if (L > 1) issue(1);
+    const InstDev* I0 = a.inst + a.pslots[J.first];
+    float hi[CPT][RR], lo[CPT][RR];
+#pragma unroll
+    for (int q = 0; q < CPT; q++)
+#pragma unroll
+        for (int r = 0; r < RR; r++) hi[q][r] = lo[q][r] = 0.0f;
+#pragma unroll 1
+    for (int i = 0; i < L; i++) {
+        if (!cta_wait_tile(&bar[i & 1], (i >> 1) & 1, a.d_status)) {
+            // the other buffer's copy must land before the CTA retires
+            if (i + 1 < L) cta_wait_tile(&bar[(i + 1) & 1], ((i + 1) >> 1) & 1, a.d_status);
+            return;
+        }
+        const TileGeom g = tile_geom(pos[L - 1 - i], 0, y0);
+        const float sc = J.factored ? 1.0f : I0->scoeff[L - 1 - i];
+        float wx[4], wy[4];
+        keys_weights(g.fx, wx);
+        keys_weights(g.fy, wy);
+        const float* tile = tiles + (i & 1) * TILE;
+#pragma unroll
+        for (int q = 0; q < CPT; q++)
+            gather_column<RR>(tile, g, wx, wy, tid + q * NT, [&](int r, float val) {
+                float s, e;
+                two_sum(hi[q][r], __fmul_rn(val, sc), s, e);
+                hi[q][r] = s;
+                lo[q][r] = __fadd_rn(lo[q][r], e);
+            });
+        __syncthreads();  // every thread has read the tile
+        if (i + 2 < L) issue(i + 2);
+    }
+    for (int m = 0; m < J.count; m++) {
+        const InstDev* I = a.inst + a.pslots[J.first + m];
+        const int off = I->off, Nout = I->Nout;
+        const size_t slot = (size_t)(step % I->ring) * I->ostride;
+        float* __restrict__ opha = I->out_pha + slot;
+        float* __restrict__ oamp = I->out_amp + slot;
+        const float sg = I->scoeff[0];
+#pragma unroll
+        for (int r = 0; r < RR; r++) {
+            const int y = y0 + r - off;
+            if (y < 0 || y >= Nout) continue;
+#pragma unroll
+            for (int q = 0; q < CPT; q++) {
+                const int x = tid + q * NT - off;
+                if (x < 0 || x >= Nout) continue;
+                const size_t o = (size_t)y * Nout + x;
+                opha[o] = J.factored ? fmaf(sg, hi[q][r], sg * lo[q][r]) : __fadd_rn(hi[q][r], lo[q][r]);
+                oamp[o] = 1.0f;
+            }
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------
 // geometric phase sum over all layers for the crop (reference array1 /
 // sarray1, AtmosphericTurbulence.c:2909-2916, 3237-3245) from the step's
 // windows in the screen orientation: per pixel the layers from the top
@@ -806,6 +885,17 @@ cudaError_t launch_pass_t(int var, dim3 grid, const PassArgs& a, const TmaSet* m
                 attr = true;
             }
             return launch_gated(k_layer_windows<N, RR>, grid, dim3(G::NT), sm, st, a, m);
+        }
+        case kVarPhases: {
+            constexpr int PR = phase_rows(N), PT = phase_threads(N);
+            constexpr size_t sm = 2 * PassGeom<N, PR>::TILE_BYTES + 128;
+            static bool attr = false;
+            if (!attr) {
+                cudaError_t e = cudaFuncSetAttribute(k_phase_frames<N, PR, PT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+                if (e != cudaSuccess) return e;
+                attr = true;
+            }
+            return launch_gated(k_phase_frames<N, PR, PT>, grid, dim3(PT), sm, st, a, m);
         }
         default: return cudaErrorInvalidValue;
     }
