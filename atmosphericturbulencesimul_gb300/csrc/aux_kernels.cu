@@ -182,6 +182,7 @@ __global__ void k_unwrap(const InstDev* __restrict__ insts, const int* __restric
     __shared__ unsigned s_max[2];
     __shared__ int s_cnt[2];
     const double kTwoPi = 2.0 * 3.14159265358979323846;
+    float vmin = 4.0f, vmax = -4.0f;  // outside the range of an angle
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
         // the fixed-point sums back to float (one rounding; the scaling by
         // 2^-kBinFrac is exact), then (float)atan2((double)im, (double)re)
@@ -191,11 +192,38 @@ __global__ void k_unwrap(const InstDev* __restrict__ insts, const int* __restric
         const float im = __ll2float_rn((long long)I.bins[n + i]) * q;
         const float v = atan2_ff(im, re, atan_tab);
         pb[i] = v;
-        ppf[i] = __double2float_rd((double)v + kTwoPi * 0.5);
+        vmin = fminf(vmin, v);
+        vmax = fmaxf(vmax, v);
         I.bins[i] = 0ull;
         I.bins[n + i] = 0ull;
     }
     if (threadIdx.x < 2) { s_max[threadIdx.x] = 0u; s_cnt[threadIdx.x] = 0; }
+    // A vote needs two bins more than pi apart.  Where all bins lie closer
+    // (the usual case: the bins hold the diffraction's mean phase, a fraction
+    // of a radian) the first iteration finds none, lowers the limit to 0.5 and
+    // is the last, and the bins stay as they are.  That takes the 48 candidate
+    // votes per bin and the FP64 thresholds out of the frame: one CTA spent
+    // about 30 us on the 102^2 bins of a 2048^2 frame.
+    for (int o = 16; o > 0; o >>= 1) {
+        vmin = fminf(vmin, __shfl_xor_sync(0xffffffffu, vmin, o));
+        vmax = fmaxf(vmax, __shfl_xor_sync(0xffffffffu, vmax, o));
+    }
+    __shared__ float s_lo[32], s_hi[32];
+    if ((threadIdx.x & 31) == 0) {
+        s_lo[threadIdx.x >> 5] = vmin;
+        s_hi[threadIdx.x >> 5] = vmax;
+    }
+    __syncthreads();
+    for (int w = 0; w < (int)(blockDim.x >> 5); w++) {
+        vmin = fminf(vmin, s_lo[w]);
+        vmax = fmaxf(vmax, s_hi[w]);
+    }
+    if (vmax - vmin < 3.14159f) {  // below pi by more than the difference's rounding
+        for (int i = threadIdx.x; i < n; i += blockDim.x) I.peak[i] = pb[i];
+        if (threadIdx.x == 0 && iters_out) iters_out[list[blockIdx.x]] = 1;
+        return;
+    }
+    for (int i = threadIdx.x; i < n; i += blockDim.x) ppf[i] = __double2float_rd((double)pb[i] + kTwoPi * 0.5);
     __syncthreads();
     int chiter = 0, chcnt0cnt = 0, par = 0;
     double plim = 1.0;
@@ -243,7 +271,7 @@ __global__ void k_unwrap(const InstDev* __restrict__ insts, const int* __restric
 }
 
 cudaError_t unwrap_bins(const InstDev* insts, const int* list, int nsci, int maxnb, unsigned* status, int* iters,
-                        const float2* atan_tab, cudaStream_t st)
+                        const float2* atan_tab, long pdl_ctas, cudaStream_t st)
 {
     if (nsci <= 0) return cudaSuccess;
     const size_t sm = (size_t)3 * maxnb * maxnb * sizeof(float);
@@ -251,7 +279,9 @@ cudaError_t unwrap_bins(const InstDev* insts, const int* list, int nsci, int max
         cudaError_t e = cudaFuncSetAttribute(k_unwrap, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
         if (e != cudaSuccess) return e;
     }
-    return launch_gated(k_unwrap, dim3(nsci), dim3(512), sm, st, insts, list, status, iters, atan_tab);
+    // about four bins per thread up to 64^2 bins, ten at the 102^2 of a 2048^2 frame
+    const int nt = maxnb <= 32 ? 256 : maxnb <= 64 ? 512 : 1024;
+    return launch_gated_up_to(pdl_ctas, k_unwrap, dim3(nsci), dim3(nt), sm, st, insts, list, status, iters, atan_tab);
 }
 
 // final science phase: pha + 2 pi round((phasum - pha - peak[bin]) / 2 pi)
@@ -266,49 +296,53 @@ __global__ void k_sci_apply(const InstDev* __restrict__ insts, const int* __rest
     const short* __restrict__ binx = I.binx;
     const float* __restrict__ peakv = I.peak;
     const float* __restrict__ psum = I.phisum;
-    // one row per block iteration; four columns per thread as 16-byte vectors
-    // when the row length allows, else one column per thread
+    // four neighbouring pixels of a row per thread as 16-byte vectors when the
+    // row length allows, else one; items run through the frame so that every
+    // thread has one whatever the row length
     const bool v4 = (Nout % 4 == 0) && ((reinterpret_cast<uintptr_t>(pha) & 15) == 0) &&
                     ((reinterpret_cast<uintptr_t>(psum) & 15) == 0);
-    for (int jj = blockIdx.x; jj < Nout; jj += gridDim.x) {
+    const int per = v4 ? 4 : 1, wrow = Nout / per, items = wrow * Nout;
+    const float sc = I.scoeff[0];
+    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < items; k += gridDim.x * blockDim.x) {
+        const int jj = k / wrow, ii = (k - jj * wrow) * per;
         const int bj = nb > 0 ? binx[jj] * nb : 0;
-        const size_t ro = (size_t)jj * Nout;
-        const float2* __restrict__ gs = I.gsum ? I.gsum + (size_t)(jj + I.off) * I.wstride + I.off : nullptr;
-        const float sc = I.scoeff[0];
-        auto one = [&](float p, float s, int ii) {
-            const float peak = nb > 0 ? peakv[bj + binx[ii]] : 0.0f;
+        const size_t o = (size_t)jj * Nout + ii;
+        const float2* __restrict__ gs = I.gsum ? I.gsum + (size_t)(jj + I.off) * I.wstride + I.off + ii : nullptr;
+        auto one = [&](float p, float s, int x) {
+            const float peak = nb > 0 ? peakv[bj + binx[x]] : 0.0f;
             float d1, e1, d2, e2;
             two_sum(s, -p, d1, e1);
             two_sum(d1, -peak, d2, e2);
             return add_2pi_multiple(p, round_2pi(d2, e1 + e2));
         };
         if (v4) {
-            for (int i4 = threadIdx.x; i4 < Nout / 4; i4 += blockDim.x) {
-                const int ii = 4 * i4;
-                const float4 p = *reinterpret_cast<const float4*>(pha + ro + ii);
-                float4 s;
-                if (gs) {
-                    const float2 g0 = gs[ii], g1 = gs[ii + 1], g2 = gs[ii + 2], g3 = gs[ii + 3];
-                    s = make_float4(fmaf(sc, g0.x, sc * g0.y), fmaf(sc, g1.x, sc * g1.y), fmaf(sc, g2.x, sc * g2.y),
-                                    fmaf(sc, g3.x, sc * g3.y));
-                } else {
-                    s = *reinterpret_cast<const float4*>(psum + ro + ii);
-                }
-                *reinterpret_cast<float4*>(pha + ro + ii) =
-                    make_float4(one(p.x, s.x, ii), one(p.y, s.y, ii + 1), one(p.z, s.z, ii + 2), one(p.w, s.w, ii + 3));
+            const float4 p = *reinterpret_cast<const float4*>(pha + o);
+            float4 s;
+            if (gs) {
+                const float2 g0 = gs[0], g1 = gs[1], g2 = gs[2], g3 = gs[3];
+                s = make_float4(fmaf(sc, g0.x, sc * g0.y), fmaf(sc, g1.x, sc * g1.y), fmaf(sc, g2.x, sc * g2.y),
+                                fmaf(sc, g3.x, sc * g3.y));
+            } else {
+                s = *reinterpret_cast<const float4*>(psum + o);
             }
+            *reinterpret_cast<float4*>(pha + o) =
+                make_float4(one(p.x, s.x, ii), one(p.y, s.y, ii + 1), one(p.z, s.z, ii + 2), one(p.w, s.w, ii + 3));
         } else {
-            for (int ii = threadIdx.x; ii < Nout; ii += blockDim.x)
-                pha[ro + ii] = one(pha[ro + ii], gs ? fmaf(sc, gs[ii].x, sc * gs[ii].y) : psum[ro + ii], ii);
+            pha[o] = one(pha[o], gs ? fmaf(sc, gs[0].x, sc * gs[0].y) : psum[o], ii);
         }
     }
 }
 
-cudaError_t sci_apply(const InstDev* insts, const int* list, int nsci, int maxnout, const int* d_step, cudaStream_t st)
+cudaError_t sci_apply(const InstDev* insts, const int* list, int nsci, int maxnout, const int* d_step, long pdl_ctas,
+                      cudaStream_t st)
 {
     if (nsci <= 0) return cudaSuccess;
-    const int bx = maxnout < 256 ? maxnout : 256;
-    return launch_gated(k_sci_apply, dim3(bx, nsci), dim3(256), 0, st, insts, list, d_step);
+    // at most 256 CTAs per instance once the instances fill the GPU, more for
+    // a few large frames (one 2048^2 frame on 256 CTAs: eight rows in turn each)
+    const long need = ((long)maxnout * maxnout / (maxnout % 4 == 0 ? 4 : 1) + 255) / 256;
+    const long cap = std::max(256L, (16L * 152 + nsci - 1) / nsci);
+    const int bx = (int)std::max(1L, std::min(need, cap));
+    return launch_gated_up_to(pdl_ctas, k_sci_apply, dim3(bx, nsci), dim3(256), 0, st, insts, list, d_step);
 }
 
 // Layer sum of one window group, from the top layer down with a two-sum
@@ -345,12 +379,13 @@ __global__ void __launch_bounds__(256) k_group_sum(const GroupSumJob* __restrict
     }
 }
 
-cudaError_t group_sums(const GroupSumJob* jobs, int njobs, int L, int maxside, cudaStream_t st)
+cudaError_t group_sums(const GroupSumJob* jobs, int njobs, int L, int maxside, long pdl_ctas, cudaStream_t st)
 {
     if (njobs <= 0) return cudaSuccess;
     const long n4 = (long)maxside * maxside / 4;
     const long b = (n4 + 255) / 256;
-    return launch_gated(k_group_sum, dim3((unsigned)(b < 1024 ? b : 1024), (unsigned)njobs), dim3(256), 0, st, jobs, L);
+    return launch_gated_up_to(pdl_ctas, k_group_sum, dim3((unsigned)(b < 1024 ? b : 1024), (unsigned)njobs), dim3(256), 0, st,
+                              jobs, L);
 }
 
 __global__ void k_step_advance(int* d_step)

@@ -349,6 +349,7 @@ struct atmwfs_ctx {
     std::vector<float*> d_pad[2];        // padded copies per layer and orientation
     std::vector<char> loaded;
     bool normalized = false, committed = false;
+    bool tuning = false;                 // the autotuner is timing its candidates
     std::vector<Class> classes;
     // window groups: instances whose layer positions are identical at every
     // step (same start positions and offsets) share the per-step bicubic
@@ -508,6 +509,11 @@ atmwfs_status make_tma_map(CUtensorMap* m, float* base, int Wp, int Hp, int box_
 // the screen's own orientation.
 int pass_orient(int k, int Q) { return (Q - k) & 1; }
 
+// Largest grid of the step launched with programmatic dependent launch.  The
+// autotuner times its candidates with plain launches: back-to-back launches
+// of one configuration that overlap there would not predict its time in a step.
+long step_pdl_ctas(const atmwfs_ctx* c) { return c->tuning ? 0 : pdl_max_ctas(); }
+
 // The window kernel over jobs [j0, j1) of class cl (the windows of the
 // groups whose side is cl's grid); optionally report its algorithmic bytes.
 atmwfs_status launch_windows(atmwfs_ctx* c, Class& cl, int j0, int j1, double* bytes, cudaStream_t st)
@@ -523,6 +529,7 @@ atmwfs_status launch_windows(atmwfs_ctx* c, Class& cl, int j0, int j1, double* b
     a.ninst_total = c->ninst;
     a.poscap = c->poscap;
     a.jobs = cl.d_jobs + j0;
+    a.pdl_ctas = step_pdl_ctas(c);
     const int RR0 = tile_cfg(cl.N, 0).rr;
     // screen tiles in (RR0 + 3 rows of the padded width) and windows out
     if (bytes) *bytes = (4.0 * (RR0 + 3) / RR0 + 4.0) * (double)cl.N * cl.N * (j1 - j0);
@@ -547,6 +554,7 @@ atmwfs_status launch_phases(atmwfs_ctx* c, Class& cl, double* bytes, cudaStream_
     a.poscap = c->poscap;
     a.pjobs = cl.d_pjobs;
     a.pslots = cl.d_pslots;
+    a.pdl_ctas = step_pdl_ctas(c);
     const int RR = phase_rows(cl.N);
     if (bytes) {
         *bytes = 4.0 * (RR + 3) / RR * c->L * (double)cl.N * cl.N * cl.pjobs.size();
@@ -574,7 +582,7 @@ atmwfs_status launch_pass(atmwfs_ctx* c, int k, Class& cl, double* bytes, cudaSt
         // sums of the others (k_phasum), from the step's windows
         double b = 0;
         if (!cl.gjobs.empty()) {
-            AW_CUDA(group_sums(cl.d_gjobs, (int)cl.gjobs.size(), c->L, cl.N, st));
+            AW_CUDA(group_sums(cl.d_gjobs, (int)cl.gjobs.size(), c->L, cl.N, step_pdl_ctas(c), st));
             b += (4.0 * c->L + 8.0) * (double)cl.N * cl.N * cl.gjobs.size();
         }
         if (!cl.need_phasum) {
@@ -589,6 +597,7 @@ atmwfs_status launch_pass(atmwfs_ctx* c, int k, Class& cl, double* bytes, cudaSt
         a.L = c->L;
         a.ninst_total = c->ninst;
         a.poscap = c->poscap;
+        a.pdl_ctas = step_pdl_ctas(c);
         int own = 0;
         for (int i : cl.members) own += c->d_gsum[c->group_of[i]] == nullptr;
         if (bytes) *bytes = b + (4.0 * c->L + 4.0) * cl.Nout * cl.Nout * own;
@@ -601,8 +610,9 @@ atmwfs_status launch_pass(atmwfs_ctx* c, int k, Class& cl, double* bytes, cudaSt
         // instance of the context (diagnostics only)
         if (bytes) *bytes = 0;
         if (c->nsci > 0) {
-            AW_CUDA(unwrap_bins(c->d_inst, c->d_sci, c->nsci, c->maxnb, c->d_status, c->d_iters, c->d_atan_tab, st));
-            AW_CUDA(sci_apply(c->d_inst, c->d_sci, c->nsci, c->maxnout, c->d_step, st));
+            AW_CUDA(unwrap_bins(c->d_inst, c->d_sci, c->nsci, c->maxnb, c->d_status, c->d_iters, c->d_atan_tab,
+                                step_pdl_ctas(c), st));
+            AW_CUDA(sci_apply(c->d_inst, c->d_sci, c->nsci, c->maxnout, c->d_step, step_pdl_ctas(c), st));
         }
         return ATMWFS_OK;
     }
@@ -623,6 +633,7 @@ atmwfs_status launch_pass(atmwfs_ctx* c, int k, Class& cl, double* bytes, cudaSt
             a.L = c->L;
             a.ninst_total = c->ninst;
             a.poscap = c->poscap;
+            a.pdl_ctas = step_pdl_ctas(c);
             a.g_lo = c->plane_lo[k - 1];
             a.g_hi = c->plane_hi[k - 1];
             a.hop1 = k - 2;
@@ -666,6 +677,16 @@ atmwfs_status launch_pass(atmwfs_ctx* c, int k, Class& cl, double* bytes, cudaSt
     return ATMWFS_OK;
 }
 
+// The science unwrap and apply of one class's instances.
+atmwfs_status launch_science(atmwfs_ctx* c, const Class& cl, cudaStream_t st)
+{
+    if (cl.nsci == 0) return ATMWFS_OK;
+    const long lim = step_pdl_ctas(c);
+    AW_CUDA(unwrap_bins(c->d_inst, c->d_sci + cl.sci0, cl.nsci, cl.maxnb, c->d_status, c->d_iters, c->d_atan_tab, lim, st));
+    AW_CUDA(sci_apply(c->d_inst, c->d_sci + cl.sci0, cl.nsci, cl.maxnout, c->d_step, lim, st));
+    return ATMWFS_OK;
+}
+
 // One step.  The screen windows of every window group come first; then the
 // graph forks: the phase sums (independent of the field) on their own
 // branch, every grid class's chain of passes on its own branch; the last pass
@@ -698,12 +719,7 @@ atmwfs_status launch_step(atmwfs_ctx* c)
         }
         // the class's science unwrap and apply on its own branch: a class that
         // finishes early unwraps beside the passes of the larger grids
-        const Class& cl = c->classes[ci];
-        if (cl.nsci > 0) {
-            AW_CUDA(unwrap_bins(c->d_inst, c->d_sci + cl.sci0, cl.nsci, cl.maxnb, c->d_status, c->d_iters,
-                                c->d_atan_tab, cs));
-            AW_CUDA(sci_apply(c->d_inst, c->d_sci + cl.sci0, cl.nsci, cl.maxnout, c->d_step, cs));
-        }
+        AW_TRY(launch_science(c, c->classes[ci], cs));
         AW_CUDA(cudaEventRecord(c->gev[2 + ci], cs));
         AW_CUDA(cudaStreamWaitEvent(c->st, c->gev[2 + ci], 0));
     }
@@ -723,9 +739,9 @@ atmwfs_status clear_bins(atmwfs_ctx* c)
     return ATMWFS_OK;
 }
 
-// Project autotuner: for every grid class time the representative pass
-// (a middle pass when there is one) in each configuration compiled for its
-// size -- radix plan and tile shape (tile_cfg) -- and keep the fastest.
+// Project autotuner: for every grid class time its chain of passes (first,
+// middle, last, weighted by their number) in each configuration compiled for
+// its size -- radix plan and tile shape (tile_cfg) -- and keep the fastest.
 // ATMWFS_TILE_CFG=<k> forces configuration k (ignored where the size has
 // none); ATMWFS_TILE_CFG=<N>:<k>[,<N>:<k>...] forces it for the listed grid
 // sizes only and tunes the others.  Science bins are cleared afterwards (a
@@ -748,15 +764,16 @@ atmwfs_status autotune(atmwfs_ctx* c)
 {
     const int Q = (int)c->plane_lo.size();
     const char* force = getenv("ATMWFS_TILE_CFG");
-    const int k = Q >= 3 ? 2 : 1;
-    // the candidates are timed with plain launches (see pdl_hold)
-    struct Hold {
-        Hold() { pdl_hold() = 1; }
-        ~Hold() { pdl_hold() = 0; }
-    } hold;
-    cudaEvent_t e0, e1;
-    AW_CUDA(cudaEventCreate(&e0));
-    AW_CUDA(cudaEventCreate(&e1));
+    std::vector<int> kinds = {1};
+    if (Q >= 3) kinds.push_back(2);
+    if (Q >= 2) kinds.push_back(Q);
+    struct Tuning {
+        atmwfs_ctx* c;
+        explicit Tuning(atmwfs_ctx* x) : c(x) { c->tuning = true; }
+        ~Tuning() { c->tuning = false; }
+    } tuning(c);
+    cudaEvent_t ev[4];
+    for (cudaEvent_t& e : ev) AW_CUDA(cudaEventCreate(&e));
     atmwfs_status s = ATMWFS_OK;
     for (Class& cl : c->classes) {
         if (!c->amplitude) {
@@ -767,23 +784,34 @@ atmwfs_status autotune(atmwfs_ctx* c)
             const int g = forced_cfg(force, cl.N);
             cl.cfg = (g < kNumTileCfg && tile_cfg(cl.N, g).rr > 0) ? g : 0;
         } else {
-            // two interleaved rounds over the configurations; each keeps its
-            // fastest reading, so one disturbed reading does not decide
+            // interleaved rounds over the configurations, two or (short passes)
+            // three; each configuration keeps its fastest reading, so one
+            // disturbed reading does not decide
             for (int g = 0; g < kNumTileCfg; g++) cl.tuned_ms[g] = 1e30f;
-            for (int round = 0; round < 2 && s == ATMWFS_OK; round++) {
+            double spent = 0;
+            for (int round = 0; round < 3 && (round < 2 || spent < 1.0) && s == ATMWFS_OK; round++) {
                 for (int g = 0; g < kNumTileCfg && s == ATMWFS_OK; g++) {
                     if (tile_cfg(cl.N, g).rr == 0) continue;  // not compiled at this size
                     cl.cfg = g;
                     cl.RR = tile_cfg(cl.N, g).rr;
-                    s = launch_pass(c, k, cl, nullptr, c->st);
+                    s = launch_pass(c, kinds[0], cl, nullptr, c->st);  // warm-up
+                    for (size_t q = 0; q < kinds.size() && s == ATMWFS_OK; q++) {
+                        cudaEventRecord(ev[q], c->st);
+                        s = launch_pass(c, kinds[q], cl, nullptr, c->st);
+                    }
                     if (s != ATMWFS_OK) break;
-                    cudaEventRecord(e0, c->st);
-                    for (int r = 0; r < 3 && s == ATMWFS_OK; r++) s = launch_pass(c, k, cl, nullptr, c->st);
-                    cudaEventRecord(e1, c->st);
-                    float ms = 0;
-                    if (cudaEventSynchronize(e1) != cudaSuccess || cudaEventElapsedTime(&ms, e0, e1) != cudaSuccess)
-                        s = fail(ATMWFS_ERR_CUDA, "autotune timing failed");
-                    if (ms / 3 < cl.tuned_ms[g]) cl.tuned_ms[g] = ms / 3;
+                    cudaEventRecord(ev[kinds.size()], c->st);
+                    float total = 0;
+                    if (cudaEventSynchronize(ev[kinds.size()]) != cudaSuccess) s = fail(ATMWFS_ERR_CUDA, "autotune timing failed");
+                    for (size_t q = 0; q < kinds.size() && s == ATMWFS_OK; q++) {
+                        float ms = 0;
+                        if (cudaEventElapsedTime(&ms, ev[q], ev[q + 1]) != cudaSuccess)
+                            s = fail(ATMWFS_ERR_CUDA, "autotune timing failed");
+                        spent += ms;
+                        total += ms * (q == 1 && Q >= 3 ? Q - 2 : 1);
+                    }
+                    total /= Q;  // mean pass
+                    if (s == ATMWFS_OK && total < cl.tuned_ms[g]) cl.tuned_ms[g] = total;
                 }
             }
             int bg = 0;
@@ -795,8 +823,7 @@ atmwfs_status autotune(atmwfs_ctx* c)
         }
         cl.RR = tile_cfg(cl.N, cl.cfg).rr;
     }
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
+    for (cudaEvent_t e : ev) cudaEventDestroy(e);
     if (s != ATMWFS_OK) return s;
     AW_TRY(clear_bins(c));
     AW_CUDA(cudaStreamSynchronize(c->st));

@@ -51,15 +51,6 @@ inline int pdl_max_ctas()
     return n;
 }
 
-// Non-zero while the autotuner times its candidates: it times each
-// configuration's launches back to back, and overlapped launches there would
-// not predict the configuration's time inside a step.
-inline int& pdl_hold()
-{
-    static int h = 0;
-    return h;
-}
-
 // Launch k<<<grid, block, sm, st>>>(args...), with programmatic stream
 // serialization when the grid has at most max_ctas CTAs; k must open with
 // pdl_gate().
@@ -76,7 +67,7 @@ cudaError_t launch_gated_up_to(long max_ctas, void (*k)(P...), dim3 grid, dim3 b
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
-    cfg.numAttrs = pdl_hold() == 0 && (long)grid.x * grid.y * grid.z <= max_ctas ? 1 : 0;
+    cfg.numAttrs = (long)grid.x * grid.y * grid.z <= max_ctas ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, k, std::forward<A>(args)...);
 }
 template <typename... P, typename... A>
@@ -216,6 +207,7 @@ struct PassArgs {
     // phase-only frames: their jobs (blockIdx.y) and the jobs' instance slots
     const PhaseJob* pjobs;
     const int* pslots;
+    long pdl_ctas;             // host: largest grid launched with programmatic dependent launch
 };
 
 // Tensor maps of the halo-padded screens: [orientation][layer].
@@ -268,7 +260,7 @@ constexpr TileCfg tile_cfg(int N, int c)
          : N == 256   ? (c == 0 ? TileCfg{16, 1, false, 0, false} : c == 1 ? TileCfg{8, 3, false, 0, false} : TileCfg{8, 4, true, 0, false})
          : N == 512   ? (c == 0 ? TileCfg{16, 1, false, 0, false} : c == 1 ? TileCfg{8, 3, false, 0, false} : TileCfg{8, 4, true, 0, false})
          : N == 1024  ? (c == 0 ? TileCfg{8, 1, false, 0, false} : c == 1 ? TileCfg{4, 3, false, 0, false} : TileCfg{4, 4, true, 0, false})
-         : N == 2048  ? (c == 0 ? TileCfg{4, 1, false, 0, false} : c == 1 ? TileCfg{2, 3, false, 0, false} : TileCfg{2, 3, true, 0, false})
+         : N == 2048  ? (c == 0 ? TileCfg{4, 1, false, 0, false} : c == 1 ? TileCfg{2, 3, false, 0, false} : TileCfg{4, 2, true, 0, false})
                       : TileCfg{0, 0, false, 0, false};
 }
 
