@@ -67,6 +67,14 @@ cudaError_t xspectral_umma(const __nv_bfloat16* Bt, int n, int k, const float* A
                            long M, unsigned* status, int swap, cudaStream_t st);
 cudaError_t spectral_umma(const __nv_bfloat16* W, int o, int c, const float* X, float* C, long P, unsigned* status,
                           int swap, cudaStream_t st);
+// fused forward kernels of the default shape (fno_fused.cu)
+bool fused_supported(int grid, int modes, int width, int proj, int nout);
+cudaError_t xdft_fused(const __nv_bfloat16* F, const float* H, float* a, int B, unsigned* status, cudaStream_t st);
+cudaError_t fourier_fused(const __nv_bfloat16* W, const __nv_bfloat16* Gt, const float* X, const float* bb, float* U,
+                          float* act, const float* bias, int B, unsigned* status, bool write_u, cudaStream_t st);
+cudaError_t project_fused(const __nv_bfloat16* W1, const float* c1, const __nv_bfloat16* W2, const float* c2,
+                          const float* X, float* qpre, float* q, float* out, int B, unsigned* status, bool keep,
+                          cudaStream_t st);
 }  // namespace atmwfs
 
 struct atmwfs_fno {
@@ -187,43 +195,88 @@ __global__ void k_mse(const float* __restrict__ out, const float* __restrict__ t
     if ((threadIdx.x & 31) == 0) atomicAdd(loss, s / (double)n);
 }
 
-// Mode mixing y[b][o][k] = sum_c R[k][o][c] z[b][c][k] (complex), one block
-// per mode k = (ky, kx).  z / y layout [2m][B w][m]: row ky holds the real
-// parts, row m + ky the imaginary parts, then (sample, channel), then kx.
-__global__ void k_modemix(const __nv_bfloat16* __restrict__ R, const float* __restrict__ z, float* __restrict__ y,
-                          int B, int w, int m)
+// Mode mixing y[b][o][k] = sum_c R[k][o][c] z[b][c][k] (complex) for KX
+// neighbouring kx of one ky (blockIdx.x = ky (m / KX) + kx / KX).  z / y
+// layout [2m][B w][m]: row ky holds the real parts, row m + ky the imaginary
+// parts, then (sample, channel), then kx, so KX neighbours are one vector.
+// FP32 FMAs bound it: 8 w^2 B m^2 operations, 7 us for a batch of 16 at the
+// default shape.  A thread owns one (mode, output channel) and kMixB samples:
+// a weight is read from shared memory once for all of them and the samples'
+// values are broadcasts, two channels to a load (one thread per output value
+// read both operands for every product: 67 us).
+constexpr int kMixB = 8;
+template <int KX>
+__global__ void __launch_bounds__(256) k_modemix(const __nv_bfloat16* __restrict__ R, const float* __restrict__ z,
+                                                 float* __restrict__ y, int B, int w, int m)
 {
-    const int k = blockIdx.x, ky = k / m, kx = k % m;
-    const long plane = m;                                     // (sample, channel) stride
+    const int groups = m / KX, ky = blockIdx.x / groups, kx0 = blockIdx.x % groups * KX;
     const long Nc = (long)B * w * m;
-    const long ore = (long)ky * Nc + kx, oim = (long)(m + ky) * Nc + kx;
-    extern __shared__ float sh[];
-    float* zs = sh;                  // [B][w][2]
-    float2* rs = reinterpret_cast<float2*>(sh + 2 * B * w);  // [w][w + 1]: R[o][c], padded rows
-    const __nv_bfloat16* Rk = R + (size_t)k * w * w * 2;
-    for (int i = threadIdx.x; i < w * w; i += blockDim.x) {
-        const __nv_bfloat162 v = reinterpret_cast<const __nv_bfloat162*>(Rk)[i];  // coalesced (re, im) pairs
-        rs[(i / w) * (w + 1) + i % w] = make_float2(__low2float(v), __high2float(v));
-    }
-    for (int i = threadIdx.x; i < B * w; i += blockDim.x) {
-        zs[2 * i] = z[i * plane + ore];
-        zs[2 * i + 1] = z[i * plane + oim];
-    }
-    __syncthreads();
-    for (int i = threadIdx.x; i < B * w; i += blockDim.x) {
-        const int bq = i / w, o = i % w;
-        const float2* r = rs + o * (w + 1);
-        const float* zb = zs + 2 * bq * w;
-        float sr = 0.0f, si = 0.0f;
-        for (int c = 0; c < w; c++) {
-            const float2 rc = r[c];
-            const float zr = zb[2 * c], zi = zb[2 * c + 1];
-            sr += rc.x * zr - rc.y * zi;
-            si += rc.x * zi + rc.y * zr;
+    const long ore = (long)ky * Nc + kx0, oim = (long)(m + ky) * Nc + kx0;
+    extern __shared__ float4 mix_smem[];
+    float* zs = reinterpret_cast<float*>(mix_smem);                                 // [KX][kMixB][w][2]
+    __nv_bfloat162* rs = reinterpret_cast<__nv_bfloat162*>(zs + KX * kMixB * w * 2);  // [KX][w][w + 1]
+    const __nv_bfloat162* Rk = reinterpret_cast<const __nv_bfloat162*>(R) + (size_t)(ky * m + kx0) * w * w;
+    for (int i = threadIdx.x; i < KX * w * w; i += blockDim.x) rs[i / w * (w + 1) + i % w] = Rk[i];
+    for (int b0 = 0; b0 < B; b0 += kMixB) {
+        const int nb = min(kMixB, B - b0);
+        __syncthreads();  // the previous samples are used
+        for (int i = threadIdx.x; i < kMixB * w; i += blockDim.x) {
+            float vr[KX], vi[KX];
+            const long o = (long)(b0 * w + i) * m;
+#pragma unroll
+            for (int k = 0; k < KX; k++) {
+                vr[k] = i < nb * w ? z[o + ore + k] : 0.0f;
+                vi[k] = i < nb * w ? z[o + oim + k] : 0.0f;
+            }
+#pragma unroll
+            for (int k = 0; k < KX; k++) reinterpret_cast<float2*>(zs)[k * kMixB * w + i] = make_float2(vr[k], vi[k]);
         }
-        y[i * plane + ore] = sr;
-        y[i * plane + oim] = si;
+        __syncthreads();
+        for (int i = threadIdx.x; i < KX * w; i += blockDim.x) {
+            const int k = i / w, o = i % w;
+            const __nv_bfloat162* r = rs + (size_t)i * (w + 1);
+            const float4* zk = reinterpret_cast<const float4*>(zs + (size_t)k * kMixB * w * 2);
+            float sr[kMixB], si[kMixB];
+#pragma unroll
+            for (int b = 0; b < kMixB; b++) sr[b] = si[b] = 0.0f;
+            for (int c = 0; c < w; c += 2) {  // w is even
+                const float2 r0 = make_float2(__low2float(r[c]), __high2float(r[c]));
+                const float2 r1 = make_float2(__low2float(r[c + 1]), __high2float(r[c + 1]));
+#pragma unroll
+                for (int b = 0; b < kMixB; b++) {
+                    const float4 v = zk[(b * w + c) / 2];
+                    sr[b] += r0.x * v.x - r0.y * v.y;
+                    si[b] += r0.x * v.y + r0.y * v.x;
+                    sr[b] += r1.x * v.z - r1.y * v.w;
+                    si[b] += r1.x * v.w + r1.y * v.z;
+                }
+            }
+            for (int b = 0; b < nb; b++) {
+                const long q = (long)((b0 + b) * w + o) * m + k;
+                y[q + ore] = sr[b];
+                y[q + oim] = si[b];
+            }
+        }
     }
+}
+
+template <int KX>
+constexpr size_t modemix_smem(int w) { return (size_t)KX * ((size_t)kMixB * w * 8 + (size_t)w * (w + 1) * 4); }
+
+// Four neighbouring modes per CTA where they fit twice into an SM, else two or one.
+cudaError_t modemix(const __nv_bfloat16* R, const float* z, float* y, int B, int w, int m, cudaStream_t st)
+{
+    auto go = [&](auto kern, size_t sm, int kx) -> cudaError_t {
+        if (sm > 48 * 1024) {
+            const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+            if (e != cudaSuccess) return e;
+        }
+        kern<<<m * m / kx, 256, sm, st>>>(R, z, y, B, w, m);
+        return cudaGetLastError();
+    };
+    if (m % 4 == 0 && modemix_smem<4>(w) <= 113 * 1024) return go(k_modemix<4>, modemix_smem<4>(w), 4);
+    if (modemix_smem<2>(w) <= 113 * 1024) return go(k_modemix<2>, modemix_smem<2>(w), 2);  // m is even
+    return go(k_modemix<1>, modemix_smem<1>(w), 1);
 }
 
 // Backward of the mode mixing: dz = R^H dy per mode, and dR += sum_b dy z^H.
@@ -529,7 +582,8 @@ static cudaError_t gemm_args(GemmArgs& g, float beta, cudaStream_t st)
     return gemm_launch(g, beta, st);
 }
 
-// spectral convolution of layer l: spec = S_l(h)
+// spectral convolution of layer l: spec = S_l(h); spec NULL: up to bb, the
+// image before the inverse transform along x (which k_fourier applies)
 atmwfs_status spectral_fwd(atmwfs_fno* f, int l, const void* h, int h_bf16, float* spec, int B, cudaStream_t st)
 {
     const atmwfs_fno_cfg& c = f->cfg;
@@ -539,7 +593,9 @@ atmwfs_status spectral_fwd(atmwfs_fno* f, int l, const void* h, int h_bf16, floa
     float* z = f->z[l];
     const bool tcx = umma_enabled() && xspectral_umma_supported(2 * m, G) && xspectral_umma_supported(G, 2 * m);
     {   // a[p][y][bc][kx] = sum_x h[bc][y][x] Fx[x][p m + kx]
-        if (tcx && !h_bf16 &&
+        if (!spec) {
+            FN_CUDA(xdft_fused(f->FxT_bf, (const float*)h, a, B, umma_status_ptr(), st));
+        } else if (tcx && !h_bf16 &&
             xspectral_umma(f->FxT_bf, 2 * m, G, (const float*)h, 0, G, 0, G, 0, a, G, Nc, m, m, (long)G * Nc, BW * G,
                            umma_status_ptr(), 0, st) == cudaSuccess) {
         } else {
@@ -560,15 +616,14 @@ atmwfs_status spectral_fwd(atmwfs_fno* f, int l, const void* h, int h_bf16, floa
     // y = R z per mode
     const size_t smf = sizeof(float) * (2 * B * w + 2 * w * (w + 1));
     if (smf > 227 * 1024) return err(ATMWFS_ERR_INVALID, "batch %d x width %d exceeds the mode-mixing shared memory", B, w);
-    if (smf > 48 * 1024) FN_CUDA(cudaFuncSetAttribute(k_modemix, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smf));
-    k_modemix<<<m * m, 256, smf, st>>>(f->pbf + f->L.R[l], z, f->y, B, w, m);
-    FN_CUDA(cudaGetLastError());
+    FN_CUDA(modemix(f->pbf + f->L.R[l], z, f->y, B, w, m, st));
     // bb = GyBig y: [2G, 2m] x [2m, Nc], on tcgen05 where compiled
     if (tc && spectral_umma_supported(2 * G, 2 * m))
         FN_CUDA(spectral_umma(f->GyBig_bf, 2 * G, 2 * m, f->y, f->bb, Nc, umma_status_ptr(), 0, st));
     else
         FN_CUDA(gemm(2 * G, (int)Nc, 2 * m, f->GyBig, 2 * m, 0, 0, f->y, Nc, 0, 0, f->bb, Nc, 0.0f, 1, 0, 0, 0, nullptr, 0,
                      st));
+    if (!spec) return ATMWFS_OK;
     {   // spec[bo][y][x] = sum_{p,kx} bb[p][y][bo][kx] Gx[p m + kx][x]: rows (bo, y), A read through its maps
         if (tcx && xspectral_umma(f->GxT_bf, G, 2 * m, f->bb, G, Nc, m, m, (long)G * Nc, spec, 0, G, 0, G, 0, BW * G,
                                   umma_status_ptr(), 0, st) == cudaSuccess) {
@@ -673,6 +728,18 @@ atmwfs_status forward(atmwfs_fno* f, const float* x, float* out, int B, cudaStre
                        ? 1
                        : 0;
     FN_CUDA(pointwise_fwd(pb + f->L.lift_W, c.width, c.nin, x, 0, f->h[0], B, P, 0.0f, pf + f->L.lift_b, st));
+    if (!bf && umma_enabled() && fused_supported(c.grid, c.modes, c.width, c.proj, c.nout)) {
+        unsigned* status = umma_status_ptr();
+        if (!status) return err(ATMWFS_ERR_CUDA, "status symbol");
+        for (int l = 0; l < c.layers; l++) {
+            FN_TRY(spectral_fwd(f, l, f->h[l], 0, nullptr, B, st));
+            FN_CUDA(fourier_fused(pb + f->L.W[l], f->GxT_bf, f->h[l], f->bb, f->u[l], l + 1 < c.layers ? f->h[l + 1] : nullptr,
+                                  pf + f->L.b[l], B, status, training, st));
+        }
+        FN_CUDA(project_fused(pb + f->L.proj1_W, pf + f->L.proj1_b, pb + f->L.proj2_W, pf + f->L.proj2_b, last_h(f), f->qpre,
+                              f->q, out, B, status, training, st));
+        return ATMWFS_OK;
+    }
     for (int l = 0; l < c.layers; l++) {
         // u = S_l(h) + W_l h + b_l; h' = gelu(u) from the same epilogue
         // (the last layer has no activation: its u is the projection's input)

@@ -1,0 +1,410 @@
+// fno_fused.cu -- the forward pass of the surrogate's default shape (grid 256,
+// 32 modes, width 64, projection 128) as kernels that fuse neighbouring
+// products on the tcgen05 tensor cores, so that the images between them are
+// not written and read back:
+//   k_xdft     the forward DFT along x, written as coalesced spectrum rows;
+//   k_fourier  pointwise mixing + inverse DFT along x + bias (+ GELU);
+//   k_project  the first projection + GELU + the 2-channel output.
+// The products keep the operands' BF16 rounding, the K order and the FP32
+// accumulation of the separate products (k_pointwise, k_rowprod, the mma.sync
+// GEMM), so a layer's results are the same bits.
+#include <cuda_bf16.h>
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+#include "atmwfs_fno.h"
+#include "fno_gemm.cuh"
+#include "umma_core.cuh"
+
+namespace atmwfs {
+namespace umma {
+
+constexpr int kG = 256;       // grid side
+constexpr int kModes = 32;    // modes per axis
+constexpr int kW = 64;        // width
+constexpr int kProj = 128;    // projection channels
+constexpr long kP = (long)kG * kG;
+
+__device__ __forceinline__ uint4 pack8(const float (&f)[8])
+{
+    __nv_bfloat162 h[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) h[q] = __floats2bfloat162_rn(f[2 * q], f[2 * q + 1]);
+    uint4 v;
+    v.x = *reinterpret_cast<uint32_t*>(&h[0]);
+    v.y = *reinterpret_cast<uint32_t*>(&h[1]);
+    v.z = *reinterpret_cast<uint32_t*>(&h[2]);
+    v.w = *reinterpret_cast<uint32_t*>(&h[3]);
+    return v;
+}
+
+// ---------------------------------------------------------------------------
+// Forward DFT along x of one line (sample b, row y), all channels:
+//   a[p][y][b w + c][kx] = sum_x F[p m + kx][x] h[b][c][y][x]
+// as D = F h^T: the 2 m = 64 rows of F are the MMA's M (rows 64 .. 127 of the
+// 128 are whatever follows in shared memory, here B, and their results are not
+// read), the channels its N, K = 256.  With the modes along the TMEM lanes a
+// channel's spectrum leaves as one 128-byte run per warp.  (k_rowprod has the
+// lines along the lanes and writes 16-byte pieces 128 bytes apart: the rate of
+// L2 requests bounds it, 138 us for a batch of 16 against 49 us of HBM time.)
+// F is staged once per CTA; a line's 64 KB are loaded into registers while the
+// previous line's products run, so a CTA keeps 64 KB in flight.
+// ---------------------------------------------------------------------------
+constexpr int kXK = kG / 8;                        // core matrices along K
+constexpr uint32_t kXBytes = 2 * kModes * kG * 2;  // F, and one line of 64 channels, in BF16: 32 KB each
+static_assert(2 * kModes == kW, "the two operands have the same shape");
+
+// piece j of thread tid: 8 consecutive x of one channel; the lanes of a warp
+// take 8 channels x 4 pieces, so that a store phase of 8 lanes fills one
+// 128-byte core matrix
+__device__ __forceinline__ void x_piece(int tid, int j, int& row, int& k8)
+{
+    const int i = tid + kThreads * j, rest = i >> 5;
+    row = (rest & 7) * 8 + (i & 7);
+    k8 = (rest >> 3) * 4 + ((i >> 3) & 3);
+}
+
+__global__ void __launch_bounds__(kThreads, 2) k_xdft(const __nv_bfloat16* __restrict__ F, const float* __restrict__ H,
+                                                      float* __restrict__ a, int nlines, long Nc, unsigned* status)
+{
+    constexpr int J = kW * kXK / kThreads;  // pieces per thread
+    extern __shared__ __align__(1024) unsigned char sm[];
+    unsigned char *sa = sm, *sb = sm + kXBytes;
+    __shared__ __align__(8) uint64_t bar;
+    __shared__ uint32_t tmem_base;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    float4 v[J][2];
+    auto load = [&](int line) {
+        const float* src = H + (size_t)(line / kG) * kW * kP + (size_t)(line % kG) * kG;
+#pragma unroll
+        for (int j = 0; j < J; j++) {
+            int row, k8;
+            x_piece(tid, j, row, k8);
+            const float4* q = reinterpret_cast<const float4*>(src + (size_t)row * kP + k8 * 8);
+            v[j][0] = __ldg(q);
+            v[j][1] = __ldg(q + 1);
+        }
+    };
+    if (blockIdx.x < nlines) load(blockIdx.x);
+    tmem_alloc(&tmem_base, 64, warp);
+    if (tid == 0) mbar_init(&bar);
+#pragma unroll
+    for (int j = 0; j < J; j++) {
+        int row, k8;
+        x_piece(tid, j, row, k8);
+        *reinterpret_cast<uint4*>(sa + kmajor_off(row, k8 * 8, kXK)) =
+            *reinterpret_cast<const uint4*>(F + (size_t)row * kG + k8 * 8);
+    }
+    fence_before();
+    __syncthreads();
+    fence_after();
+    const uint32_t tmem = tmem_base, a_addr = smem_addr(sa), b_addr = smem_addr(sb);
+    uint32_t parity = 0;
+    for (int line = blockIdx.x; line < nlines; line += gridDim.x) {
+#pragma unroll
+        for (int j = 0; j < J; j++) {
+            int row, k8;
+            x_piece(tid, j, row, k8);
+            const float f[8] = {v[j][0].x, v[j][0].y, v[j][0].z, v[j][0].w, v[j][1].x, v[j][1].y, v[j][1].z, v[j][1].w};
+            *reinterpret_cast<uint4*>(sb + kmajor_off(row, k8 * 8, kXK)) = pack8(f);
+        }
+        publish_smem();
+        if (line + (int)gridDim.x < nlines) load(line + gridDim.x);
+        if (tid == 0) {
+#pragma unroll
+            for (int ks = 0; ks < kG / 16; ks++)
+                mma_bf16(tmem, smem_desc(a_addr + ks * 256, 128, kXK * 128), smem_desc(b_addr + ks * 256, 128, kXK * 128),
+                         instr_desc(kW), ks > 0);
+            mma_commit(&bar);
+        }
+        if (!mma_wait(&bar, parity, status)) break;
+        parity ^= 1;
+        const int p = warp & 3, half = warp >> 2;
+        if (p < 2) {
+            const int b = line / kG, y = line % kG;
+            float* o = a + (size_t)p * kG * Nc + (size_t)y * Nc + (size_t)b * kW * kModes + lane;
+#pragma unroll
+            for (int c0 = half * (kW / 2); c0 < (half + 1) * (kW / 2); c0 += 16) {
+                float r[16];
+                tmem_ld16(tmem + ((uint32_t)(p * 32) << 16) + c0, r);
+#pragma unroll
+                for (int q = 0; q < 16; q++) o[(size_t)(c0 + q) * kModes] = r[q];
+            }
+        }
+        retire_tile();
+    }
+    tmem_free(tmem, 64, warp);
+}
+
+// ---------------------------------------------------------------------------
+// A Fourier layer's output u = W h + b + S, S the inverse DFT along x of the
+// planar spectrum bb, and act = gelu(u): for 128 pixels of a line (sample b,
+// row y, half of x)
+//   D1 = X^T W^T   (128 pixels x 64 channels, K = 64 channels)
+//   D2 = Gx^T B^T  (128 pixels x 64 channels, K = 64: re and im of 32 modes)
+// in two ranges of tensor memory, added in the epilogue in the order of the
+// separate products.  The inverse DFT's image is 268 MB per layer and batch
+// of 16: it was written in 16-byte pieces (126 us) and read back by the
+// pointwise product (161 us); both now run as one pass over h and bb.
+// Gx^T and W are staged once per CTA; a tile's 32 channel values per thread
+// and the line's spectrum are loaded while the previous tile's products run.
+// ---------------------------------------------------------------------------
+constexpr int kFK = kW / 8;  // core matrices along K (both products)
+constexpr uint32_t kFW = 0, kFG = kFW + kW * kW * 2, kFA = kFG + kG * kW * 2, kFB = kFA + kM * kW * 2,
+                   kFBytes = kFB + kW * kW * 2;
+
+__global__ void __launch_bounds__(kThreads, 2)
+    k_fourier(const __nv_bfloat16* __restrict__ W, const __nv_bfloat16* __restrict__ Gt, const float* __restrict__ X,
+              const float* __restrict__ bb, float* __restrict__ U, float* __restrict__ act,
+              const float* __restrict__ bias, int nlines, long Nc, unsigned* status, int write_u)
+{
+    extern __shared__ __align__(1024) unsigned char sm[];
+    __shared__ __align__(8) uint64_t bar;
+    __shared__ uint32_t tmem_base;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int m = tid % kM, kc0 = tid / kM;  // this thread's pixel and first channel group (of 8): kc0, kc0 + 2, ...
+    const int so = (tid >> 6) * 8 + (tid & 7), sk = (tid >> 3) & 7;  // its spectrum rows so, so + 32, piece sk
+    float x[4][8];
+    float4 s[2][2];
+    auto load_x = [&](int line, int half) {
+        const float* src = X + (size_t)(line / kG) * kW * kP + (size_t)(line % kG) * kG + half * kM + m;
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+#pragma unroll
+            for (int q = 0; q < 8; q++) x[j][q] = __ldg(src + (size_t)((kc0 + 2 * j) * 8 + q) * kP);
+    };
+    auto load_s = [&](int line) {
+        const float* src = bb + (size_t)(sk >> 2) * kG * Nc + (size_t)(line % kG) * Nc +
+                           (size_t)(line / kG) * kW * kModes + (sk & 3) * 8;
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+            const float4* q = reinterpret_cast<const float4*>(src + (size_t)(so + 32 * j) * kModes);
+            s[j][0] = __ldg(q);
+            s[j][1] = __ldg(q + 1);
+        }
+    };
+    if (blockIdx.x < nlines) {
+        load_x(blockIdx.x, 0);
+        load_s(blockIdx.x);
+    }
+    tmem_alloc(&tmem_base, 128, warp);
+    if (tid == 0) mbar_init(&bar);
+    // the weights: element loads (a parameter block carries no alignment guarantee)
+    for (int i = tid; i < kW * kW; i += kThreads)
+        *reinterpret_cast<__nv_bfloat16*>(sm + kFW + kmajor_off(i / kW, i % kW, kFK)) = W[i];
+    for (int i = tid; i < kG * kFK; i += kThreads) {
+        const int row = (i >> 6) * 8 + (i & 7), k8 = (i >> 3) & 7;
+        *reinterpret_cast<uint4*>(sm + kFG + kmajor_off(row, k8 * 8, kFK)) =
+            *reinterpret_cast<const uint4*>(Gt + (size_t)row * kW + k8 * 8);
+    }
+    fence_before();
+    __syncthreads();
+    fence_after();
+    const uint32_t tmem = tmem_base, base = smem_addr(sm);
+    uint32_t parity = 0;
+    const int ntiles = 2 * nlines;
+    // tiles in pairs: both halves of a line, then the CTA's next line
+    for (int tile = 2 * blockIdx.x; tile < ntiles; tile += (tile & 1) ? 2 * (int)gridDim.x - 1 : 1) {
+        const int line = tile >> 1, half = tile & 1;
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+            *reinterpret_cast<uint4*>(sm + kFA + kmajor_off(m, (kc0 + 2 * j) * 8, kFK)) = pack8(x[j]);
+        if (half == 0) {
+#pragma unroll
+            for (int j = 0; j < 2; j++) {
+                const float f[8] = {s[j][0].x, s[j][0].y, s[j][0].z, s[j][0].w, s[j][1].x, s[j][1].y, s[j][1].z, s[j][1].w};
+                *reinterpret_cast<uint4*>(sm + kFB + kmajor_off(so + 32 * j, sk * 8, kFK)) = pack8(f);
+            }
+        }
+        publish_smem();
+        if (half == 0) {
+            load_x(line, 1);
+        } else if (line + (int)gridDim.x < nlines) {
+            load_x(line + gridDim.x, 0);
+            load_s(line + gridDim.x);
+        }
+        if (tid == 0) {
+#pragma unroll
+            for (int ks = 0; ks < kW / 16; ks++)
+                mma_bf16(tmem, smem_desc(base + kFA + ks * 256, 128, kFK * 128),
+                         smem_desc(base + kFW + ks * 256, 128, kFK * 128), instr_desc(kW), ks > 0);
+#pragma unroll
+            for (int ks = 0; ks < kW / 16; ks++)
+                mma_bf16(tmem + kW, smem_desc(base + kFG + half * (kM / 8) * kFK * 128 + ks * 256, 128, kFK * 128),
+                         smem_desc(base + kFB + ks * 256, 128, kFK * 128), instr_desc(kW), ks > 0);
+            mma_commit(&bar);
+        }
+        if (!mma_wait(&bar, parity, status)) break;
+        parity ^= 1;
+        const int g = warp & 3, ch = warp >> 2;
+        const uint32_t trow = tmem + ((uint32_t)(g * 32) << 16);
+        const size_t o0 = (size_t)(line / kG) * kW * kP + (size_t)(line % kG) * kG + half * kM + g * 32 + lane;
+#pragma unroll 1
+        for (int c0 = ch * (kW / 2); c0 < (ch + 1) * (kW / 2); c0 += 16) {
+            float r[16], sp[16];
+            tmem_ld16(trow + c0, r);
+            tmem_ld16(trow + kW + c0, sp);
+#pragma unroll
+            for (int q = 0; q < 16; q++) {
+                const size_t o = o0 + (size_t)(c0 + q) * kP;
+                const float u = (r[q] + __ldg(bias + c0 + q)) + sp[q];
+                if (write_u) U[o] = u;
+                if (act) act[o] = gelu_f(u);
+            }
+        }
+        retire_tile();
+    }
+    tmem_free(tmem, 128, warp);
+}
+
+// ---------------------------------------------------------------------------
+// The projection head: q = gelu(W1 h + c1) (128 channels), out = W2 q + c2 (2
+// channels).  The 2-channel product is two FMAs per value in the epilogue of
+// the first, on q rounded to BF16 as the product rounds it, so inference
+// neither stores q (537 MB per batch of 16) nor reads it back: 230 us for the
+// first product and 381 us for a GEMM of N = 2 before.  keep: training also
+// stores the pre-activation and q for the backward pass.
+// ---------------------------------------------------------------------------
+constexpr uint32_t kPA = kProj * kW * 2, kPBytes = kPA + kM * kW * 2;
+
+__global__ void __launch_bounds__(kThreads, 3)
+    k_project(const __nv_bfloat16* __restrict__ W1, const float* __restrict__ c1, const __nv_bfloat16* __restrict__ W2,
+              const float* __restrict__ c2, const float* __restrict__ X, float* __restrict__ qpre, float* __restrict__ qact,
+              float* __restrict__ out, int ntiles, unsigned* status, int keep)
+{
+    extern __shared__ __align__(1024) unsigned char sm[];
+    __shared__ __align__(8) uint64_t bar;
+    __shared__ uint32_t tmem_base;
+    __shared__ float s_c1[kProj], s_w2[2][kProj], s_half[2][kM];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int m = tid % kM, kc0 = tid / kM;
+    float x[4][8];
+    auto load_x = [&](int tile) {
+        const float* src = X + (size_t)(tile / (int)(kP / kM)) * kW * kP + (size_t)(tile % (int)(kP / kM)) * kM + m;
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+#pragma unroll
+            for (int q = 0; q < 8; q++) x[j][q] = __ldg(src + (size_t)((kc0 + 2 * j) * 8 + q) * kP);
+    };
+    if (blockIdx.x < ntiles) load_x(blockIdx.x);
+    tmem_alloc(&tmem_base, 128, warp);
+    if (tid == 0) mbar_init(&bar);
+    for (int i = tid; i < kProj * kW; i += kThreads)
+        *reinterpret_cast<__nv_bfloat16*>(sm + kmajor_off(i / kW, i % kW, kFK)) = W1[i];
+    if (tid < kProj) {
+        s_c1[tid] = c1[tid];
+        s_w2[0][tid] = __bfloat162float(W2[tid]);
+        s_w2[1][tid] = __bfloat162float(W2[kProj + tid]);
+    }
+    fence_before();
+    __syncthreads();
+    fence_after();
+    const uint32_t tmem = tmem_base, base = smem_addr(sm);
+    const float o0 = c2[0], o1 = c2[1];
+    uint32_t parity = 0;
+    for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+            *reinterpret_cast<uint4*>(sm + kPA + kmajor_off(m, (kc0 + 2 * j) * 8, kFK)) = pack8(x[j]);
+        publish_smem();
+        if (tile + (int)gridDim.x < ntiles) load_x(tile + gridDim.x);
+        if (tid == 0) {
+#pragma unroll
+            for (int ks = 0; ks < kW / 16; ks++)
+                mma_bf16(tmem, smem_desc(base + kPA + ks * 256, 128, kFK * 128),
+                         smem_desc(base + ks * 256, 128, kFK * 128), instr_desc(kProj), ks > 0);
+            mma_commit(&bar);
+        }
+        if (!mma_wait(&bar, parity, status)) break;
+        parity ^= 1;
+        const int g = warp & 3, ch = warp >> 2;
+        const uint32_t trow = tmem + ((uint32_t)(g * 32) << 16);
+        const size_t b = tile / (int)(kP / kM), p = (size_t)(tile % (int)(kP / kM)) * kM + g * 32 + lane;
+        float y0 = 0.0f, y1 = 0.0f;
+#pragma unroll 1
+        for (int c0 = ch * (kProj / 2); c0 < (ch + 1) * (kProj / 2); c0 += 16) {
+            float r[16];
+            tmem_ld16(trow + c0, r);
+#pragma unroll
+            for (int q = 0; q < 16; q++) {
+                const float u = r[q] + s_c1[c0 + q], v = gelu_f(u);
+                if (keep) {
+                    const size_t o = (b * kProj + c0 + q) * kP + p;
+                    qpre[o] = u;
+                    qact[o] = v;
+                }
+                const float vb = __bfloat162float(__float2bfloat16_rn(v));
+                y0 = fmaf(s_w2[0][c0 + q], vb, y0);
+                y1 = fmaf(s_w2[1][c0 + q], vb, y1);
+            }
+        }
+        if (ch == 1) {
+            s_half[0][g * 32 + lane] = y0;
+            s_half[1][g * 32 + lane] = y1;
+        }
+        retire_tile();  // (also orders the upper half's sums)
+        if (ch == 0) {
+            out[(b * 2) * kP + p] = (y0 + s_half[0][g * 32 + lane]) + o0;
+            out[(b * 2 + 1) * kP + p] = (y1 + s_half[1][g * 32 + lane]) + o1;
+        }
+    }
+    tmem_free(tmem, 128, warp);
+}
+
+template <typename K>
+cudaError_t allow_smem(K k, uint32_t bytes)
+{
+    return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+}
+
+int sm_count()
+{
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        return 1;
+    return sms;
+}
+
+}  // namespace umma
+
+// The shape the fused forward kernels are compiled for.
+bool fused_supported(int grid, int modes, int width, int proj, int nout)
+{
+    return grid == umma::kG && modes == umma::kModes && width == umma::kW && proj == umma::kProj && nout == 2;
+}
+
+cudaError_t xdft_fused(const __nv_bfloat16* F, const float* H, float* a, int B, unsigned* status, cudaStream_t st)
+{
+    using namespace umma;
+    const cudaError_t e = allow_smem(k_xdft, 2 * kXBytes);
+    if (e != cudaSuccess) return e;
+    const int lines = B * kG, grid = lines < 2 * sm_count() ? lines : 2 * sm_count();
+    k_xdft<<<grid, kThreads, 2 * kXBytes, st>>>(F, H, a, lines, (long)B * kW * kModes, status);
+    return cudaGetLastError();
+}
+
+cudaError_t fourier_fused(const __nv_bfloat16* W, const __nv_bfloat16* Gt, const float* X, const float* bb, float* U,
+                          float* act, const float* bias, int B, unsigned* status, bool write_u, cudaStream_t st)
+{
+    using namespace umma;
+    const cudaError_t e = allow_smem(k_fourier, kFBytes);
+    if (e != cudaSuccess) return e;
+    const int lines = B * kG, grid = lines < 2 * sm_count() ? lines : 2 * sm_count();
+    k_fourier<<<grid, kThreads, kFBytes, st>>>(W, Gt, X, bb, U, act, bias, lines, (long)B * kW * kModes, status,
+                                               write_u || !act);
+    return cudaGetLastError();
+}
+
+cudaError_t project_fused(const __nv_bfloat16* W1, const float* c1, const __nv_bfloat16* W2, const float* c2,
+                          const float* X, float* qpre, float* q, float* out, int B, unsigned* status, bool keep,
+                          cudaStream_t st)
+{
+    using namespace umma;
+    const cudaError_t e = allow_smem(k_project, kPBytes);
+    if (e != cudaSuccess) return e;
+    const int tiles = (int)(B * (kP / kM)), grid = tiles < 3 * sm_count() ? tiles : 3 * sm_count();
+    k_project<<<grid, kThreads, kPBytes, st>>>(W1, c1, W2, c2, X, qpre, q, out, tiles, status, keep);
+    return cudaGetLastError();
+}
+
+}  // namespace atmwfs
