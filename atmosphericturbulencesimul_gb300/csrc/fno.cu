@@ -75,6 +75,10 @@ cudaError_t fourier_fused(const __nv_bfloat16* W, const __nv_bfloat16* Gt, const
 cudaError_t project_fused(const __nv_bfloat16* W1, const float* c1, const __nv_bfloat16* W2, const float* c2,
                           const float* X, float* qpre, float* q, float* out, int B, unsigned* status, bool keep,
                           cudaStream_t st);
+cudaError_t fourier_bwd_fused(const __nv_bfloat16* W, const __nv_bfloat16* Fx, const float* dU, const float* da, float* dX,
+                              int B, unsigned* status, cudaStream_t st);
+cudaError_t layer_bwd_fused(const __nv_bfloat16* Gx, const float* dh, const float* u, const float* h, float* du, float* dbb,
+                            float* dW, float* db, int B, unsigned* status, cudaStream_t st);
 }  // namespace atmwfs
 
 struct atmwfs_fno {
@@ -91,6 +95,8 @@ struct atmwfs_fno {
     float *Fx = nullptr, *FyAB = nullptr, *GyBig = nullptr, *Gx = nullptr;
     __nv_bfloat16 *FyAB_bf = nullptr, *GyBig_bf = nullptr;
     __nv_bfloat16 *FxT_bf = nullptr, *GxT_bf = nullptr;  // the x transforms transposed (N x K)
+    // the transposed products of the backward pass
+    __nv_bfloat16 *Fx_bf = nullptr, *Gx_bf = nullptr, *FyABT_bf = nullptr;
     // activations for one batch size
     int cap = 0;
     std::vector<float*> h, u, a, z;     // h[0..nl], u[0..nl-1], a/z per layer
@@ -140,20 +146,6 @@ atmwfs_status dalloc(atmwfs_fno* f, void** p, size_t bytes)
 // ---------------------------------------------------------------------------
 // elementwise kernels
 // ---------------------------------------------------------------------------
-// GELU (gelu_f, fno_gemm.cuh) and its derivative
-__device__ __forceinline__ float gelu_d(float x)
-{
-    const float c = 0.7978845608028654f;
-    const float t = tanhf(c * (x + 0.044715f * x * x * x));
-    return 0.5f * (1.0f + t) + 0.5f * x * (1.0f - t * t) * c * (1.0f + 3.0f * 0.044715f * x * x);
-}
-
-__global__ void k_gelu(const float* __restrict__ in, float* __restrict__ out, long n)
-{
-    for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x)
-        out[i] = gelu_f(in[i]);
-}
-
 __global__ void k_gelu_bwd(const float* __restrict__ dy, const float* __restrict__ x, float* __restrict__ dx, long n)
 {
     for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x)
@@ -196,9 +188,12 @@ __global__ void k_mse(const float* __restrict__ out, const float* __restrict__ t
 }
 
 // Mode mixing y[b][o][k] = sum_c R[k][o][c] z[b][c][k] (complex) for KX
-// neighbouring kx of one ky (blockIdx.x = ky (m / KX) + kx / KX).  z / y
-// layout [2m][B w][m]: row ky holds the real parts, row m + ky the imaginary
-// parts, then (sample, channel), then kx, so KX neighbours are one vector.
+// neighbouring kx of one ky (blockIdx.x = ky (m / KX) + kx / KX).  z / y: row ky
+// holds the real parts, row m + ky the imaginary parts; in a row mode kx of
+// (sample, channel) bc is at kx sk + bc sc: [B w][m] (sk = 1, sc = m) or, at the
+// shape of the fused kernels, [m][B w] (sk = B w, sc = 1), whose loads and
+// stores are whole runs (the scattered 4-byte stores of the first took most of
+// 75 us).
 // FP32 FMAs bound it: 8 w^2 B m^2 operations, 7 us for a batch of 16 at the
 // default shape.  A thread owns one (mode, output channel) and kMixB samples:
 // a weight is read from shared memory once for all of them and the samples'
@@ -207,11 +202,11 @@ __global__ void k_mse(const float* __restrict__ out, const float* __restrict__ t
 constexpr int kMixB = 8;
 template <int KX>
 __global__ void __launch_bounds__(256) k_modemix(const __nv_bfloat16* __restrict__ R, const float* __restrict__ z,
-                                                 float* __restrict__ y, int B, int w, int m)
+                                                 float* __restrict__ y, int B, int w, int m, long sk, long sc)
 {
     const int groups = m / KX, ky = blockIdx.x / groups, kx0 = blockIdx.x % groups * KX;
     const long Nc = (long)B * w * m;
-    const long ore = (long)ky * Nc + kx0, oim = (long)(m + ky) * Nc + kx0;
+    const long ore = (long)ky * Nc + kx0 * sk, oim = (long)(m + ky) * Nc + kx0 * sk;
     extern __shared__ float4 mix_smem[];
     float* zs = reinterpret_cast<float*>(mix_smem);                                 // [KX][kMixB][w][2]
     __nv_bfloat162* rs = reinterpret_cast<__nv_bfloat162*>(zs + KX * kMixB * w * 2);  // [KX][w][w + 1]
@@ -222,11 +217,11 @@ __global__ void __launch_bounds__(256) k_modemix(const __nv_bfloat16* __restrict
         __syncthreads();  // the previous samples are used
         for (int i = threadIdx.x; i < kMixB * w; i += blockDim.x) {
             float vr[KX], vi[KX];
-            const long o = (long)(b0 * w + i) * m;
+            const long o = (long)(b0 * w + i) * sc;
 #pragma unroll
             for (int k = 0; k < KX; k++) {
-                vr[k] = i < nb * w ? z[o + ore + k] : 0.0f;
-                vi[k] = i < nb * w ? z[o + oim + k] : 0.0f;
+                vr[k] = i < nb * w ? z[o + ore + k * sk] : 0.0f;
+                vi[k] = i < nb * w ? z[o + oim + k * sk] : 0.0f;
             }
 #pragma unroll
             for (int k = 0; k < KX; k++) reinterpret_cast<float2*>(zs)[k * kMixB * w + i] = make_float2(vr[k], vi[k]);
@@ -252,7 +247,7 @@ __global__ void __launch_bounds__(256) k_modemix(const __nv_bfloat16* __restrict
                 }
             }
             for (int b = 0; b < nb; b++) {
-                const long q = (long)((b0 + b) * w + o) * m + k;
+                const long q = (long)((b0 + b) * w + o) * sc + k * sk;
                 y[q + ore] = sr[b];
                 y[q + oim] = si[b];
             }
@@ -264,14 +259,14 @@ template <int KX>
 constexpr size_t modemix_smem(int w) { return (size_t)KX * ((size_t)kMixB * w * 8 + (size_t)w * (w + 1) * 4); }
 
 // Four neighbouring modes per CTA where they fit twice into an SM, else two or one.
-cudaError_t modemix(const __nv_bfloat16* R, const float* z, float* y, int B, int w, int m, cudaStream_t st)
+cudaError_t modemix(const __nv_bfloat16* R, const float* z, float* y, int B, int w, int m, long sk, long sc, cudaStream_t st)
 {
     auto go = [&](auto kern, size_t sm, int kx) -> cudaError_t {
         if (sm > 48 * 1024) {
             const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
             if (e != cudaSuccess) return e;
         }
-        kern<<<m * m / kx, 256, sm, st>>>(R, z, y, B, w, m);
+        kern<<<m * m / kx, 256, sm, st>>>(R, z, y, B, w, m, sk, sc);
         return cudaGetLastError();
     };
     if (m % 4 == 0 && modemix_smem<4>(w) <= 113 * 1024) return go(k_modemix<4>, modemix_smem<4>(w), 4);
@@ -332,6 +327,75 @@ __global__ void k_modemix_bwd(const __nv_bfloat16* __restrict__ R, const float* 
         dRk[i * 2] += sr;
         dRk[i * 2 + 1] += si;
     }
+}
+
+size_t modemix_bwd_smem(int B, int w) { return sizeof(float) * (4 * (size_t)B * w + 2 * (size_t)w * (w + 1)); }
+
+// The same at the fused kernels' shape (width 64, images [.][m][B w]): one
+// mode per CTA, whose z, dy and dz are runs of B w values.  A thread owns an
+// input channel c and 16 output channels: dR[o][c] stays in registers over the
+// samples (z of its channel in registers, dy a broadcast), is added to the
+// gradient once, and is read early.  HBM bounds it: 75 MB per layer at a batch
+// of 8, 33 us; the form above took 75 us (two shared loads per product, 4-byte
+// accesses 128 bytes apart).
+template <int NB>
+__global__ void __launch_bounds__(256) k_modemix_bwd64(const __nv_bfloat16* __restrict__ R, const float* __restrict__ z,
+                                                       const float* __restrict__ dy, float* __restrict__ dz,
+                                                       float* __restrict__ dR, int B, int m)
+{
+    constexpr int w = 64;
+    const int k = blockIdx.x, ky = k / m, kx = k % m, tid = threadIdx.x;
+    const long BW = (long)B * w, Nc = BW * m;
+    const long ore = (long)ky * Nc + kx * BW, oim = (long)(m + ky) * Nc + kx * BW;
+    __shared__ float2 ds[NB * w];
+    __shared__ __nv_bfloat162 rs[w * w];
+    const __nv_bfloat162* Rk = reinterpret_cast<const __nv_bfloat162*>(R) + (size_t)k * w * w;
+    float2* dRk = reinterpret_cast<float2*>(dR) + (size_t)k * w * w;
+    const int c = tid % w, og = tid / w * 16;
+    float2 g[16], acc[16];
+#pragma unroll
+    for (int q = 0; q < 16; q++) {
+        g[q] = dRk[(og + q) * w + c];
+        acc[q] = make_float2(0.0f, 0.0f);
+    }
+    for (int i = tid; i < w * w; i += 256) rs[i] = Rk[i];
+    for (int b0 = 0; b0 < B; b0 += NB) {
+        const int nb = min(NB, B - b0);
+        __syncthreads();  // the previous samples are used
+        for (int i = tid; i < NB * w; i += 256)
+            ds[i] = i < nb * w ? make_float2(dy[ore + b0 * w + i], dy[oim + b0 * w + i]) : make_float2(0.0f, 0.0f);
+        float zr[NB], zi[NB];
+#pragma unroll
+        for (int b = 0; b < NB; b++) {
+            zr[b] = b < nb ? z[ore + (b0 + b) * w + c] : 0.0f;
+            zi[b] = b < nb ? z[oim + (b0 + b) * w + c] : 0.0f;
+        }
+        __syncthreads();
+        // dR[o][c] += sum_b dy[b][o] conj(z[b][c])
+#pragma unroll
+        for (int q = 0; q < 16; q++)
+#pragma unroll
+            for (int b = 0; b < NB; b++) {
+                const float2 d = ds[b * w + og + q];
+                acc[q].x += d.x * zr[b] + d.y * zi[b];
+                acc[q].y += d.y * zr[b] - d.x * zi[b];
+            }
+        // dz[b][c] = sum_o conj(R[o][c]) dy[b][o]: samples tid / 64, + 4, ...
+        for (int b = tid / w; b < nb; b += 4) {
+            float sr = 0.0f, si = 0.0f;
+#pragma unroll 8
+            for (int o = 0; o < w; o++) {
+                const float2 rc = make_float2(__low2float(rs[o * w + c]), __high2float(rs[o * w + c]));
+                const float dr = ds[b * w + o].x, di = ds[b * w + o].y;
+                sr += rc.x * dr + rc.y * di;
+                si += rc.x * di - rc.y * dr;
+            }
+            dz[ore + (b0 + b) * w + c] = sr;
+            dz[oim + (b0 + b) * w + c] = si;
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < 16; q++) dRk[(og + q) * w + c] = make_float2(g[q].x + acc[q].x, g[q].y + acc[q].y);
 }
 
 __global__ void k_to_bf16(const float* __restrict__ in, __nv_bfloat16* __restrict__ out, long n)
@@ -511,8 +575,12 @@ atmwfs_status build_dft(atmwfs_fno* f)
             FxT[(size_t)n * G + x] = Fx[(size_t)x * 2 * m + n];
             GxT[(size_t)x * 2 * m + n] = Gx[(size_t)n * G + x];
         }
+    std::vector<float> FyABT((size_t)2 * G * 2 * m);
+    for (int r = 0; r < 2 * m; r++)
+        for (int k = 0; k < 2 * G; k++) FyABT[(size_t)k * 2 * m + r] = FyAB[(size_t)r * 2 * G + k];
     struct MB { __nv_bfloat16** d; std::vector<float>* h; } bmats[] = {
-        {&f->FyAB_bf, &FyAB}, {&f->GyBig_bf, &GyBig}, {&f->FxT_bf, &FxT}, {&f->GxT_bf, &GxT}};
+        {&f->FyAB_bf, &FyAB}, {&f->GyBig_bf, &GyBig}, {&f->FxT_bf, &FxT}, {&f->GxT_bf, &GxT},
+        {&f->Fx_bf, &Fx},     {&f->Gx_bf, &Gx},       {&f->FyABT_bf, &FyABT}};
     for (auto& mm : bmats) {
         std::vector<__nv_bfloat16> hb(mm.h->size());
         for (size_t i = 0; i < hb.size(); i++) hb[i] = __float2bfloat16_rn((*mm.h)[i]);
@@ -616,7 +684,7 @@ atmwfs_status spectral_fwd(atmwfs_fno* f, int l, const void* h, int h_bf16, floa
     // y = R z per mode
     const size_t smf = sizeof(float) * (2 * B * w + 2 * w * (w + 1));
     if (smf > 227 * 1024) return err(ATMWFS_ERR_INVALID, "batch %d x width %d exceeds the mode-mixing shared memory", B, w);
-    FN_CUDA(modemix(f->pbf + f->L.R[l], z, f->y, B, w, m, st));
+    FN_CUDA(modemix(f->pbf + f->L.R[l], z, f->y, B, w, m, spec ? 1 : BW, spec ? m : 1, st));
     // bb = GyBig y: [2G, 2m] x [2m, Nc], on tcgen05 where compiled
     if (tc && spectral_umma_supported(2 * G, 2 * m))
         FN_CUDA(spectral_umma(f->GyBig_bf, 2 * G, 2 * m, f->y, f->bb, Nc, umma_status_ptr(), 0, st));
@@ -656,7 +724,7 @@ atmwfs_status spectral_bwd(atmwfs_fno* f, int l, const float* ds, float* dh, int
     FN_CUDA(gemm(2 * m, (int)Nc, 2 * G, f->GyBig, 2 * m, 1, 0, f->dbb, Nc, 0, 0, f->dy, Nc, 0.0f, 1, 0, 0, 0, nullptr, 0,
                  st));
     // dz, dR
-    const size_t smb = sizeof(float) * (4 * B * w + 2 * w * (w + 1));
+    const size_t smb = modemix_bwd_smem(B, w);
     if (smb > 227 * 1024) return err(ATMWFS_ERR_INVALID, "batch %d x width %d exceeds the mode-mixing shared memory", B, w);
     if (smb > 48 * 1024) FN_CUDA(cudaFuncSetAttribute(k_modemix_bwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smb));
     k_modemix_bwd<<<m * m, 256, smb, st>>>(f->pbf + f->L.R[l], f->z[l], f->dy, f->dz, f->grads + f->L.R[l], B, w, m);
@@ -689,6 +757,13 @@ bool umma_enabled()
         return !(e && e[0] == '0');
     }();
     return use;
+}
+
+// Whether the fused kernels run the network (their shape only; the spectral
+// images then have the channels fastest, in both passes).
+bool fused_shape(const atmwfs_fno_cfg& c)
+{
+    return umma_enabled() && fused_supported(c.grid, c.modes, c.width, c.proj, c.nout);
 }
 
 // keep_c = false (inference with an activation output): the pre-activation C
@@ -728,7 +803,7 @@ atmwfs_status forward(atmwfs_fno* f, const float* x, float* out, int B, cudaStre
                        ? 1
                        : 0;
     FN_CUDA(pointwise_fwd(pb + f->L.lift_W, c.width, c.nin, x, 0, f->h[0], B, P, 0.0f, pf + f->L.lift_b, st));
-    if (!bf && umma_enabled() && fused_supported(c.grid, c.modes, c.width, c.proj, c.nout)) {
+    if (!bf && fused_shape(c)) {
         unsigned* status = umma_status_ptr();
         if (!status) return err(ATMWFS_ERR_CUDA, "status symbol");
         for (int l = 0; l < c.layers; l++) {
@@ -755,6 +830,30 @@ atmwfs_status forward(atmwfs_fno* f, const float* x, float* out, int B, cudaStre
     return ATMWFS_OK;
 }
 
+// A Fourier layer's backward at the fused shape: dh (dL/dh[l + 1]) -> dX
+// (dL/dh[l]), the layer's gradients accumulated.
+atmwfs_status layer_bwd(atmwfs_fno* f, int l, const float* dh, float* dX, int B, unsigned* status, cudaStream_t st)
+{
+    const atmwfs_fno_cfg& c = f->cfg;
+    const int G = c.grid, m = c.modes;
+    const long Nc = (long)B * c.width * m;
+    const bool act = l + 1 < c.layers;
+    const float* du = act ? f->du : dh;
+    if (modemix_bwd_smem(B, c.width) > 227 * 1024)  // the batches the unfused mixing takes
+        return err(ATMWFS_ERR_INVALID, "batch %d x width %d exceeds the mode-mixing shared memory", B, c.width);
+    FN_CUDA(layer_bwd_fused(f->Gx_bf, dh, act ? f->u[l] : nullptr, f->h[l], f->du, f->dbb, f->grads + f->L.W[l],
+                            f->grads + f->L.b[l], B, status, st));
+    // dy = GyBig^T dbb: [2m, 2G] x [2G, Nc]
+    FN_CUDA(gemm(2 * m, (int)Nc, 2 * G, f->GyBig, 2 * m, 1, 0, f->dbb, Nc, 0, 0, f->dy, Nc, 0.0f, 1, 0, 0, 0, nullptr, 0,
+                 st));
+    k_modemix_bwd64<8><<<m * m, 256, 0, st>>>(f->pbf + f->L.R[l], f->z[l], f->dy, f->dz, f->grads + f->L.R[l], B, m);
+    FN_CUDA(cudaGetLastError());
+    // da = FyAB^T dz: [2G, 2m] x [2m, Nc]
+    FN_CUDA(spectral_umma(f->FyABT_bf, 2 * G, 2 * m, f->dz, f->da, Nc, status, 0, st));
+    FN_CUDA(fourier_bwd_fused(f->pbf + f->L.W[l], f->Fx_bf, du, f->da, dX, B, status, st));
+    return ATMWFS_OK;
+}
+
 atmwfs_status backward(atmwfs_fno* f, const float* x, const float* dout, int B, cudaStream_t st)
 {
     const atmwfs_fno_cfg& c = f->cfg;
@@ -772,7 +871,15 @@ atmwfs_status backward(atmwfs_fno* f, const float* x, const float* dout, int B, 
     k_rowsum<<<dim3(rs.x, c.proj), 256, 0, st>>>(f->dq, g + f->L.proj1_b, B, c.proj, P);
     FN_CUDA(pointwise_dx(pb + f->L.proj1_W, c.proj, c.width, f->dq, f->dh, B, P, 0.0f, st));
     // Fourier layers, last to first: dh holds dL/dh[l+1]
+    const bool fused = fused_shape(c);
+    unsigned* status = fused ? umma_status_ptr() : nullptr;
+    if (fused && !status) return err(ATMWFS_ERR_CUDA, "status symbol");
     for (int l = c.layers - 1; l >= 0; l--) {
+        if (fused) {
+            FN_TRY(layer_bwd(f, l, f->dh, f->dh2, B, status, st));
+            std::swap(f->dh, f->dh2);
+            continue;
+        }
         if (l + 1 < c.layers) k_gelu_bwd<<<grid_for(nact), 256, 0, st>>>(f->dh, f->u[l], f->du, nact);
         else FN_CUDA(cudaMemcpyAsync(f->du, f->dh, sizeof(float) * nact, cudaMemcpyDeviceToDevice, st));
         FN_CUDA(pointwise_dw(c.width, c.width, f->du, f->h[l], g + f->L.W[l], B, P, st));

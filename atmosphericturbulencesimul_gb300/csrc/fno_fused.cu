@@ -1,13 +1,23 @@
-// fno_fused.cu -- the forward pass of the surrogate's default shape (grid 256,
-// 32 modes, width 64, projection 128) as kernels that fuse neighbouring
-// products on the tcgen05 tensor cores, so that the images between them are
-// not written and read back:
+// fno_fused.cu -- the surrogate's default shape (grid 256, 32 modes, width 64,
+// projection 128) as kernels that fuse neighbouring products on the tcgen05
+// tensor cores, so that the images between them are not written and read
+// back:
 //   k_xdft     the forward DFT along x, written as coalesced spectrum rows;
-//   k_fourier  pointwise mixing + inverse DFT along x + bias (+ GELU);
-//   k_project  the first projection + GELU + the 2-channel output.
+//   k_fourier  pointwise mixing + inverse DFT along x (+ bias, GELU), and the
+//              same pair of the backward pass;
+//   k_project  the first projection + GELU + the 2-channel output;
+//   k_layer_bwd  a layer's GELU gradient, its weight and bias gradients and
+//              the transposed inverse DFT along x, from one read of the line.
 // The products keep the operands' BF16 rounding, the K order and the FP32
 // accumulation of the separate products (k_pointwise, k_rowprod, the mma.sync
-// GEMM), so a layer's results are the same bits.
+// GEMM), so a layer's activations and gradients are the same bits (sums over
+// pixels, which were atomic before, are not).
+//
+// Spectral images here are planar with the channels fastest, so that a
+// mode's values of every channel are one run (the mode mixing) and a
+// warp's channels store as one (k_xdft): with BW = B w,
+//   a, bb : [2][G][m][BW]  (real / imaginary plane, row y, kx, channel)
+//   z, y  : [2 m][m][BW]   (row ky: real parts, row m + ky: imaginary parts)
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -40,13 +50,14 @@ __device__ __forceinline__ uint4 pack8(const float (&f)[8])
 
 // ---------------------------------------------------------------------------
 // Forward DFT along x of one line (sample b, row y), all channels:
-//   a[p][y][b w + c][kx] = sum_x F[p m + kx][x] h[b][c][y][x]
-// as D = F h^T: the 2 m = 64 rows of F are the MMA's M (rows 64 .. 127 of the
-// 128 are whatever follows in shared memory, here B, and their results are not
-// read), the channels its N, K = 256.  With the modes along the TMEM lanes a
-// channel's spectrum leaves as one 128-byte run per warp.  (k_rowprod has the
-// lines along the lanes and writes 16-byte pieces 128 bytes apart: the rate of
-// L2 requests bounds it, 138 us for a batch of 16 against 49 us of HBM time.)
+//   a[p][y][kx][b w + c] = sum_x h[b][c][y][x] F[p m + kx][x]
+// as D = h F^T: the 64 channels are the MMA's M (rows 64 .. 127 of the 128 are
+// whatever follows in shared memory, here F, and their results are not read),
+// the 64 rows of F its N, K = 256.  With the channels along the TMEM lanes a
+// mode's values leave as one 128-byte run per warp.  (k_rowprod has the lines
+// of all channels along the lanes and writes 16-byte pieces 128 bytes apart:
+// the rate of L2 requests bounds it, 138 us for a batch of 16 against 49 us of
+// HBM time; this form takes 57 us.)
 // F is staged once per CTA; a line's 64 KB are loaded into registers while the
 // previous line's products run, so a CTA keeps 64 KB in flight.
 // ---------------------------------------------------------------------------
@@ -64,12 +75,29 @@ __device__ __forceinline__ void x_piece(int tid, int j, int& row, int& k8)
     k8 = (rest >> 3) * 4 + ((i >> 3) & 3);
 }
 
+// The 64 x 64 spectrum of a line from tensor memory (lanes 0 .. 63: channels,
+// columns: re and im of the modes) into the planar image; warps 0, 1, 4 and 5
+// (warp w: lanes 32 (w % 4) .., plane w / 4).
+__device__ __forceinline__ void store_spectrum(uint32_t tmem, float* __restrict__ a, int line, long Nc, int warp, int lane)
+{
+    const int cb = (warp & 3) * 32, p = warp >> 2, b = line / kG, y = line % kG;
+    const size_t BW = (size_t)Nc / kModes;
+    float* o = a + (size_t)p * kG * Nc + (size_t)y * Nc + (size_t)b * kW + cb + lane;
+#pragma unroll
+    for (int c0 = 0; c0 < kModes; c0 += 16) {
+        float r[16];
+        tmem_ld16(tmem + ((uint32_t)cb << 16) + p * kModes + c0, r);
+#pragma unroll
+        for (int q = 0; q < 16; q++) o[(c0 + q) * BW] = r[q];
+    }
+}
+
 __global__ void __launch_bounds__(kThreads, 2) k_xdft(const __nv_bfloat16* __restrict__ F, const float* __restrict__ H,
                                                       float* __restrict__ a, int nlines, long Nc, unsigned* status)
 {
     constexpr int J = kW * kXK / kThreads;  // pieces per thread
     extern __shared__ __align__(1024) unsigned char sm[];
-    unsigned char *sa = sm, *sb = sm + kXBytes;
+    unsigned char *sa = sm, *sb = sm + kXBytes;  // the line, F
     __shared__ __align__(8) uint64_t bar;
     __shared__ uint32_t tmem_base;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -92,7 +120,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_xdft(const __nv_bfloat16* __res
     for (int j = 0; j < J; j++) {
         int row, k8;
         x_piece(tid, j, row, k8);
-        *reinterpret_cast<uint4*>(sa + kmajor_off(row, k8 * 8, kXK)) =
+        *reinterpret_cast<uint4*>(sb + kmajor_off(row, k8 * 8, kXK)) =
             *reinterpret_cast<const uint4*>(F + (size_t)row * kG + k8 * 8);
     }
     fence_before();
@@ -106,7 +134,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_xdft(const __nv_bfloat16* __res
             int row, k8;
             x_piece(tid, j, row, k8);
             const float f[8] = {v[j][0].x, v[j][0].y, v[j][0].z, v[j][0].w, v[j][1].x, v[j][1].y, v[j][1].z, v[j][1].w};
-            *reinterpret_cast<uint4*>(sb + kmajor_off(row, k8 * 8, kXK)) = pack8(f);
+            *reinterpret_cast<uint4*>(sa + kmajor_off(row, k8 * 8, kXK)) = pack8(f);
         }
         publish_smem();
         if (line + (int)gridDim.x < nlines) load(line + gridDim.x);
@@ -119,18 +147,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_xdft(const __nv_bfloat16* __res
         }
         if (!mma_wait(&bar, parity, status)) break;
         parity ^= 1;
-        const int p = warp & 3, half = warp >> 2;
-        if (p < 2) {
-            const int b = line / kG, y = line % kG;
-            float* o = a + (size_t)p * kG * Nc + (size_t)y * Nc + (size_t)b * kW * kModes + lane;
-#pragma unroll
-            for (int c0 = half * (kW / 2); c0 < (half + 1) * (kW / 2); c0 += 16) {
-                float r[16];
-                tmem_ld16(tmem + ((uint32_t)(p * 32) << 16) + c0, r);
-#pragma unroll
-                for (int q = 0; q < 16; q++) o[(size_t)(c0 + q) * kModes] = r[q];
-            }
-        }
+        if ((warp & 3) < 2) store_spectrum(tmem, a, line, Nc, warp, lane);
         retire_tile();
     }
     tmem_free(tmem, 64, warp);
@@ -148,11 +165,14 @@ __global__ void __launch_bounds__(kThreads, 2) k_xdft(const __nv_bfloat16* __res
 // pointwise product (161 us); both now run as one pass over h and bb.
 // Gx^T and W are staged once per CTA; a tile's 32 channel values per thread
 // and the line's spectrum are loaded while the previous tile's products run.
+// The backward pass of a layer ends with the same pair: dh = W^T du + Fx da
+// (TW: W transposed; Gt = Fx; no bias).
 // ---------------------------------------------------------------------------
 constexpr int kFK = kW / 8;  // core matrices along K (both products)
 constexpr uint32_t kFW = 0, kFG = kFW + kW * kW * 2, kFA = kFG + kG * kW * 2, kFB = kFA + kM * kW * 2,
                    kFBytes = kFB + kW * kW * 2;
 
+template <bool TW>
 __global__ void __launch_bounds__(kThreads, 2)
     k_fourier(const __nv_bfloat16* __restrict__ W, const __nv_bfloat16* __restrict__ Gt, const float* __restrict__ X,
               const float* __restrict__ bb, float* __restrict__ U, float* __restrict__ act,
@@ -163,9 +183,9 @@ __global__ void __launch_bounds__(kThreads, 2)
     __shared__ uint32_t tmem_base;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int m = tid % kM, kc0 = tid / kM;  // this thread's pixel and first channel group (of 8): kc0, kc0 + 2, ...
-    const int so = (tid >> 6) * 8 + (tid & 7), sk = (tid >> 3) & 7;  // its spectrum rows so, so + 32, piece sk
-    float x[4][8];
-    float4 s[2][2];
+    const int so = tid & 63, sk = tid >> 6;  // its spectrum channel, and mode groups (of 8) sk, sk + 4
+    const size_t BW = (size_t)Nc / kModes;
+    float x[4][8], s[2][8];
     auto load_x = [&](int line, int half) {
         const float* src = X + (size_t)(line / kG) * kW * kP + (size_t)(line % kG) * kG + half * kM + m;
 #pragma unroll
@@ -174,14 +194,11 @@ __global__ void __launch_bounds__(kThreads, 2)
             for (int q = 0; q < 8; q++) x[j][q] = __ldg(src + (size_t)((kc0 + 2 * j) * 8 + q) * kP);
     };
     auto load_s = [&](int line) {
-        const float* src = bb + (size_t)(sk >> 2) * kG * Nc + (size_t)(line % kG) * Nc +
-                           (size_t)(line / kG) * kW * kModes + (sk & 3) * 8;
+        const float* src = bb + (size_t)(line % kG) * Nc + (size_t)sk * 8 * BW + (size_t)(line / kG) * kW + so;
 #pragma unroll
-        for (int j = 0; j < 2; j++) {
-            const float4* q = reinterpret_cast<const float4*>(src + (size_t)(so + 32 * j) * kModes);
-            s[j][0] = __ldg(q);
-            s[j][1] = __ldg(q + 1);
-        }
+        for (int j = 0; j < 2; j++)  // j: real, imaginary plane
+#pragma unroll
+            for (int q = 0; q < 8; q++) s[j][q] = __ldg(src + (size_t)j * kG * Nc + q * BW);
     };
     if (blockIdx.x < nlines) {
         load_x(blockIdx.x, 0);
@@ -191,7 +208,7 @@ __global__ void __launch_bounds__(kThreads, 2)
     if (tid == 0) mbar_init(&bar);
     // the weights: element loads (a parameter block carries no alignment guarantee)
     for (int i = tid; i < kW * kW; i += kThreads)
-        *reinterpret_cast<__nv_bfloat16*>(sm + kFW + kmajor_off(i / kW, i % kW, kFK)) = W[i];
+        *reinterpret_cast<__nv_bfloat16*>(sm + kFW + (TW ? kmajor_off(i % kW, i / kW, kFK) : kmajor_off(i / kW, i % kW, kFK))) = W[i];
     for (int i = tid; i < kG * kFK; i += kThreads) {
         const int row = (i >> 6) * 8 + (i & 7), k8 = (i >> 3) & 7;
         *reinterpret_cast<uint4*>(sm + kFG + kmajor_off(row, k8 * 8, kFK)) =
@@ -211,10 +228,8 @@ __global__ void __launch_bounds__(kThreads, 2)
             *reinterpret_cast<uint4*>(sm + kFA + kmajor_off(m, (kc0 + 2 * j) * 8, kFK)) = pack8(x[j]);
         if (half == 0) {
 #pragma unroll
-            for (int j = 0; j < 2; j++) {
-                const float f[8] = {s[j][0].x, s[j][0].y, s[j][0].z, s[j][0].w, s[j][1].x, s[j][1].y, s[j][1].z, s[j][1].w};
-                *reinterpret_cast<uint4*>(sm + kFB + kmajor_off(so + 32 * j, sk * 8, kFK)) = pack8(f);
-            }
+            for (int j = 0; j < 2; j++)
+                *reinterpret_cast<uint4*>(sm + kFB + kmajor_off(so, (sk + 4 * j) * 8, kFK)) = pack8(s[j]);
         }
         publish_smem();
         if (half == 0) {
@@ -247,13 +262,126 @@ __global__ void __launch_bounds__(kThreads, 2)
 #pragma unroll
             for (int q = 0; q < 16; q++) {
                 const size_t o = o0 + (size_t)(c0 + q) * kP;
-                const float u = (r[q] + __ldg(bias + c0 + q)) + sp[q];
+                const float u = (r[q] + (bias ? __ldg(bias + c0 + q) : 0.0f)) + sp[q];
                 if (write_u) U[o] = u;
                 if (act) act[o] = gelu_f(u);
             }
         }
         retire_tile();
     }
+    tmem_free(tmem, 128, warp);
+}
+
+// ---------------------------------------------------------------------------
+// A layer's backward products over one line (sample b, row y), from one read
+// of dh, u and h:
+//   du = dh gelu'(u)                              (ACT; else du = dh, not written)
+//   dbb = the transposed inverse DFT along x: D1 = du Gx^T (64 channels x 64, K = 256 x)
+//   dW += du h^T                              D2 (64 x 64, K = 256 x, over lines)
+//   db += sum_x du
+// HBM bounds it: 0.57 GB for a batch of 8.  As separate kernels the gradient
+// (74 us), the weight product (93), the bias sums (37) and the DFT (67) read du
+// three times more.  The line's du is the A operand of both products (rows 64
+// .. 127 of the MMA's M are what follows in shared memory and are not read);
+// D2 stays in tensor memory for kFlush lines (K = 1024, the longest run of the
+// split product it replaces) and is then added to FP32 registers, one atomic
+// per element and CTA at the end.
+// ---------------------------------------------------------------------------
+constexpr int kFlush = 4;
+
+template <bool ACT>
+__global__ void __launch_bounds__(kThreads, 2)
+    k_layer_bwd(const __nv_bfloat16* __restrict__ Gx, const float* __restrict__ dh, const float* __restrict__ u,
+                const float* __restrict__ h, float* __restrict__ du, float* __restrict__ dbb, float* __restrict__ dW,
+                float* __restrict__ db, int nlines, long Nc, unsigned* status)
+{
+    constexpr int J = kW * kXK / kThreads;
+    extern __shared__ __align__(1024) unsigned char sm[];
+    unsigned char *sd = sm, *sg = sm + kXBytes, *sh = sm + 2 * kXBytes;  // du, Gx, h
+    __shared__ __align__(8) uint64_t bar;
+    __shared__ uint32_t tmem_base;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    tmem_alloc(&tmem_base, 128, warp);
+    if (tid == 0) mbar_init(&bar);
+#pragma unroll
+    for (int j = 0; j < J; j++) {
+        int row, k8;
+        x_piece(tid, j, row, k8);
+        *reinterpret_cast<uint4*>(sg + kmajor_off(row, k8 * 8, kXK)) =
+            *reinterpret_cast<const uint4*>(Gx + (size_t)row * kG + k8 * 8);
+    }
+    fence_before();
+    __syncthreads();
+    fence_after();
+    const uint32_t tmem = tmem_base, d_addr = smem_addr(sd), g_addr = smem_addr(sg), h_addr = smem_addr(sh);
+    uint32_t parity = 0;
+    float bsum = 0.0f;  // every piece of a thread has the same channel
+    float acc[32];      // dW of (o = lane's channel, 32 columns): the four warps that read tensor memory
+#pragma unroll
+    for (int q = 0; q < 32; q++) acc[q] = 0.0f;
+    const bool reads = (warp & 3) < 2;
+    const uint32_t trow = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+    int held = 0;  // lines in D2
+    for (int line = blockIdx.x; line < nlines; line += gridDim.x) {
+        const size_t o0 = (size_t)(line / kG) * kW * kP + (size_t)(line % kG) * kG;
+#pragma unroll 2
+        for (int j = 0; j < J; j++) {
+            int row, k8;
+            x_piece(tid, j, row, k8);
+            const size_t o = o0 + (size_t)row * kP + k8 * 8;
+            const float4 a0 = __ldg(reinterpret_cast<const float4*>(dh + o)), a1 = __ldg(reinterpret_cast<const float4*>(dh + o) + 1);
+            const float4 h0 = __ldg(reinterpret_cast<const float4*>(h + o)), h1 = __ldg(reinterpret_cast<const float4*>(h + o) + 1);
+            float f[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+            if constexpr (ACT) {
+                const float4 u0 = __ldg(reinterpret_cast<const float4*>(u + o)), u1 = __ldg(reinterpret_cast<const float4*>(u + o) + 1);
+                const float g[8] = {u0.x, u0.y, u0.z, u0.w, u1.x, u1.y, u1.z, u1.w};
+#pragma unroll
+                for (int q = 0; q < 8; q++) f[q] *= gelu_d(g[q]);
+                reinterpret_cast<float4*>(du + o)[0] = make_float4(f[0], f[1], f[2], f[3]);
+                reinterpret_cast<float4*>(du + o)[1] = make_float4(f[4], f[5], f[6], f[7]);
+            }
+            bsum += ((f[0] + f[1]) + (f[2] + f[3])) + ((f[4] + f[5]) + (f[6] + f[7]));
+            *reinterpret_cast<uint4*>(sd + kmajor_off(row, k8 * 8, kXK)) = pack8(f);
+            const float hv[8] = {h0.x, h0.y, h0.z, h0.w, h1.x, h1.y, h1.z, h1.w};
+            *reinterpret_cast<uint4*>(sh + kmajor_off(row, k8 * 8, kXK)) = pack8(hv);
+        }
+        publish_smem();
+        if (tid == 0) {
+#pragma unroll
+            for (int ks = 0; ks < kG / 16; ks++) {
+                const uint64_t da = smem_desc(d_addr + ks * 256, 128, kXK * 128);
+                mma_bf16(tmem, da, smem_desc(g_addr + ks * 256, 128, kXK * 128), instr_desc(kW), ks > 0);
+                mma_bf16(tmem + kW, da, smem_desc(h_addr + ks * 256, 128, kXK * 128), instr_desc(kW), ks > 0 || held > 0);
+            }
+            mma_commit(&bar);
+        }
+        if (!mma_wait(&bar, parity, status)) break;
+        parity ^= 1;
+        const bool flush = ++held == kFlush || line + (int)gridDim.x >= nlines;
+        if (reads) {
+            store_spectrum(tmem, dbb, line, Nc, warp, lane);
+            if (flush) {
+#pragma unroll
+                for (int c0 = 0; c0 < 32; c0 += 16) {
+                    float r[16];
+                    tmem_ld16(trow + kW + (warp >> 2) * 32 + c0, r);
+#pragma unroll
+                    for (int q = 0; q < 16; q++) acc[c0 + q] += r[q];
+                }
+            }
+        }
+        if (flush) held = 0;
+        retire_tile();
+    }
+    if (reads) {
+        float* o = dW + ((warp & 3) * 32 + lane) * kW + (warp >> 2) * 32;
+#pragma unroll
+        for (int q = 0; q < 32; q++) atomicAdd(o + q, acc[q]);
+    }
+    // the four lanes of a channel: lanes l, l + 8, l + 16, l + 24
+    bsum += __shfl_xor_sync(0xffffffffu, bsum, 8);
+    bsum += __shfl_xor_sync(0xffffffffu, bsum, 16);
+    if (lane < 8) atomicAdd(db + warp * 8 + lane, bsum);
     tmem_free(tmem, 128, warp);
 }
 
@@ -387,11 +515,43 @@ cudaError_t fourier_fused(const __nv_bfloat16* W, const __nv_bfloat16* Gt, const
                           float* act, const float* bias, int B, unsigned* status, bool write_u, cudaStream_t st)
 {
     using namespace umma;
-    const cudaError_t e = allow_smem(k_fourier, kFBytes);
+    const cudaError_t e = allow_smem(k_fourier<false>, kFBytes);
     if (e != cudaSuccess) return e;
     const int lines = B * kG, grid = lines < 2 * sm_count() ? lines : 2 * sm_count();
-    k_fourier<<<grid, kThreads, kFBytes, st>>>(W, Gt, X, bb, U, act, bias, lines, (long)B * kW * kModes, status,
-                                               write_u || !act);
+    k_fourier<false><<<grid, kThreads, kFBytes, st>>>(W, Gt, X, bb, U, act, bias, lines, (long)B * kW * kModes, status,
+                                                      write_u || !act);
+    return cudaGetLastError();
+}
+
+// dX = W^T dU + the transposed forward DFT along x of da (Fx: G x 2 m)
+cudaError_t fourier_bwd_fused(const __nv_bfloat16* W, const __nv_bfloat16* Fx, const float* dU, const float* da, float* dX,
+                              int B, unsigned* status, cudaStream_t st)
+{
+    using namespace umma;
+    const cudaError_t e = allow_smem(k_fourier<true>, kFBytes);
+    if (e != cudaSuccess) return e;
+    const int lines = B * kG, grid = lines < 2 * sm_count() ? lines : 2 * sm_count();
+    k_fourier<true><<<grid, kThreads, kFBytes, st>>>(W, Fx, dU, da, dX, nullptr, nullptr, lines, (long)B * kW * kModes,
+                                                     status, 1);
+    return cudaGetLastError();
+}
+
+// u NULL: no activation (du is dh and is not written).  dW and db accumulate.
+cudaError_t layer_bwd_fused(const __nv_bfloat16* Gx, const float* dh, const float* u, const float* h, float* du, float* dbb,
+                            float* dW, float* db, int B, unsigned* status, cudaStream_t st)
+{
+    using namespace umma;
+    const int lines = B * kG, grid = lines < 2 * sm_count() ? lines : 2 * sm_count();
+    const long Nc = (long)B * kW * kModes;
+    if (u) {
+        const cudaError_t e = allow_smem(k_layer_bwd<true>, 3 * kXBytes);
+        if (e != cudaSuccess) return e;
+        k_layer_bwd<true><<<grid, kThreads, 3 * kXBytes, st>>>(Gx, dh, u, h, du, dbb, dW, db, lines, Nc, status);
+    } else {
+        const cudaError_t e = allow_smem(k_layer_bwd<false>, 3 * kXBytes);
+        if (e != cudaSuccess) return e;
+        k_layer_bwd<false><<<grid, kThreads, 3 * kXBytes, st>>>(Gx, dh, nullptr, h, nullptr, dbb, dW, db, lines, Nc, status);
+    }
     return cudaGetLastError();
 }
 

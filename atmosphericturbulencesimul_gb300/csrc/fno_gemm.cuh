@@ -53,6 +53,14 @@ __device__ __forceinline__ float gelu_f(float x)
     return 0.5f * x * (1.0f + tanhf(c * (x + 0.044715f * x * x * x)));
 }
 
+// Its derivative.
+__device__ __forceinline__ float gelu_d(float x)
+{
+    const float c = 0.7978845608028654f;
+    const float t = tanhf(c * (x + 0.044715f * x * x * x));
+    return 0.5f * (1.0f + t) + 0.5f * x * (1.0f - t * t) * c * (1.0f + 3.0f * 0.044715f * x * x);
+}
+
 namespace gemm {
 
 constexpr int BK = 32;
