@@ -73,8 +73,13 @@ cudaError_t xdft_fused(const __nv_bfloat16* F, const float* H, float* a, int B, 
 cudaError_t fourier_fused(const __nv_bfloat16* W, const __nv_bfloat16* Gt, const float* X, const float* bb, float* U,
                           float* act, const float* bias, int B, unsigned* status, bool write_u, cudaStream_t st);
 cudaError_t project_fused(const __nv_bfloat16* W1, const float* c1, const __nv_bfloat16* W2, const float* c2,
-                          const float* X, float* qpre, float* q, float* out, int B, unsigned* status, bool keep,
+                          const float* X, float* qpre, float* out, int B, unsigned* status, bool keep,
                           cudaStream_t st);
+bool lift_bwd_supported(int nin);
+cudaError_t lift_bwd_fused(const float* dh, const float* x, float* dW, float* db, int B, unsigned* status, cudaStream_t st);
+cudaError_t project_bwd_fused(const __nv_bfloat16* W1, const __nv_bfloat16* W2, const float* dout, const float* qpre,
+                              const float* u, float* dh, float* dW1, float* dc1, float* dW2, float* dc2, int B,
+                              unsigned* status, cudaStream_t st);
 cudaError_t fourier_bwd_fused(const __nv_bfloat16* W, const __nv_bfloat16* Fx, const float* dU, const float* da, float* dX,
                               int B, unsigned* status, cudaStream_t st);
 cudaError_t layer_bwd_fused(const __nv_bfloat16* Gx, const float* dh, const float* u, const float* h, float* du, float* dbb,
@@ -183,8 +188,16 @@ __global__ void k_mse(const float* __restrict__ out, const float* __restrict__ t
         dout[i] = inv * d;
         s += (double)d * d;
     }
+    // one atomic per CTA: every one goes to the same address (one per warp of
+    // 2432 CTAs took 35 us)
+    __shared__ double red[32];
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if ((threadIdx.x & 31) == 0) atomicAdd(loss, s / (double)n);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (unsigned w = 1; w < blockDim.x >> 5; w++) s += red[w];
+        atomicAdd(loss, s / (double)n);
+    }
 }
 
 // Mode mixing y[b][o][k] = sum_c R[k][o][c] z[b][c][k] (complex) for KX
@@ -269,7 +282,8 @@ cudaError_t modemix(const __nv_bfloat16* R, const float* z, float* y, int B, int
         kern<<<m * m / kx, 256, sm, st>>>(R, z, y, B, w, m, sk, sc);
         return cudaGetLastError();
     };
-    if (m % 4 == 0 && modemix_smem<4>(w) <= 113 * 1024) return go(k_modemix<4>, modemix_smem<4>(w), 4);
+    // (whole runs per mode, sc = 1, need no neighbours: two modes make twice the CTAs)
+    if (sc != 1 && m % 4 == 0 && modemix_smem<4>(w) <= 113 * 1024) return go(k_modemix<4>, modemix_smem<4>(w), 4);
     if (modemix_smem<2>(w) <= 113 * 1024) return go(k_modemix<2>, modemix_smem<2>(w), 2);  // m is even
     return go(k_modemix<1>, modemix_smem<1>(w), 1);
 }
@@ -334,12 +348,12 @@ size_t modemix_bwd_smem(int B, int w) { return sizeof(float) * (4 * (size_t)B * 
 // The same at the fused kernels' shape (width 64, images [.][m][B w]): one
 // mode per CTA, whose z, dy and dz are runs of B w values.  A thread owns an
 // input channel c and 16 output channels: dR[o][c] stays in registers over the
-// samples (z of its channel in registers, dy a broadcast), is added to the
-// gradient once, and is read early.  HBM bounds it: 75 MB per layer at a batch
+// samples (z of its channel in registers, dy a broadcast) and is added to the
+// gradient once.  HBM bounds it: 75 MB per layer at a batch
 // of 8, 33 us; the form above took 75 us (two shared loads per product, 4-byte
 // accesses 128 bytes apart).
 template <int NB>
-__global__ void __launch_bounds__(256) k_modemix_bwd64(const __nv_bfloat16* __restrict__ R, const float* __restrict__ z,
+__global__ void __launch_bounds__(256, 3) k_modemix_bwd64(const __nv_bfloat16* __restrict__ R, const float* __restrict__ z,
                                                        const float* __restrict__ dy, float* __restrict__ dz,
                                                        float* __restrict__ dR, int B, int m)
 {
@@ -352,12 +366,9 @@ __global__ void __launch_bounds__(256) k_modemix_bwd64(const __nv_bfloat16* __re
     const __nv_bfloat162* Rk = reinterpret_cast<const __nv_bfloat162*>(R) + (size_t)k * w * w;
     float2* dRk = reinterpret_cast<float2*>(dR) + (size_t)k * w * w;
     const int c = tid % w, og = tid / w * 16;
-    float2 g[16], acc[16];
+    float2 acc[16];
 #pragma unroll
-    for (int q = 0; q < 16; q++) {
-        g[q] = dRk[(og + q) * w + c];
-        acc[q] = make_float2(0.0f, 0.0f);
-    }
+    for (int q = 0; q < 16; q++) acc[q] = make_float2(0.0f, 0.0f);
     for (int i = tid; i < w * w; i += 256) rs[i] = Rk[i];
     for (int b0 = 0; b0 < B; b0 += NB) {
         const int nb = min(NB, B - b0);
@@ -395,7 +406,10 @@ __global__ void __launch_bounds__(256) k_modemix_bwd64(const __nv_bfloat16* __re
         }
     }
 #pragma unroll
-    for (int q = 0; q < 16; q++) dRk[(og + q) * w + c] = make_float2(g[q].x + acc[q].x, g[q].y + acc[q].y);
+    for (int q = 0; q < 16; q++) {
+        const float2 g = dRk[(og + q) * w + c];
+        dRk[(og + q) * w + c] = make_float2(g.x + acc[q].x, g.y + acc[q].y);
+    }
 }
 
 __global__ void k_to_bf16(const float* __restrict__ in, __nv_bfloat16* __restrict__ out, long n)
@@ -812,7 +826,7 @@ atmwfs_status forward(atmwfs_fno* f, const float* x, float* out, int B, cudaStre
                                   pf + f->L.b[l], B, status, training, st));
         }
         FN_CUDA(project_fused(pb + f->L.proj1_W, pf + f->L.proj1_b, pb + f->L.proj2_W, pf + f->L.proj2_b, last_h(f), f->qpre,
-                              f->q, out, B, status, training, st));
+                              out, B, status, training, st));
         return ATMWFS_OK;
     }
     for (int l = 0; l < c.layers; l++) {
@@ -862,18 +876,23 @@ atmwfs_status backward(atmwfs_fno* f, const float* x, const float* dout, int B, 
     const __nv_bfloat16* pb = f->pbf;
     float* g = f->grads;
     const dim3 rs((unsigned)std::min<long>((P + 255) / 256, 64), 1);
-    // projection
-    FN_CUDA(pointwise_dw(c.nout, c.proj, dout, f->q, g + f->L.proj2_W, B, P, st));
-    k_rowsum<<<dim3(rs.x, c.nout), 256, 0, st>>>(dout, g + f->L.proj2_b, B, c.nout, P);
-    FN_CUDA(pointwise_dx(pb + f->L.proj2_W, c.nout, c.proj, dout, f->dq, B, P, 0.0f, st));
-    k_gelu_bwd<<<grid_for(nq), 256, 0, st>>>(f->dq, f->qpre, f->dq, nq);
-    FN_CUDA(pointwise_dw(c.proj, c.width, f->dq, last_h(f), g + f->L.proj1_W, B, P, st));
-    k_rowsum<<<dim3(rs.x, c.proj), 256, 0, st>>>(f->dq, g + f->L.proj1_b, B, c.proj, P);
-    FN_CUDA(pointwise_dx(pb + f->L.proj1_W, c.proj, c.width, f->dq, f->dh, B, P, 0.0f, st));
-    // Fourier layers, last to first: dh holds dL/dh[l+1]
     const bool fused = fused_shape(c);
     unsigned* status = fused ? umma_status_ptr() : nullptr;
     if (fused && !status) return err(ATMWFS_ERR_CUDA, "status symbol");
+    // projection
+    if (fused) {
+        FN_CUDA(project_bwd_fused(pb + f->L.proj1_W, pb + f->L.proj2_W, dout, f->qpre, last_h(f), f->dh, g + f->L.proj1_W,
+                                  g + f->L.proj1_b, g + f->L.proj2_W, g + f->L.proj2_b, B, status, st));
+    } else {
+        FN_CUDA(pointwise_dw(c.nout, c.proj, dout, f->q, g + f->L.proj2_W, B, P, st));
+        k_rowsum<<<dim3(rs.x, c.nout), 256, 0, st>>>(dout, g + f->L.proj2_b, B, c.nout, P);
+        FN_CUDA(pointwise_dx(pb + f->L.proj2_W, c.nout, c.proj, dout, f->dq, B, P, 0.0f, st));
+        k_gelu_bwd<<<grid_for(nq), 256, 0, st>>>(f->dq, f->qpre, f->dq, nq);
+        FN_CUDA(pointwise_dw(c.proj, c.width, f->dq, last_h(f), g + f->L.proj1_W, B, P, st));
+        k_rowsum<<<dim3(rs.x, c.proj), 256, 0, st>>>(f->dq, g + f->L.proj1_b, B, c.proj, P);
+        FN_CUDA(pointwise_dx(pb + f->L.proj1_W, c.proj, c.width, f->dq, f->dh, B, P, 0.0f, st));
+    }
+    // Fourier layers, last to first: dh holds dL/dh[l+1]
     for (int l = c.layers - 1; l >= 0; l--) {
         if (fused) {
             FN_TRY(layer_bwd(f, l, f->dh, f->dh2, B, status, st));
@@ -889,6 +908,10 @@ atmwfs_status backward(atmwfs_fno* f, const float* x, const float* dout, int B, 
         std::swap(f->dh, f->dh2);
     }
     // lift
+    if (fused && lift_bwd_supported(c.nin) && (reinterpret_cast<uintptr_t>(x) & 15) == 0) {
+        FN_CUDA(lift_bwd_fused(f->dh, x, g + f->L.lift_W, g + f->L.lift_b, B, status, st));
+        return ATMWFS_OK;
+    }
     FN_CUDA(pointwise_dw(c.width, c.nin, f->dh, x, g + f->L.lift_W, B, P, st));
     k_rowsum<<<dim3(rs.x, c.width), 256, 0, st>>>(f->dh, g + f->L.lift_b, B, c.width, P);
     FN_CUDA(cudaGetLastError());
@@ -1009,7 +1032,7 @@ atmwfs_status atmwfs_fno_loss_grad(atmwfs_fno* f, const float* in, const float* 
     FN_TRY(forward(f, in, out, batch, st, true));
     const long n = (long)batch * f->cfg.nout * f->cfg.grid * f->cfg.grid;
     FN_CUDA(cudaMemsetAsync(f->d_loss, 0, sizeof(double), st));
-    k_mse<<<grid_for(n), 256, 0, st>>>(out, target, f->dout, n, f->d_loss);
+    k_mse<<<std::min(grid_for(n), 2u * 152u), 256, 0, st>>>(out, target, f->dout, n, f->d_loss);
     FN_CUDA(cudaGetLastError());
     FN_TRY(backward(f, in, f->dout, batch, st));
     if (loss) {

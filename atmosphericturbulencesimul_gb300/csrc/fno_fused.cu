@@ -7,7 +7,8 @@
 //              same pair of the backward pass;
 //   k_project  the first projection + GELU + the 2-channel output;
 //   k_layer_bwd  a layer's GELU gradient, its weight and bias gradients and
-//              the transposed inverse DFT along x, from one read of the line.
+//              the transposed inverse DFT along x, from one read of the line;
+//   k_project_bwd  every gradient of the head, without storing dq.
 // The products keep the operands' BF16 rounding, the K order and the FP32
 // accumulation of the separate products (k_pointwise, k_rowprod, the mma.sync
 // GEMM), so a layer's activations and gradients are the same bits (sums over
@@ -68,27 +69,31 @@ static_assert(2 * kModes == kW, "the two operands have the same shape");
 // piece j of thread tid: 8 consecutive x of one channel; the lanes of a warp
 // take 8 channels x 4 pieces, so that a store phase of 8 lanes fills one
 // 128-byte core matrix
+template <int NT = kThreads>
 __device__ __forceinline__ void x_piece(int tid, int j, int& row, int& k8)
 {
-    const int i = tid + kThreads * j, rest = i >> 5;
+    const int i = tid + NT * j, rest = i >> 5;
     row = (rest & 7) * 8 + (i & 7);
     k8 = (rest >> 3) * 4 + ((i >> 3) & 3);
 }
 
 // The 64 x 64 spectrum of a line from tensor memory (lanes 0 .. 63: channels,
-// columns: re and im of the modes) into the planar image; warps 0, 1, 4 and 5
-// (warp w: lanes 32 (w % 4) .., plane w / 4).
+// columns: re and im of the modes) into the planar image, by the warps of the
+// lower two lane blocks: warp w takes lanes 32 (w % 4) .. and the w / 4-th of
+// S equal ranges of columns.
+template <int S>
 __device__ __forceinline__ void store_spectrum(uint32_t tmem, float* __restrict__ a, int line, long Nc, int warp, int lane)
 {
-    const int cb = (warp & 3) * 32, p = warp >> 2, b = line / kG, y = line % kG;
+    const int cb = (warp & 3) * 32, b = line / kG, y = line % kG;
     const size_t BW = (size_t)Nc / kModes;
-    float* o = a + (size_t)p * kG * Nc + (size_t)y * Nc + (size_t)b * kW + cb + lane;
 #pragma unroll
-    for (int c0 = 0; c0 < kModes; c0 += 16) {
+    for (int c0 = 0; c0 < kW / S; c0 += 16) {
+        const int n = (warp >> 2) * (kW / S) + c0, p = n / kModes, kx = n % kModes;
+        float* o = a + (size_t)p * kG * Nc + (size_t)y * Nc + kx * BW + (size_t)b * kW + cb + lane;
         float r[16];
-        tmem_ld16(tmem + ((uint32_t)cb << 16) + p * kModes + c0, r);
+        tmem_ld16(tmem + ((uint32_t)cb << 16) + n, r);
 #pragma unroll
-        for (int q = 0; q < 16; q++) o[(c0 + q) * BW] = r[q];
+        for (int q = 0; q < 16; q++) o[q * BW] = r[q];
     }
 }
 
@@ -147,7 +152,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_xdft(const __nv_bfloat16* __res
         }
         if (!mma_wait(&bar, parity, status)) break;
         parity ^= 1;
-        if ((warp & 3) < 2) store_spectrum(tmem, a, line, Nc, warp, lane);
+        if ((warp & 3) < 2) store_spectrum<2>(tmem, a, line, Nc, warp, lane);
         retire_tile();
     }
     tmem_free(tmem, 64, warp);
@@ -287,28 +292,70 @@ __global__ void __launch_bounds__(kThreads, 2)
 // split product it replaces) and is then added to FP32 registers, one atomic
 // per element and CTA at the end.
 // ---------------------------------------------------------------------------
+// HC = 8 without SPEC is the lift's weight and bias gradient (no DFT, K the
+// input planes padded to 16 zero rows).
+//
+// One CTA of 512 threads per SM: a line's operands (up to 192 KB) are loaded
+// into registers while the previous line's products run.
 constexpr int kFlush = 4;
+constexpr int kBT = 512;
 
-template <bool ACT>
-__global__ void __launch_bounds__(kThreads, 2)
+__device__ __forceinline__ void ld8(float (&f)[8], const float* p)
+{
+    const float4 a = __ldg(reinterpret_cast<const float4*>(p)), b = __ldg(reinterpret_cast<const float4*>(p) + 1);
+    f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w;
+    f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w;
+}
+
+template <bool ACT, bool SPEC, int HC>
+__global__ void __launch_bounds__(kBT, 1)
     k_layer_bwd(const __nv_bfloat16* __restrict__ Gx, const float* __restrict__ dh, const float* __restrict__ u,
                 const float* __restrict__ h, float* __restrict__ du, float* __restrict__ dbb, float* __restrict__ dW,
                 float* __restrict__ db, int nlines, long Nc, unsigned* status)
 {
-    constexpr int J = kW * kXK / kThreads;
+    constexpr int J = kW * kXK / kBT;            // pieces of the line per thread
+    constexpr int HN = HC < 16 ? 16 : HC;        // N of the weight product
+    constexpr int JH = HC == kW ? J : 1;         // pieces of h per thread
+    constexpr int CN = HN / 4;                   // dW columns per reading thread (4 warps per lane block)
+    static_assert(HC == kW || HC * kXK <= kBT, "h in one piece per thread");
     extern __shared__ __align__(1024) unsigned char sm[];
     unsigned char *sd = sm, *sg = sm + kXBytes, *sh = sm + 2 * kXBytes;  // du, Gx, h
     __shared__ __align__(8) uint64_t bar;
     __shared__ uint32_t tmem_base;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    float d[J][8], g[ACT ? J : 1][8], hv[JH][8];
+    const int hrow = tid & 7, hk8 = tid >> 3;    // HC = 8: this thread's piece of h
+    auto load = [&](int line) {
+        const size_t o0 = (size_t)(line / kG) * kW * kP + (size_t)(line % kG) * kG;
+#pragma unroll
+        for (int j = 0; j < J; j++) {
+            int row, k8;
+            x_piece<kBT>(tid, j, row, k8);
+            const size_t o = o0 + (size_t)row * kP + k8 * 8;
+            ld8(d[j], dh + o);
+            if constexpr (ACT) ld8(g[j], u + o);
+            if constexpr (HC == kW) ld8(hv[j], h + o);
+        }
+        if constexpr (HC != kW)
+            if (tid < HC * kXK)
+                ld8(hv[0], h + (size_t)(line / kG) * HC * kP + (size_t)(line % kG) * kG + (size_t)hrow * kP + hk8 * 8);
+    };
+    if (blockIdx.x < nlines) load(blockIdx.x);
     tmem_alloc(&tmem_base, 128, warp);
     if (tid == 0) mbar_init(&bar);
+    if constexpr (SPEC) {
 #pragma unroll
-    for (int j = 0; j < J; j++) {
-        int row, k8;
-        x_piece(tid, j, row, k8);
-        *reinterpret_cast<uint4*>(sg + kmajor_off(row, k8 * 8, kXK)) =
-            *reinterpret_cast<const uint4*>(Gx + (size_t)row * kG + k8 * 8);
+        for (int j = 0; j < J; j++) {
+            int row, k8;
+            x_piece<kBT>(tid, j, row, k8);
+            *reinterpret_cast<uint4*>(sg + kmajor_off(row, k8 * 8, kXK)) =
+                *reinterpret_cast<const uint4*>(Gx + (size_t)row * kG + k8 * 8);
+        }
+    }
+    if constexpr (HC != kW) {
+        static_assert(HC == kW || HC == 8, "one group of valid rows, one of zeros");
+        if (tid < 8 * kXK)
+            *reinterpret_cast<uint4*>(sh + kmajor_off(8 + hrow, hk8 * 8, kXK)) = make_uint4(0u, 0u, 0u, 0u);
     }
     fence_before();
     __syncthreads();
@@ -316,42 +363,40 @@ __global__ void __launch_bounds__(kThreads, 2)
     const uint32_t tmem = tmem_base, d_addr = smem_addr(sd), g_addr = smem_addr(sg), h_addr = smem_addr(sh);
     uint32_t parity = 0;
     float bsum = 0.0f;  // every piece of a thread has the same channel
-    float acc[32];      // dW of (o = lane's channel, 32 columns): the four warps that read tensor memory
+    float acc[CN];      // dW of o = the lane's channel: the warps that read tensor memory
 #pragma unroll
-    for (int q = 0; q < 32; q++) acc[q] = 0.0f;
+    for (int q = 0; q < CN; q++) acc[q] = 0.0f;
     const bool reads = (warp & 3) < 2;
     const uint32_t trow = tmem + ((uint32_t)((warp & 3) * 32) << 16);
     int held = 0;  // lines in D2
     for (int line = blockIdx.x; line < nlines; line += gridDim.x) {
         const size_t o0 = (size_t)(line / kG) * kW * kP + (size_t)(line % kG) * kG;
-#pragma unroll 2
+#pragma unroll
         for (int j = 0; j < J; j++) {
             int row, k8;
-            x_piece(tid, j, row, k8);
-            const size_t o = o0 + (size_t)row * kP + k8 * 8;
-            const float4 a0 = __ldg(reinterpret_cast<const float4*>(dh + o)), a1 = __ldg(reinterpret_cast<const float4*>(dh + o) + 1);
-            const float4 h0 = __ldg(reinterpret_cast<const float4*>(h + o)), h1 = __ldg(reinterpret_cast<const float4*>(h + o) + 1);
-            float f[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+            x_piece<kBT>(tid, j, row, k8);
             if constexpr (ACT) {
-                const float4 u0 = __ldg(reinterpret_cast<const float4*>(u + o)), u1 = __ldg(reinterpret_cast<const float4*>(u + o) + 1);
-                const float g[8] = {u0.x, u0.y, u0.z, u0.w, u1.x, u1.y, u1.z, u1.w};
 #pragma unroll
-                for (int q = 0; q < 8; q++) f[q] *= gelu_d(g[q]);
-                reinterpret_cast<float4*>(du + o)[0] = make_float4(f[0], f[1], f[2], f[3]);
-                reinterpret_cast<float4*>(du + o)[1] = make_float4(f[4], f[5], f[6], f[7]);
+                for (int q = 0; q < 8; q++) d[j][q] *= gelu_d(g[j][q]);
+                float4* o = reinterpret_cast<float4*>(du + o0 + (size_t)row * kP + k8 * 8);
+                o[0] = make_float4(d[j][0], d[j][1], d[j][2], d[j][3]);
+                o[1] = make_float4(d[j][4], d[j][5], d[j][6], d[j][7]);
             }
-            bsum += ((f[0] + f[1]) + (f[2] + f[3])) + ((f[4] + f[5]) + (f[6] + f[7]));
-            *reinterpret_cast<uint4*>(sd + kmajor_off(row, k8 * 8, kXK)) = pack8(f);
-            const float hv[8] = {h0.x, h0.y, h0.z, h0.w, h1.x, h1.y, h1.z, h1.w};
-            *reinterpret_cast<uint4*>(sh + kmajor_off(row, k8 * 8, kXK)) = pack8(hv);
+            bsum += ((d[j][0] + d[j][1]) + (d[j][2] + d[j][3])) + ((d[j][4] + d[j][5]) + (d[j][6] + d[j][7]));
+            *reinterpret_cast<uint4*>(sd + kmajor_off(row, k8 * 8, kXK)) = pack8(d[j]);
+            if constexpr (HC == kW) *reinterpret_cast<uint4*>(sh + kmajor_off(row, k8 * 8, kXK)) = pack8(hv[j]);
         }
+        if constexpr (HC != kW)
+            if (tid < HC * kXK) *reinterpret_cast<uint4*>(sh + kmajor_off(hrow, hk8 * 8, kXK)) = pack8(hv[0]);
         publish_smem();
+        if (line + (int)gridDim.x < nlines) load(line + gridDim.x);
         if (tid == 0) {
 #pragma unroll
             for (int ks = 0; ks < kG / 16; ks++) {
                 const uint64_t da = smem_desc(d_addr + ks * 256, 128, kXK * 128);
-                mma_bf16(tmem, da, smem_desc(g_addr + ks * 256, 128, kXK * 128), instr_desc(kW), ks > 0);
-                mma_bf16(tmem + kW, da, smem_desc(h_addr + ks * 256, 128, kXK * 128), instr_desc(kW), ks > 0 || held > 0);
+                if constexpr (SPEC)
+                    mma_bf16(tmem, da, smem_desc(g_addr + ks * 256, 128, kXK * 128), instr_desc(kW), ks > 0);
+                mma_bf16(tmem + kW, da, smem_desc(h_addr + ks * 256, 128, kXK * 128), instr_desc(HN), ks > 0 || held > 0);
             }
             mma_commit(&bar);
         }
@@ -359,30 +404,208 @@ __global__ void __launch_bounds__(kThreads, 2)
         parity ^= 1;
         const bool flush = ++held == kFlush || line + (int)gridDim.x >= nlines;
         if (reads) {
-            store_spectrum(tmem, dbb, line, Nc, warp, lane);
+            if constexpr (SPEC) store_spectrum<4>(tmem, dbb, line, Nc, warp, lane);
             if (flush) {
+                float r[16];
+                tmem_ld16(trow + kW + (HN == 16 ? 0 : (warp >> 2) * CN), r);
+                if constexpr (HN == 16) {
 #pragma unroll
-                for (int c0 = 0; c0 < 32; c0 += 16) {
-                    float r[16];
-                    tmem_ld16(trow + kW + (warp >> 2) * 32 + c0, r);
+                    for (int q = 0; q < CN; q++) acc[q] += (warp >> 2) < 2 ? r[((warp >> 2) & 1) * CN + q] : 0.0f;
+                } else {
 #pragma unroll
-                    for (int q = 0; q < 16; q++) acc[c0 + q] += r[q];
+                    for (int q = 0; q < CN; q++) acc[q] += r[q];
                 }
             }
         }
         if (flush) held = 0;
         retire_tile();
     }
-    if (reads) {
-        float* o = dW + ((warp & 3) * 32 + lane) * kW + (warp >> 2) * 32;
+    if (reads && (warp >> 2) * CN < HC) {
+        float* o = dW + ((warp & 3) * 32 + lane) * HC + (warp >> 2) * CN;
 #pragma unroll
-        for (int q = 0; q < 32; q++) atomicAdd(o + q, acc[q]);
+        for (int q = 0; q < CN; q++) atomicAdd(o + q, acc[q]);
     }
-    // the four lanes of a channel: lanes l, l + 8, l + 16, l + 24
+    // a channel's lanes: l, l + 8, l + 16, l + 24 of warps w and w + 8
     bsum += __shfl_xor_sync(0xffffffffu, bsum, 8);
     bsum += __shfl_xor_sync(0xffffffffu, bsum, 16);
-    if (lane < 8) atomicAdd(db + warp * 8 + lane, bsum);
+    if (lane < 8) atomicAdd(db + (warp & 7) * 8 + lane, bsum);
     tmem_free(tmem, 128, warp);
+}
+
+// ---------------------------------------------------------------------------
+// Backward of the projection head over one line (sample b, row y):
+//   dq = (W2^T dout) gelu'(qpre)         (128 channels)
+//   dh = W1^T dq                         D3 (256 pixels x 64 channels, K = 128)
+//   dW1 += dq u^T, dc1 += sum dq         D2 (128 x 64, K = 256 pixels, over lines)
+//   dW2 += dout q^T, dc2 += sum dout     q = gelu(qpre), from the same tanh
+// from one read of qpre, u and dout; dq stays on the SM (as BF16, as every
+// product rounds it; its bias sums are FP32).  HBM bounds it: 0.54 GB for a
+// batch of 8.  Before: a GEMM of K = 2 writing dq (129 us), its GELU gradient
+// (120), three products reading dq or q (104 + 130 + 244) and the bias sums
+// (75).  dq is stored twice in shared memory, [channel][pixel] for dW1 and
+// [pixel][channel] for dh (each K-major); the second's 8-row groups are 32
+// bytes apart from a multiple of 128 so that its 2-byte stores spread over the
+// banks.
+// ---------------------------------------------------------------------------
+constexpr uint32_t kQA = 0;                                   // dq [128][256 px]
+constexpr uint32_t kQU = kQA + kProj * kG * 2;                // u [64][256 px]
+constexpr uint32_t kQTs = kProj / 8 * 128 + 32;               // bytes between 8-pixel groups of dq^T
+constexpr uint32_t kQT = kQU + kW * kG * 2;                   // dq^T [256 px][128]
+constexpr uint32_t kQW = kQT + kG / 8 * kQTs;                 // W1^T [64][128]
+constexpr uint32_t kQBytes = kQW + kW * kProj * 2;
+
+__global__ void __launch_bounds__(kBT, 1)
+    k_project_bwd(const __nv_bfloat16* __restrict__ W1, const __nv_bfloat16* __restrict__ W2, const float* __restrict__ dout,
+                  const float* __restrict__ qpre, const float* __restrict__ u, float* __restrict__ dh, float* __restrict__ dW1,
+                  float* __restrict__ dc1, float* __restrict__ dW2, float* __restrict__ dc2, int nlines, unsigned* status)
+{
+    constexpr int J = kW * kXK / kBT;  // pieces of 64 channels of a line per thread
+    extern __shared__ __align__(1024) unsigned char sm[];
+    __shared__ __align__(8) uint64_t bar;
+    __shared__ uint32_t tmem_base;
+    __shared__ __align__(16) float s_d[2][2][kG];  // dout of a line, rounded to BF16, double-buffered
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int ch = (warp & 7) * 8 + (lane & 7);    // every piece of a thread has channel ch or ch + 64
+    float q[2][J][8];
+    float dv = 0.0f, dsum = 0.0f;                  // this thread's dout value (plane tid / 256, pixel tid % 256), its sum
+    auto load = [&](int line) {
+        const size_t o0 = (size_t)(line / kG) * kProj * kP + (size_t)(line % kG) * kG;
+#pragma unroll
+        for (int hf = 0; hf < 2; hf++)
+#pragma unroll
+            for (int j = 0; j < J; j++) {
+                int row, k8;
+                x_piece<kBT>(tid, j, row, k8);
+                ld8(q[hf][j], qpre + o0 + (size_t)(row + 64 * hf) * kP + k8 * 8);
+            }
+        dv = __ldg(dout + ((size_t)(line / kG) * 2 + tid / kG) * kP + (size_t)(line % kG) * kG + tid % kG);
+    };
+    if (blockIdx.x < nlines) load(blockIdx.x);
+    tmem_alloc(&tmem_base, 256, warp);
+    if (tid == 0) mbar_init(&bar);
+    for (int i = tid; i < kProj * kW; i += kBT)  // W1 is [128][64]: element (o, c) to row c, K index o
+        *reinterpret_cast<__nv_bfloat16*>(sm + kQW + kmajor_off(i % kW, i / kW, kProj / 8)) = W1[i];
+    float w2[2][2], bs[2] = {0.0f, 0.0f}, g2[2][2] = {{0.0f, 0.0f}, {0.0f, 0.0f}};
+#pragma unroll
+    for (int hf = 0; hf < 2; hf++)
+#pragma unroll
+        for (int k = 0; k < 2; k++) w2[hf][k] = __bfloat162float(W2[k * kProj + ch + 64 * hf]);
+    float acc[16];  // dW1 of channel (warp % 4) 32 + lane, 16 columns
+#pragma unroll
+    for (int k = 0; k < 16; k++) acc[k] = 0.0f;
+    fence_before();
+    __syncthreads();
+    fence_after();
+    const uint32_t tmem = tmem_base, base = smem_addr(sm);
+    const uint32_t trow = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+    uint32_t parity = 0;
+    int held = 0, buf = 0;
+    for (int line = blockIdx.x; line < nlines; line += gridDim.x) {
+        const size_t o0 = (size_t)(line / kG) * kW * kP + (size_t)(line % kG) * kG;
+        dsum += dv;
+        s_d[buf][tid / kG][tid % kG] = __bfloat162float(__float2bfloat16_rn(dv));
+#pragma unroll
+        for (int j = 0; j < J; j++) {  // u: loaded here, its latency under the first channels' arithmetic
+            int row, k8;
+            x_piece<kBT>(tid, j, row, k8);
+            float f[8];
+            ld8(f, u + o0 + (size_t)row * kP + k8 * 8);
+            *reinterpret_cast<uint4*>(sm + kQU + kmajor_off(row, k8 * 8, kXK)) = pack8(f);
+        }
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < J; j++) {
+            int row, k8;
+            x_piece<kBT>(tid, j, row, k8);
+            const float4 *p0 = reinterpret_cast<const float4*>(&s_d[buf][0][k8 * 8]), *p1 = reinterpret_cast<const float4*>(&s_d[buf][1][k8 * 8]);
+            const float4 a0 = p0[0], a1 = p0[1], b0 = p1[0], b1 = p1[1];
+            const float d0[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+            const float d1[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+#pragma unroll
+            for (int hf = 0; hf < 2; hf++) {
+                float f[8];
+#pragma unroll
+                for (int k = 0; k < 8; k++) {
+                    float v, dg;
+                    gelu_both(q[hf][j][k], v, dg);
+                    f[k] = fmaf(w2[hf][1], d1[k], w2[hf][0] * d0[k]) * dg;
+                    const float vb = __bfloat162float(__float2bfloat16_rn(v));
+                    g2[hf][0] = fmaf(d0[k], vb, g2[hf][0]);
+                    g2[hf][1] = fmaf(d1[k], vb, g2[hf][1]);
+                    bs[hf] += f[k];
+                }
+                const uint4 pk = pack8(f);
+                const int o = row + 64 * hf;
+                *reinterpret_cast<uint4*>(sm + kQA + kmajor_off(o, k8 * 8, kXK)) = pk;
+                unsigned short* t = reinterpret_cast<unsigned short*>(sm + kQT + k8 * kQTs + (o >> 3) * 128 + (o & 7) * 2);
+                const uint32_t w[4] = {pk.x, pk.y, pk.z, pk.w};
+#pragma unroll
+                for (int k = 0; k < 8; k++) t[k * 8] = (unsigned short)(w[k >> 1] >> (16 * (k & 1)));
+            }
+        }
+        publish_smem();
+        if (line + (int)gridDim.x < nlines) load(line + gridDim.x);
+        if (tid == 0) {
+#pragma unroll
+            for (int ks = 0; ks < kG / 16; ks++)  // dW1: K = 256 pixels
+                mma_bf16(tmem + 128, smem_desc(base + kQA + ks * 256, 128, kXK * 128),
+                         smem_desc(base + kQU + ks * 256, 128, kXK * 128), instr_desc(kW), ks > 0 || held > 0);
+#pragma unroll
+            for (int half = 0; half < 2; half++)
+#pragma unroll
+                for (int ks = 0; ks < kProj / 16; ks++)  // dh: K = 128 channels, 128 pixels each
+                    mma_bf16(tmem + half * kW, smem_desc(base + kQT + half * (kM / 8) * kQTs + ks * 256, 128, kQTs),
+                             smem_desc(base + kQW + ks * 256, 128, kProj / 8 * 128), instr_desc(kW), ks > 0);
+            mma_commit(&bar);
+        }
+        if (!mma_wait(&bar, parity, status)) break;
+        parity ^= 1;
+        const bool flush = ++held == kFlush || line + (int)gridDim.x >= nlines;
+        {
+            // warp w: pixels 32 (w % 4) .. of half (w / 4) % 2, channels 32 (w / 8) ..
+            const int half = (warp >> 2) & 1, c0 = (warp >> 3) * 32;
+            float* o = dh + o0 + half * kM + (warp & 3) * 32 + lane;
+#pragma unroll
+            for (int c = 0; c < 32; c += 16) {
+                float r[16];
+                tmem_ld16(trow + half * kW + c0 + c, r);
+#pragma unroll
+                for (int k = 0; k < 16; k++) o[(size_t)(c0 + c + k) * kP] = r[k];
+            }
+        }
+        if (flush) {
+            float r[16];
+            tmem_ld16(trow + 128 + (warp >> 2) * 16, r);
+#pragma unroll
+            for (int k = 0; k < 16; k++) acc[k] += r[k];
+            held = 0;
+        }
+        buf ^= 1;
+        retire_tile();
+    }
+    {
+        float* o = dW1 + ((warp & 3) * 32 + lane) * kW + (warp >> 2) * 16;
+#pragma unroll
+        for (int k = 0; k < 16; k++) atomicAdd(o + k, acc[k]);
+    }
+#pragma unroll
+    for (int o = 8; o < 32; o <<= 1)
+#pragma unroll
+        for (int hf = 0; hf < 2; hf++) {
+            bs[hf] += __shfl_xor_sync(0xffffffffu, bs[hf], o);
+            g2[hf][0] += __shfl_xor_sync(0xffffffffu, g2[hf][0], o);
+            g2[hf][1] += __shfl_xor_sync(0xffffffffu, g2[hf][1], o);
+        }
+    if (lane < 8)
+#pragma unroll
+        for (int hf = 0; hf < 2; hf++) {
+            atomicAdd(dc1 + ch + 64 * hf, bs[hf]);
+            atomicAdd(dW2 + ch + 64 * hf, g2[hf][0]);
+            atomicAdd(dW2 + kProj + ch + 64 * hf, g2[hf][1]);
+        }
+    for (int o = 16; o > 0; o >>= 1) dsum += __shfl_xor_sync(0xffffffffu, dsum, o);
+    if (lane == 0) atomicAdd(dc2 + tid / kG, dsum);
+    tmem_free(tmem, 256, warp);
 }
 
 // ---------------------------------------------------------------------------
@@ -390,15 +613,15 @@ __global__ void __launch_bounds__(kThreads, 2)
 // channels).  The 2-channel product is two FMAs per value in the epilogue of
 // the first, on q rounded to BF16 as the product rounds it, so inference
 // neither stores q (537 MB per batch of 16) nor reads it back: 230 us for the
-// first product and 381 us for a GEMM of N = 2 before.  keep: training also
-// stores the pre-activation and q for the backward pass.
+// first product and 381 us for a GEMM of N = 2 before.  keep: training stores
+// the pre-activation, from which the backward pass forms q again.
 // ---------------------------------------------------------------------------
 constexpr uint32_t kPA = kProj * kW * 2, kPBytes = kPA + kM * kW * 2;
 
 __global__ void __launch_bounds__(kThreads, 3)
     k_project(const __nv_bfloat16* __restrict__ W1, const float* __restrict__ c1, const __nv_bfloat16* __restrict__ W2,
-              const float* __restrict__ c2, const float* __restrict__ X, float* __restrict__ qpre, float* __restrict__ qact,
-              float* __restrict__ out, int ntiles, unsigned* status, int keep)
+              const float* __restrict__ c2, const float* __restrict__ X, float* __restrict__ qpre, float* __restrict__ out,
+              int ntiles, unsigned* status, int keep)
 {
     extern __shared__ __align__(1024) unsigned char sm[];
     __shared__ __align__(8) uint64_t bar;
@@ -456,11 +679,7 @@ __global__ void __launch_bounds__(kThreads, 3)
 #pragma unroll
             for (int q = 0; q < 16; q++) {
                 const float u = r[q] + s_c1[c0 + q], v = gelu_f(u);
-                if (keep) {
-                    const size_t o = (b * kProj + c0 + q) * kP + p;
-                    qpre[o] = u;
-                    qact[o] = v;
-                }
+                if (keep) qpre[(b * kProj + c0 + q) * kP + p] = u;
                 const float vb = __bfloat162float(__float2bfloat16_rn(v));
                 y0 = fmaf(s_w2[0][c0 + q], vb, y0);
                 y1 = fmaf(s_w2[1][c0 + q], vb, y1);
@@ -541,29 +760,52 @@ cudaError_t layer_bwd_fused(const __nv_bfloat16* Gx, const float* dh, const floa
                             float* dW, float* db, int B, unsigned* status, cudaStream_t st)
 {
     using namespace umma;
-    const int lines = B * kG, grid = lines < 2 * sm_count() ? lines : 2 * sm_count();
+    const int lines = B * kG, grid = lines < sm_count() ? lines : sm_count();
     const long Nc = (long)B * kW * kModes;
-    if (u) {
-        const cudaError_t e = allow_smem(k_layer_bwd<true>, 3 * kXBytes);
+    auto go = [&](auto kern) {
+        const cudaError_t e = allow_smem(kern, 3 * kXBytes);
         if (e != cudaSuccess) return e;
-        k_layer_bwd<true><<<grid, kThreads, 3 * kXBytes, st>>>(Gx, dh, u, h, du, dbb, dW, db, lines, Nc, status);
-    } else {
-        const cudaError_t e = allow_smem(k_layer_bwd<false>, 3 * kXBytes);
-        if (e != cudaSuccess) return e;
-        k_layer_bwd<false><<<grid, kThreads, 3 * kXBytes, st>>>(Gx, dh, nullptr, h, nullptr, dbb, dW, db, lines, Nc, status);
-    }
+        kern<<<grid, kBT, 3 * kXBytes, st>>>(Gx, dh, u, h, du, dbb, dW, db, lines, Nc, status);
+        return cudaGetLastError();
+    };
+    return u ? go(k_layer_bwd<true, true, kW>) : go(k_layer_bwd<false, true, kW>);
+}
+
+// The lift's gradients: dW (64 x nin) += dh x^T, db += sum dh.
+bool lift_bwd_supported(int nin) { return nin == 8; }
+
+cudaError_t lift_bwd_fused(const float* dh, const float* x, float* dW, float* db, int B, unsigned* status, cudaStream_t st)
+{
+    using namespace umma;
+    const cudaError_t e = allow_smem(k_layer_bwd<false, false, 8>, 3 * kXBytes);
+    if (e != cudaSuccess) return e;
+    const int lines = B * kG, grid = lines < sm_count() ? lines : sm_count();
+    k_layer_bwd<false, false, 8><<<grid, kBT, 3 * kXBytes, st>>>(nullptr, dh, nullptr, x, nullptr, nullptr, dW, db, lines,
+                                                                 (long)B * kW * kModes, status);
+    return cudaGetLastError();
+}
+
+cudaError_t project_bwd_fused(const __nv_bfloat16* W1, const __nv_bfloat16* W2, const float* dout, const float* qpre,
+                              const float* u, float* dh, float* dW1, float* dc1, float* dW2, float* dc2, int B,
+                              unsigned* status, cudaStream_t st)
+{
+    using namespace umma;
+    const cudaError_t e = allow_smem(k_project_bwd, kQBytes);
+    if (e != cudaSuccess) return e;
+    const int lines = B * kG, grid = lines < sm_count() ? lines : sm_count();
+    k_project_bwd<<<grid, kBT, kQBytes, st>>>(W1, W2, dout, qpre, u, dh, dW1, dc1, dW2, dc2, lines, status);
     return cudaGetLastError();
 }
 
 cudaError_t project_fused(const __nv_bfloat16* W1, const float* c1, const __nv_bfloat16* W2, const float* c2,
-                          const float* X, float* qpre, float* q, float* out, int B, unsigned* status, bool keep,
+                          const float* X, float* qpre, float* out, int B, unsigned* status, bool keep,
                           cudaStream_t st)
 {
     using namespace umma;
     const cudaError_t e = allow_smem(k_project, kPBytes);
     if (e != cudaSuccess) return e;
     const int tiles = (int)(B * (kP / kM)), grid = tiles < 3 * sm_count() ? tiles : 3 * sm_count();
-    k_project<<<grid, kThreads, kPBytes, st>>>(W1, c1, W2, c2, X, qpre, q, out, tiles, status, keep);
+    k_project<<<grid, kThreads, kPBytes, st>>>(W1, c1, W2, c2, X, qpre, out, tiles, status, keep);
     return cudaGetLastError();
 }
 

@@ -61,6 +61,15 @@ __device__ __forceinline__ float gelu_d(float x)
     return 0.5f * (1.0f + t) + 0.5f * x * (1.0f - t * t) * c * (1.0f + 3.0f * 0.044715f * x * x);
 }
 
+// Both, from one tanh.
+__device__ __forceinline__ void gelu_both(float x, float& v, float& d)
+{
+    const float c = 0.7978845608028654f;
+    const float t = tanhf(c * (x + 0.044715f * x * x * x));
+    v = 0.5f * x * (1.0f + t);
+    d = 0.5f * (1.0f + t) + 0.5f * x * (1.0f - t * t) * c * (1.0f + 3.0f * 0.044715f * x * x);
+}
+
 namespace gemm {
 
 constexpr int BK = 32;
