@@ -107,18 +107,17 @@ __global__ void __launch_bounds__(kThreads, 2) k_xdft(const __nv_bfloat16* __res
     __shared__ uint32_t tmem_base;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     float4 v[J][2];
-    auto load = [&](int line) {
-        const float* src = H + (size_t)(line / kG) * kW * kP + (size_t)(line % kG) * kG;
-#pragma unroll
-        for (int j = 0; j < J; j++) {
-            int row, k8;
-            x_piece(tid, j, row, k8);
-            const float4* q = reinterpret_cast<const float4*>(src + (size_t)row * kP + k8 * 8);
-            v[j][0] = __ldg(q);
-            v[j][1] = __ldg(q + 1);
-        }
+    auto load = [&](int line, int j) {
+        int row, k8;
+        x_piece(tid, j, row, k8);
+        const float4* q = reinterpret_cast<const float4*>(H + (size_t)(line / kG) * kW * kP + (size_t)(line % kG) * kG +
+                                                          (size_t)row * kP + k8 * 8);
+        v[j][0] = __ldg(q);
+        v[j][1] = __ldg(q + 1);
     };
-    if (blockIdx.x < nlines) load(blockIdx.x);
+    if (blockIdx.x < nlines)
+#pragma unroll
+        for (int j = 0; j < J; j++) load(blockIdx.x, j);
     tmem_alloc(&tmem_base, 64, warp);
     if (tid == 0) mbar_init(&bar);
 #pragma unroll
@@ -140,9 +139,9 @@ __global__ void __launch_bounds__(kThreads, 2) k_xdft(const __nv_bfloat16* __res
             x_piece(tid, j, row, k8);
             const float f[8] = {v[j][0].x, v[j][0].y, v[j][0].z, v[j][0].w, v[j][1].x, v[j][1].y, v[j][1].z, v[j][1].w};
             *reinterpret_cast<uint4*>(sa + kmajor_off(row, k8 * 8, kXK)) = pack8(f);
+            if (line + (int)gridDim.x < nlines) load(line + gridDim.x, j);
         }
         publish_smem();
-        if (line + (int)gridDim.x < nlines) load(line + gridDim.x);
         if (tid == 0) {
 #pragma unroll
             for (int ks = 0; ks < kG / 16; ks++)
@@ -296,7 +295,7 @@ __global__ void __launch_bounds__(kThreads, 2)
 // input planes padded to 16 zero rows).
 //
 // One CTA of 512 threads per SM: a line's operands (up to 192 KB) are loaded
-// into registers while the previous line's products run.
+// into registers, each piece as soon as the previous line's is used.
 constexpr int kFlush = 4;
 constexpr int kBT = 512;
 
@@ -325,22 +324,25 @@ __global__ void __launch_bounds__(kBT, 1)
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     float d[J][8], g[ACT ? J : 1][8], hv[JH][8];
     const int hrow = tid & 7, hk8 = tid >> 3;    // HC = 8: this thread's piece of h
-    auto load = [&](int line) {
+    auto load = [&](int line, int j) {
         const size_t o0 = (size_t)(line / kG) * kW * kP + (size_t)(line % kG) * kG;
-#pragma unroll
-        for (int j = 0; j < J; j++) {
-            int row, k8;
-            x_piece<kBT>(tid, j, row, k8);
-            const size_t o = o0 + (size_t)row * kP + k8 * 8;
-            ld8(d[j], dh + o);
-            if constexpr (ACT) ld8(g[j], u + o);
-            if constexpr (HC == kW) ld8(hv[j], h + o);
-        }
+        int row, k8;
+        x_piece<kBT>(tid, j, row, k8);
+        const size_t o = o0 + (size_t)row * kP + k8 * 8;
+        ld8(d[j], dh + o);
+        if constexpr (ACT) ld8(g[j], u + o);
+        if constexpr (HC == kW) ld8(hv[j], h + o);
+    };
+    auto load_h = [&](int line) {
         if constexpr (HC != kW)
             if (tid < HC * kXK)
                 ld8(hv[0], h + (size_t)(line / kG) * HC * kP + (size_t)(line % kG) * kG + (size_t)hrow * kP + hk8 * 8);
     };
-    if (blockIdx.x < nlines) load(blockIdx.x);
+    if (blockIdx.x < nlines) {
+#pragma unroll
+        for (int j = 0; j < J; j++) load(blockIdx.x, j);
+        load_h(blockIdx.x);
+    }
     tmem_alloc(&tmem_base, 128, warp);
     if (tid == 0) mbar_init(&bar);
     if constexpr (SPEC) {
@@ -385,11 +387,14 @@ __global__ void __launch_bounds__(kBT, 1)
             bsum += ((d[j][0] + d[j][1]) + (d[j][2] + d[j][3])) + ((d[j][4] + d[j][5]) + (d[j][6] + d[j][7]));
             *reinterpret_cast<uint4*>(sd + kmajor_off(row, k8 * 8, kXK)) = pack8(d[j]);
             if constexpr (HC == kW) *reinterpret_cast<uint4*>(sh + kmajor_off(row, k8 * 8, kXK)) = pack8(hv[j]);
+            // the piece's registers are free: the next line's values come in
+            // under the remaining pieces' arithmetic and the products
+            if (line + (int)gridDim.x < nlines) load(line + gridDim.x, j);
         }
         if constexpr (HC != kW)
             if (tid < HC * kXK) *reinterpret_cast<uint4*>(sh + kmajor_off(hrow, hk8 * 8, kXK)) = pack8(hv[0]);
+        if (line + (int)gridDim.x < nlines) load_h(line + gridDim.x);
         publish_smem();
-        if (line + (int)gridDim.x < nlines) load(line + gridDim.x);
         if (tid == 0) {
 #pragma unroll
             for (int ks = 0; ks < kG / 16; ks++) {
@@ -468,19 +473,22 @@ __global__ void __launch_bounds__(kBT, 1)
     const int ch = (warp & 7) * 8 + (lane & 7);    // every piece of a thread has channel ch or ch + 64
     float q[2][J][8];
     float dv = 0.0f, dsum = 0.0f;                  // this thread's dout value (plane tid / 256, pixel tid % 256), its sum
-    auto load = [&](int line) {
+    auto load = [&](int line, int hf, int j) {
         const size_t o0 = (size_t)(line / kG) * kProj * kP + (size_t)(line % kG) * kG;
+        int row, k8;
+        x_piece<kBT>(tid, j, row, k8);
+        ld8(q[hf][j], qpre + o0 + (size_t)(row + 64 * hf) * kP + k8 * 8);
+    };
+    auto load_d = [&](int line) {
+        dv = __ldg(dout + ((size_t)(line / kG) * 2 + tid / kG) * kP + (size_t)(line % kG) * kG + tid % kG);
+    };
+    if (blockIdx.x < nlines) {
 #pragma unroll
         for (int hf = 0; hf < 2; hf++)
 #pragma unroll
-            for (int j = 0; j < J; j++) {
-                int row, k8;
-                x_piece<kBT>(tid, j, row, k8);
-                ld8(q[hf][j], qpre + o0 + (size_t)(row + 64 * hf) * kP + k8 * 8);
-            }
-        dv = __ldg(dout + ((size_t)(line / kG) * 2 + tid / kG) * kP + (size_t)(line % kG) * kG + tid % kG);
-    };
-    if (blockIdx.x < nlines) load(blockIdx.x);
+            for (int j = 0; j < J; j++) load(blockIdx.x, hf, j);
+        load_d(blockIdx.x);
+    }
     tmem_alloc(&tmem_base, 256, warp);
     if (tid == 0) mbar_init(&bar);
     for (int i = tid; i < kProj * kW; i += kBT)  // W1 is [128][64]: element (o, c) to row c, K index o
@@ -504,6 +512,7 @@ __global__ void __launch_bounds__(kBT, 1)
         const size_t o0 = (size_t)(line / kG) * kW * kP + (size_t)(line % kG) * kG;
         dsum += dv;
         s_d[buf][tid / kG][tid % kG] = __bfloat162float(__float2bfloat16_rn(dv));
+        if (line + (int)gridDim.x < nlines) load_d(line + gridDim.x);
 #pragma unroll
         for (int j = 0; j < J; j++) {  // u: loaded here, its latency under the first channels' arithmetic
             int row, k8;
@@ -534,6 +543,7 @@ __global__ void __launch_bounds__(kBT, 1)
                     g2[hf][1] = fmaf(d1[k], vb, g2[hf][1]);
                     bs[hf] += f[k];
                 }
+                if (line + (int)gridDim.x < nlines) load(line + gridDim.x, hf, j);  // the piece's registers are free
                 const uint4 pk = pack8(f);
                 const int o = row + 64 * hf;
                 *reinterpret_cast<uint4*>(sm + kQA + kmajor_off(o, k8 * 8, kXK)) = pk;
@@ -544,7 +554,6 @@ __global__ void __launch_bounds__(kBT, 1)
             }
         }
         publish_smem();
-        if (line + (int)gridDim.x < nlines) load(line + gridDim.x);
         if (tid == 0) {
 #pragma unroll
             for (int ks = 0; ks < kG / 16; ks++)  // dW1: K = 256 pixels
