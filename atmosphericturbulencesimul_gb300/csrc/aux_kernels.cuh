@@ -42,12 +42,12 @@ cudaError_t chromat_sum(const float* I, int S, int n, const float* coeff, const 
                         cudaStream_t st);
 cudaError_t fft2d_large(const float2* in, float2* out, float2* tmp, int M, int sign, cudaStream_t st);
 
-cudaError_t launch_pass_64(int var, dim3 grid, const PassArgs& a, const TmaSet* maps, const float2* tw, cudaStream_t st);
-cudaError_t launch_pass_128(int var, dim3 grid, const PassArgs& a, const TmaSet* maps, const float2* tw, cudaStream_t st);
-cudaError_t launch_pass_256(int var, dim3 grid, const PassArgs& a, const TmaSet* maps, const float2* tw, cudaStream_t st);
-cudaError_t launch_pass_512(int var, dim3 grid, const PassArgs& a, const TmaSet* maps, const float2* tw, cudaStream_t st);
-cudaError_t launch_pass_1024(int var, dim3 grid, const PassArgs& a, const TmaSet* maps, const float2* tw, cudaStream_t st);
-cudaError_t launch_pass_2048(int var, dim3 grid, const PassArgs& a, const TmaSet* maps, const float2* tw, cudaStream_t st);
+cudaError_t launch_pass_64(int var, dim3 grid, const PassArgs& a, const float2* tw, cudaStream_t st);
+cudaError_t launch_pass_128(int var, dim3 grid, const PassArgs& a, const float2* tw, cudaStream_t st);
+cudaError_t launch_pass_256(int var, dim3 grid, const PassArgs& a, const float2* tw, cudaStream_t st);
+cudaError_t launch_pass_512(int var, dim3 grid, const PassArgs& a, const float2* tw, cudaStream_t st);
+cudaError_t launch_pass_1024(int var, dim3 grid, const PassArgs& a, const float2* tw, cudaStream_t st);
+cudaError_t launch_pass_2048(int var, dim3 grid, const PassArgs& a, const float2* tw, cudaStream_t st);
 
 cudaError_t launch_pass_cfg_64(int cfg, int var, dim3 grid, const PassArgs& a, const TmaSet* maps, const float2* tw,
                                 cudaStream_t st);
@@ -62,12 +62,12 @@ cudaError_t launch_pass_cfg_1024(int cfg, int var, dim3 grid, const PassArgs& a,
 cudaError_t launch_pass_cfg_2048(int cfg, int var, dim3 grid, const PassArgs& a, const TmaSet* maps, const float2* tw,
                                 cudaStream_t st);
 
-cudaError_t launch_pass_half_64(int var, dim3 grid, const PassArgs& a, const TmaSet* maps, const void* tw, cudaStream_t st);
-cudaError_t launch_pass_half_128(int var, dim3 grid, const PassArgs& a, const TmaSet* maps, const void* tw, cudaStream_t st);
-cudaError_t launch_pass_half_256(int var, dim3 grid, const PassArgs& a, const TmaSet* maps, const void* tw, cudaStream_t st);
-cudaError_t launch_pass_half_512(int var, dim3 grid, const PassArgs& a, const TmaSet* maps, const void* tw, cudaStream_t st);
-cudaError_t launch_pass_half_1024(int var, dim3 grid, const PassArgs& a, const TmaSet* maps, const void* tw, cudaStream_t st);
-cudaError_t launch_pass_half_2048(int var, dim3 grid, const PassArgs& a, const TmaSet* maps, const void* tw, cudaStream_t st);
+cudaError_t launch_pass_half_64(int var, dim3 grid, const PassArgs& a, const void* tw, cudaStream_t st);
+cudaError_t launch_pass_half_128(int var, dim3 grid, const PassArgs& a, const void* tw, cudaStream_t st);
+cudaError_t launch_pass_half_256(int var, dim3 grid, const PassArgs& a, const void* tw, cudaStream_t st);
+cudaError_t launch_pass_half_512(int var, dim3 grid, const PassArgs& a, const void* tw, cudaStream_t st);
+cudaError_t launch_pass_half_1024(int var, dim3 grid, const PassArgs& a, const void* tw, cudaStream_t st);
+cudaError_t launch_pass_half_2048(int var, dim3 grid, const PassArgs& a, const void* tw, cudaStream_t st);
 
 // Per-layer phase windows (W x W, screen orientation) of global instance
 // gidx at the last completed step, scaled by the instance's Scoeff.

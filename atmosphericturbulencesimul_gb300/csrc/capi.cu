@@ -298,10 +298,10 @@ struct Class {
     // this class's science instances: entries [sci0, sci0 + nsci) of the
     // context's science list, their largest bin grid and crop
     int sci0 = 0, nsci = 0, maxnb = 0, maxnout = 0;
-    TmaSet maps[kNumTileCfg];  // per configuration: the box height is RR + 3
+    TmaSet maps;               // of the windows (box height win_rows + 3) or phase-only frames (phase_rows + 3)
     double tuned_ms[kNumTileCfg] = {};
     // windows of the groups whose side is this class's N (the class that
-    // owns the TMA maps of that size computes them), tile configuration 0
+    // owns the TMA maps of that size computes them)
     std::vector<WinJob> jobs;
     WinJob* d_jobs = nullptr;
     // layer sums of the same groups (those with a factoring Scoeff), and
@@ -530,10 +530,10 @@ atmwfs_status launch_windows(atmwfs_ctx* c, Class& cl, int j0, int j1, double* b
     a.poscap = c->poscap;
     a.jobs = cl.d_jobs + j0;
     a.pdl_ctas = step_pdl_ctas(c);
-    const int RR0 = tile_cfg(cl.N, 0).rr;
+    const int RR0 = win_rows(cl.N);
     // screen tiles in (RR0 + 3 rows of the padded width) and windows out
     if (bytes) *bytes = (4.0 * (RR0 + 3) / RR0 + 4.0) * (double)cl.N * cl.N * (j1 - j0);
-    AW_CUDA(pass_launcher_cfg(cl.N)(0, kVarWindows, dim3(cl.N / RR0, (unsigned)(j1 - j0)), a, &cl.maps[0], nullptr, st));
+    AW_CUDA(pass_launcher_cfg(cl.N)(0, kVarWindows, dim3(cl.N / RR0, (unsigned)(j1 - j0)), a, &cl.maps, nullptr, st));
     return ATMWFS_OK;
 }
 
@@ -560,7 +560,7 @@ atmwfs_status launch_phases(atmwfs_ctx* c, Class& cl, double* bytes, cudaStream_
         *bytes = 4.0 * (RR + 3) / RR * c->L * (double)cl.N * cl.N * cl.pjobs.size();
         for (int q : cl.pslots) *bytes += 8.0 * c->hinst[q].Nout * c->hinst[q].Nout;
     }
-    AW_CUDA(pass_launcher_cfg(cl.N)(0, kVarPhases, dim3(cl.N / RR, (unsigned)cl.pjobs.size()), a, &cl.maps[0], nullptr, st));
+    AW_CUDA(pass_launcher_cfg(cl.N)(0, kVarPhases, dim3(cl.N / RR, (unsigned)cl.pjobs.size()), a, &cl.maps, nullptr, st));
     return ATMWFS_OK;
 }
 
@@ -668,9 +668,9 @@ atmwfs_status launch_pass(atmwfs_ctx* c, int k, Class& cl, double* bytes, cudaSt
                 *bytes = b * cnt;
             }
             if (c->fp16 && var != kVarSingle)
-                AW_CUDA(pass_launcher_half(cl.N)(var, grid, a, &cl.maps[cl.cfg], twiddles_half(cl.N), st));
+                AW_CUDA(pass_launcher_half(cl.N)(var, grid, a, twiddles_half(cl.N), st));
             else
-                AW_CUDA(pass_launcher_cfg(cl.N)(cl.cfg, var, grid, a, &cl.maps[cl.cfg],
+                AW_CUDA(pass_launcher_cfg(cl.N)(cl.cfg, var, grid, a, nullptr,
                                                 twiddles(cl.N, tile_cfg(cl.N, cl.cfg).plan), st));
         }
     }
@@ -964,13 +964,11 @@ atmwfs_status commit(atmwfs_ctx* c)
     }
     AW_CUDA(cudaMemcpyAsync(c->d_inst, c->hinst.data(), sizeof(InstDev) * c->hinst.size(), cudaMemcpyHostToDevice, c->st));
     for (Class& cl : c->classes) {
-        memset(cl.maps, 0, sizeof cl.maps);
-        for (int g = 0; g < kNumTileCfg; g++)
-            for (int o = 0; o < 2; o++)
-                for (int l = 0; l < c->L; l++)
-                    if (c->d_pad[o][l] && tile_cfg(cl.N, g).rr > 0)
-                        AW_TRY(make_tma_map(&cl.maps[g].m[o][l], c->d_pad[o][l], c->Wp, c->Hp,
-                                            (c->amplitude ? tile_cfg(cl.N, g).rr : phase_rows(cl.N)) + 3));
+        memset(&cl.maps, 0, sizeof cl.maps);
+        const int rows = (c->amplitude ? win_rows(cl.N) : phase_rows(cl.N)) + 3;
+        for (int o = 0; o < 2; o++)
+            for (int l = 0; l < c->L; l++)
+                if (c->d_pad[o][l]) AW_TRY(make_tma_map(&cl.maps.m[o][l], c->d_pad[o][l], c->Wp, c->Hp, rows));
     }
     AW_CUDA(cudaStreamSynchronize(c->st));
     AW_TRY(autotune(c));
@@ -1699,11 +1697,11 @@ static atmwfs_status two_pass(const void* in, void* out, long n, int var, const 
     a.H2 = H;
     a.ext_in = (const float2*)in;
     a.ext_out = tmp;
-    cudaError_t e = fn(var, dim3((unsigned)(n / RR), 1), a, nullptr, tw, st);
+    cudaError_t e = fn(var, dim3((unsigned)(n / RR), 1), a, tw, st);
     if (e == cudaSuccess) {
         a.ext_in = tmp;
         a.ext_out = (float2*)out;
-        e = fn(var, dim3((unsigned)(n / RR), 1), a, nullptr, tw, st);
+        e = fn(var, dim3((unsigned)(n / RR), 1), a, tw, st);
     }
     cudaFreeAsync(tmp, st);
     AW_CUDA(e);

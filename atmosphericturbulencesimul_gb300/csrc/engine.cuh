@@ -222,9 +222,9 @@ constexpr int kPadY = 1;
 constexpr int kBoxW = 32;  // TMA box width (floats)
 
 // Host-side launch entry of one row pass for grid size N (defined per N).
-typedef cudaError_t (*PassLauncher)(int var, dim3 grid, const PassArgs& a, const TmaSet* maps,
-                                    const float2* tw, cudaStream_t st);
-// Same, for tile configuration `cfg` (see tile_cfg).
+typedef cudaError_t (*PassLauncher)(int var, dim3 grid, const PassArgs& a, const float2* tw, cudaStream_t st);
+// Same, for tile configuration `cfg` (see tile_cfg); maps: the screens'
+// tensor maps (window kernel and phase-only frames only).
 typedef cudaError_t (*PassLauncherCfg)(int cfg, int var, dim3 grid, const PassArgs& a, const TmaSet* maps,
                                        const float2* tw, cudaStream_t st);
 
@@ -264,11 +264,14 @@ constexpr TileCfg tile_cfg(int N, int c)
                       : TileCfg{0, 0, false, 0, false};
 }
 
-// Phase-only frames: rows per CTA and threads.  Eight rows cost 11 / 8 of the
-// horizontal sums and leave four CTAs per SM at 512; 2048 takes four so that
-// two tiles fit the shared memory.
+// Window kernel and phase-only frames: rows per CTA and threads (four columns
+// each; a warp at least).  Eight rows cost 11 / 8 of the horizontal sums.  At
+// 2048 the phase-only frames take four, so that their two tiles leave room for
+// a second CTA per SM.
+constexpr int win_rows(int) { return 8; }
+constexpr int win_threads(int N) { return N < 128 ? 32 : N / 4; }
 constexpr int phase_rows(int N) { return N <= 1024 ? 8 : 4; }
-constexpr int phase_threads(int N) { return N < 256 ? N : 256; }
+constexpr int phase_threads(int N) { return N < 128 ? 32 : N < 1024 ? N / 4 : 256; }
 
 // Threads of a phase-sum CTA and CTAs per instance of its launch.
 constexpr int kPhasumThreads = 256;
@@ -298,8 +301,7 @@ constexpr int kUnitPdlWaves = 8;
 PassLauncher pass_launcher(int N);
 PassLauncherCfg pass_launcher_cfg(int N);
 // FP16-transform series passes (tile configuration 2); tw = FP16 twiddles
-typedef cudaError_t (*PassLauncherHalf)(int var, dim3 grid, const PassArgs& a, const TmaSet* maps, const void* tw,
-                                        cudaStream_t st);
+typedef cudaError_t (*PassLauncherHalf)(int var, dim3 grid, const PassArgs& a, const void* tw, cudaStream_t st);
 PassLauncherHalf pass_launcher_half(int N);
 
 }  // namespace atmwfs

@@ -157,11 +157,11 @@ extern "C" atmwfs_status atmwfs_fresnel_noalloc(const void* in, void* out, long 
     a.ext_in = (const float2*)in;
     a.ext_out = s->field;
     const dim3 grid((unsigned)(n / unit_rows((int)n)), 1);
-    e = fn(kVarUnitProp, grid, a, nullptr, s->twiddle, cs);
+    e = fn(kVarUnitProp, grid, a, s->twiddle, cs);
     if (e == cudaSuccess) {
         a.ext_in = s->field;
         a.ext_out = (float2*)out;
-        e = fn(kVarUnitProp, grid, a, nullptr, s->twiddle, cs);
+        e = fn(kVarUnitProp, grid, a, s->twiddle, cs);
     }
     if (e != cudaSuccess) return err(ATMWFS_ERR_CUDA, cudaGetErrorString(e));
     return ATMWFS_OK;

@@ -346,7 +346,7 @@ __device__ __forceinline__ void two_sum(float a, float b, float& s, float& e)
 
 template <int N, int RR, int MINB, int OPS, bool ALIAS, bool HP = false, int V = 0, bool HS = false>
 __global__ void __launch_bounds__(Plan<N, V>::T* RR, MINB)
-    k_pass(const __grid_constant__ PassArgs a, const __grid_constant__ TmaSet maps, const float2* __restrict__ tw)
+    k_pass(const __grid_constant__ PassArgs a, const float2* __restrict__ tw)
 {
     using G = PassGeom<N, RR, V>;
     static_assert(!HP || V == 0, "FP16 transforms use the default plan");
@@ -652,12 +652,10 @@ __global__ void __launch_bounds__(Plan<N, V>::T* RR, MINB)
 // instance of a group (the wavelengths of one direction) then reads the same
 // samples instead of interpolating the screen itself.
 // ---------------------------------------------------------------------------
-template <int N, int RR>
-__global__ void __launch_bounds__(PassGeom<N, RR>::NT)
+template <int N, int RR, int NT>
+__global__ void __launch_bounds__(NT)
     k_layer_windows(const __grid_constant__ PassArgs a, const __grid_constant__ TmaSet maps)
 {
-    using G = PassGeom<N, RR>;
-    constexpr int NT = G::NT;
     extern __shared__ __align__(1024) unsigned char sm[];
     float* tile = reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(sm) + 127) & ~uintptr_t(127));
     __shared__ __align__(8) uint64_t bar;
@@ -672,9 +670,15 @@ __global__ void __launch_bounds__(PassGeom<N, RR>::NT)
     __syncthreads();
     tma_issue_layer<N, RR>(maps, J.orient, J.layer, g, tile, &bar, tid, NT);
     if (!cta_wait_tile(&bar, 0, a.d_status)) return;
-    float* out = J.out + (size_t)y0 * J.stride;
+    float* out = J.out + (size_t)y0 * J.stride;  // rows of the group's side: multiples of 16 bytes
     const int stride = J.stride;
-    gather_tile<N, RR, NT>(tile, g, 1.0f, tid, [=](int r, int x, float val) { out[(size_t)r * stride + x] = val; });
+    float wx[4], wy[4];
+    keys_weights(g.fx, wx);
+    keys_weights(g.fy, wy);
+    for (int x = 4 * tid; x < N; x += 4 * NT)
+        gather_quad<RR>(tile, g, wx, wy, x, [&](int r, float v0, float v1, float v2, float v3) {
+            *reinterpret_cast<float4*>(out + (size_t)r * stride + x) = make_float4(v0, v1, v2, v3);
+        });
 }
 
 // ---------------------------------------------------------------------------
@@ -686,15 +690,15 @@ __global__ void __launch_bounds__(PassGeom<N, RR>::NT)
 // the two-sum of every pixel there and writes the frames of the group's
 // instances.  The same samples and sums as k_layer_windows + k_group_sum (or
 // k_phasum where Scoeff depends on the layer) and an output pass, bit for bit.
-// Issue bounds it: about 18 instructions per pixel and layer.  16 directions
+// Issue bounds it: about 16 instructions per pixel and layer.  16 directions
 // of 512^2 through 10 layers: windows 60 + sums 45 + output pass 46 us before.
 // ---------------------------------------------------------------------------
 template <int N, int RR, int NT>
 __global__ void __launch_bounds__(NT) k_phase_frames(const __grid_constant__ PassArgs a, const __grid_constant__ TmaSet maps)
 {
     using G = PassGeom<N, RR>;
-    constexpr int CPT = N / NT;  // columns per thread
-    static_assert(N % NT == 0, "whole columns");
+    constexpr int QPT = N < 4 * NT ? 1 : N / (4 * NT);  // quads of columns per thread
+    static_assert(N % (4 * NT) == 0 || N < 4 * NT, "whole quads");
     extern __shared__ __align__(1024) unsigned char sm[];
     float* tiles = reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(sm) + 127) & ~uintptr_t(127));
     constexpr int TILE = (int)(G::TILE_BYTES / 4);
@@ -716,11 +720,13 @@ __global__ void __launch_bounds__(NT) k_phase_frames(const __grid_constant__ Pas
     issue(0);
     if (L > 1) issue(1);
     const InstDev* I0 = a.inst + a.pslots[J.first];
-    float hi[CPT][RR], lo[CPT][RR];
+    float hi[QPT][RR][4], lo[QPT][RR][4];
 #pragma unroll
-    for (int q = 0; q < CPT; q++)
+    for (int q = 0; q < QPT; q++)
 #pragma unroll
-        for (int r = 0; r < RR; r++) hi[q][r] = lo[q][r] = 0.0f;
+        for (int r = 0; r < RR; r++)
+#pragma unroll
+            for (int k = 0; k < 4; k++) hi[q][r][k] = lo[q][r][k] = 0.0f;
 #pragma unroll 1
     for (int i = 0; i < L; i++) {
         if (!cta_wait_tile(&bar[i & 1], (i >> 1) & 1, a.d_status)) {
@@ -735,13 +741,20 @@ __global__ void __launch_bounds__(NT) k_phase_frames(const __grid_constant__ Pas
         keys_weights(g.fy, wy);
         const float* tile = tiles + (i & 1) * TILE;
 #pragma unroll
-        for (int q = 0; q < CPT; q++)
-            gather_column<RR>(tile, g, wx, wy, tid + q * NT, [&](int r, float val) {
-                float s, e;
-                two_sum(hi[q][r], __fmul_rn(val, sc), s, e);
-                hi[q][r] = s;
-                lo[q][r] = __fadd_rn(lo[q][r], e);
+        for (int q = 0; q < QPT; q++) {
+            const int x = 4 * (tid + q * NT);
+            if (x >= N) break;
+            gather_quad<RR>(tile, g, wx, wy, x, [&](int r, float v0, float v1, float v2, float v3) {
+                const float v[4] = {v0, v1, v2, v3};
+#pragma unroll
+                for (int k = 0; k < 4; k++) {
+                    float s, e;
+                    two_sum(hi[q][r][k], __fmul_rn(v[k], sc), s, e);
+                    hi[q][r][k] = s;
+                    lo[q][r][k] = __fadd_rn(lo[q][r][k], e);
+                }
             });
+        }
         __syncthreads();  // every thread has read the tile
         if (i + 2 < L) issue(i + 2);
     }
@@ -752,17 +765,32 @@ __global__ void __launch_bounds__(NT) k_phase_frames(const __grid_constant__ Pas
         float* __restrict__ opha = I->out_pha + slot;
         float* __restrict__ oamp = I->out_amp + slot;
         const float sg = I->scoeff[0];
+        const bool v4 = (off % 4) == 0 && (Nout % 4) == 0 && (reinterpret_cast<uintptr_t>(opha) & 15) == 0 &&
+                        (reinterpret_cast<uintptr_t>(oamp) & 15) == 0;
 #pragma unroll
         for (int r = 0; r < RR; r++) {
             const int y = y0 + r - off;
             if (y < 0 || y >= Nout) continue;
 #pragma unroll
-            for (int q = 0; q < CPT; q++) {
-                const int x = tid + q * NT - off;
-                if (x < 0 || x >= Nout) continue;
+            for (int q = 0; q < QPT; q++) {
+                const int x = 4 * (tid + q * NT) - off;
+                float p[4];
+#pragma unroll
+                for (int k = 0; k < 4; k++)
+                    p[k] = J.factored ? fmaf(sg, hi[q][r][k], sg * lo[q][r][k]) : __fadd_rn(hi[q][r][k], lo[q][r][k]);
                 const size_t o = (size_t)y * Nout + x;
-                opha[o] = J.factored ? fmaf(sg, hi[q][r], sg * lo[q][r]) : __fadd_rn(hi[q][r], lo[q][r]);
-                oamp[o] = 1.0f;
+                if (v4) {  // off and Nout multiples of 4: a quad is inside the crop or outside
+                    if (x < 0 || x >= Nout) continue;
+                    *reinterpret_cast<float4*>(opha + o) = make_float4(p[0], p[1], p[2], p[3]);
+                    *reinterpret_cast<float4*>(oamp + o) = make_float4(1.0f, 1.0f, 1.0f, 1.0f);
+                } else {
+#pragma unroll
+                    for (int k = 0; k < 4; k++) {
+                        if (x + k < 0 || x + k >= Nout) continue;
+                        opha[o + k] = p[k];
+                        oamp[o + k] = 1.0f;
+                    }
+                }
             }
         }
     }
@@ -838,8 +866,6 @@ template <int N, int RR, int MINB, bool ALIAS, bool HP = false, int V = 0, bool 
 cudaError_t launch_pass_t(int var, dim3 grid, const PassArgs& a, const TmaSet* maps, const float2* tw, cudaStream_t st)
 {
     using G = PassGeom<N, RR, V>;
-    static TmaSet empty_maps;  // unit passes gather nothing
-    const TmaSet& m = maps ? *maps : empty_maps;
     dim3 block(G::NT);
 #define AW_CASE(VAR)                                                                                   \
     case VAR: {                                                                                        \
@@ -850,7 +876,7 @@ cudaError_t launch_pass_t(int var, dim3 grid, const PassArgs& a, const TmaSet* m
             if (e != cudaSuccess) return e;                                                            \
             attr = true;                                                                               \
         }                                                                                              \
-        return launch_gated_up_to(I_SERIES(VAR) ? a.pdl_ctas : kUnitPdlWaves * pdl_max_ctas(), k_pass<N, RR, MINB, VAR, ALIAS, HP, V, HS>, grid, block, sm, st, a, m, tw); \
+        return launch_gated_up_to(I_SERIES(VAR) ? a.pdl_ctas : kUnitPdlWaves * pdl_max_ctas(), k_pass<N, RR, MINB, VAR, ALIAS, HP, V, HS>, grid, block, sm, st, a, tw); \
     }
     if constexpr (UNIT) {
         switch (var) {
@@ -879,14 +905,15 @@ cudaError_t launch_pass_t(int var, dim3 grid, const PassArgs& a, const TmaSet* m
             return launch_gated_up_to(a.pdl_ctas, k_phasum<N>, grid, dim3(kPhasumThreads), 0, st, a);
         }
         case kVarWindows: {
-            constexpr size_t sm = G::TILE_BYTES + 128;
+            constexpr int WR = win_rows(N), WT = win_threads(N);
+            constexpr size_t sm = PassGeom<N, WR>::TILE_BYTES + 128;
             static bool attr = false;
             if (!attr) {
-                cudaError_t e = cudaFuncSetAttribute(k_layer_windows<N, RR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+                cudaError_t e = cudaFuncSetAttribute(k_layer_windows<N, WR, WT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
                 if (e != cudaSuccess) return e;
                 attr = true;
             }
-            return launch_gated_up_to(a.pdl_ctas, k_layer_windows<N, RR>, grid, dim3(G::NT), sm, st, a, m);
+            return launch_gated_up_to(a.pdl_ctas, k_layer_windows<N, WR, WT>, grid, dim3(WT), sm, st, a, *maps);
         }
         case kVarPhases: {
             constexpr int PR = phase_rows(N), PT = phase_threads(N);
@@ -897,7 +924,7 @@ cudaError_t launch_pass_t(int var, dim3 grid, const PassArgs& a, const TmaSet* m
                 if (e != cudaSuccess) return e;
                 attr = true;
             }
-            return launch_gated_up_to(a.pdl_ctas, k_phase_frames<N, PR, PT>, grid, dim3(PT), sm, st, a, m);
+            return launch_gated_up_to(a.pdl_ctas, k_phase_frames<N, PR, PT>, grid, dim3(PT), sm, st, a, *maps);
         }
         default: return cudaErrorInvalidValue;
     }
@@ -906,17 +933,17 @@ cudaError_t launch_pass_t(int var, dim3 grid, const PassArgs& a, const TmaSet* m
 }
 
 template <int N>
-cudaError_t launch_pass_n(int var, dim3 grid, const PassArgs& a, const TmaSet* maps, const float2* tw, cudaStream_t st)
+cudaError_t launch_pass_n(int var, dim3 grid, const PassArgs& a, const float2* tw, cudaStream_t st)
 {
-    return launch_pass_t<N, unit_rows(N), 1, false, false, 0, false, false, true>(var, grid, a, maps, tw, st);
+    return launch_pass_t<N, unit_rows(N), 1, false, false, 0, false, false, true>(var, grid, a, nullptr, tw, st);
 }
 
 // FP16-transform passes: tile configuration 2, tw = the FP16 twiddle table
 template <int N>
-cudaError_t launch_pass_hn(int var, dim3 grid, const PassArgs& a, const TmaSet* maps, const void* tw, cudaStream_t st)
+cudaError_t launch_pass_hn(int var, dim3 grid, const PassArgs& a, const void* tw, cudaStream_t st)
 {
     constexpr TileCfg c2 = tile_cfg(N, 2);
-    return launch_pass_t<N, c2.rr, c2.minb, c2.alias, true>(var, grid, a, maps, reinterpret_cast<const float2*>(tw), st);
+    return launch_pass_t<N, c2.rr, c2.minb, c2.alias, true>(var, grid, a, nullptr, reinterpret_cast<const float2*>(tw), st);
 }
 
 template <int N>
