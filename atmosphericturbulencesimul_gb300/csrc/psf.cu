@@ -17,6 +17,7 @@
 // frame (amplitude + phase) read, 2 x 16 W^2 B of intermediate written and
 // read, and 8 (2W)^2 / batch B of accumulator update.
 #include <algorithm>
+#include <cfloat>
 #include <cmath>
 #include <cstdio>
 #include <vector>
@@ -24,13 +25,16 @@
 #include "atmwfs_psf.h"
 #include "aux_kernels.cuh"
 #include "pass_impl.cuh"
+#include "atan_ff.cuh"
 
 namespace atmwfs {
 
 void set_error_message(const char* msg);
 
-// rows per CTA: 128 threads per CTA at every size
-template <int N> struct PsfRows { static constexpr int RR = N <= 128 ? 16 : N <= 512 ? 8 : N == 1024 ? 4 : 2; };
+// Rows per CTA of the row pass: 128 threads below 1024, 256 from there, so that
+// the transposed store writes runs of at least 32 bytes at every size (1024:
+// eight rows 205 us per 64-frame exposure of 512^2 against 213 with four).
+template <int N> struct PsfRows { static constexpr int RR = N <= 128 ? 16 : N <= 1024 ? 8 : 4; };
 
 // Row pass.  Field b: rows and columns [0, W) hold amp * exp(i c_b pha), the
 // rest is zero (PAD: W = N / 2, else W = N).  The reference places an exposure
@@ -38,13 +42,14 @@ template <int N> struct PsfRows { static constexpr int RR = N <= 128 ? 16 : N <=
 // which |F|^2 is kept, and at offset 0 a thread's values are all frame or all
 // padding.  Writes G[b][kx][y], y < W.
 template <int N, bool PAD>
-__global__ void __launch_bounds__(Plan<N>::T * PsfRows<N>::RR)
+__global__ void __launch_bounds__(Plan<N>::T * PsfRows<N>::RR, N >= 1024 ? 2 : 1)
 k_psf_rows(const float* __restrict__ amp, long amp_fstride, const float* __restrict__ pha, long pha_fstride,
            const float* __restrict__ cscale, float2* __restrict__ G, const float2* __restrict__ tw)
 {
     constexpr int RR = PsfRows<N>::RR, T = Plan<N>::T, E = Plan<N>::E, NT = T * RR, RS = row_stride<N>();
     constexpr int RL = last_radix<N>(), W = PAD ? N / 2 : N;
-    __shared__ __align__(16) float2 xb[RR * RS];
+    extern __shared__ __align__(16) float2 psf_smem[];
+    float2* xb = psf_smem;  // [RR][RS]
     const int tid = threadIdx.x, t = tid % T, rr = tid / T;
     const int b = blockIdx.y;
     const int yb = blockIdx.x * RR + rr;
@@ -79,14 +84,15 @@ k_psf_rows(const float* __restrict__ amp, long amp_fstride, const float* __restr
 
 // Column pass over the B fields of G: one column per CTA, the fields spread
 // over F frame lanes of the CTA (lane f takes fields f, f + F, ...), so that
-// a batch of fields keeps F transforms of the column in flight per CTA (a
-// column per CTA with the fields in sequence left a 1024-column transform
-// with 1.7 CTAs of four warps per SM).  PAD (exposure): acc[kx][ky] +=
+// a batch of fields keeps F transforms of the column in flight per CTA: there
+// are only N CTAs, so the smaller the transform the more lanes (200 frames of
+// 128^2: 16 lanes 77 us against 93 with four; 1024-point columns gain nothing
+// from more than four).  PAD (exposure): acc[kx][ky] +=
 // |F_b[ky][kx]|^2 for b = 0..B-1: each lane sums its fields in order, then
 // the lanes' partial sums are added to the accumulator in lane order (the
 // accumulator is kept transposed and uncentred so that these updates are
 // coalesced).  Else (chromatic): I[b][kx][ky] = |F_b[ky][kx]|^2.
-template <int N> struct PsfLanes { static constexpr int F = Plan<N>::T >= 64 ? 2 : 4; };
+template <int N> struct PsfLanes { static constexpr int F = N <= 256 ? 16 : N == 512 ? 8 : N == 1024 ? 4 : 2; };
 
 template <int N, bool PAD>
 __global__ void __launch_bounds__(Plan<N>::T * PsfLanes<N>::F, 4)
@@ -161,36 +167,73 @@ __global__ void k_expo_layout(const float* __restrict__ src, float* __restrict__
 // weights follow the reference's double and float expressions, and the
 // accumulation is in float.  I_s is centred on read: I(j, i) =
 // I_s[(i + h) % n][(j + h) % n].
-__global__ void k_chromat_sum(const float* __restrict__ I, int S, int n, const float* __restrict__ coeff,
-                              const float* __restrict__ mcoeff, float* __restrict__ out)
+//
+// The reference's double expressions, (1 - u)(1 - t) v00 and two more, each
+// rounded to float, are evaluated in float-float: 1 - u as an exact pair, the
+// products as exact two-products, one rounding at the end -- the float of the
+// double expression except when that lies within about 2^-46 of a midpoint.
+// In doubles the FP64 pipe bounded the sum, and with the lanes along ii every
+// tap was a gather over 32 rows of I_s (lanes now run along jj): 365 us for 40
+// steps of 512^2.
+__device__ __forceinline__ void ff_mul_f(float ah, float al, float b, float& h, float& l)
 {
-    const long np = (long)n * n;
-    const int h = n / 2;
-    for (long p = blockIdx.x * (long)blockDim.x + threadIdx.x; p < np; p += (long)gridDim.x * blockDim.x) {
-        const int ii = (int)(p % n), jj = (int)(p / n);
-        float acc = out[p];
-        for (int s = 0; s < S; s++) {
-            const float c = coeff[s];
-            const float x = fmaf((float)(ii - h), c, (float)h);
-            const float y = fmaf((float)(jj - h), c, (float)h);
-            const int i = (int)x, j = (int)y;
+    h = ff_mul(ah, b);
+    l = ff_fma(ah, b, -h);
+    l = ff_fma(al, b, l);
+}
+
+// (ah + al) (bh + bl) v as a pair: the weight is exact to 2^-48, v a float.  An
+// infinite or undefined product keeps its value (its error term has none).
+__device__ __forceinline__ void tap(float ah, float al, float bh, float bl, float v, float& h, float& l)
+{
+    float wh = ff_mul(ah, bh);
+    float wl = ff_fma(ah, bh, -wh);
+    wl = ff_fma(ah, bl, ff_fma(al, bh, wl));
+    ff_mul_f(wh, wl, v, h, l);
+    if (!(fabsf(h) <= FLT_MAX)) l = 0.0f;
+}
+
+// float(t + (h + l))
+__device__ __forceinline__ float add_pair(float t, float h, float l)
+{
+    float s, e;
+    ff_two_sum(t, h, s, e);
+    return fabsf(s) <= FLT_MAX ? ff_add(s, ff_add(e, l)) : s;
+}
+
+__global__ void __launch_bounds__(256) k_chromat_sum(const float* __restrict__ I, int S, int n, const float* __restrict__ coeff,
+                                                     const float* __restrict__ mcoeff, float* __restrict__ out)
+{
+    // a CTA covers 32 jj (lanes) x 8 ii; n is a power of two >= 64
+    const int h = n / 2, mk = n - 1;
+    const int jj = blockIdx.x * 32 + threadIdx.x % 32, ii = blockIdx.y * 8 + threadIdx.x / 32;
+    const size_t np = (size_t)n * n, p = (size_t)jj * n + ii;
+    float acc = out[p];
+    for (int s = 0; s < S; s++) {
+        const float c = coeff[s];
+        const float x = fmaf((float)(ii - h), c, (float)h);
+        const float y = fmaf((float)(jj - h), c, (float)h);
+        const int i = (int)x, j = (int)y;
+        if (i < n - 1 && j < n - 1 && i > -1 && j > -1) {
             const float u = x - (float)i, t = y - (float)j;
-            if (i < n - 1 && j < n - 1 && i > -1 && j > -1) {
-                const float* Is = I + (size_t)s * np;
-                const float v00 = Is[(size_t)((i + h) % n) * n + (j + h) % n];
-                const float v01 = Is[(size_t)((i + h) % n) * n + (j + 1 + h) % n];
-                const float v10 = Is[(size_t)((i + 1 + h) % n) * n + (j + h) % n];
-                const float v11 = Is[(size_t)((i + 1 + h) % n) * n + (j + 1 + h) % n];
-                const double du = 1.0 - (double)u, dt = 1.0 - (double)t;
-                float tmp = (float)(du * dt * (double)v00);
-                tmp = (float)((double)tmp + du * (double)t * (double)v01);
-                tmp = (float)((double)tmp + (double)u * dt * (double)v10);
-                tmp = __fadd_rn(tmp, __fmul_rn(__fmul_rn(u, t), v11));   // u * t * F: float arithmetic
-                acc = __fadd_rn(acc, __fdiv_rn(__fdiv_rn(__fmul_rn(mcoeff[s], tmp), c), c));
-            }
+            const float* r0 = I + (size_t)s * np + (size_t)((i + h) & mk) * n;
+            const float* r1 = I + (size_t)s * np + (size_t)((i + 1 + h) & mk) * n;
+            const int j0 = (j + h) & mk, j1 = (j + 1 + h) & mk;
+            const float v00 = r0[j0], v01 = r0[j1], v10 = r1[j0], v11 = r1[j1];
+            float duh, dul, dth, dtl, a, b;
+            ff_two_sum(1.0f, -u, duh, dul);
+            ff_two_sum(1.0f, -t, dth, dtl);
+            tap(duh, dul, dth, dtl, v00, a, b);
+            float tmp = ff_add(a, b);
+            tap(duh, dul, t, 0.0f, v01, a, b);
+            tmp = add_pair(tmp, a, b);
+            tap(u, 0.0f, dth, dtl, v10, a, b);
+            tmp = add_pair(tmp, a, b);
+            tmp = __fadd_rn(tmp, __fmul_rn(__fmul_rn(u, t), v11));   // u * t * F: float arithmetic
+            acc = __fadd_rn(acc, __fdiv_rn(__fdiv_rn(__fmul_rn(mcoeff[s], tmp), c), c));
         }
-        out[p] = acc;
     }
+    out[p] = acc;
 }
 
 template <int N, bool PAD>
@@ -199,7 +242,12 @@ static cudaError_t psf_rows_n(const float* amp, long as, const float* pha, long 
 {
     constexpr int RR = PsfRows<N>::RR, W = PAD ? N / 2 : N;
     static_assert(W % RR == 0, "whole CTAs of rows");
-    k_psf_rows<N, PAD><<<dim3((unsigned)(W / RR), (unsigned)B), Plan<N>::T * RR, 0, st>>>(amp, as, pha, ps, cs, G, tw);
+    constexpr int sm = RR * row_stride<N>() * (int)sizeof(float2);
+    if (sm > 48 * 1024) {
+        const cudaError_t e = cudaFuncSetAttribute(k_psf_rows<N, PAD>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+        if (e != cudaSuccess) return e;
+    }
+    k_psf_rows<N, PAD><<<dim3((unsigned)(W / RR), (unsigned)B), Plan<N>::T * RR, sm, st>>>(amp, as, pha, ps, cs, G, tw);
     return cudaGetLastError();
 }
 
@@ -242,7 +290,7 @@ cudaError_t psf_cols(int N, const float2* G, int B, float* out, const float2* tw
 cudaError_t chromat_sum(const float* I, int S, int n, const float* coeff, const float* mcoeff, float* out,
                         cudaStream_t st)
 {
-    k_chromat_sum<<<4 * 152, 256, 0, st>>>(I, S, n, coeff, mcoeff, out);
+    k_chromat_sum<<<dim3((unsigned)(n / 32), (unsigned)(n / 8)), 256, 0, st>>>(I, S, n, coeff, mcoeff, out);
     return cudaGetLastError();
 }
 
@@ -273,9 +321,11 @@ atmwfs_status psf_cuda(cudaError_t e, const char* what)
 bool pow2_between(long n, long lo, long hi) { return n >= lo && n <= hi && (n & (n - 1)) == 0; }
 
 // Fields per launch, 1..64: a batch's intermediate (N x W complex values per
-// field) is written by the row pass and read by the column pass.
-long psf_mb() { const char* e = getenv("PSF_MB"); return e ? atol(e) : 64; }
-long psf_batch(long N, long W) { return std::max(1L, std::min(64L, (psf_mb() << 20) / (N * W * 8))); }
+// field) is written by the row pass and read by the column pass.  About 256
+// MB: a batch that stayed in L2 (64 MB) wins back less in the row pass than the
+// column pass loses with fewer fields per CTA (64 frames of 512^2: 242 against
+// 199 us).
+long psf_batch(long N, long W) { return std::max(1L, std::min(64L, (256L << 20) / (N * W * 8))); }
 
 // Step coefficients and weights with the reference's types (psf.c:86-99):
 // float coeff, x and mcoeff from double expressions.
