@@ -19,6 +19,7 @@
 #include "atmwfs.h"
 #include "aux_kernels.cuh"
 #include "atan_ff.cuh"
+#include "workspace.cuh"
 
 namespace atmwfs {
 
@@ -370,6 +371,7 @@ struct atmwfs_ctx {
     float* d_out_amp = nullptr;
     int* d_step = nullptr;
     unsigned* d_status = nullptr;
+    unsigned* h_status = nullptr;        // pinned: where check_status reads it
     int* d_iters = nullptr;
     int* d_sci = nullptr;
     float2* d_atan_tab = nullptr;  // atan(k / 1024) pairs of the science unwrap
@@ -1002,9 +1004,9 @@ atmwfs_status commit(atmwfs_ctx* c)
 
 atmwfs_status check_status(atmwfs_ctx* c)
 {
-    unsigned st = 0;
-    AW_CUDA(cudaMemcpyAsync(&st, c->d_status, sizeof st, cudaMemcpyDeviceToHost, c->st));
+    AW_CUDA(cudaMemcpyAsync(c->h_status, c->d_status, sizeof(unsigned), cudaMemcpyDeviceToHost, c->st));
     AW_CUDA(cudaStreamSynchronize(c->st));
+    const unsigned st = *c->h_status;
     if (st & kStatTmaTimeout) return fail(ATMWFS_ERR_TIMEOUT, "a screen tile load did not complete within 1 s");
     if (st) return fail(ATMWFS_ERR_CUDA, "device status 0x%x", st);
     return ATMWFS_OK;
@@ -1225,6 +1227,7 @@ atmwfs_status atmwfs_create(const atmwfs_params* p, atmwfs_ctx** out)
         CKC(cudaMemset(c->d_step, 0, sizeof(int)));
         CK(dalloc(c, (void**)&c->d_status, sizeof(unsigned)));
         CKC(cudaMemset(c->d_status, 0, sizeof(unsigned)));
+        CKC(cudaHostAlloc((void**)&c->h_status, sizeof(unsigned), cudaHostAllocDefault));
         CK(dalloc(c, (void**)&c->d_iters, sizeof(int) * c->ninst * 0 + sizeof(int) * (c->hinst.size() + 1)));
         const size_t posn = (size_t)c->poscap * c->ninst * c->L;
         CK(dalloc(c, (void**)&c->d_pos, sizeof(LayerPos) * posn));
@@ -1283,7 +1286,9 @@ void atmwfs_destroy(atmwfs_ctx* c)
     for (auto e : c->ev_copied)
         if (e) cudaEventDestroy(e);
     if (c->st) cudaStreamDestroy(c->st);
+    if (c->h_status) cudaFreeHost(c->h_status);
     delete c;
+    workspace_release();
 }
 
 static atmwfs_status load_common(atmwfs_ctx* c, int layer, const float* src, long M, cudaMemcpyKind kind)
@@ -1396,7 +1401,10 @@ atmwfs_status atmwfs_run(atmwfs_ctx* c, long nsteps, const atmwfs_sink* sink)
     AW_TRY(commit(c));
     const size_t per = (size_t)c->ninst * c->L;
     const bool copies = sink && (sink->pha || sink->amp);
-    if (copies && !c->out_st) {
+    // with one ring slot the copy and the next step take turns anyway: it goes
+    // on the step's own stream, without the events between two
+    const bool inline_copy = copies && c->ring == 1;
+    if (copies && !inline_copy && !c->out_st) {
         // the copy stream has the highest priority: its few CTAs take the
         // next free SM slots ahead of the queued pass and phase-sum CTAs, so a
         // step's frames leave while the next step computes
@@ -1459,34 +1467,37 @@ atmwfs_status atmwfs_run(atmwfs_ctx* c, long nsteps, const atmwfs_sink* sink)
             const long slot = (g0 + i) % c->ring;
             // the slot is free once its previous copy is done (a no-op for a
             // slot never copied); with ring >= 2 this copy overlaps the next step
-            if (copies) AW_CUDA(cudaStreamWaitEvent(c->st, c->ev_copied[slot], 0));
+            if (copies && !inline_copy) AW_CUDA(cudaStreamWaitEvent(c->st, c->ev_copied[slot], 0));
             AW_CUDA(cudaGraphLaunch(c->gexec, c->st));
             if (copies) {
-                AW_CUDA(cudaEventRecord(c->ev_written[slot], c->st));
-                AW_CUDA(cudaStreamWaitEvent(c->out_st, c->ev_written[slot], 0));
+                const cudaStream_t cst = inline_copy ? c->st : c->out_st;
+                if (!inline_copy) {
+                    AW_CUDA(cudaEventRecord(c->ev_written[slot], c->st));
+                    AW_CUDA(cudaStreamWaitEvent(c->out_st, c->ev_written[slot], 0));
+                }
                 const long hs = sink->nslots > 0 ? (s + i) % sink->nslots : (s + i);
                 const size_t ff = c->frame_floats;
                 if (by_kernel) {
                     auto f4 = [](const float* q) { return reinterpret_cast<const float4*>(q); };
                     auto h4 = [&](float* q) { return q ? reinterpret_cast<float4*>(q + (size_t)hs * ff) : nullptr; };
                     AW_CUDA(copy_out(f4(c->d_out_pha + slot * ff), h4(dev_sink[0]), (long)(ff / 4),
-                                     f4(c->d_out_amp + slot * ff), h4(dev_sink[1]), (long)(ff / 4), device_sink, c->out_st));
+                                     f4(c->d_out_amp + slot * ff), h4(dev_sink[1]), (long)(ff / 4), device_sink, cst));
                 } else {
                     if (sink->pha)
                         AW_CUDA(cudaMemcpyAsync(sink->pha + (size_t)hs * ff, c->d_out_pha + slot * ff, sizeof(float) * ff,
-                                                cudaMemcpyDefault, c->out_st));
+                                                cudaMemcpyDefault, cst));
                     if (sink->amp)
                         AW_CUDA(cudaMemcpyAsync(sink->amp + (size_t)hs * ff, c->d_out_amp + slot * ff, sizeof(float) * ff,
-                                                cudaMemcpyDefault, c->out_st));
+                                                cudaMemcpyDefault, cst));
                 }
-                AW_CUDA(cudaEventRecord(c->ev_copied[slot], c->out_st));
+                if (!inline_copy) AW_CUDA(cudaEventRecord(c->ev_copied[slot], c->out_st));
             }
         }
         s += chunk;
         b ^= 1;
     }
     // the caller's buffers hold every frame on return
-    if (copies) AW_CUDA(cudaStreamSynchronize(c->out_st));
+    if (copies && !inline_copy) AW_CUDA(cudaStreamSynchronize(c->out_st));
     return check_status(c);
 }
 
@@ -1688,8 +1699,9 @@ static atmwfs_status two_pass(const void* in, void* out, long n, int var, const 
     if (!fn) return fail(ATMWFS_ERR_INVALID, "size %ld unsupported (power of two 64..2048)", n);
     const float2* tw = twiddles((int)n);
     if (!tw) return fail(ATMWFS_ERR_NOMEM, "twiddle allocation failed");
-    float2* tmp = nullptr;
-    AW_CUDA(cudaMallocAsync((void**)&tmp, sizeof(float2) * n * n, st));
+    Workspace ws(sizeof(float2) * n * n, st);
+    AW_CUDA(ws.error());
+    float2* tmp = ws.as<float2>();
     const int RR = unit_rows((int)n);
     PassArgs a;
     memset(&a, 0, sizeof a);
@@ -1703,7 +1715,6 @@ static atmwfs_status two_pass(const void* in, void* out, long n, int var, const 
         a.ext_out = (float2*)out;
         e = fn(var, dim3((unsigned)(n / RR), 1), a, tw, st);
     }
-    cudaFreeAsync(tmp, st);
     AW_CUDA(e);
     return ATMWFS_OK;
 }
@@ -1715,12 +1726,12 @@ atmwfs_status atmwfs_fresnel_dev(const void* in, void* out, long n, double dx, d
     cudaStream_t st = (cudaStream_t)stream;
     std::vector<float2> h(n);
     transfer_table(h.data(), (int)n, dx, z, lambda);
-    float2* dh = nullptr;
-    AW_CUDA(cudaMallocAsync((void**)&dh, sizeof(float2) * n, st));
+    Workspace ws(sizeof(float2) * n, st);
+    AW_CUDA(ws.error());
+    float2* dh = ws.as<float2>();
     cudaError_t e = cudaMemcpyAsync(dh, h.data(), sizeof(float2) * n, cudaMemcpyHostToDevice, st);
     atmwfs_status s = e == cudaSuccess ? two_pass(in, out, n, kVarUnitProp, dh, st)
                                        : fail(ATMWFS_ERR_CUDA, "copy failed: %s", cudaGetErrorString(e));
-    cudaFreeAsync(dh, st);
     // the host table must outlive the asynchronous copy
     cudaStreamSynchronize(st);
     return s;
@@ -1732,11 +1743,9 @@ atmwfs_status atmwfs_fft2d_dev(const void* in, void* out, long n, int sign, void
     if (sign != -1 && sign != 1) return fail(ATMWFS_ERR_INVALID, "sign must be -1 or +1");
     if (fft2d_large_supported(n)) {
         cudaStream_t st = (cudaStream_t)stream;
-        float2* tmp = nullptr;
-        AW_CUDA(cudaMallocAsync((void**)&tmp, sizeof(float2) * n * n, st));
-        const cudaError_t e = fft2d_large((const float2*)in, (float2*)out, tmp, (int)n, sign, st);
-        cudaFreeAsync(tmp, st);
-        AW_CUDA(e);
+        Workspace ws(sizeof(float2) * n * n, st);
+        AW_CUDA(ws.error());
+        AW_CUDA(fft2d_large((const float2*)in, (float2*)out, ws.as<float2>(), (int)n, sign, st));
         return ATMWFS_OK;
     }
     return two_pass(in, out, n, sign < 0 ? kVarUnitFwd : kVarUnitInv, nullptr, (cudaStream_t)stream);
@@ -1753,18 +1762,16 @@ static atmwfs_status host_unit(const float* in, float* out, long n,
         return fail(ATMWFS_ERR_INVALID, "size %ld unsupported (power of two 64..2048%s)", n,
                     fn == fft_thunk ? ", 4096 or 8192" : "");
     const size_t bytes = sizeof(float2) * n * n;
-    void *din = nullptr, *dout = nullptr;
-    AW_CUDA(cudaMalloc(&din, bytes));
-    if (cudaMalloc(&dout, bytes) != cudaSuccess) {
-        cudaFree(din);
-        return fail(ATMWFS_ERR_NOMEM, "cudaMalloc failed");
+    Workspace win(bytes, nullptr), wout(bytes, nullptr);
+    if (win.error() != cudaSuccess || wout.error() != cudaSuccess) {
+        cudaGetLastError();
+        return fail(ATMWFS_ERR_NOMEM, "device allocation failed");
     }
+    void *din = win.as<void>(), *dout = wout.as<void>();
     atmwfs_status s = ATMWFS_OK;
     if (cudaMemcpy(din, in, bytes, cudaMemcpyHostToDevice) != cudaSuccess) s = fail(ATMWFS_ERR_CUDA, "H2D failed");
     if (s == ATMWFS_OK) s = fn(din, dout, n, nullptr, arg);
     if (s == ATMWFS_OK && cudaMemcpy(out, dout, bytes, cudaMemcpyDeviceToHost) != cudaSuccess) s = fail(ATMWFS_ERR_CUDA, "D2H failed");
-    cudaFree(din);
-    cudaFree(dout);
     return s;
 }
 
@@ -1801,16 +1808,17 @@ atmwfs_status atmwfs_master_screen(uint64_t seed, uint32_t stream, long M, doubl
     if (!pow2_in(M, 64, 8192)) return fail(ATMWFS_ERR_INVALID, "M=%ld unsupported (power of two 64..8192)", M);
     if (!(outer_pix > 0) || !(inner_pix > 0)) return fail(ATMWFS_ERR_INVALID, "scales must be > 0");
     const size_t n = (size_t)M * M;
-    float2 *C = nullptr, *F = nullptr;
-    double* acc = nullptr;
-    float *o1 = nullptr, *o2 = nullptr;
     atmwfs_status s = ATMWFS_OK;
     cudaStream_t st = nullptr;
-    if (cudaMalloc(&C, n * sizeof(float2)) != cudaSuccess || cudaMalloc(&F, n * sizeof(float2)) != cudaSuccess ||
-        cudaMalloc(&acc, 8 * sizeof(double)) != cudaSuccess || cudaMalloc(&o1, n * sizeof(float)) != cudaSuccess ||
-        cudaMalloc(&o2, n * sizeof(float)) != cudaSuccess) {
-        s = fail(ATMWFS_ERR_NOMEM, "cudaMalloc failed");
+    // the spectrum's buffer takes the two screens once it is transformed
+    Workspace wc(n * sizeof(float2), st), wf(n * sizeof(float2), st), wa(8 * sizeof(double), st);
+    if (wc.error() != cudaSuccess || wf.error() != cudaSuccess || wa.error() != cudaSuccess) {
+        cudaGetLastError();
+        s = fail(ATMWFS_ERR_NOMEM, "device allocation failed");
     }
+    float2 *C = wc.as<float2>(), *F = wf.as<float2>();
+    double* acc = wa.as<double>();
+    float *o1 = wc.as<float>(), *o2 = o1 ? o1 + n : nullptr;
     // f0 = M / L0pix, fi = (5.92 / 2 pi) M / l0pix (:679-680)
     const double fo = 1.0 * M / outer_pix;
     const double fi = (5.92 / (2.0 * kPi)) * M / inner_pix;
@@ -1838,7 +1846,6 @@ atmwfs_status atmwfs_master_screen(uint64_t seed, uint32_t stream, long M, doubl
     if (s == ATMWFS_OK && out1 && cudaMemcpy(out1, o1, n * sizeof(float), cudaMemcpyDeviceToHost) != cudaSuccess) s = fail(ATMWFS_ERR_CUDA, "D2H failed");
     if (s == ATMWFS_OK && out2 && cudaMemcpy(out2, o2, n * sizeof(float), cudaMemcpyDeviceToHost) != cudaSuccess) s = fail(ATMWFS_ERR_CUDA, "D2H failed");
     if (s == ATMWFS_OK && cfit) { cfit[0] = C12[0]; cfit[1] = C12[1]; }
-    cudaFree(C); cudaFree(F); cudaFree(acc); cudaFree(o1); cudaFree(o2);
     return s;
 }
 

@@ -23,6 +23,7 @@
 #include "atmwfs.h"
 #include "atmwfs_fno.h"
 #include "fno_gemm.cuh"
+#include "workspace.cuh"
 
 namespace atmwfs {
 void set_error_message(const char* msg);
@@ -982,6 +983,7 @@ void atmwfs_fno_destroy(atmwfs_fno* f)
     for (void* p : f->allocs)
         if (p) cudaFree(p);
     delete f;
+    workspace_release();
 }
 
 long atmwfs_fno_num_params(const atmwfs_fno* f) { return f ? f->L.total : 0; }

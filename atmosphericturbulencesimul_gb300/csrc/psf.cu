@@ -26,6 +26,7 @@
 #include "aux_kernels.cuh"
 #include "pass_impl.cuh"
 #include "atan_ff.cuh"
+#include "workspace.cuh"
 
 namespace atmwfs {
 
@@ -365,16 +366,16 @@ atmwfs_status atmwfs_psf_expo_accumulate_dev(const float* amp, long amp_fstride,
     const float2* tw = stage_twiddles((int)N);
     if (!tw) return psf_fail(ATMWFS_ERR_NOMEM, "twiddle allocation failed");
     const long B = std::min(psf_batch(N, W), nframes);
-    float2* G = nullptr;
-    atmwfs_status s = psf_cuda(cudaMallocAsync((void**)&G, sizeof(float2) * B * N * W, st), "intermediate allocation");
+    Workspace ws(sizeof(float2) * B * N * W, st);
+    atmwfs_status s = psf_cuda(ws.error(), "intermediate allocation");
     if (s != ATMWFS_OK) return s;
+    float2* G = ws.as<float2>();
     for (long f0 = 0; f0 < nframes && s == ATMWFS_OK; f0 += B) {
         const long b = std::min(B, nframes - f0);
         s = psf_cuda(psf_rows<true>((int)N, amp + f0 * amp_fstride, amp_fstride, pha + f0 * W * W, W * W, nullptr, (int)b, G,
                                     tw, st), "row pass");
         if (s == ATMWFS_OK) s = psf_cuda(psf_cols<true>((int)N, G, (int)b, acc, tw, st), "column pass");
     }
-    cudaFreeAsync(G, st);
     return s;
 }
 
@@ -400,11 +401,13 @@ atmwfs_status atmwfs_psf_expo_accumulate(const float* amp, long amp_fstride, con
     if (nframes < 0 || amp_fstride < 0) return psf_fail(ATMWFS_ERR_INVALID, "negative frame count or stride");
     const long N = 2 * W;
     const long namp = (amp_fstride && nframes > 0) ? amp_fstride * (nframes - 1) + W * W : W * W;
-    float *da = nullptr, *dp = nullptr, *dimg = nullptr, *dacc = nullptr;
-    atmwfs_status s = psf_cuda(cudaMalloc(&da, sizeof(float) * namp), "allocation");
-    if (s == ATMWFS_OK) s = psf_cuda(cudaMalloc(&dp, sizeof(float) * std::max(nframes, 1L) * W * W), "allocation");
-    if (s == ATMWFS_OK) s = psf_cuda(cudaMalloc(&dimg, sizeof(float) * N * N), "allocation");
-    if (s == ATMWFS_OK) s = psf_cuda(cudaMalloc(&dacc, sizeof(float) * N * N), "allocation");
+    const size_t nb[4] = {sizeof(float) * (size_t)namp, sizeof(float) * std::max(nframes, 1L) * W * W, sizeof(float) * N * N,
+                          sizeof(float) * N * N};
+    Workspace w0(nb[0], nullptr), w1(nb[1], nullptr), w2(nb[2], nullptr), w3(nb[3], nullptr);
+    atmwfs_status s = ATMWFS_OK;
+    for (const Workspace* w : {&w0, &w1, &w2, &w3})
+        if (s == ATMWFS_OK) s = psf_cuda(w->error(), "allocation");
+    float *da = w0.as<float>(), *dp = w1.as<float>(), *dimg = w2.as<float>(), *dacc = w3.as<float>();
     if (s == ATMWFS_OK) s = psf_cuda(cudaMemcpy(da, amp, sizeof(float) * namp, cudaMemcpyHostToDevice), "copy");
     if (s == ATMWFS_OK && nframes > 0)
         s = psf_cuda(cudaMemcpy(dp, pha, sizeof(float) * nframes * W * W, cudaMemcpyHostToDevice), "copy");
@@ -413,10 +416,6 @@ atmwfs_status atmwfs_psf_expo_accumulate(const float* amp, long amp_fstride, con
     if (s == ATMWFS_OK) s = atmwfs_psf_expo_accumulate_dev(da, amp_fstride, dp, W, nframes, dacc, nullptr);
     if (s == ATMWFS_OK) s = atmwfs_psf_expo_image_dev(dacc, W, dimg, nullptr);
     if (s == ATMWFS_OK) s = psf_cuda(cudaMemcpy(psf, dimg, sizeof(float) * N * N, cudaMemcpyDeviceToHost), "copy");
-    cudaFree(da);
-    cudaFree(dp);
-    cudaFree(dimg);
-    cudaFree(dacc);
     return s;
 }
 
@@ -431,15 +430,15 @@ atmwfs_status atmwfs_chromat_psf(const float* amp, const float* pha, long n, flo
     const float2* tw = stage_twiddles((int)n);
     if (!tw) return psf_fail(ATMWFS_ERR_NOMEM, "twiddle allocation failed");
     const long B = std::min(psf_batch(n, n), nbstep);
-    float *da = nullptr, *dp = nullptr, *dI = nullptr, *dout = nullptr, *dc = nullptr, *dm = nullptr;
-    float2* G = nullptr;
-    atmwfs_status s = psf_cuda(cudaMalloc(&da, sizeof(float) * n * n), "allocation");
-    if (s == ATMWFS_OK) s = psf_cuda(cudaMalloc(&dp, sizeof(float) * n * n), "allocation");
-    if (s == ATMWFS_OK) s = psf_cuda(cudaMalloc(&dI, sizeof(float) * B * n * n), "allocation");
-    if (s == ATMWFS_OK) s = psf_cuda(cudaMalloc(&G, sizeof(float2) * B * n * n), "allocation");
-    if (s == ATMWFS_OK) s = psf_cuda(cudaMalloc(&dout, sizeof(float) * n * n), "allocation");
-    if (s == ATMWFS_OK) s = psf_cuda(cudaMalloc(&dc, sizeof(float) * nbstep), "allocation");
-    if (s == ATMWFS_OK) s = psf_cuda(cudaMalloc(&dm, sizeof(float) * nbstep), "allocation");
+    const size_t im = sizeof(float) * (size_t)n * n;
+    Workspace w0(im, nullptr), w1(im, nullptr), w2(im * B, nullptr), w3(2 * im * B, nullptr), w4(im, nullptr),
+        w5(sizeof(float) * nbstep, nullptr), w6(sizeof(float) * nbstep, nullptr);
+    atmwfs_status s = ATMWFS_OK;
+    for (const Workspace* w : {&w0, &w1, &w2, &w3, &w4, &w5, &w6})
+        if (s == ATMWFS_OK) s = psf_cuda(w->error(), "allocation");
+    float *da = w0.as<float>(), *dp = w1.as<float>(), *dI = w2.as<float>(), *dout = w4.as<float>(), *dc = w5.as<float>(),
+          *dm = w6.as<float>();
+    float2* G = w3.as<float2>();
     if (s == ATMWFS_OK) s = psf_cuda(cudaMemcpy(da, amp, sizeof(float) * n * n, cudaMemcpyHostToDevice), "copy");
     if (s == ATMWFS_OK) s = psf_cuda(cudaMemcpy(dp, pha, sizeof(float) * n * n, cudaMemcpyHostToDevice), "copy");
     if (s == ATMWFS_OK) s = psf_cuda(cudaMemcpy(dc, c.data(), sizeof(float) * nbstep, cudaMemcpyHostToDevice), "copy");
@@ -452,13 +451,6 @@ atmwfs_status atmwfs_chromat_psf(const float* amp, const float* pha, long n, flo
         if (s == ATMWFS_OK) s = psf_cuda(chromat_sum(dI, (int)b, (int)n, dc + s0, dm + s0, dout, nullptr), "zoom sum");
     }
     if (s == ATMWFS_OK) s = psf_cuda(cudaMemcpy(out, dout, sizeof(float) * n * n, cudaMemcpyDeviceToHost), "copy");
-    cudaFree(da);
-    cudaFree(dp);
-    cudaFree(dI);
-    cudaFree(G);
-    cudaFree(dout);
-    cudaFree(dc);
-    cudaFree(dm);
     return s;
 }
 

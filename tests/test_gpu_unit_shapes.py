@@ -42,3 +42,45 @@ def test_fft2d_dev_launch_shapes(lib, n, sign, off_in, off_out, in_place):
     got = _run(lib, a, sign, off_in, off_out, in_place)
     ref = np.fft.fft2(a.astype(np.complex128)) if sign < 0 else np.fft.ifft2(a.astype(np.complex128)) * n * n
     assert np.abs(got - ref).max() / np.abs(ref).max() < TOL
+
+
+def test_workspaces_of_concurrent_and_captured_calls(lib):
+    """The calls' device workspaces come from one pool: transforms of several
+    sizes issued by two host threads on streams of their own give the results
+    of calls made one by one, and a captured call can be replayed."""
+    import threading
+
+    import torch
+    from atmosphericturbulencesimul_gb300 import _lib
+
+    def call(a, out, st):
+        _lib.check(lib.atmwfs_fft2d_dev(C.c_void_p(a.data_ptr()), C.c_void_p(out.data_ptr()), a.shape[0], -1, C.c_void_p(st)))
+
+    sizes = [64, 4096, 512, 256, 4096, 1024]
+    g = torch.Generator(device="cuda").manual_seed(5)
+    ins = [torch.randn((n, n), dtype=torch.complex64, device="cuda", generator=g) for n in sizes]
+    want = [torch.empty_like(a) for a in ins]
+    for a, o in zip(ins, want):
+        call(a, o, 0)
+    torch.cuda.synchronize()
+    outs = [[torch.zeros_like(a) for a in ins] for _ in range(2)]
+
+    def work(k):
+        st = torch.cuda.Stream()
+        for _ in range(5):
+            for a, o in zip(ins, outs[k]):
+                call(a, o, st.cuda_stream)
+        st.synchronize()
+
+    ts = [threading.Thread(target=work, args=(k,)) for k in range(2)]
+    [t.start() for t in ts]
+    [t.join() for t in ts]
+    for k in range(2):
+        assert all(torch.equal(o, w) for o, w in zip(outs[k], want))
+    graph, out = torch.cuda.CUDAGraph(), torch.zeros_like(ins[2])
+    with torch.cuda.graph(graph):
+        call(ins[2], out, torch.cuda.current_stream().cuda_stream)
+    out.zero_()
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(out, want[2])
