@@ -510,13 +510,19 @@ cudaError_t screen_spectrum(uint64_t seed, uint32_t stream, int M, double fo, do
 // as an exact product plus the cross term, accumulated by two-sums (about
 // 46 bits, against the 53 of a double sum); the FP64 pipe, slow on this
 // part, is used only for the per-warp totals.
-__global__ void k_strf(const float2* __restrict__ F, int M, double* acc)
+//
+// FP32 issue bounds it (about 20 operations per lag and part).  A thread walks
+// kStrfRows rows down one column, so that the two neighbours of the row two
+// below are the next row's one below: three loads per pixel instead of five,
+// and no index arithmetic in the loop (one pixel after the other with five
+// loads: 72 us at 2048^2).
+constexpr int kStrfRows = 32;
+__global__ void __launch_bounds__(256) k_strf(const float2* __restrict__ F, int M, double* acc)
 {
     float hi[8], lo[8];
 #pragma unroll
     for (int q = 0; q < 8; q++) hi[q] = lo[q] = 0.0f;
-    const long n = (long)M * M;
-    const int lg = __ffs(M) - 1, mk = M - 1;  // M is a power of two
+    const int mk = M - 1;  // M is a power of two
     auto add_sq = [&](int q, float a, float b) {
         float dh, dl;
         ff_two_sum(a, -b, dh, dl);
@@ -527,18 +533,28 @@ __global__ void k_strf(const float2* __restrict__ F, int M, double* acc)
         hi[q] = s;
         lo[q] = ff_add(lo[q], ff_add(e, pe));
     };
-    for (long p = blockIdx.x * (long)blockDim.x + threadIdx.x; p < n; p += (long)gridDim.x * blockDim.x) {
-        const int x = (int)p & mk, y = (int)(p >> lg);
-        const float2 a = F[p];
-#pragma unroll
-        for (int q = 0; q < 4; q++) {
-            const int lx = 1 + (q & 1), ly = 1 + (q >> 1);
-            const float2 b = F[(size_t)((y + ly) & mk) * M + ((x + lx) & mk)];
-            add_sq(q, a.x, b.x);
-            add_sq(4 + q, a.y, b.y);
-        }
+    const int x = blockIdx.x * blockDim.x + threadIdx.x, y0 = blockIdx.y * kStrfRows;
+    const int x1 = (x + 1) & mk, x2 = (x + 2) & mk;
+    auto row = [&](int y) { return F + (size_t)(y & mk) * M; };
+    float2 b1 = row(y0 + 1)[x1], b2 = row(y0 + 1)[x2];  // the row below, at x + 1 and x + 2
+#pragma unroll 4
+    for (int y = y0; y < y0 + kStrfRows; y++) {
+        const float2 a = row(y)[x], c1 = row(y + 2)[x1], c2 = row(y + 2)[x2];
+        add_sq(0, a.x, b1.x);
+        add_sq(4, a.y, b1.y);
+        add_sq(1, a.x, b2.x);
+        add_sq(5, a.y, b2.y);
+        add_sq(2, a.x, c1.x);
+        add_sq(6, a.y, c1.y);
+        add_sq(3, a.x, c2.x);
+        add_sq(7, a.y, c2.y);
+        b1 = c1;
+        b2 = c2;
     }
-    // warp totals in float-float, then one double atomic per warp and sum
+    // warp totals in float-float, then one double atomic per CTA and sum (all
+    // atomics of a sum go to one address: one per warp took 45 of 65 us)
+    __shared__ double red[8][8];
+    const int warp = threadIdx.x >> 5;
 #pragma unroll
     for (int q = 0; q < 8; q++) {
         float h = hi[q], l = lo[q];
@@ -549,13 +565,20 @@ __global__ void k_strf(const float2* __restrict__ F, int M, double* acc)
             h = s;
             l = ff_add(l, ff_add(l2, e));
         }
-        if ((threadIdx.x & 31) == 0) atomicAdd(&acc[q], (double)h + (double)l);
+        if ((threadIdx.x & 31) == 0) red[warp][q] = (double)h + (double)l;
+    }
+    __syncthreads();
+    if (threadIdx.x < 8) {
+        double t = 0.0;
+        for (int w = 0; w < (int)(blockDim.x >> 5); w++) t += red[w][threadIdx.x];
+        atomicAdd(&acc[threadIdx.x], t);
     }
 }
 
 cudaError_t strf_lags(const float2* F, int M, double* acc, cudaStream_t st)
 {
-    k_strf<<<4 * 152, 256, 0, st>>>(F, M, acc);
+    const int nt = M < 256 ? M : 256;  // M is a power of two >= 64
+    k_strf<<<dim3((unsigned)(M / nt), (unsigned)(M / kStrfRows)), nt, 0, st>>>(F, M, acc);
     return cudaGetLastError();
 }
 
