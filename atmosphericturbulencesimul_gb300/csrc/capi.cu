@@ -516,6 +516,19 @@ int pass_orient(int k, int Q) { return (Q - k) & 1; }
 // of one configuration that overlap there would not predict its time in a step.
 long step_pdl_ctas(const atmwfs_ctx* c) { return c->tuning ? 0 : pdl_max_ctas(); }
 
+// The same for the propagation passes.  They let their successor be scheduled
+// only when their transforms are done, so its CTAs find the slots of finished
+// ones and spread evenly; a context of one grid class, whose chain has no
+// branch of passes beside it, therefore takes them up to four CTAs per SM (a
+// step of 4 x 256^2 57 -> 50 us, 512^2 84 -> 77, 8 x 512^2 164 -> 149, 1024^2
+// 137 -> 129).  Scheduled from the start of the predecessor instead, grids
+// above one CTA per SM pile up on some SMs (4 x 512^2: 107 -> 145 us).
+long pass_pdl_ctas(const atmwfs_ctx* c)
+{
+    if (c->tuning) return 0;
+    return (c->classes.size() == 1 ? 4L : 1L) * pdl_max_ctas();
+}
+
 // The window kernel over jobs [j0, j1) of class cl (the windows of the
 // groups whose side is cl's grid); optionally report its algorithmic bytes.
 atmwfs_status launch_windows(atmwfs_ctx* c, Class& cl, int j0, int j1, double* bytes, cudaStream_t st)
@@ -635,7 +648,7 @@ atmwfs_status launch_pass(atmwfs_ctx* c, int k, Class& cl, double* bytes, cudaSt
             a.L = c->L;
             a.ninst_total = c->ninst;
             a.poscap = c->poscap;
-            a.pdl_ctas = step_pdl_ctas(c);
+            a.pdl_ctas = pass_pdl_ctas(c);
             a.g_lo = c->plane_lo[k - 1];
             a.g_hi = c->plane_hi[k - 1];
             a.hop1 = k - 2;

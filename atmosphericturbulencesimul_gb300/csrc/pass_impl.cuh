@@ -357,7 +357,8 @@ __global__ void __launch_bounds__(Plan<N, V>::T* RR, MINB)
     extern __shared__ __align__(1024) unsigned char sm[];
     float2* xb = reinterpret_cast<float2*>(sm);
     float* wrows = reinterpret_cast<float*>(sm + G::win_offset());  // [RR][N]
-    pdl_gate();
+    pdl_wait();
+    if constexpr (!I_SERIES(OPS)) pdl_trigger();
 
     const int tid = threadIdx.x;
     const int t = tid % T;
@@ -484,6 +485,8 @@ __global__ void __launch_bounds__(Plan<N, V>::T* RR, MINB)
         }
     }
 
+    // (series passes: the successor's CTAs are scheduled from here, see pass_pdl_ctas)
+    if constexpr (I_SERIES(OPS)) pdl_trigger();
     if constexpr (kEpi) {
         // Outputs of the crop.  The geometric phase sum over all layers
         // (reference array1 / sarray1) comes from k_phasum.  The field is
