@@ -71,6 +71,8 @@ cudaError_t spectral_umma(const __nv_bfloat16* W, int o, int c, const float* X, 
 // fused forward kernels of the default shape (fno_fused.cu)
 bool fused_supported(int grid, int modes, int width, int proj, int nout);
 cudaError_t xdft_fused(const __nv_bfloat16* F, const float* H, float* a, int B, unsigned* status, cudaStream_t st);
+cudaError_t yfwd_fused(const __nv_bfloat16* F, const float* a, float* z, int B, unsigned* status, cudaStream_t st);
+cudaError_t yinv_fused(const __nv_bfloat16* G, const float* y, float* bb, int B, unsigned* status, cudaStream_t st);
 cudaError_t fourier_fused(const __nv_bfloat16* W, const __nv_bfloat16* Gt, const float* X, const float* bb, float* U,
                           float* act, const float* bias, int B, unsigned* status, bool write_u, cudaStream_t st);
 cudaError_t project_fused(const __nv_bfloat16* W1, const float* c1, const __nv_bfloat16* W2, const float* c2,
@@ -214,17 +216,21 @@ __global__ void k_mse(const float* __restrict__ out, const float* __restrict__ t
 // values are broadcasts, two channels to a load (one thread per output value
 // read both operands for every product: 67 us).
 constexpr int kMixB = 8;
-template <int KX>
+// WC: the width as a constant (0: the argument); the staging loops divide by it.
+template <int KX, int WC>
 __global__ void __launch_bounds__(256) k_modemix(const __nv_bfloat16* __restrict__ R, const float* __restrict__ z,
-                                                 float* __restrict__ y, int B, int w, int m, long sk, long sc)
+                                                 float* __restrict__ y, int B, int width, int m, long sk, long sc)
 {
+    const int w = WC ? WC : width;
     const int groups = m / KX, ky = blockIdx.x / groups, kx0 = blockIdx.x % groups * KX;
     const long Nc = (long)B * w * m;
     const long ore = (long)ky * Nc + kx0 * sk, oim = (long)(m + ky) * Nc + kx0 * sk;
+    constexpr int NB = WC ? kMixB / 2 : kMixB;  // samples per thread: two threads share a channel where w is known
     extern __shared__ float4 mix_smem[];
     float* zs = reinterpret_cast<float*>(mix_smem);                                 // [KX][kMixB][w][2]
     __nv_bfloat162* rs = reinterpret_cast<__nv_bfloat162*>(zs + KX * kMixB * w * 2);  // [KX][w][w + 1]
     const __nv_bfloat162* Rk = reinterpret_cast<const __nv_bfloat162*>(R) + (size_t)(ky * m + kx0) * w * w;
+#pragma unroll 8
     for (int i = threadIdx.x; i < KX * w * w; i += blockDim.x) rs[i / w * (w + 1) + i % w] = Rk[i];
     for (int b0 = 0; b0 < B; b0 += kMixB) {
         const int nb = min(kMixB, B - b0);
@@ -241,18 +247,20 @@ __global__ void __launch_bounds__(256) k_modemix(const __nv_bfloat16* __restrict
             for (int k = 0; k < KX; k++) reinterpret_cast<float2*>(zs)[k * kMixB * w + i] = make_float2(vr[k], vi[k]);
         }
         __syncthreads();
-        for (int i = threadIdx.x; i < KX * w; i += blockDim.x) {
+        for (int it = threadIdx.x; it < KX * w * (kMixB / NB); it += blockDim.x) {
+            const int i = it % (KX * w), bg = it / (KX * w) * NB;  // (mode, output channel), first sample
             const int k = i / w, o = i % w;
             const __nv_bfloat162* r = rs + (size_t)i * (w + 1);
-            const float4* zk = reinterpret_cast<const float4*>(zs + (size_t)k * kMixB * w * 2);
-            float sr[kMixB], si[kMixB];
+            const float4* zk = reinterpret_cast<const float4*>(zs + ((size_t)k * kMixB + bg) * w * 2);
+            float sr[NB], si[NB];
 #pragma unroll
-            for (int b = 0; b < kMixB; b++) sr[b] = si[b] = 0.0f;
+            for (int b = 0; b < NB; b++) sr[b] = si[b] = 0.0f;
+#pragma unroll 4
             for (int c = 0; c < w; c += 2) {  // w is even
                 const float2 r0 = make_float2(__low2float(r[c]), __high2float(r[c]));
                 const float2 r1 = make_float2(__low2float(r[c + 1]), __high2float(r[c + 1]));
 #pragma unroll
-                for (int b = 0; b < kMixB; b++) {
+                for (int b = 0; b < NB; b++) {
                     const float4 v = zk[(b * w + c) / 2];
                     sr[b] += r0.x * v.x - r0.y * v.y;
                     si[b] += r0.x * v.y + r0.y * v.x;
@@ -260,8 +268,10 @@ __global__ void __launch_bounds__(256) k_modemix(const __nv_bfloat16* __restrict
                     si[b] += r1.x * v.w + r1.y * v.z;
                 }
             }
-            for (int b = 0; b < nb; b++) {
-                const long q = (long)((b0 + b) * w + o) * sc + k * sk;
+#pragma unroll
+            for (int b = 0; b < NB; b++) {
+                if (bg + b >= nb) break;
+                const long q = (long)((b0 + bg + b) * w + o) * sc + k * sk;
                 y[q + ore] = sr[b];
                 y[q + oim] = si[b];
             }
@@ -283,10 +293,11 @@ cudaError_t modemix(const __nv_bfloat16* R, const float* z, float* y, int B, int
         kern<<<m * m / kx, 256, sm, st>>>(R, z, y, B, w, m, sk, sc);
         return cudaGetLastError();
     };
-    // (whole runs per mode, sc = 1, need no neighbours: two modes make twice the CTAs)
-    if (sc != 1 && m % 4 == 0 && modemix_smem<4>(w) <= 113 * 1024) return go(k_modemix<4>, modemix_smem<4>(w), 4);
-    if (modemix_smem<2>(w) <= 113 * 1024) return go(k_modemix<2>, modemix_smem<2>(w), 2);  // m is even
-    return go(k_modemix<1>, modemix_smem<1>(w), 1);
+    // (whole runs per mode need no neighbours: two modes make twice the CTAs)
+    if (sc == 1 && w == 64) return go(k_modemix<2, 64>, modemix_smem<2>(w), 2);
+    if (m % 4 == 0 && modemix_smem<4>(w) <= 113 * 1024) return go(k_modemix<4, 0>, modemix_smem<4>(w), 4);
+    if (modemix_smem<2>(w) <= 113 * 1024) return go(k_modemix<2, 0>, modemix_smem<2>(w), 2);  // m is even
+    return go(k_modemix<1, 0>, modemix_smem<1>(w), 1);
 }
 
 // Backward of the mode mixing: dz = R^H dy per mode, and dR += sum_b dy z^H.
@@ -692,7 +703,9 @@ atmwfs_status spectral_fwd(atmwfs_fno* f, int l, const void* h, int h_bf16, floa
     }
     // z = FyAB a: [2m, 2G] x [2G, Nc], on tcgen05 where compiled
     const bool tc = umma_enabled() && Nc % 8 == 0;
-    if (tc && spectral_umma_supported(2 * m, 2 * G))
+    if (!spec)
+        FN_CUDA(yfwd_fused(f->FyAB_bf, a, z, B, umma_status_ptr(), st));
+    else if (tc && spectral_umma_supported(2 * m, 2 * G))
         FN_CUDA(spectral_umma(f->FyAB_bf, 2 * m, 2 * G, a, z, Nc, umma_status_ptr(), 0, st));
     else
         FN_CUDA(gemm(2 * m, (int)Nc, 2 * G, f->FyAB, 2 * G, 0, 0, a, Nc, 0, 0, z, Nc, 0.0f, 1, 0, 0, 0, nullptr, 0, st));
@@ -701,7 +714,9 @@ atmwfs_status spectral_fwd(atmwfs_fno* f, int l, const void* h, int h_bf16, floa
     if (smf > 227 * 1024) return err(ATMWFS_ERR_INVALID, "batch %d x width %d exceeds the mode-mixing shared memory", B, w);
     FN_CUDA(modemix(f->pbf + f->L.R[l], z, f->y, B, w, m, spec ? 1 : BW, spec ? m : 1, st));
     // bb = GyBig y: [2G, 2m] x [2m, Nc], on tcgen05 where compiled
-    if (tc && spectral_umma_supported(2 * G, 2 * m))
+    if (!spec)
+        FN_CUDA(yinv_fused(f->GyBig_bf, f->y, f->bb, B, umma_status_ptr(), st));
+    else if (tc && spectral_umma_supported(2 * G, 2 * m))
         FN_CUDA(spectral_umma(f->GyBig_bf, 2 * G, 2 * m, f->y, f->bb, Nc, umma_status_ptr(), 0, st));
     else
         FN_CUDA(gemm(2 * G, (int)Nc, 2 * m, f->GyBig, 2 * m, 0, 0, f->y, Nc, 0, 0, f->bb, Nc, 0.0f, 1, 0, 0, 0, nullptr, 0,
@@ -864,7 +879,7 @@ atmwfs_status layer_bwd(atmwfs_fno* f, int l, const float* dh, float* dX, int B,
     k_modemix_bwd64<8><<<m * m, 256, 0, st>>>(f->pbf + f->L.R[l], f->z[l], f->dy, f->dz, f->grads + f->L.R[l], B, m);
     FN_CUDA(cudaGetLastError());
     // da = FyAB^T dz: [2G, 2m] x [2m, Nc]
-    FN_CUDA(spectral_umma(f->FyABT_bf, 2 * G, 2 * m, f->dz, f->da, Nc, status, 0, st));
+    FN_CUDA(yinv_fused(f->FyABT_bf, f->dz, f->da, B, status, st));
     FN_CUDA(fourier_bwd_fused(f->pbf + f->L.W[l], f->Fx_bf, du, f->da, dX, B, status, st));
     return ATMWFS_OK;
 }

@@ -3,6 +3,7 @@
 // tensor cores, so that the images between them are not written and read
 // back:
 //   k_xdft     the forward DFT along x, written as coalesced spectrum rows;
+//   k_yfwd, k_yinv  the DFTs along y;
 //   k_fourier  pointwise mixing + inverse DFT along x (+ bias, GELU), and the
 //              same pair of the backward pass;
 //   k_project  the first projection + GELU + the 2-channel output;
@@ -155,6 +156,162 @@ __global__ void __launch_bounds__(kThreads, 2) k_xdft(const __nv_bfloat16* __res
         retire_tile();
     }
     tmem_free(tmem, 64, warp);
+}
+
+// ---------------------------------------------------------------------------
+// The DFTs along y over the P = m B w columns of the planar images:
+//   k_yfwd  z (64 x P) = F (64 x 512) a (512 x P)     (64 rows: re, im of the kept ky)
+//   k_yinv  bb (512 x P) = G (512 x 64) y (64 x P)
+// 128 columns per tile along the TMEM lanes.  An image is 67 MB at a batch of 16
+// (10 us of HBM time, or L2): latency is what has to be hidden.  k_yfwd takes
+// K in four chunks of 128 whose next values are loaded into registers as the
+// current ones are stored (eight staged chunks of 64 before: 31-33 us).  k_yinv
+// gives each CTA a quarter of the output rows, so that four CTAs share an SM
+// and its 512 columns of tensor memory (one CTA per SM held all 512 rows
+// before, 256 tiles on 152 CTAs: 31 us).
+// ---------------------------------------------------------------------------
+constexpr int kYK = 2 * kG;                      // K of the forward product
+constexpr int kYC = 128;                         // its chunk
+constexpr uint32_t kYA = 2 * kModes * kYK * 2;   // F: 64 KB, then the chunk's A tile: 32 KB
+constexpr uint32_t kYBytes = kYA + kM * kYC * 2;
+
+__global__ void __launch_bounds__(kThreads, 2) k_yfwd(const __nv_bfloat16* __restrict__ F, const float* __restrict__ X,
+                                                      float* __restrict__ Z, long P, int ntiles, unsigned* status)
+{
+    constexpr int J = kYC / 16;       // pieces of 8 rows per thread
+    constexpr int NC = kYK / kYC;
+    extern __shared__ __align__(1024) unsigned char sm[];
+    __shared__ __align__(8) uint64_t bar;
+    __shared__ uint32_t tmem_base;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int m = tid % kM, kc0 = tid / kM;
+    float x[J][8];
+    auto load = [&](int tile, int chunk, int j) {
+        const float* src = X + (size_t)(chunk * kYC + (kc0 + 2 * j) * 8) * P + (size_t)tile * kM + m;
+#pragma unroll
+        for (int q = 0; q < 8; q++) x[j][q] = __ldg(src + (size_t)q * P);
+    };
+    if (blockIdx.x < ntiles)
+#pragma unroll
+        for (int j = 0; j < J; j++) load(blockIdx.x, 0, j);
+    tmem_alloc(&tmem_base, 64, warp);
+    if (tid == 0) mbar_init(&bar);
+    for (int i = tid; i < 2 * kModes * kYK / 8; i += kThreads) {
+        const int row = (i >> 9) * 8 + (i & 7), k8 = (i >> 3) & 63;
+        *reinterpret_cast<uint4*>(sm + kmajor_off(row, k8 * 8, kYK / 8)) =
+            *reinterpret_cast<const uint4*>(F + (size_t)row * kYK + k8 * 8);
+    }
+    fence_before();
+    __syncthreads();
+    fence_after();
+    const uint32_t tmem = tmem_base, base = smem_addr(sm);
+    uint32_t parity = 0;
+    bool failed = false;
+    for (int tile = blockIdx.x; tile < ntiles && !failed; tile += gridDim.x) {
+#pragma unroll 1
+        for (int c = 0; c < NC; c++) {
+            const bool more = c + 1 < NC || tile + (int)gridDim.x < ntiles;
+            const int nt = c + 1 < NC ? tile : tile + gridDim.x, nc = c + 1 < NC ? c + 1 : 0;
+#pragma unroll
+            for (int j = 0; j < J; j++) {
+                *reinterpret_cast<uint4*>(sm + kYA + kmajor_off(m, (kc0 + 2 * j) * 8, kYC / 8)) = pack8(x[j]);
+                if (more) load(nt, nc, j);
+            }
+            publish_smem();
+            if (tid == 0) {
+#pragma unroll
+                for (int ks = 0; ks < kYC / 16; ks++)
+                    mma_bf16(tmem, smem_desc(base + kYA + ks * 256, 128, kYC / 8 * 128),
+                             smem_desc(base + c * (kYC / 8) * 128 + ks * 256, 128, kYK / 8 * 128), instr_desc(2 * kModes),
+                             c > 0 || ks > 0);
+                mma_commit(&bar);
+            }
+            // the chunk's products are done before its A tile is overwritten
+            if (!mma_wait(&bar, parity, status)) {
+                failed = true;
+                break;
+            }
+            parity ^= 1;
+        }
+        if (failed) break;
+        const int g = warp & 3, half = warp >> 2;
+        float* o = Z + (size_t)tile * kM + g * 32 + lane;
+#pragma unroll
+        for (int c0 = half * kModes; c0 < (half + 1) * kModes; c0 += 16) {
+            float r[16];
+            tmem_ld16(tmem + ((uint32_t)(g * 32) << 16) + c0, r);
+#pragma unroll
+            for (int q = 0; q < 16; q++) o[(size_t)(c0 + q) * P] = r[q];
+        }
+        retire_tile();
+    }
+    tmem_free(tmem, 64, warp);
+}
+
+constexpr int kYQ = kYK / 4;                              // output rows per CTA
+constexpr uint32_t kIA = kYQ * 2 * kModes * 2;            // its rows of G: 16 KB, then the A tile: 16 KB
+constexpr uint32_t kIBytes = kIA + kM * 2 * kModes * 2;
+
+__global__ void __launch_bounds__(kThreads, 4) k_yinv(const __nv_bfloat16* __restrict__ Gy, const float* __restrict__ X,
+                                                      float* __restrict__ bb, long P, int ntiles, unsigned* status)
+{
+    constexpr int K = 2 * kModes, J = K / 16;
+    extern __shared__ __align__(1024) unsigned char sm[];
+    __shared__ __align__(8) uint64_t bar;
+    __shared__ uint32_t tmem_base;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int m = tid % kM, kc0 = tid / kM;
+    const int quarter = blockIdx.x & 3, step = gridDim.x >> 2;
+    float x[J][8];
+    auto load = [&](int tile, int j) {
+        const float* src = X + (size_t)((kc0 + 2 * j) * 8) * P + (size_t)tile * kM + m;
+#pragma unroll
+        for (int q = 0; q < 8; q++) x[j][q] = __ldg(src + (size_t)q * P);
+    };
+    const int first = blockIdx.x >> 2;
+    if (first < ntiles)
+#pragma unroll
+        for (int j = 0; j < J; j++) load(first, j);
+    tmem_alloc(&tmem_base, kYQ, warp);
+    if (tid == 0) mbar_init(&bar);
+    for (int i = tid; i < kYQ * K / 8; i += kThreads) {
+        const int row = (i >> 6) * 8 + (i & 7), k8 = (i >> 3) & 7;
+        *reinterpret_cast<uint4*>(sm + kmajor_off(row, k8 * 8, K / 8)) =
+            *reinterpret_cast<const uint4*>(Gy + (size_t)(quarter * kYQ + row) * K + k8 * 8);
+    }
+    fence_before();
+    __syncthreads();
+    fence_after();
+    const uint32_t tmem = tmem_base, base = smem_addr(sm);
+    uint32_t parity = 0;
+    for (int tile = first; tile < ntiles; tile += step) {
+#pragma unroll
+        for (int j = 0; j < J; j++) {
+            *reinterpret_cast<uint4*>(sm + kIA + kmajor_off(m, (kc0 + 2 * j) * 8, K / 8)) = pack8(x[j]);
+            if (tile + step < ntiles) load(tile + step, j);
+        }
+        publish_smem();
+        if (tid == 0) {
+#pragma unroll
+            for (int ks = 0; ks < K / 16; ks++)
+                mma_bf16(tmem, smem_desc(base + kIA + ks * 256, 128, K / 8 * 128), smem_desc(base + ks * 256, 128, K / 8 * 128),
+                         instr_desc(kYQ), ks > 0);
+            mma_commit(&bar);
+        }
+        if (!mma_wait(&bar, parity, status)) break;
+        parity ^= 1;
+        const int g = warp & 3, half = warp >> 2;
+        float* o = bb + (size_t)quarter * kYQ * P + (size_t)tile * kM + g * 32 + lane;
+#pragma unroll 1
+        for (int c0 = half * (kYQ / 2); c0 < (half + 1) * (kYQ / 2); c0 += 16) {
+            float r[16];
+            tmem_ld16(tmem + ((uint32_t)(g * 32) << 16) + c0, r);
+#pragma unroll
+            for (int q = 0; q < 16; q++) o[(size_t)(c0 + q) * P] = r[q];
+        }
+        retire_tile();
+    }
+    tmem_free(tmem, kYQ, warp);
 }
 
 // ---------------------------------------------------------------------------
@@ -736,6 +893,30 @@ cudaError_t xdft_fused(const __nv_bfloat16* F, const float* H, float* a, int B, 
     if (e != cudaSuccess) return e;
     const int lines = B * kG, grid = lines < 2 * sm_count() ? lines : 2 * sm_count();
     k_xdft<<<grid, kThreads, 2 * kXBytes, st>>>(F, H, a, lines, (long)B * kW * kModes, status);
+    return cudaGetLastError();
+}
+
+// z = F a, F 64 x 512 (FyAB)
+cudaError_t yfwd_fused(const __nv_bfloat16* F, const float* a, float* z, int B, unsigned* status, cudaStream_t st)
+{
+    using namespace umma;
+    const cudaError_t e = allow_smem(k_yfwd, kYBytes);
+    if (e != cudaSuccess) return e;
+    const long P = (long)B * kW * kModes;
+    const int tiles = (int)(P / kM), grid = tiles < 2 * sm_count() ? tiles : 2 * sm_count();
+    k_yfwd<<<grid, kThreads, kYBytes, st>>>(F, a, z, P, tiles, status);
+    return cudaGetLastError();
+}
+
+// bb = G y, G 512 x 64 (GyBig, FyAB^T)
+cudaError_t yinv_fused(const __nv_bfloat16* G, const float* y, float* bb, int B, unsigned* status, cudaStream_t st)
+{
+    using namespace umma;
+    const cudaError_t e = allow_smem(k_yinv, kIBytes);
+    if (e != cudaSuccess) return e;
+    const long P = (long)B * kW * kModes;
+    const int tiles = (int)(P / kM), grid = 4 * (tiles < sm_count() ? tiles : sm_count());
+    k_yinv<<<grid, kThreads, kIBytes, st>>>(G, y, bb, P, tiles, status);
     return cudaGetLastError();
 }
 
