@@ -163,34 +163,52 @@ __device__ float bin_votes(const float* pb, const float* ppf, int nb, int bx, in
     return ch;
 }
 
-// Bin phases of one instance into pb[n], by the whole CTA: the fixed-point sums
-// back to float (one rounding; the scaling by 2^-kBinFrac is exact), then
-// (float)atan2((double)im, (double)re) without FP64 (atan_ff.cuh).  Returns
-// whether any vote can fire.
-//
-// A vote needs two bins more than pi apart.  Where all bins lie closer (the
-// usual case: the bins hold the diffraction's mean phase, a fraction of a
-// radian) the first iteration finds none, lowers the limit to 0.5 and is the
-// last, and the bins stay as they are.  That takes the 48 candidate votes per
-// bin and the FP64 thresholds out of the frame: one CTA spent about 30 us on
-// the 102^2 bins of a 2048^2 frame.
-__device__ __forceinline__ bool load_bins(const unsigned long long* bins, int n, float* pb, const float2* __restrict__ atan_tab)
+__global__ void k_unwrap(const InstDev* __restrict__ insts, const int* __restrict__ list, unsigned* status,
+                         int* iters_out, const float2* __restrict__ atan_tab)
 {
-    __shared__ float s_lo[32], s_hi[32];
+    pdl_gate();
+    const InstDev& I = insts[list[blockIdx.x]];
+    const int nb = I.nb;
+    if (nb <= 0) return;
+    const int n = nb * nb;
+    extern __shared__ float sh[];
+    float* pb = sh;
+    float* ch = sh + n;
+    float* ppf = sh + 2 * n;
+    // vote maximum and flip count, double-buffered by iteration parity so
+    // that one iteration needs two barriers: the counters of iteration it-1
+    // are cleared in iteration it after its first barrier, when every thread
+    // has read them, and are next written after its second barrier
+    __shared__ unsigned s_max[2];
+    __shared__ int s_cnt[2];
+    const double kTwoPi = 2.0 * 3.14159265358979323846;
     float vmin = 4.0f, vmax = -4.0f;  // outside the range of an angle
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
+        // the fixed-point sums back to float (one rounding; the scaling by
+        // 2^-kBinFrac is exact), then (float)atan2((double)im, (double)re)
+        // without FP64 (atan_ff.cuh)
         const float q = 1.0f / (float)(1ull << kBinFrac);
-        const float re = __ll2float_rn((long long)bins[i]) * q;
-        const float im = __ll2float_rn((long long)bins[n + i]) * q;
+        const float re = __ll2float_rn((long long)I.bins[i]) * q;
+        const float im = __ll2float_rn((long long)I.bins[n + i]) * q;
         const float v = atan2_ff(im, re, atan_tab);
         pb[i] = v;
         vmin = fminf(vmin, v);
         vmax = fmaxf(vmax, v);
+        I.bins[i] = 0ull;
+        I.bins[n + i] = 0ull;
     }
+    if (threadIdx.x < 2) { s_max[threadIdx.x] = 0u; s_cnt[threadIdx.x] = 0; }
+    // A vote needs two bins more than pi apart.  Where all bins lie closer
+    // (the usual case: the bins hold the diffraction's mean phase, a fraction
+    // of a radian) the first iteration finds none, lowers the limit to 0.5 and
+    // is the last, and the bins stay as they are.  That takes the 48 candidate
+    // votes per bin and the FP64 thresholds out of the frame: one CTA spent
+    // about 30 us on the 102^2 bins of a 2048^2 frame.
     for (int o = 16; o > 0; o >>= 1) {
         vmin = fminf(vmin, __shfl_xor_sync(0xffffffffu, vmin, o));
         vmax = fmaxf(vmax, __shfl_xor_sync(0xffffffffu, vmax, o));
     }
+    __shared__ float s_lo[32], s_hi[32];
     if ((threadIdx.x & 31) == 0) {
         s_lo[threadIdx.x >> 5] = vmin;
         s_hi[threadIdx.x >> 5] = vmax;
@@ -200,22 +218,11 @@ __device__ __forceinline__ bool load_bins(const unsigned long long* bins, int n,
         vmin = fminf(vmin, s_lo[w]);
         vmax = fmaxf(vmax, s_hi[w]);
     }
-    return !(vmax - vmin < 3.14159f);  // below pi by more than the difference's rounding
-}
-
-// The relaxation of the bin phases pb by the whole CTA (ch, ppf: scratch);
-// returns its iterations.
-__device__ __forceinline__ int relax_bins(float* pb, float* ch, float* ppf, int nb)
-{
-    const int n = nb * nb;
-    // vote maximum and flip count, double-buffered by iteration parity so
-    // that one iteration needs two barriers: the counters of iteration it-1
-    // are cleared in iteration it after its first barrier, when every thread
-    // has read them, and are next written after its second barrier
-    __shared__ unsigned s_max[2];
-    __shared__ int s_cnt[2];
-    const double kTwoPi = 2.0 * 3.14159265358979323846;
-    if (threadIdx.x < 2) { s_max[threadIdx.x] = 0u; s_cnt[threadIdx.x] = 0; }
+    if (vmax - vmin < 3.14159f) {  // below pi by more than the difference's rounding
+        for (int i = threadIdx.x; i < n; i += blockDim.x) I.peak[i] = pb[i];
+        if (threadIdx.x == 0 && iters_out) iters_out[list[blockIdx.x]] = 1;
+        return;
+    }
     for (int i = threadIdx.x; i < n; i += blockDim.x) ppf[i] = __double2float_rd((double)pb[i] + kTwoPi * 0.5);
     __syncthreads();
     int chiter = 0, chcnt0cnt = 0, par = 0;
@@ -259,23 +266,8 @@ __device__ __forceinline__ int relax_bins(float* pb, float* ch, float* ppf, int 
         else chcnt0cnt = 0;
         par ^= 1;
     }
-    return chiter;
-}
-
-__global__ void k_unwrap(const InstDev* __restrict__ insts, const int* __restrict__ list, unsigned* status,
-                         int* iters_out, const float2* __restrict__ atan_tab)
-{
-    pdl_gate();
-    const InstDev& I = insts[list[blockIdx.x]];
-    const int nb = I.nb;
-    if (nb <= 0) return;
-    const int n = nb * nb;
-    extern __shared__ float sh[];
-    const bool votes = load_bins(I.bins, n, sh, atan_tab);
-    for (int i = threadIdx.x; i < 2 * n; i += blockDim.x) I.bins[i] = 0ull;  // (past a barrier: every sum is read)
-    const int iters = votes ? relax_bins(sh, sh + n, sh + 2 * n, nb) : 1;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) I.peak[i] = sh[i];
-    if (threadIdx.x == 0 && iters_out) iters_out[list[blockIdx.x]] = iters;
+    for (int i = threadIdx.x; i < n; i += blockDim.x) I.peak[i] = pb[i];
+    if (threadIdx.x == 0 && iters_out) iters_out[list[blockIdx.x]] = chiter;
 }
 
 cudaError_t unwrap_bins(const InstDev* insts, const int* list, int nsci, int maxnb, unsigned* status, int* iters,
@@ -294,11 +286,15 @@ cudaError_t unwrap_bins(const InstDev* insts, const int* list, int nsci, int max
 
 // final science phase: pha + 2 pi round((phasum - pha - peak[bin]) / 2 pi)
 // (AtmosphericTurbulence.c:3918-3941)
-__device__ __forceinline__ void apply_peaks(const InstDev& I, int step, const float* peakv)
+__global__ void k_sci_apply(const InstDev* __restrict__ insts, const int* __restrict__ list, const int* d_step)
 {
+    pdl_gate();
+    const InstDev& I = insts[list[blockIdx.y]];
     const int Nout = I.Nout, nb = I.nb;
+    const int step = d_step ? *d_step : 0;
     float* pha = I.out_pha + (size_t)(step % I.ring) * I.ostride;
     const short* __restrict__ binx = I.binx;
+    const float* __restrict__ peakv = I.peak;
     const float* __restrict__ psum = I.phisum;
     // four neighbouring pixels of a row per thread as 16-byte vectors when the
     // row length allows, else one; items run through the frame so that every
@@ -335,63 +331,6 @@ __device__ __forceinline__ void apply_peaks(const InstDev& I, int step, const fl
             pha[o] = one(pha[o], gs ? fmaf(sc, gs[0].x, sc * gs[0].y) : psum[o], ii);
         }
     }
-}
-
-__global__ void k_sci_apply(const InstDev* __restrict__ insts, const int* __restrict__ list, const int* d_step)
-{
-    pdl_gate();
-    const InstDev& I = insts[list[blockIdx.y]];
-    apply_peaks(I, d_step ? *d_step : 0, I.peak);
-}
-
-// Unwrap, apply and step counter in one kernel, for a context whose chain of
-// passes is alone in the step and whose frames have few bins (kFinishBins per
-// side): there the three launches cost as much as the work (256^2: 4.8 + 2 of
-// 25 us per step).  Every CTA evaluates the instance's bin phases for itself
-// (and relaxes them where a vote can fire: the same operations, the same
-// result).  The last CTA of an instance to have read the bins clears them; the
-// last instance of the step advances the counter, which every CTA has read by
-// then.  tickets: [instances + 1], zero between launches.
-__global__ void __launch_bounds__(256) k_sci_finish(const InstDev* __restrict__ insts, const int* __restrict__ list,
-                                                    int* d_step, int* iters_out, const float2* __restrict__ atan_tab,
-                                                    unsigned* tickets)
-{
-    pdl_gate();
-    const InstDev& I = insts[list[blockIdx.y]];
-    const int nb = I.nb, n = nb * nb;
-    const int step = *d_step;
-    extern __shared__ float sh[];
-    __shared__ bool s_last;
-    int iters = -1;
-    if (nb > 0) iters = load_bins(I.bins, n, sh, atan_tab) ? relax_bins(sh, sh + n, sh + 2 * n, nb) : 1;
-    __syncthreads();  // the CTA has read the bins and the step
-    if (threadIdx.x == 0) {
-        __threadfence();
-        s_last = atomicAdd(&tickets[blockIdx.y], 1u) == gridDim.x - 1;
-    }
-    apply_peaks(I, step, sh);
-    __syncthreads();
-    if (!s_last) return;
-    for (int i = threadIdx.x; i < 2 * n; i += blockDim.x) I.bins[i] = 0ull;
-    if (threadIdx.x == 0) {
-        if (nb > 0 && iters_out) iters_out[list[blockIdx.y]] = iters;
-        tickets[blockIdx.y] = 0u;
-        if (atomicAdd(&tickets[gridDim.y], 1u) == gridDim.y - 1) {
-            tickets[gridDim.y] = 0u;
-            *d_step = step + 1;
-        }
-    }
-}
-
-cudaError_t sci_finish(const InstDev* insts, const int* list, int nsci, int maxnb, int maxnout, int* d_step, int* iters,
-                       const float2* atan_tab, unsigned* tickets, long pdl_ctas, cudaStream_t st)
-{
-    // about two CTAs per SM in all: each repeats the instance's bin phases
-    const long need = ((long)maxnout * maxnout / (maxnout % 4 == 0 ? 4 : 1) + 255) / 256;
-    const int bx = (int)std::max(1L, std::min(need, (2L * 152 + nsci - 1) / nsci));
-    const size_t sm = (size_t)3 * maxnb * maxnb * sizeof(float);
-    return launch_gated_up_to(pdl_ctas, k_sci_finish, dim3(bx, nsci), dim3(256), sm, st, insts, list, d_step, iters, atan_tab,
-                              tickets);
 }
 
 cudaError_t sci_apply(const InstDev* insts, const int* list, int nsci, int maxnout, const int* d_step, long pdl_ctas,

@@ -11,10 +11,6 @@ cudaError_t scale_screen(float* S, long n, double f, cudaStream_t st);
 cudaError_t unwrap_bins(const InstDev* insts, const int* list, int nsci, int maxnb, unsigned* status, int* iters,
                         const float2* atan_tab, long pdl_ctas, cudaStream_t st);
 cudaError_t sci_apply(const InstDev* insts, const int* list, int nsci, int maxnout, const int* d_step, long pdl_ctas, cudaStream_t st);
-// Bins per side up to which sci_finish keeps its scratch in 48 KB.
-constexpr int kFinishBins = 32;
-cudaError_t sci_finish(const InstDev* insts, const int* list, int nsci, int maxnb, int maxnout, int* d_step, int* iters,
-                       const float2* atan_tab, unsigned* tickets, long pdl_ctas, cudaStream_t st);
 cudaError_t step_advance(int* d_step, cudaStream_t st);
 // Compensated layer sums of the window groups with a layer-independent
 // Scoeff (one job per group, maxside the largest side).

@@ -373,7 +373,6 @@ struct atmwfs_ctx {
     unsigned* d_status = nullptr;
     unsigned* h_status = nullptr;        // pinned: where check_status reads it
     int* d_iters = nullptr;
-    unsigned* d_tickets = nullptr;       // of sci_finish
     int* d_sci = nullptr;
     float2* d_atan_tab = nullptr;  // atan(k / 1024) pairs of the science unwrap
     int nsci = 0, maxnb = 0, maxnout = 0;
@@ -693,13 +692,6 @@ atmwfs_status launch_pass(atmwfs_ctx* c, int k, Class& cl, double* bytes, cudaSt
     return ATMWFS_OK;
 }
 
-// Whether one kernel finishes the step (sci_finish): one grid class with
-// science instances of few bins.
-bool finish_step(const atmwfs_ctx* c)
-{
-    return c->classes.size() == 1 && c->classes[0].nsci > 0 && c->classes[0].maxnb <= kFinishBins;
-}
-
 // The science unwrap and apply of one class's instances.
 atmwfs_status launch_science(atmwfs_ctx* c, const Class& cl, cudaStream_t st)
 {
@@ -742,17 +734,11 @@ atmwfs_status launch_step(atmwfs_ctx* c)
         }
         // the class's science unwrap and apply on its own branch: a class that
         // finishes early unwraps beside the passes of the larger grids
-        if (finish_step(c)) {
-            const Class& cl = c->classes[0];
-            AW_CUDA(sci_finish(c->d_inst, c->d_sci, cl.nsci, cl.maxnb, cl.maxnout, c->d_step, c->d_iters, c->d_atan_tab,
-                               c->d_tickets, pass_pdl_ctas(c), cs));
-        } else {
-            AW_TRY(launch_science(c, c->classes[ci], cs));
-        }
+        AW_TRY(launch_science(c, c->classes[ci], cs));
         AW_CUDA(cudaEventRecord(c->gev[2 + ci], cs));
         AW_CUDA(cudaStreamWaitEvent(c->st, c->gev[2 + ci], 0));
     }
-    if (!finish_step(c)) AW_CUDA(step_advance(c->d_step, c->st));
+    AW_CUDA(step_advance(c->d_step, c->st));
     return ATMWFS_OK;
 }
 
@@ -1243,8 +1229,6 @@ atmwfs_status atmwfs_create(const atmwfs_params* p, atmwfs_ctx** out)
         CKC(cudaMemcpy(c->d_inst, c->hinst.data(), sizeof(InstDev) * c->hinst.size(), cudaMemcpyHostToDevice));
         c->nsci = (int)sci.size();
         if (c->nsci) {
-            CK(dalloc(c, (void**)&c->d_tickets, sizeof(unsigned) * (sci.size() + 1)));
-            CKC(cudaMemset(c->d_tickets, 0, sizeof(unsigned) * (sci.size() + 1)));
             CK(dalloc(c, (void**)&c->d_sci, sizeof(int) * sci.size()));
             CKC(cudaMemcpy(c->d_sci, sci.data(), sizeof(int) * sci.size(), cudaMemcpyHostToDevice));
             std::vector<float2> tab(kAtanTabN + 1);
