@@ -73,8 +73,12 @@ bool fused_supported(int grid, int modes, int width, int proj, int nout);
 cudaError_t xdft_fused(const __nv_bfloat16* F, const float* H, float* a, int B, unsigned* status, cudaStream_t st);
 cudaError_t yfwd_fused(const __nv_bfloat16* F, const float* a, float* z, int B, unsigned* status, cudaStream_t st);
 cudaError_t yinv_fused(const __nv_bfloat16* G, const float* y, float* bb, int B, unsigned* status, cudaStream_t st);
+bool lift_supported(int nin);
+cudaError_t lift_fused(const __nv_bfloat16* W, const float* X, float* h, const float* bias, const __nv_bfloat16* F, float* a,
+                       int B, unsigned* status, cudaStream_t st);
 cudaError_t fourier_fused(const __nv_bfloat16* W, const __nv_bfloat16* Gt, const float* X, const float* bb, float* U,
-                          float* act, const float* bias, int B, unsigned* status, bool write_u, cudaStream_t st);
+                          float* act, const float* bias, const __nv_bfloat16* F, float* a, int B, unsigned* status,
+                          bool write_u, cudaStream_t st);
 cudaError_t project_fused(const __nv_bfloat16* W1, const float* c1, const __nv_bfloat16* W2, const float* c2,
                           const float* X, float* qpre, float* out, int B, unsigned* status, bool keep,
                           cudaStream_t st);
@@ -676,8 +680,9 @@ static cudaError_t gemm_args(GemmArgs& g, float beta, cudaStream_t st)
     return gemm_launch(g, beta, st);
 }
 
-// spectral convolution of layer l: spec = S_l(h); spec NULL: up to bb, the
-// image before the inverse transform along x (which k_fourier applies)
+// spectral convolution of layer l: spec = S_l(h); spec NULL: from a, the DFT
+// along x that came with h, to bb, the image before the inverse transform along
+// x (which k_fourier applies)
 atmwfs_status spectral_fwd(atmwfs_fno* f, int l, const void* h, int h_bf16, float* spec, int B, cudaStream_t st)
 {
     const atmwfs_fno_cfg& c = f->cfg;
@@ -687,8 +692,7 @@ atmwfs_status spectral_fwd(atmwfs_fno* f, int l, const void* h, int h_bf16, floa
     float* z = f->z[l];
     const bool tcx = umma_enabled() && xspectral_umma_supported(2 * m, G) && xspectral_umma_supported(G, 2 * m);
     {   // a[p][y][bc][kx] = sum_x h[bc][y][x] Fx[x][p m + kx]
-        if (!spec) {
-            FN_CUDA(xdft_fused(f->FxT_bf, (const float*)h, a, B, umma_status_ptr(), st));
+        if (!spec) {  // written with h
         } else if (tcx && !h_bf16 &&
             xspectral_umma(f->FxT_bf, 2 * m, G, (const float*)h, 0, G, 0, G, 0, a, G, Nc, m, m, (long)G * Nc, BW * G,
                            umma_status_ptr(), 0, st) == cudaSuccess) {
@@ -832,14 +836,21 @@ atmwfs_status forward(atmwfs_fno* f, const float* x, float* out, int B, cudaStre
                     pointwise_umma_supported(c.proj, c.width))
                        ? 1
                        : 0;
-    FN_CUDA(pointwise_fwd(pb + f->L.lift_W, c.width, c.nin, x, 0, f->h[0], B, P, 0.0f, pf + f->L.lift_b, st));
-    if (!bf && fused_shape(c)) {
-        unsigned* status = umma_status_ptr();
-        if (!status) return err(ATMWFS_ERR_CUDA, "status symbol");
+    const bool fused = !bf && fused_shape(c);
+    unsigned* status = fused ? umma_status_ptr() : nullptr;
+    if (fused && !status) return err(ATMWFS_ERR_CUDA, "status symbol");
+    if (fused && lift_supported(c.nin)) {
+        FN_CUDA(lift_fused(pb + f->L.lift_W, x, f->h[0], pf + f->L.lift_b, f->FxT_bf, f->a[0], B, status, st));
+    } else {
+        FN_CUDA(pointwise_fwd(pb + f->L.lift_W, c.width, c.nin, x, 0, f->h[0], B, P, 0.0f, pf + f->L.lift_b, st));
+        if (fused) FN_CUDA(xdft_fused(f->FxT_bf, f->h[0], f->a[0], B, status, st));
+    }
+    if (fused) {
         for (int l = 0; l < c.layers; l++) {
             FN_TRY(spectral_fwd(f, l, f->h[l], 0, nullptr, B, st));
-            FN_CUDA(fourier_fused(pb + f->L.W[l], f->GxT_bf, f->h[l], f->bb, f->u[l], l + 1 < c.layers ? f->h[l + 1] : nullptr,
-                                  pf + f->L.b[l], B, status, training, st));
+            const bool act = l + 1 < c.layers;
+            FN_CUDA(fourier_fused(pb + f->L.W[l], f->GxT_bf, f->h[l], f->bb, f->u[l], act ? f->h[l + 1] : nullptr,
+                                  pf + f->L.b[l], f->FxT_bf, act ? f->a[l + 1] : nullptr, B, status, training, st));
         }
         FN_CUDA(project_fused(pb + f->L.proj1_W, pf + f->L.proj1_b, pb + f->L.proj2_W, pf + f->L.proj2_b, last_h(f), f->qpre,
                               out, B, status, training, st));

@@ -2,10 +2,12 @@
 // projection 128) as kernels that fuse neighbouring products on the tcgen05
 // tensor cores, so that the images between them are not written and read
 // back:
-//   k_xdft     the forward DFT along x, written as coalesced spectrum rows;
+//   k_xdft     the forward DFT along x, written as coalesced spectrum rows
+//              (of the lift's output, for a number of input planes other than 8);
 //   k_yfwd, k_yinv  the DFTs along y;
-//   k_fourier  pointwise mixing + inverse DFT along x (+ bias, GELU), and the
-//              same pair of the backward pass;
+//   k_fourier  pointwise mixing + inverse DFT along x (+ bias, GELU, and the
+//              next layer's forward DFT along x), the lift with its DFT, and
+//              the same pair of the backward pass;
 //   k_project  the first projection + GELU + the 2-channel output;
 //   k_layer_bwd  a layer's GELU gradient, its weight and bias gradients and
 //              the transposed inverse DFT along x, from one read of the line;
@@ -102,7 +104,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_xdft(const __nv_bfloat16* __res
                                                       float* __restrict__ a, int nlines, long Nc, unsigned* status)
 {
     constexpr int J = kW * kXK / kThreads;  // pieces per thread
-    extern __shared__ __align__(1024) unsigned char sm[];
+    extern __shared__ __align__(128) unsigned char sm[];
     unsigned char *sa = sm, *sb = sm + kXBytes;  // the line, F
     __shared__ __align__(8) uint64_t bar;
     __shared__ uint32_t tmem_base;
@@ -180,7 +182,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_yfwd(const __nv_bfloat16* __res
 {
     constexpr int J = kYC / 16;       // pieces of 8 rows per thread
     constexpr int NC = kYK / kYC;
-    extern __shared__ __align__(1024) unsigned char sm[];
+    extern __shared__ __align__(128) unsigned char sm[];
     __shared__ __align__(8) uint64_t bar;
     __shared__ uint32_t tmem_base;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -256,7 +258,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_yinv(const __nv_bfloat16* __res
                                                       float* __restrict__ bb, long P, int ntiles, unsigned* status)
 {
     constexpr int K = 2 * kModes, J = K / 16;
-    extern __shared__ __align__(1024) unsigned char sm[];
+    extern __shared__ __align__(128) unsigned char sm[];
     __shared__ __align__(8) uint64_t bar;
     __shared__ uint32_t tmem_base;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -328,33 +330,66 @@ __global__ void __launch_bounds__(kThreads, 4) k_yinv(const __nv_bfloat16* __res
 // and the line's spectrum are loaded while the previous tile's products run.
 // The backward pass of a layer ends with the same pair: dh = W^T du + Fx da
 // (TW: W transposed; Gt = Fx; no bias).
+//
+// DFT: the next layer's forward DFT along x, from the same registers:
+//   D3 = act F^T   (64 channels x 64, K = 256 x, half a line per tile)
+// The epilogue leaves the tile's BF16 values in shared memory (two pixels of
+// a channel per word: neighbouring lanes trade one value), their products are
+// issued with the next tile's and the line's spectrum is stored after them, so
+// that nothing more is waited for.  At a batch of 16, k_fourier 137 us and a
+// k_xdft of 76 us (which read 268 MB again) became 193 us; the lift, 72 us
+// and 76, became 70 us.
+// KX = 8 without SPEC is the lift (K padded to 16 with zero channels; no
+// activation).
 // ---------------------------------------------------------------------------
-constexpr int kFK = kW / 8;  // core matrices along K (both products)
-constexpr uint32_t kFW = 0, kFG = kFW + kW * kW * 2, kFA = kFG + kG * kW * 2, kFB = kFA + kM * kW * 2,
-                   kFBytes = kFB + kW * kW * 2;
+constexpr int kFK = kW / 8;  // core matrices along a K of 64
 
-template <bool TW>
-__global__ void __launch_bounds__(kThreads, 2)
+// A stored pixel pair is one word per lane: 8-pixel groups 1056 bytes apart
+// put a warp's four groups x two channels into all 32 banks.
+constexpr uint32_t kHL = kW / 8 * 128 + 32;
+__device__ __forceinline__ uint32_t h_off(int ch, int px)
+{
+    return (uint32_t)((px >> 3) * kHL + (ch >> 3) * 128 + (ch & 7) * 16 + (px & 7) * 2);
+}
+
+// shared-memory offsets: W, Gt, the tile's X, the line's spectrum, then the
+// tile's outputs (whose MMA rows 64 .. 127 read on into F) and F
+template <bool SPEC, int KX, bool DFT>
+struct FourierSmem {
+    static constexpr int K = KX < 16 ? 16 : KX, KC = K / 8;
+    static constexpr uint32_t w = 0, g = w + kW * K * 2, x = g + (SPEC ? kG * kW * 2 : 0), s = x + kM * K * 2,
+                              h = s + (SPEC ? kW * kW * 2 : 0), f = h + (DFT ? kM / 8 * kHL : 0),
+                              bytes = f + (DFT ? kXBytes : 0);
+};
+
+template <bool TW, bool SPEC, int KX, bool DFT>
+__global__ void __launch_bounds__(kThreads, SPEC ? 2 : 3)
     k_fourier(const __nv_bfloat16* __restrict__ W, const __nv_bfloat16* __restrict__ Gt, const float* __restrict__ X,
               const float* __restrict__ bb, float* __restrict__ U, float* __restrict__ act,
-              const float* __restrict__ bias, int nlines, long Nc, unsigned* status, int write_u)
+              const float* __restrict__ bias, const __nv_bfloat16* __restrict__ F, float* __restrict__ a, int nlines,
+              long Nc, unsigned* status, int write_u)
 {
-    extern __shared__ __align__(1024) unsigned char sm[];
+    using S = FourierSmem<SPEC, KX, DFT>;
+    constexpr int KC = S::KC, J = S::K / 16, GC = kFK;
+    constexpr uint32_t kD3 = SPEC ? 2 * kW : kW, kCols = DFT && SPEC ? 256 : 128;
+    extern __shared__ __align__(128) unsigned char sm[];
     __shared__ __align__(8) uint64_t bar;
     __shared__ uint32_t tmem_base;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int m = tid % kM, kc0 = tid / kM;  // this thread's pixel and first channel group (of 8): kc0, kc0 + 2, ...
     const int so = tid & 63, sk = tid >> 6;  // its spectrum channel, and mode groups (of 8) sk, sk + 4
     const size_t BW = (size_t)Nc / kModes;
-    float x[4][8], s[2][8];
+    float x[J][8], s[2][8];
     auto load_x = [&](int line, int half) {
-        const float* src = X + (size_t)(line / kG) * kW * kP + (size_t)(line % kG) * kG + half * kM + m;
+        const float* src = X + (size_t)(line / kG) * KX * kP + (size_t)(line % kG) * kG + half * kM + m;
 #pragma unroll
-        for (int j = 0; j < 4; j++)
+        for (int j = 0; j < J; j++)
 #pragma unroll
-            for (int q = 0; q < 8; q++) x[j][q] = __ldg(src + (size_t)((kc0 + 2 * j) * 8 + q) * kP);
+            for (int q = 0; q < 8; q++)
+                x[j][q] = KX >= 16 || kc0 == 0 ? __ldg(src + (size_t)((kc0 + 2 * j) * 8 + q) * kP) : 0.0f;
     };
     auto load_s = [&](int line) {
+        if (!SPEC) return;
         const float* src = bb + (size_t)(line % kG) * Nc + (size_t)sk * 8 * BW + (size_t)(line / kG) * kW + so;
 #pragma unroll
         for (int j = 0; j < 2; j++)  // j: real, imaginary plane
@@ -365,32 +400,53 @@ __global__ void __launch_bounds__(kThreads, 2)
         load_x(blockIdx.x, 0);
         load_s(blockIdx.x);
     }
-    tmem_alloc(&tmem_base, 128, warp);
+    tmem_alloc(&tmem_base, kCols, warp);
     if (tid == 0) mbar_init(&bar);
     // the weights: element loads (a parameter block carries no alignment guarantee)
-    for (int i = tid; i < kW * kW; i += kThreads)
-        *reinterpret_cast<__nv_bfloat16*>(sm + kFW + (TW ? kmajor_off(i % kW, i / kW, kFK) : kmajor_off(i / kW, i % kW, kFK))) = W[i];
-    for (int i = tid; i < kG * kFK; i += kThreads) {
-        const int row = (i >> 6) * 8 + (i & 7), k8 = (i >> 3) & 7;
-        *reinterpret_cast<uint4*>(sm + kFG + kmajor_off(row, k8 * 8, kFK)) =
-            *reinterpret_cast<const uint4*>(Gt + (size_t)row * kW + k8 * 8);
+    for (int i = tid; i < kW * S::K; i += kThreads) {
+        const int row = i / S::K, k = i % S::K;  // TW: of W^T
+        *reinterpret_cast<__nv_bfloat16*>(sm + S::w + kmajor_off(TW ? k : row, TW ? row : k, KC)) =
+            k < KX ? W[row * KX + k] : __float2bfloat16_rn(0.0f);
     }
+    if (SPEC)
+        for (int i = tid; i < kG * GC; i += kThreads) {
+            const int row = (i >> 6) * 8 + (i & 7), k8 = (i >> 3) & 7;
+            *reinterpret_cast<uint4*>(sm + S::g + kmajor_off(row, k8 * 8, GC)) =
+                *reinterpret_cast<const uint4*>(Gt + (size_t)row * kW + k8 * 8);
+        }
+    if (DFT)
+        for (int i = tid; i < 2 * kModes * kXK; i += kThreads) {
+            int row, k8;
+            x_piece(tid, i / kThreads, row, k8);
+            *reinterpret_cast<uint4*>(sm + S::f + kmajor_off(row, k8 * 8, kXK)) =
+                *reinterpret_cast<const uint4*>(F + (size_t)row * kG + k8 * 8);
+        }
     fence_before();
     __syncthreads();
     fence_after();
     const uint32_t tmem = tmem_base, base = smem_addr(sm);
+    // the products of the last tile's outputs, K = its half of x (one thread issues)
+    auto dft = [&](int half) {
+#pragma unroll
+        for (int ks = 0; ks < kM / 16; ks++)
+            mma_bf16(tmem + kD3, smem_desc(base + S::h + ks * 2 * kHL, kHL, 128),
+                     smem_desc(base + S::f + half * (kM / 8) * 128 + ks * 256, 128, kXK * 128), instr_desc(kW),
+                     half > 0 || ks > 0);
+    };
     uint32_t parity = 0;
+    bool failed = false;
+    int last = -1;  // the line whose second half is in shared memory
     const int ntiles = 2 * nlines;
     // tiles in pairs: both halves of a line, then the CTA's next line
     for (int tile = 2 * blockIdx.x; tile < ntiles; tile += (tile & 1) ? 2 * (int)gridDim.x - 1 : 1) {
         const int line = tile >> 1, half = tile & 1;
 #pragma unroll
-        for (int j = 0; j < 4; j++)
-            *reinterpret_cast<uint4*>(sm + kFA + kmajor_off(m, (kc0 + 2 * j) * 8, kFK)) = pack8(x[j]);
-        if (half == 0) {
+        for (int j = 0; j < J; j++)
+            *reinterpret_cast<uint4*>(sm + S::x + kmajor_off(m, (kc0 + 2 * j) * 8, KC)) = pack8(x[j]);
+        if (SPEC && half == 0) {
 #pragma unroll
             for (int j = 0; j < 2; j++)
-                *reinterpret_cast<uint4*>(sm + kFB + kmajor_off(so, (sk + 4 * j) * 8, kFK)) = pack8(s[j]);
+                *reinterpret_cast<uint4*>(sm + S::s + kmajor_off(so, (sk + 4 * j) * 8, GC)) = pack8(s[j]);
         }
         publish_smem();
         if (half == 0) {
@@ -401,17 +457,24 @@ __global__ void __launch_bounds__(kThreads, 2)
         }
         if (tid == 0) {
 #pragma unroll
-            for (int ks = 0; ks < kW / 16; ks++)
-                mma_bf16(tmem, smem_desc(base + kFA + ks * 256, 128, kFK * 128),
-                         smem_desc(base + kFW + ks * 256, 128, kFK * 128), instr_desc(kW), ks > 0);
+            for (int ks = 0; ks < S::K / 16; ks++)
+                mma_bf16(tmem, smem_desc(base + S::x + ks * 256, 128, KC * 128),
+                         smem_desc(base + S::w + ks * 256, 128, KC * 128), instr_desc(kW), ks > 0);
+            if (SPEC) {
 #pragma unroll
-            for (int ks = 0; ks < kW / 16; ks++)
-                mma_bf16(tmem + kW, smem_desc(base + kFG + half * (kM / 8) * kFK * 128 + ks * 256, 128, kFK * 128),
-                         smem_desc(base + kFB + ks * 256, 128, kFK * 128), instr_desc(kW), ks > 0);
+                for (int ks = 0; ks < kW / 16; ks++)
+                    mma_bf16(tmem + kW, smem_desc(base + S::g + half * (kM / 8) * GC * 128 + ks * 256, 128, GC * 128),
+                             smem_desc(base + S::s + ks * 256, 128, GC * 128), instr_desc(kW), ks > 0);
+            }
+            if (DFT && (half == 1 || last >= 0)) dft(half ^ 1);
             mma_commit(&bar);
         }
-        if (!mma_wait(&bar, parity, status)) break;
+        if (!mma_wait(&bar, parity, status)) {
+            failed = true;
+            break;
+        }
         parity ^= 1;
+        if (DFT && half == 0 && last >= 0 && (warp & 3) < 2) store_spectrum<2>(tmem + kD3, a, last, Nc, warp, lane);
         const int g = warp & 3, ch = warp >> 2;
         const uint32_t trow = tmem + ((uint32_t)(g * 32) << 16);
         const size_t o0 = (size_t)(line / kG) * kW * kP + (size_t)(line % kG) * kG + half * kM + g * 32 + lane;
@@ -419,18 +482,39 @@ __global__ void __launch_bounds__(kThreads, 2)
         for (int c0 = ch * (kW / 2); c0 < (ch + 1) * (kW / 2); c0 += 16) {
             float r[16], sp[16];
             tmem_ld16(trow + c0, r);
-            tmem_ld16(trow + kW + c0, sp);
+            if (SPEC) tmem_ld16(trow + kW + c0, sp);
 #pragma unroll
             for (int q = 0; q < 16; q++) {
                 const size_t o = o0 + (size_t)(c0 + q) * kP;
-                const float u = (r[q] + (bias ? __ldg(bias + c0 + q) : 0.0f)) + sp[q];
+                float u = r[q] + (bias ? __ldg(bias + c0 + q) : 0.0f);
+                if (SPEC) u += sp[q];
                 if (write_u) U[o] = u;
-                if (act) act[o] = gelu_f(u);
+                if (SPEC && act) act[o] = u = gelu_f(u);
+                r[q] = u;
+            }
+            if (DFT) {
+                const bool odd = lane & 1;
+#pragma unroll
+                for (int q = 0; q < 16; q += 2) {  // even lanes: channel q, odd lanes: q + 1; pixels lane & ~1, + 1
+                    const float other = __shfl_xor_sync(0xFFFFFFFFu, odd ? r[q] : r[q + 1], 1);
+                    *reinterpret_cast<__nv_bfloat162*>(sm + S::h + h_off(c0 + q + odd, g * 32 + (lane & ~1))) =
+                        __floats2bfloat162_rn(odd ? other : r[q], odd ? r[q + 1] : other);
+                }
             }
         }
+        if (half == 1) last = line;
         retire_tile();
     }
-    tmem_free(tmem, 128, warp);
+    if (DFT && !failed && last >= 0) {  // the CTA's last line
+        publish_smem();
+        if (tid == 0) {
+            dft(1);
+            mma_commit(&bar);
+        }
+        if (mma_wait(&bar, parity, status) && (warp & 3) < 2) store_spectrum<2>(tmem + kD3, a, last, Nc, warp, lane);
+        fence_before();
+    }
+    tmem_free(tmem, kCols, warp);
 }
 
 // ---------------------------------------------------------------------------
@@ -474,7 +558,7 @@ __global__ void __launch_bounds__(kBT, 1)
     constexpr int JH = HC == kW ? J : 1;         // pieces of h per thread
     constexpr int CN = HN / 4;                   // dW columns per reading thread (4 warps per lane block)
     static_assert(HC == kW || HC * kXK <= kBT, "h in one piece per thread");
-    extern __shared__ __align__(1024) unsigned char sm[];
+    extern __shared__ __align__(128) unsigned char sm[];
     unsigned char *sd = sm, *sg = sm + kXBytes, *sh = sm + 2 * kXBytes;  // du, Gx, h
     __shared__ __align__(8) uint64_t bar;
     __shared__ uint32_t tmem_base;
@@ -622,7 +706,7 @@ __global__ void __launch_bounds__(kBT, 1)
                   float* __restrict__ dc1, float* __restrict__ dW2, float* __restrict__ dc2, int nlines, unsigned* status)
 {
     constexpr int J = kW * kXK / kBT;  // pieces of 64 channels of a line per thread
-    extern __shared__ __align__(1024) unsigned char sm[];
+    extern __shared__ __align__(128) unsigned char sm[];
     __shared__ __align__(8) uint64_t bar;
     __shared__ uint32_t tmem_base;
     __shared__ __align__(16) float s_d[2][2][kG];  // dout of a line, rounded to BF16, double-buffered
@@ -789,7 +873,7 @@ __global__ void __launch_bounds__(kThreads, 3)
               const float* __restrict__ c2, const float* __restrict__ X, float* __restrict__ qpre, float* __restrict__ out,
               int ntiles, unsigned* status, int keep)
 {
-    extern __shared__ __align__(1024) unsigned char sm[];
+    extern __shared__ __align__(128) unsigned char sm[];
     __shared__ __align__(8) uint64_t bar;
     __shared__ uint32_t tmem_base;
     __shared__ float s_c1[kProj], s_w2[2][kProj], s_half[2][kM];
@@ -920,29 +1004,48 @@ cudaError_t yinv_fused(const __nv_bfloat16* G, const float* y, float* bb, int B,
     return cudaGetLastError();
 }
 
-cudaError_t fourier_fused(const __nv_bfloat16* W, const __nv_bfloat16* Gt, const float* X, const float* bb, float* U,
-                          float* act, const float* bias, int B, unsigned* status, bool write_u, cudaStream_t st)
+namespace umma {
+template <bool TW, bool SPEC, int KX, bool DFT>
+cudaError_t launch_fourier(const __nv_bfloat16* W, const __nv_bfloat16* Gt, const float* X, const float* bb, float* U, float* act,
+                           const float* bias, const __nv_bfloat16* F, float* a, int B, unsigned* status, bool write_u,
+                           cudaStream_t st)
 {
-    using namespace umma;
-    const cudaError_t e = allow_smem(k_fourier<false>, kFBytes);
+    constexpr uint32_t bytes = FourierSmem<SPEC, KX, DFT>::bytes;
+    const auto kern = k_fourier<TW, SPEC, KX, DFT>;
+    const cudaError_t e = allow_smem(kern, bytes);
     if (e != cudaSuccess) return e;
-    const int lines = B * kG, grid = lines < 2 * sm_count() ? lines : 2 * sm_count();
-    k_fourier<false><<<grid, kThreads, kFBytes, st>>>(W, Gt, X, bb, U, act, bias, lines, (long)B * kW * kModes, status,
-                                                      write_u || !act);
+    const int lines = B * kG, ctas = (SPEC ? 2 : 3) * sm_count(), grid = lines < ctas ? lines : ctas;
+    kern<<<grid, kThreads, bytes, st>>>(W, Gt, X, bb, U, act, bias, F, a, lines, (long)B * kW * kModes, status, write_u);
     return cudaGetLastError();
+}
+}  // namespace umma
+
+// h = W x + bias of 8 input planes, and its forward DFT along x (F: 2 m x G).
+bool lift_supported(int nin) { return nin == 8; }
+
+cudaError_t lift_fused(const __nv_bfloat16* W, const float* X, float* h, const float* bias, const __nv_bfloat16* F, float* a,
+                       int B, unsigned* status, cudaStream_t st)
+{
+    return umma::launch_fourier<false, false, 8, true>(W, nullptr, X, nullptr, h, nullptr, bias, F, a, B, status, true, st);
+}
+
+// act NULL: the last layer (no activation, and no layer that wants its DFT).
+cudaError_t fourier_fused(const __nv_bfloat16* W, const __nv_bfloat16* Gt, const float* X, const float* bb, float* U,
+                          float* act, const float* bias, const __nv_bfloat16* F, float* a, int B, unsigned* status,
+                          bool write_u, cudaStream_t st)
+{
+    if (!act)
+        return umma::launch_fourier<false, true, umma::kW, false>(W, Gt, X, bb, U, act, bias, nullptr, nullptr, B, status, true,
+                                                                  st);
+    return umma::launch_fourier<false, true, umma::kW, true>(W, Gt, X, bb, U, act, bias, F, a, B, status, write_u, st);
 }
 
 // dX = W^T dU + the transposed forward DFT along x of da (Fx: G x 2 m)
 cudaError_t fourier_bwd_fused(const __nv_bfloat16* W, const __nv_bfloat16* Fx, const float* dU, const float* da, float* dX,
                               int B, unsigned* status, cudaStream_t st)
 {
-    using namespace umma;
-    const cudaError_t e = allow_smem(k_fourier<true>, kFBytes);
-    if (e != cudaSuccess) return e;
-    const int lines = B * kG, grid = lines < 2 * sm_count() ? lines : 2 * sm_count();
-    k_fourier<true><<<grid, kThreads, kFBytes, st>>>(W, Fx, dU, da, dX, nullptr, nullptr, lines, (long)B * kW * kModes,
-                                                     status, 1);
-    return cudaGetLastError();
+    return umma::launch_fourier<true, true, umma::kW, false>(W, Fx, dU, da, dX, nullptr, nullptr, nullptr, nullptr, B, status,
+                                                             true, st);
 }
 
 // u NULL: no activation (du is dh and is not written).  dW and db accumulate.
