@@ -71,7 +71,7 @@ cudaError_t spectral_umma(const __nv_bfloat16* W, int o, int c, const float* X, 
 // fused forward kernels of the default shape (fno_fused.cu)
 bool fused_supported(int grid, int modes, int width, int proj, int nout);
 cudaError_t xdft_fused(const __nv_bfloat16* F, const float* H, float* a, int B, unsigned* status, cudaStream_t st);
-cudaError_t yfwd_fused(const __nv_bfloat16* F, const float* a, float* z, int B, unsigned* status, cudaStream_t st);
+cudaError_t yfwd_fused(const __nv_bfloat16* F, const float* a, float* z, int B, unsigned* status, bool split, cudaStream_t st);
 cudaError_t yinv_fused(const __nv_bfloat16* G, const float* y, float* bb, int B, unsigned* status, cudaStream_t st);
 bool lift_supported(int nin);
 cudaError_t lift_fused(const __nv_bfloat16* W, const float* X, float* h, const float* bias, const __nv_bfloat16* F, float* a,
@@ -108,7 +108,7 @@ struct atmwfs_fno {
     __nv_bfloat16 *FyAB_bf = nullptr, *GyBig_bf = nullptr;
     __nv_bfloat16 *FxT_bf = nullptr, *GxT_bf = nullptr;  // the x transforms transposed (N x K)
     // the transposed products of the backward pass
-    __nv_bfloat16 *Fx_bf = nullptr, *Gx_bf = nullptr, *FyABT_bf = nullptr;
+    __nv_bfloat16 *Fx_bf = nullptr, *Gx_bf = nullptr;
     // activations for one batch size
     int cap = 0;
     std::vector<float*> h, u, a, z;     // h[0..nl], u[0..nl-1], a/z per layer
@@ -605,12 +605,9 @@ atmwfs_status build_dft(atmwfs_fno* f)
             FxT[(size_t)n * G + x] = Fx[(size_t)x * 2 * m + n];
             GxT[(size_t)x * 2 * m + n] = Gx[(size_t)n * G + x];
         }
-    std::vector<float> FyABT((size_t)2 * G * 2 * m);
-    for (int r = 0; r < 2 * m; r++)
-        for (int k = 0; k < 2 * G; k++) FyABT[(size_t)k * 2 * m + r] = FyAB[(size_t)r * 2 * G + k];
     struct MB { __nv_bfloat16** d; std::vector<float>* h; } bmats[] = {
         {&f->FyAB_bf, &FyAB}, {&f->GyBig_bf, &GyBig}, {&f->FxT_bf, &FxT}, {&f->GxT_bf, &GxT},
-        {&f->Fx_bf, &Fx},     {&f->Gx_bf, &Gx},       {&f->FyABT_bf, &FyABT}};
+        {&f->Fx_bf, &Fx},     {&f->Gx_bf, &Gx}};
     for (auto& mm : bmats) {
         std::vector<__nv_bfloat16> hb(mm.h->size());
         for (size_t i = 0; i < hb.size(); i++) hb[i] = __float2bfloat16_rn((*mm.h)[i]);
@@ -708,7 +705,7 @@ atmwfs_status spectral_fwd(atmwfs_fno* f, int l, const void* h, int h_bf16, floa
     // z = FyAB a: [2m, 2G] x [2G, Nc], on tcgen05 where compiled
     const bool tc = umma_enabled() && Nc % 8 == 0;
     if (!spec)
-        FN_CUDA(yfwd_fused(f->FyAB_bf, a, z, B, umma_status_ptr(), st));
+        FN_CUDA(yfwd_fused(f->FyAB_bf, a, z, B, umma_status_ptr(), false, st));
     else if (tc && spectral_umma_supported(2 * m, 2 * G))
         FN_CUDA(spectral_umma(f->FyAB_bf, 2 * m, 2 * G, a, z, Nc, umma_status_ptr(), 0, st));
     else
@@ -884,13 +881,12 @@ atmwfs_status layer_bwd(atmwfs_fno* f, int l, const float* dh, float* dX, int B,
         return err(ATMWFS_ERR_INVALID, "batch %d x width %d exceeds the mode-mixing shared memory", B, c.width);
     FN_CUDA(layer_bwd_fused(f->Gx_bf, dh, act ? f->u[l] : nullptr, f->h[l], f->du, f->dbb, f->grads + f->L.W[l],
                             f->grads + f->L.b[l], B, status, st));
-    // dy = GyBig^T dbb: [2m, 2G] x [2G, Nc]
-    FN_CUDA(gemm(2 * m, (int)Nc, 2 * G, f->GyBig, 2 * m, 1, 0, f->dbb, Nc, 0, 0, f->dy, Nc, 0.0f, 1, 0, 0, 0, nullptr, 0,
-                 st));
+    // dy = GyBig^T dbb: [2m, 2G] x [2G, Nc] (GyBig^T = FyAB)
+    FN_CUDA(yfwd_fused(f->FyAB_bf, f->dbb, f->dy, B, status, true, st));
     k_modemix_bwd64<8><<<m * m, 256, 0, st>>>(f->pbf + f->L.R[l], f->z[l], f->dy, f->dz, f->grads + f->L.R[l], B, m);
     FN_CUDA(cudaGetLastError());
-    // da = FyAB^T dz: [2G, 2m] x [2m, Nc]
-    FN_CUDA(yinv_fused(f->FyABT_bf, f->dz, f->da, B, status, st));
+    // da = FyAB^T dz: [2G, 2m] x [2m, Nc] (FyAB^T = GyBig)
+    FN_CUDA(yinv_fused(f->GyBig_bf, f->dz, f->da, B, status, st));
     FN_CUDA(fourier_bwd_fused(f->pbf + f->L.W[l], f->Fx_bf, du, f->da, dX, B, status, st));
     return ATMWFS_OK;
 }

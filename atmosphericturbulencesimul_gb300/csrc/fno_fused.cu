@@ -171,17 +171,24 @@ __global__ void __launch_bounds__(kThreads, 2) k_xdft(const __nv_bfloat16* __res
 // gives each CTA a quarter of the output rows, so that four CTAs share an SM
 // and its 512 columns of tensor memory (one CTA per SM held all 512 rows
 // before, 256 tiles on 152 CTAs: 31 us).
+// The backward pass has the same two: dy = GyBig^T dbb, da = FyAB^T dz, and
+// GyBig^T is FyAB, value by value.  SPLIT (dy) keeps a chunk's products in an
+// accumulator of their own and adds the four in FP32, as the split product
+// did that this replaces (K = 128 per run, four atomic adds into a cleared dy:
+// 45 us for a batch of 8, now 21).
 // ---------------------------------------------------------------------------
 constexpr int kYK = 2 * kG;                      // K of the forward product
 constexpr int kYC = 128;                         // its chunk
 constexpr uint32_t kYA = 2 * kModes * kYK * 2;   // F: 64 KB, then the chunk's A tile: 32 KB
 constexpr uint32_t kYBytes = kYA + kM * kYC * 2;
 
+template <bool SPLIT>
 __global__ void __launch_bounds__(kThreads, 2) k_yfwd(const __nv_bfloat16* __restrict__ F, const float* __restrict__ X,
                                                       float* __restrict__ Z, long P, int ntiles, unsigned* status)
 {
     constexpr int J = kYC / 16;       // pieces of 8 rows per thread
     constexpr int NC = kYK / kYC;
+    constexpr int NA = SPLIT ? NC : 1;  // accumulators, 64 columns each
     extern __shared__ __align__(128) unsigned char sm[];
     __shared__ __align__(8) uint64_t bar;
     __shared__ uint32_t tmem_base;
@@ -196,7 +203,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_yfwd(const __nv_bfloat16* __res
     if (blockIdx.x < ntiles)
 #pragma unroll
         for (int j = 0; j < J; j++) load(blockIdx.x, 0, j);
-    tmem_alloc(&tmem_base, 64, warp);
+    tmem_alloc(&tmem_base, 64 * NA, warp);
     if (tid == 0) mbar_init(&bar);
     for (int i = tid; i < 2 * kModes * kYK / 8; i += kThreads) {
         const int row = (i >> 9) * 8 + (i & 7), k8 = (i >> 3) & 63;
@@ -223,9 +230,9 @@ __global__ void __launch_bounds__(kThreads, 2) k_yfwd(const __nv_bfloat16* __res
             if (tid == 0) {
 #pragma unroll
                 for (int ks = 0; ks < kYC / 16; ks++)
-                    mma_bf16(tmem, smem_desc(base + kYA + ks * 256, 128, kYC / 8 * 128),
+                    mma_bf16(tmem + (SPLIT ? c * 64 : 0), smem_desc(base + kYA + ks * 256, 128, kYC / 8 * 128),
                              smem_desc(base + c * (kYC / 8) * 128 + ks * 256, 128, kYK / 8 * 128), instr_desc(2 * kModes),
-                             c > 0 || ks > 0);
+                             (!SPLIT && c > 0) || ks > 0);
                 mma_commit(&bar);
             }
             // the chunk's products are done before its A tile is overwritten
@@ -243,11 +250,18 @@ __global__ void __launch_bounds__(kThreads, 2) k_yfwd(const __nv_bfloat16* __res
             float r[16];
             tmem_ld16(tmem + ((uint32_t)(g * 32) << 16) + c0, r);
 #pragma unroll
+            for (int p = 1; p < NA; p++) {
+                float t[16];
+                tmem_ld16(tmem + ((uint32_t)(g * 32) << 16) + p * 64 + c0, t);
+#pragma unroll
+                for (int q = 0; q < 16; q++) r[q] += t[q];
+            }
+#pragma unroll
             for (int q = 0; q < 16; q++) o[(size_t)(c0 + q) * P] = r[q];
         }
         retire_tile();
     }
-    tmem_free(tmem, 64, warp);
+    tmem_free(tmem, 64 * NA, warp);
 }
 
 constexpr int kYQ = kYK / 4;                              // output rows per CTA
@@ -980,19 +994,20 @@ cudaError_t xdft_fused(const __nv_bfloat16* F, const float* H, float* a, int B, 
     return cudaGetLastError();
 }
 
-// z = F a, F 64 x 512 (FyAB)
-cudaError_t yfwd_fused(const __nv_bfloat16* F, const float* a, float* z, int B, unsigned* status, cudaStream_t st)
+// z = F a, F 64 x 512 (FyAB); split: K in four runs of 128 (dy)
+cudaError_t yfwd_fused(const __nv_bfloat16* F, const float* a, float* z, int B, unsigned* status, bool split, cudaStream_t st)
 {
     using namespace umma;
-    const cudaError_t e = allow_smem(k_yfwd, kYBytes);
+    const auto kern = split ? k_yfwd<true> : k_yfwd<false>;
+    const cudaError_t e = allow_smem(kern, kYBytes);
     if (e != cudaSuccess) return e;
     const long P = (long)B * kW * kModes;
     const int tiles = (int)(P / kM), grid = tiles < 2 * sm_count() ? tiles : 2 * sm_count();
-    k_yfwd<<<grid, kThreads, kYBytes, st>>>(F, a, z, P, tiles, status);
+    kern<<<grid, kThreads, kYBytes, st>>>(F, a, z, P, tiles, status);
     return cudaGetLastError();
 }
 
-// bb = G y, G 512 x 64 (GyBig, FyAB^T)
+// bb = G y, G 512 x 64 (GyBig)
 cudaError_t yinv_fused(const __nv_bfloat16* G, const float* y, float* bb, int B, unsigned* status, cudaStream_t st)
 {
     using namespace umma;
