@@ -351,8 +351,10 @@ __global__ void __launch_bounds__(kThreads, 4) k_yinv(const __nv_bfloat16* __res
 // a channel per word: neighbouring lanes trade one value), their products are
 // issued with the next tile's and the line's spectrum is stored after them, so
 // that nothing more is waited for.  At a batch of 16, k_fourier 137 us and a
-// k_xdft of 76 us (which read 268 MB again) became 193 us; the lift, 72 us
-// and 76, became 70 us.
+// k_xdft of 76 us (which read 268 MB again) became 168 us; the lift, 72 us
+// and 76, became 70 us.  The bias is read from shared memory: the tiles take
+// the L1 that the operands leave (28 KB), so each read of the global array went
+// to L2 (193 us).
 // KX = 8 without SPEC is the lift (K padded to 16 with zero channels; no
 // activation).
 // ---------------------------------------------------------------------------
@@ -389,6 +391,7 @@ __global__ void __launch_bounds__(kThreads, SPEC ? 2 : 3)
     extern __shared__ __align__(128) unsigned char sm[];
     __shared__ __align__(8) uint64_t bar;
     __shared__ uint32_t tmem_base;
+    __shared__ float s_bias[kW];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int m = tid % kM, kc0 = tid / kM;  // this thread's pixel and first channel group (of 8): kc0, kc0 + 2, ...
     const int so = tid & 63, sk = tid >> 6;  // its spectrum channel, and mode groups (of 8) sk, sk + 4
@@ -416,6 +419,7 @@ __global__ void __launch_bounds__(kThreads, SPEC ? 2 : 3)
     }
     tmem_alloc(&tmem_base, kCols, warp);
     if (tid == 0) mbar_init(&bar);
+    if (tid < kW) s_bias[tid] = bias ? bias[tid] : 0.0f;
     // the weights: element loads (a parameter block carries no alignment guarantee)
     for (int i = tid; i < kW * S::K; i += kThreads) {
         const int row = i / S::K, k = i % S::K;  // TW: of W^T
@@ -500,7 +504,7 @@ __global__ void __launch_bounds__(kThreads, SPEC ? 2 : 3)
 #pragma unroll
             for (int q = 0; q < 16; q++) {
                 const size_t o = o0 + (size_t)(c0 + q) * kP;
-                float u = r[q] + (bias ? __ldg(bias + c0 + q) : 0.0f);
+                float u = r[q] + s_bias[c0 + q];
                 if (SPEC) u += sp[q];
                 if (write_u) U[o] = u;
                 if (SPEC && act) act[o] = u = gelu_f(u);
