@@ -218,11 +218,14 @@ __global__ void k_mse(const float* __restrict__ out, const float* __restrict__ t
 // default shape.  A thread owns one (mode, output channel) and kMixB samples:
 // a weight is read from shared memory once for all of them and the samples'
 // values are broadcasts, two channels to a load (one thread per output value
-// read both operands for every product: 67 us).
+// read both operands for every product: 67 us).  Where the width is known the
+// weights, the first samples and, under the products, the next samples are
+// loaded in one go each: 25 us, and 29 with the weights in four batches and
+// the samples behind a barrier.
 constexpr int kMixB = 8;
 // WC: the width as a constant (0: the argument); the staging loops divide by it.
 template <int KX, int WC>
-__global__ void __launch_bounds__(256) k_modemix(const __nv_bfloat16* __restrict__ R, const float* __restrict__ z,
+__global__ void __launch_bounds__(256, WC ? 4 : 1) k_modemix(const __nv_bfloat16* __restrict__ R, const float* __restrict__ z,
                                                  float* __restrict__ y, int B, int width, int m, long sk, long sc)
 {
     const int w = WC ? WC : width;
@@ -234,21 +237,52 @@ __global__ void __launch_bounds__(256) k_modemix(const __nv_bfloat16* __restrict
     float* zs = reinterpret_cast<float*>(mix_smem);                                 // [KX][kMixB][w][2]
     __nv_bfloat162* rs = reinterpret_cast<__nv_bfloat162*>(zs + KX * kMixB * w * 2);  // [KX][w][w + 1]
     const __nv_bfloat162* Rk = reinterpret_cast<const __nv_bfloat162*>(R) + (size_t)(ky * m + kx0) * w * w;
+    // a block of samples' values: loaded (all in flight), then stored as (re, im)
+    constexpr int NV = WC ? kMixB * WC / 256 : 1;
+    float vr[NV][KX], vi[NV][KX];
+    auto load_z = [&](int b0, int i, int j) {
+        const long o = (long)(b0 * w + i) * sc;
+        const bool in = i < min(kMixB, B - b0) * w;
+#pragma unroll
+        for (int k = 0; k < KX; k++) {
+            vr[j][k] = in ? z[o + ore + k * sk] : 0.0f;
+            vi[j][k] = in ? z[o + oim + k * sk] : 0.0f;
+        }
+    };
+    auto store_z = [&](int i, int j) {
+#pragma unroll
+        for (int k = 0; k < KX; k++) reinterpret_cast<float2*>(zs)[k * kMixB * w + i] = make_float2(vr[j][k], vi[j][k]);
+    };
+    if constexpr (WC != 0) {
+        constexpr int NR = KX * WC * WC / 256;
+        __nv_bfloat162 rk[NR];
+#pragma unroll
+        for (int j = 0; j < NR; j++) rk[j] = Rk[threadIdx.x + 256 * j];
+#pragma unroll
+        for (int j = 0; j < NV; j++) load_z(0, threadIdx.x + 256 * j, j);
+#pragma unroll
+        for (int j = 0; j < NR; j++) {
+            const int i = threadIdx.x + 256 * j;
+            rs[i / w * (w + 1) + i % w] = rk[j];
+        }
+    } else {
 #pragma unroll 8
-    for (int i = threadIdx.x; i < KX * w * w; i += blockDim.x) rs[i / w * (w + 1) + i % w] = Rk[i];
+        for (int i = threadIdx.x; i < KX * w * w; i += blockDim.x) rs[i / w * (w + 1) + i % w] = Rk[i];
+    }
     for (int b0 = 0; b0 < B; b0 += kMixB) {
         const int nb = min(kMixB, B - b0);
         __syncthreads();  // the previous samples are used
-        for (int i = threadIdx.x; i < kMixB * w; i += blockDim.x) {
-            float vr[KX], vi[KX];
-            const long o = (long)(b0 * w + i) * sc;
+        if constexpr (WC != 0) {
 #pragma unroll
-            for (int k = 0; k < KX; k++) {
-                vr[k] = i < nb * w ? z[o + ore + k * sk] : 0.0f;
-                vi[k] = i < nb * w ? z[o + oim + k * sk] : 0.0f;
+            for (int j = 0; j < NV; j++) store_z(threadIdx.x + 256 * j, j);
+            if (b0 + kMixB < B)
+#pragma unroll
+                for (int j = 0; j < NV; j++) load_z(b0 + kMixB, threadIdx.x + 256 * j, j);
+        } else {
+            for (int i = threadIdx.x; i < kMixB * w; i += blockDim.x) {
+                load_z(b0, i, 0);
+                store_z(i, 0);
             }
-#pragma unroll
-            for (int k = 0; k < KX; k++) reinterpret_cast<float2*>(zs)[k * kMixB * w + i] = make_float2(vr[k], vi[k]);
         }
         __syncthreads();
         for (int it = threadIdx.x; it < KX * w * (kMixB / NB); it += blockDim.x) {
