@@ -4,7 +4,7 @@
 // do2dfft on the full M x M spectrum, :783).
 //
 // Rows: one CTA of 256 threads owns one row; each thread holds M / 256 values
-// in registers and the engine's Stockham stages (fft_rt) run three in-register
+// in registers and the engine's Stockham stages (fft3_ct) run three in-register
 // radix stages (16 x 16 x 16 for 4096, 32 x 16 x 16 for 8192) with two
 // exchanges through one padded shared row (68 KB at 8192).
 // Columns: in place of the array's layout, as two passes of short transforms
@@ -19,10 +19,19 @@
 
 namespace atmwfs {
 
-// One row per CTA; ds = -1 forward, +1 inverse.
+// One row per CTA; ds = -1 forward, +1 inverse.  HBM should bound it (1.07 GB at
+// 8192^2, 158 us); it takes 194 us (4096^2: 49).  The last radix stage leaves
+// neighbouring outputs in neighbouring threads, so they are stored from
+// registers: a third exchange to reorder them cost 25 us.  With the stages
+// compiled for the size and the registers bounded for kRowCtas CTAs per SM the
+// exchange addresses are constants and a second row's loads run under the
+// first's stages: 305 us on the runtime stage loop, 267 unbounded (one CTA of
+// 183 registers); three CTAs per SM spill at 8192 (362).
+template <int N> constexpr int kRowCtas = N > 4096 ? 2 : 4;
 template <int N>
-__global__ void __launch_bounds__(Plan<N>::T) k_fft_row_plan(const float2* __restrict__ in, float2* __restrict__ out,
-                                                             const float2* __restrict__ tw, float ds)
+__global__ void __launch_bounds__(Plan<N>::T, kRowCtas<N>) k_fft_row_plan(const float2* __restrict__ in,
+                                                                          float2* __restrict__ out,
+                                                                          const float2* __restrict__ tw, float ds)
 {
     constexpr int T = Plan<N>::T, E = Plan<N>::E, RL = last_radix<N>();
     extern __shared__ float4 big_smem[];
@@ -32,13 +41,11 @@ __global__ void __launch_bounds__(Plan<N>::T) k_fft_row_plan(const float2* __res
     float2 v[E];
 #pragma unroll
     for (int e = 0; e < E; e++) v[e] = in[row + t + e * T];
-    fft_rt<N, T, E>(v, xrow, t, tw, ds, 0);
-    __syncthreads();
+    if (ds > 0.0f) conj_all<E>(v);  // inverse = conj(forward(conj))
+    fft3_ct<N, T, E, Stages<N>::R0, Stages<N>::R1, Stages<N>::R2>(v, xrow, t, tw + tw_offset<N>(0, 1), tw + tw_offset<N>(0, 2));
+    if (ds > 0.0f) conj_all<E>(v);
 #pragma unroll
-    for (int s = 0; s < E; s++) xrow[padi(last_index<N, T, RL>(t, s))] = v[s];
-    __syncthreads();
-#pragma unroll
-    for (int e = 0; e < E; e++) out[row + t + e * T] = xrow[padi(t + e * T)];
+    for (int s = 0; s < E; s++) out[row + last_index<N, T, RL>(t, s)] = v[s];
 }
 
 // Column transforms of the M x M grid, M = N1 N2:
