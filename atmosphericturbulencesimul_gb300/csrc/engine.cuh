@@ -18,8 +18,9 @@ namespace atmwfs {
 // predecessor grids have completed and their memory is visible, and
 // launch_dependents then lets its own successors be scheduled.  The gate
 // comes before any global read and before any early return, so ordering
-// stays transitive along a chain.  Launched without the attribute, both
-// instructions return at once.
+// stays transitive along a chain.  (A propagation pass waits there too, but
+// lets its successor go only after its transforms: pass_pdl_ctas.)  Launched
+// without the attribute, both instructions return at once.
 #if defined(__CUDACC__)
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
@@ -35,8 +36,9 @@ __device__ __forceinline__ void pdl_gate()
 // hides (a 256^2 single-frame step: 29.1 -> 25.0 us).  Larger grids are
 // bound by throughput.  There, early-scheduled CTAs that wait resident take
 // SM slots from the step's concurrent branches: a 7-layer 512^2 step went
-// 0.107 -> 0.149 ms with the attribute on every launch.  ATMWFS_PDL=0 turns
-// the attribute off.
+// 0.107 -> 0.149 ms with the attribute on every launch.  (The propagation
+// passes and the unit operators go further, pass_pdl_ctas and kUnitPdlWaves.)
+// ATMWFS_PDL=0 turns the attribute off.
 inline int pdl_max_ctas()
 {
     static const int n = [] {

@@ -224,9 +224,7 @@ AW_HD void stage_store(const float2* v, float2* buf, int t)
     }
 }
 
-// The same with the stride NS known at run time (ns is a power of two): the
-// stage loop below runs every stage of every transform through one copy of
-// the code of each radix.  The stages are always forward (compile-time
+// The same with the stride NS known at run time (ns is a power of two).  The stages are always forward (compile-time
 // butterfly constants, the +-i rotations free); an inverse transform is the
 // conjugate of the forward transform of the conjugate.
 // tws: the stage's twiddle table tws[r * ns + k] = exp(-2 pi i k r / (ns R))
@@ -371,7 +369,9 @@ inline void build_twiddles(float2* out)
 }
 
 // Stage body (twiddles + butterflies) of radix r and stride ns for one
-// thread; a uniform branch selects the code of the radix.
+// thread, and the exchange between stages, with radix and stride at run time:
+// for a transform as a loop over its stages, as the CPU emulation has it (the
+// kernels compile the stages of their size).
 template <int N, int T, int E, int V = 0>
 AW_HD void stage_compute(float2* v, int t, const float2* tw, int r, int ns)
 {

@@ -156,12 +156,6 @@ __device__ __forceinline__ void tma_issue_layer(const TmaSet& maps, int orient, 
     for (int k = w; k < G::NBOX; k += nw) tma_load_2d(tile + k * G::TROWS * kBoxW, m, g.xs + k * kBoxW, g.ys, bar);
 }
 
-// One 1-D transform of the row in v through a runtime stage loop: every
-// stage of every transform of the kernel runs through the same code of its
-// radix, which keeps the kernel inside the instruction cache.  ds = -1
-// forward, +1 inverse; rev walks the radix sequence backwards (the inverse of
-// a propagation, which starts from the forward's register layout and ends in
-// the natural layout x[t + e T]).
 // Two-stage plans (N <= 1024) with the radices, strides and exchange
 // indices known at compile time: stage A (stride 1, no twiddles), the
 // exchange, stage B (stride RA).
@@ -206,7 +200,8 @@ __device__ __forceinline__ void fft2_ct_r(float2* v, float2* xrow, int t, const 
     stage_dft<E, RB, -1>(v);
 }
 
-// Three-stage plans with compile-time radices and strides (the alternative
+// Three-stage plans with compile-time radices and strides (2048, the large 2-D
+// transforms, and the alternative
 // plans, see Plan): stage A (stride 1), exchange, stage B (stride RA),
 // exchange, stage C (stride RA RB); twsB / twsC are the stage tables.
 template <int N, int T, int E, int RA, int RB, int RC>
@@ -228,21 +223,21 @@ __device__ __forceinline__ void fft3_ct(float2* v, float2* xrow, int t, const fl
     stage_dft<E, RC, -1>(v);
 }
 
+// One 1-D transform of the row in v.  ds = -1 forward, +1 inverse; rev walks
+// the radix sequence backwards (the inverse of a propagation, which starts
+// from the forward's register layout and ends in the natural layout
+// x[t + e T]).
 template <int N, int T, int E, bool RT = false, int V = 0>
 __device__ __forceinline__ void fft_rt(float2* v, float2* xrow, int t, const float2* __restrict__ tw, float ds, int rev,
                                        const float2* twr = nullptr)
 {
     if (ds > 0.0f) conj_all<E>(v);     // inverse = conj(forward(conj))
-    // (the whole-row transforms above 2048 keep the stage loop: 8192^2 882 us
-    // against 933 with this form)
-    if constexpr (Stages<N, V>::S == 3 && N <= 2048) {
+    static_assert(Stages<N, V>::S == 2 || Stages<N, V>::S == 3, "two- and three-stage plans");
+    if constexpr (Stages<N, V>::S == 3) {
         constexpr int R0 = Stages<N, V>::R0, R1 = Stages<N, V>::R1, R2 = Stages<N, V>::R2;
         if (rev) fft3_ct<N, T, E, R2, R1, R0>(v, xrow, t, tw + tw_offset<N, V>(1, 1), tw + tw_offset<N, V>(1, 2));
         else fft3_ct<N, T, E, R0, R1, R2>(v, xrow, t, tw + tw_offset<N, V>(0, 1), tw + tw_offset<N, V>(0, 2));
-        if (ds > 0.0f) conj_all<E>(v);
-        return;
-    }
-    if constexpr (Stages<N>::S == 2) {
+    } else {
         constexpr int R0 = Stages<N>::R0, R1 = Stages<N>::R1;
         if constexpr (RT && reg_twiddles<N>()) {
             fft2_ct_r<N, T, E, R0, R1>(v, xrow, t, twr);
@@ -252,23 +247,6 @@ __device__ __forceinline__ void fft_rt(float2* v, float2* xrow, int t, const flo
             if (rev) fft2_ct<N, T, E, R1, R0>(v, xrow, t, tw + tw_offset<N>(1, 1));
             else fft2_ct<N, T, E, R0, R1>(v, xrow, t, tw + tw_offset<N>(0, 1));
         }
-        if (ds > 0.0f) conj_all<E>(v);
-        return;
-    }
-    int ns = 1, rp = 0, nsp = 1;
-#pragma unroll 1
-    for (int st = 0; st < Stages<N>::S; st++) {
-        const int r = stage_radix<N>(st, rev);
-        if (st > 0) {
-            row_sync<T>();
-            stage_exchange_store<N, T, E>(v, xrow, t, rp, nsp);
-            row_sync<T>();
-            stage_exchange_load<N, T, E>(v, xrow, t, r);
-        }
-        stage_compute<N, T, E>(v, t, tw + tw_offset<N>(rev, st), r, ns);
-        rp = r;
-        nsp = ns;
-        ns *= r;
     }
     if (ds > 0.0f) conj_all<E>(v);
 }
