@@ -282,12 +282,16 @@ def frame_flops(cfg: FnoConfig) -> float:
 
 
 def frame_bytes(cfg: FnoConfig, bf16_act: bool | None = None) -> float:
-    """HBM bytes one inference frame moves in the library's dataflow: FP32
-    spectral images and pre-activations, each product reading its operands
-    and writing its result once, the residual add and the activation in the
-    pointwise epilogue, pre-activations that only training reads not stored;
-    with bf16_act (ATMWFS_FNO_BF16_ACT=1; off by default) the activations
-    between Fourier layers (h[1..]) and of the projection (q) stored as BF16.
+    """HBM bytes one inference frame moves in the library's dataflow, each
+    kernel reading its operands and writing its results once, in FP32;
+    pre-activations that only training reads are not stored.  The shape of the
+    fused kernels (grid 256, 32 modes, width 64, projection 128, 2 outputs): a
+    layer's output is written with its DFT along x, the inverse DFT along x is
+    added where the output is formed, the projection keeps its activations on
+    chip.  Other shapes, and ATMWFS_FNO_BF16_ACT=1 (bf16_act: the activations
+    between Fourier layers, h[1..], and of the projection, q, stored as BF16)
+    or ATMWFS_FNO_UMMA=0: one kernel per product, the residual add and the
+    activation in the pointwise epilogue.
     The algorithmic figure of the surrogate's HBM roofline."""
     if bf16_act is None:
         bf16_act = os.environ.get("ATMWFS_FNO_BF16_ACT", "0") == "1"
@@ -295,6 +299,18 @@ def frame_bytes(cfg: FnoConfig, bf16_act: bool | None = None) -> float:
     G, m, w, P = cfg.grid, cfg.modes, cfg.width, cfg.grid * cfg.grid
     spec_rows = 4.0 * w * G * 2 * m           # one x-DFT image (2m columns per row)
     modes = 4.0 * w * 2 * m * m               # one mode image (complex m x m per channel)
+    if not bf16_act and (G, m, w, cfg.proj, cfg.nout) == (256, 32, 64, 128, 2) and \
+            not os.environ.get("ATMWFS_FNO_UMMA", "").startswith("0"):
+        b = 4.0 * cfg.nin * P + 4.0 * w * P + spec_rows  # lift: x in, h[0] and its a out
+        if cfg.nin != 8:                      # the lift and the DFT along x as two kernels
+            b += 4.0 * w * P
+        for l in range(cfg.layers):
+            b += (spec_rows + modes           # a -> z
+                  + 2 * modes                 # z -> y (mode mixing)
+                  + modes + spec_rows         # y -> bb
+                  + spec_rows + 8.0 * w * P   # bb, h -> the layer's output
+                  + (spec_rows if l + 1 < cfg.layers else 0.0))  # and its a
+        return b + 4.0 * w * P + 4.0 * cfg.nout * P  # projection
     b = 4.0 * cfg.nin * P + 4.0 * w * P       # lift: x in, h[0] out (FP32)
     for l in range(cfg.layers):
         eh = 4.0 if l == 0 else ea            # bytes of one element of h[l]

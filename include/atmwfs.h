@@ -123,10 +123,10 @@ atmwfs_status atmwfs_normalize_screens_ext(atmwfs_ctx* ctx, float lambda_ref, fl
                                            long nextra, double* r0_pix);
 
 /* Run nsteps time steps (the frame loop, :2561-4345).  Frames of step s of
- * this call are written at offset s * wf_size^2 of the sink buffers.  The
- * copies into the sink run on a stream of their own: with ring >= 2 the
- * copy of step s overlaps the computation of step s + 1 (with ring = 1 they
- * alternate).  Every frame is in the sink when the call returns. */
+ * this call are written at offset s * wf_size^2 of the sink buffers.  With
+ * ring >= 2 the copies into the sink run on a stream of their own and the copy
+ * of step s overlaps the computation of step s + 1; with ring = 1 they follow
+ * each step in its stream.  Every frame is in the sink when the call returns. */
 atmwfs_status atmwfs_run(atmwfs_ctx* ctx, long nsteps, const atmwfs_sink* sink);
 
 /* Advance nsteps time steps (window positions and the step counter) without
@@ -176,7 +176,8 @@ void* atmwfs_stream(atmwfs_ctx* ctx);
  * for the instances of grid class c `reps` times, timed with CUDA events on
  * the context stream.  Returns the mean duration [ms], the algorithmic bytes
  * of one launch (field in/out, window rows, outputs), and the class's grid
- * size and instance count.  Does not advance the simulation. */
+ * size and instance count.  A phase-only context has one kernel per class,
+ * k = 1; other k take no time.  Does not advance the simulation. */
 atmwfs_status atmwfs_time_pass(atmwfs_ctx* ctx, int k, int c, int reps, double* ms, double* bytes, int* n,
                                int* count);
 int atmwfs_num_classes(const atmwfs_ctx* ctx);
@@ -191,9 +192,9 @@ int atmwfs_num_classes(const atmwfs_ctx* ctx);
 #define ATMWFS_NUM_TILE_CFG 6
 
 /* Grid class ci (instances sharing wf_raw_size and wf_size): sizes, member
- * count, the rows per CTA the autotuner chose, and the mean time [ms] of the
- * tuned pass in each of the ATMWFS_NUM_TILE_CFG tile configurations (0 if
- * forced). */
+ * count, the rows per CTA the autotuner chose, and the mean time [ms] of a
+ * pass of the class's chain (all its passes, timed together) in each of the
+ * ATMWFS_NUM_TILE_CFG tile configurations (0 if forced or not compiled). */
 atmwfs_status atmwfs_class_info(const atmwfs_ctx* ctx, int ci, int* n, int* nout, int* count, int* rows_per_cta,
                                 double* tuned_ms);
 
@@ -236,7 +237,8 @@ atmwfs_status atmwfs_fresnel_noalloc(const void* in, void* out, long n, double d
 
 /* do2dfft / do2dffti (src/fft/fft.c:1298-1315): unnormalised 2-D complex
  * DFT, sign -1 forward, +1 inverse.  n is a power of two in 64..2048, or
- * 4096 / 8192 (rows in shared memory, columns through a transpose). */
+ * 4096 / 8192 (rows in shared memory, then the columns in two passes of
+ * shorter transforms). */
 atmwfs_status atmwfs_fft2d(const float* in, float* out, long n, int sign);
 atmwfs_status atmwfs_fft2d_dev(const void* in, void* out, long n, int sign, void* stream);
 
