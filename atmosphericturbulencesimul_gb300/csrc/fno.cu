@@ -83,14 +83,14 @@ cudaError_t project_fused(const __nv_bfloat16* W1, const float* c1, const __nv_b
                           const float* X, float* qpre, float* out, int B, unsigned* status, bool keep,
                           cudaStream_t st);
 bool lift_bwd_supported(int nin);
-cudaError_t lift_bwd_fused(const float* dh, const float* x, float* dW, float* db, int B, unsigned* status, cudaStream_t st);
+cudaError_t lift_bwd_fused(const float* dh, const float* x, float* dW, double* db, int B, unsigned* status, cudaStream_t st);
 cudaError_t project_bwd_fused(const __nv_bfloat16* W1, const __nv_bfloat16* W2, const float* dout, const float* qpre,
-                              const float* u, float* dh, float* dW1, float* dc1, float* dW2, float* dc2, int B,
+                              const float* u, float* dh, float* dW1, double* dc1, double* dW2, double* dc2, int B,
                               unsigned* status, cudaStream_t st);
 cudaError_t fourier_bwd_fused(const __nv_bfloat16* W, const __nv_bfloat16* Fx, const float* dU, const float* da, float* dX,
                               int B, unsigned* status, cudaStream_t st);
 cudaError_t layer_bwd_fused(const __nv_bfloat16* Gx, const float* dh, const float* u, const float* h, float* du, float* dbb,
-                            float* dW, float* db, int B, unsigned* status, cudaStream_t st);
+                            float* dW, double* db, int B, unsigned* status, cudaStream_t st);
 }  // namespace atmwfs
 
 struct atmwfs_fno {
@@ -116,6 +116,10 @@ struct atmwfs_fno {
     float *dh = nullptr, *dh2 = nullptr, *du = nullptr, *dq = nullptr, *dz = nullptr, *dy = nullptr, *da = nullptr, *dbb = nullptr;
     float* dout = nullptr;               // gradient of the loss at the output, [B][nout][G][G]
     double* d_loss = nullptr;
+    // fused backward: FP64 sums over pixels behind the loss (cleared with it):
+    // every layer's b, lift_b, proj1_b, proj2_W, proj2_b; and where they belong
+    std::vector<long> sums;
+    long* d_sums = nullptr;
     std::vector<void*> allocs;
 };
 
@@ -182,6 +186,13 @@ __global__ void k_rowsum(const float* __restrict__ d, float* __restrict__ db, in
         for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
         if (threadIdx.x == 0) atomicAdd(&db[c], s);
     }
+}
+
+// grads[where[i]] += sums[i]
+__global__ void k_add_sums(float* __restrict__ grads, const double* __restrict__ sums, const long* __restrict__ where, int n)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) grads[where[i]] = (float)((double)grads[where[i]] + sums[i]);
 }
 
 // mean squared error and its gradient: dout = 2 (out - t) / n
@@ -928,7 +939,7 @@ atmwfs_status layer_bwd(atmwfs_fno* f, int l, const float* dh, float* dX, int B,
     if (modemix_bwd_smem(B, c.width) > 227 * 1024)  // the batches the unfused mixing takes
         return err(ATMWFS_ERR_INVALID, "batch %d x width %d exceeds the mode-mixing shared memory", B, c.width);
     FN_CUDA(layer_bwd_fused(f->Gx_bf, dh, act ? f->u[l] : nullptr, f->h[l], f->du, f->dbb, f->grads + f->L.W[l],
-                            f->grads + f->L.b[l], B, status, st));
+                            f->d_loss + 1 + (long)l * c.width, B, status, st));
     // dy = GyBig^T dbb: [2m, 2G] x [2G, Nc] (GyBig^T = FyAB)
     FN_CUDA(yfwd_fused(f->FyAB_bf, f->dbb, f->dy, B, status, true, st));
     k_modemix_bwd64<8><<<m * m, 256, 0, st>>>(f->pbf + f->L.R[l], f->z[l], f->dy, f->dz, f->grads + f->L.R[l], B, m);
@@ -951,9 +962,10 @@ atmwfs_status backward(atmwfs_fno* f, const float* x, const float* dout, int B, 
     unsigned* status = fused ? umma_status_ptr() : nullptr;
     if (fused && !status) return err(ATMWFS_ERR_CUDA, "status symbol");
     // projection
+    double *s_lift = f->d_loss + 1 + (long)c.layers * c.width, *s_proj = s_lift + c.width;
     if (fused) {
         FN_CUDA(project_bwd_fused(pb + f->L.proj1_W, pb + f->L.proj2_W, dout, f->qpre, last_h(f), f->dh, g + f->L.proj1_W,
-                                  g + f->L.proj1_b, g + f->L.proj2_W, g + f->L.proj2_b, B, status, st));
+                                  s_proj, s_proj + c.proj, s_proj + (1 + c.nout) * c.proj, B, status, st));
     } else {
         FN_CUDA(pointwise_dw(c.nout, c.proj, dout, f->q, g + f->L.proj2_W, B, P, st));
         k_rowsum<<<dim3(rs.x, c.nout), 256, 0, st>>>(dout, g + f->L.proj2_b, B, c.nout, P);
@@ -980,11 +992,15 @@ atmwfs_status backward(atmwfs_fno* f, const float* x, const float* dout, int B, 
     }
     // lift
     if (fused && lift_bwd_supported(c.nin) && (reinterpret_cast<uintptr_t>(x) & 15) == 0) {
-        FN_CUDA(lift_bwd_fused(f->dh, x, g + f->L.lift_W, g + f->L.lift_b, B, status, st));
-        return ATMWFS_OK;
+        FN_CUDA(lift_bwd_fused(f->dh, x, g + f->L.lift_W, s_lift, B, status, st));
+    } else {
+        FN_CUDA(pointwise_dw(c.width, c.nin, f->dh, x, g + f->L.lift_W, B, P, st));
+        k_rowsum<<<dim3(rs.x, c.width), 256, 0, st>>>(f->dh, g + f->L.lift_b, B, c.width, P);
     }
-    FN_CUDA(pointwise_dw(c.width, c.nin, f->dh, x, g + f->L.lift_W, B, P, st));
-    k_rowsum<<<dim3(rs.x, c.width), 256, 0, st>>>(f->dh, g + f->L.lift_b, B, c.width, P);
+    if (fused) {
+        const int n = (int)f->sums.size();
+        k_add_sums<<<(n + 255) / 256, 256, 0, st>>>(g, f->d_loss + 1, f->d_sums, n);
+    }
     FN_CUDA(cudaGetLastError());
     return ATMWFS_OK;
 }
@@ -1027,7 +1043,20 @@ atmwfs_status atmwfs_fno_create(const atmwfs_fno_cfg* cfg, uint64_t seed, atmwfs
     if ((s = dalloc(f, (void**)&f->grads, sizeof(float) * n)) != ATMWFS_OK) return fail(s);
     if ((s = dalloc(f, (void**)&f->adam_m, sizeof(float) * n)) != ATMWFS_OK) return fail(s);
     if ((s = dalloc(f, (void**)&f->adam_v, sizeof(float) * n)) != ATMWFS_OK) return fail(s);
-    if ((s = dalloc(f, (void**)&f->d_loss, sizeof(double))) != ATMWFS_OK) return fail(s);
+    if (fused_shape(c)) {
+        auto add = [&](long off, long count) {
+            for (long i = 0; i < count; i++) f->sums.push_back(off + i);
+        };
+        for (int l = 0; l < c.layers; l++) add(f->L.b[l], c.width);
+        add(f->L.lift_b, c.width);
+        add(f->L.proj1_b, c.proj);
+        add(f->L.proj2_W, (long)c.nout * c.proj);
+        add(f->L.proj2_b, c.nout);
+        if ((s = dalloc(f, (void**)&f->d_sums, sizeof(long) * f->sums.size())) != ATMWFS_OK) return fail(s);
+        if (cudaMemcpy(f->d_sums, f->sums.data(), sizeof(long) * f->sums.size(), cudaMemcpyHostToDevice) != cudaSuccess)
+            return fail(err(ATMWFS_ERR_CUDA, "gradient index copy failed"));
+    }
+    if ((s = dalloc(f, (void**)&f->d_loss, sizeof(double) * (1 + f->sums.size()))) != ATMWFS_OK) return fail(s);
     if ((s = build_dft(f)) != ATMWFS_OK) return fail(s);
     // initialisation: pointwise weights U(+-1/sqrt(fan_in)), spectral weights U(+-1/w) scaled down
     std::vector<float> h(n, 0.0f);
@@ -1103,7 +1132,7 @@ atmwfs_status atmwfs_fno_loss_grad(atmwfs_fno* f, const float* in, const float* 
     cudaStream_t st = (cudaStream_t)stream;
     FN_TRY(forward(f, in, out, batch, st, true));
     const long n = (long)batch * f->cfg.nout * f->cfg.grid * f->cfg.grid;
-    FN_CUDA(cudaMemsetAsync(f->d_loss, 0, sizeof(double), st));
+    FN_CUDA(cudaMemsetAsync(f->d_loss, 0, sizeof(double) * (1 + f->sums.size()), st));
     k_mse<<<std::min(grid_for(n), 2u * 152u), 256, 0, st>>>(out, target, f->dout, n, f->d_loss);
     FN_CUDA(cudaGetLastError());
     FN_TRY(backward(f, in, f->dout, batch, st));

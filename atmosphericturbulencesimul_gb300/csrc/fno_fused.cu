@@ -24,6 +24,7 @@
 //   z, y  : [2 m][m][BW]   (row ky: real parts, row m + ky: imaginary parts)
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
+#include <float.h>
 #include <stdint.h>
 
 #include "atmwfs_fno.h"
@@ -549,6 +550,12 @@ __global__ void __launch_bounds__(kThreads, SPEC ? 2 : 3)
 // D2 stays in tensor memory for kFlush lines (K = 1024, the longest run of the
 // split product it replaces) and is then added to FP32 registers, one atomic
 // per element and CTA at the end.
+// db (and the head's sums over pixels, below): a line's values are added in
+// FP32, the lines to a pair in shared memory (the registers are taken) and the
+// CTAs' totals in FP64, 2^-24 of the sum in all.  One FP32 register per thread
+// for all lines and FP32 atomics of 152 CTAs were twice as far from the exact
+// sums as k_rowsum's 64 CTAs (up to 22 times for dc2); FP64 additions per line
+// would share the part's few FP64 lanes with nothing to gain.
 // ---------------------------------------------------------------------------
 // HC = 8 without SPEC is the lift's weight and bias gradient (no DFT, K the
 // input planes padded to 16 zero rows).
@@ -565,11 +572,29 @@ __device__ __forceinline__ void ld8(float (&f)[8], const float* p)
     f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w;
 }
 
+// A thread's sum over lines as hi + lo; an overflowed or undefined hi is the value.
+__device__ __forceinline__ void pair_add(float2& s, float v)
+{
+    const float t = s.x + v, b = t - s.x;
+    s.y += (s.x - (t - b)) + (v - b);
+    s.x = t;
+}
+__device__ __forceinline__ double pair_value(float2 s)
+{
+    return fabsf(s.x) <= FLT_MAX ? (double)s.x + (double)s.y : (double)s.x;
+}
+__device__ __forceinline__ float sum8(const float (&f)[8])
+{
+    return ((f[0] + f[1]) + (f[2] + f[3])) + ((f[4] + f[5]) + (f[6] + f[7]));
+}
+
+constexpr uint32_t kLBytes = 3 * kXBytes + kBT * 8;  // du, Gx, h, the threads' bias sums
+
 template <bool ACT, bool SPEC, int HC>
 __global__ void __launch_bounds__(kBT, 1)
     k_layer_bwd(const __nv_bfloat16* __restrict__ Gx, const float* __restrict__ dh, const float* __restrict__ u,
                 const float* __restrict__ h, float* __restrict__ du, float* __restrict__ dbb, float* __restrict__ dW,
-                float* __restrict__ db, int nlines, long Nc, unsigned* status)
+                double* __restrict__ db, int nlines, long Nc, unsigned* status)
 {
     constexpr int J = kW * kXK / kBT;            // pieces of the line per thread
     constexpr int HN = HC < 16 ? 16 : HC;        // N of the weight product
@@ -578,6 +603,8 @@ __global__ void __launch_bounds__(kBT, 1)
     static_assert(HC == kW || HC * kXK <= kBT, "h in one piece per thread");
     extern __shared__ __align__(128) unsigned char sm[];
     unsigned char *sd = sm, *sg = sm + kXBytes, *sh = sm + 2 * kXBytes;  // du, Gx, h
+    float2& bsum = reinterpret_cast<float2*>(sm + 3 * kXBytes)[threadIdx.x];  // every piece of a thread has the same channel
+    bsum = make_float2(0.0f, 0.0f);
     __shared__ __align__(8) uint64_t bar;
     __shared__ uint32_t tmem_base;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -623,7 +650,6 @@ __global__ void __launch_bounds__(kBT, 1)
     fence_after();
     const uint32_t tmem = tmem_base, d_addr = smem_addr(sd), g_addr = smem_addr(sg), h_addr = smem_addr(sh);
     uint32_t parity = 0;
-    float bsum = 0.0f;  // every piece of a thread has the same channel
     float acc[CN];      // dW of o = the lane's channel: the warps that read tensor memory
 #pragma unroll
     for (int q = 0; q < CN; q++) acc[q] = 0.0f;
@@ -632,6 +658,7 @@ __global__ void __launch_bounds__(kBT, 1)
     int held = 0;  // lines in D2
     for (int line = blockIdx.x; line < nlines; line += gridDim.x) {
         const size_t o0 = (size_t)(line / kG) * kW * kP + (size_t)(line % kG) * kG;
+        float ls = 0.0f;
 #pragma unroll
         for (int j = 0; j < J; j++) {
             int row, k8;
@@ -643,13 +670,14 @@ __global__ void __launch_bounds__(kBT, 1)
                 o[0] = make_float4(d[j][0], d[j][1], d[j][2], d[j][3]);
                 o[1] = make_float4(d[j][4], d[j][5], d[j][6], d[j][7]);
             }
-            bsum += ((d[j][0] + d[j][1]) + (d[j][2] + d[j][3])) + ((d[j][4] + d[j][5]) + (d[j][6] + d[j][7]));
+            ls += sum8(d[j]);
             *reinterpret_cast<uint4*>(sd + kmajor_off(row, k8 * 8, kXK)) = pack8(d[j]);
             if constexpr (HC == kW) *reinterpret_cast<uint4*>(sh + kmajor_off(row, k8 * 8, kXK)) = pack8(hv[j]);
             // the piece's registers are free: the next line's values come in
             // under the remaining pieces' arithmetic and the products
             if (line + (int)gridDim.x < nlines) load(line + gridDim.x, j);
         }
+        pair_add(bsum, ls);
         if constexpr (HC != kW)
             if (tid < HC * kXK) *reinterpret_cast<uint4*>(sh + kmajor_off(hrow, hk8 * 8, kXK)) = pack8(hv[0]);
         if (line + (int)gridDim.x < nlines) load_h(line + gridDim.x);
@@ -690,9 +718,10 @@ __global__ void __launch_bounds__(kBT, 1)
         for (int q = 0; q < CN; q++) atomicAdd(o + q, acc[q]);
     }
     // a channel's lanes: l, l + 8, l + 16, l + 24 of warps w and w + 8
-    bsum += __shfl_xor_sync(0xffffffffu, bsum, 8);
-    bsum += __shfl_xor_sync(0xffffffffu, bsum, 16);
-    if (lane < 8) atomicAdd(db + (warp & 7) * 8 + lane, bsum);
+    double bs = pair_value(bsum);
+    bs += __shfl_xor_sync(0xffffffffu, bs, 8);
+    bs += __shfl_xor_sync(0xffffffffu, bs, 16);
+    if (lane < 8) atomicAdd(db + (warp & 7) * 8 + lane, bs);
     tmem_free(tmem, 128, warp);
 }
 
@@ -716,12 +745,14 @@ constexpr uint32_t kQU = kQA + kProj * kG * 2;                // u [64][256 px]
 constexpr uint32_t kQTs = kProj / 8 * 128 + 32;               // bytes between 8-pixel groups of dq^T
 constexpr uint32_t kQT = kQU + kW * kG * 2;                   // dq^T [256 px][128]
 constexpr uint32_t kQW = kQT + kG / 8 * kQTs;                 // W1^T [64][128]
-constexpr uint32_t kQBytes = kQW + kW * kProj * 2;
+constexpr uint32_t kQS = kQW + kW * kProj * 2;                // the threads' sums: dc1 and dW2 of two channels, dc2
+constexpr int kQSums = 7;
+constexpr uint32_t kQBytes = kQS + kQSums * kBT * 8;
 
 __global__ void __launch_bounds__(kBT, 1)
     k_project_bwd(const __nv_bfloat16* __restrict__ W1, const __nv_bfloat16* __restrict__ W2, const float* __restrict__ dout,
                   const float* __restrict__ qpre, const float* __restrict__ u, float* __restrict__ dh, float* __restrict__ dW1,
-                  float* __restrict__ dc1, float* __restrict__ dW2, float* __restrict__ dc2, int nlines, unsigned* status)
+                  double* __restrict__ dc1, double* __restrict__ dW2, double* __restrict__ dc2, int nlines, unsigned* status)
 {
     constexpr int J = kW * kXK / kBT;  // pieces of 64 channels of a line per thread
     extern __shared__ __align__(128) unsigned char sm[];
@@ -731,7 +762,10 @@ __global__ void __launch_bounds__(kBT, 1)
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int ch = (warp & 7) * 8 + (lane & 7);    // every piece of a thread has channel ch or ch + 64
     float q[2][J][8];
-    float dv = 0.0f, dsum = 0.0f;                  // this thread's dout value (plane tid / 256, pixel tid % 256), its sum
+    float dv = 0.0f;                               // this thread's dout value (plane tid / 256, pixel tid % 256)
+    float2* sums = reinterpret_cast<float2*>(sm + kQS) + tid;  // [kQSums], kBT apart: bs, g2 of channel ch; of ch + 64; dout
+#pragma unroll
+    for (int k = 0; k < kQSums; k++) sums[k * kBT] = make_float2(0.0f, 0.0f);
     auto load = [&](int line, int hf, int j) {
         const size_t o0 = (size_t)(line / kG) * kProj * kP + (size_t)(line % kG) * kG;
         int row, k8;
@@ -752,7 +786,7 @@ __global__ void __launch_bounds__(kBT, 1)
     if (tid == 0) mbar_init(&bar);
     for (int i = tid; i < kProj * kW; i += kBT)  // W1 is [128][64]: element (o, c) to row c, K index o
         *reinterpret_cast<__nv_bfloat16*>(sm + kQW + kmajor_off(i % kW, i / kW, kProj / 8)) = W1[i];
-    float w2[2][2], bs[2] = {0.0f, 0.0f}, g2[2][2] = {{0.0f, 0.0f}, {0.0f, 0.0f}};
+    float w2[2][2];
 #pragma unroll
     for (int hf = 0; hf < 2; hf++)
 #pragma unroll
@@ -769,7 +803,7 @@ __global__ void __launch_bounds__(kBT, 1)
     int held = 0, buf = 0;
     for (int line = blockIdx.x; line < nlines; line += gridDim.x) {
         const size_t o0 = (size_t)(line / kG) * kW * kP + (size_t)(line % kG) * kG;
-        dsum += dv;
+        pair_add(sums[6 * kBT], dv);
         s_d[buf][tid / kG][tid % kG] = __bfloat162float(__float2bfloat16_rn(dv));
         if (line + (int)gridDim.x < nlines) load_d(line + gridDim.x);
 #pragma unroll
@@ -781,6 +815,7 @@ __global__ void __launch_bounds__(kBT, 1)
             *reinterpret_cast<uint4*>(sm + kQU + kmajor_off(row, k8 * 8, kXK)) = pack8(f);
         }
         __syncthreads();
+        float bs[2] = {0.0f, 0.0f}, g2[2][2] = {{0.0f, 0.0f}, {0.0f, 0.0f}};  // of this line
 #pragma unroll
         for (int j = 0; j < J; j++) {
             int row, k8;
@@ -800,8 +835,8 @@ __global__ void __launch_bounds__(kBT, 1)
                     const float vb = __bfloat162float(__float2bfloat16_rn(v));
                     g2[hf][0] = fmaf(d0[k], vb, g2[hf][0]);
                     g2[hf][1] = fmaf(d1[k], vb, g2[hf][1]);
-                    bs[hf] += f[k];
                 }
+                bs[hf] += sum8(f);
                 if (line + (int)gridDim.x < nlines) load(line + gridDim.x, hf, j);  // the piece's registers are free
                 const uint4 pk = pack8(f);
                 const int o = row + 64 * hf;
@@ -811,6 +846,12 @@ __global__ void __launch_bounds__(kBT, 1)
 #pragma unroll
                 for (int k = 0; k < 8; k++) t[k * 8] = (unsigned short)(w[k >> 1] >> (16 * (k & 1)));
             }
+        }
+#pragma unroll
+        for (int hf = 0; hf < 2; hf++) {
+            pair_add(sums[(3 * hf) * kBT], bs[hf]);
+            pair_add(sums[(3 * hf + 1) * kBT], g2[hf][0]);
+            pair_add(sums[(3 * hf + 2) * kBT], g2[hf][1]);
         }
         publish_smem();
         if (tid == 0) {
@@ -857,22 +898,16 @@ __global__ void __launch_bounds__(kBT, 1)
         for (int k = 0; k < 16; k++) atomicAdd(o + k, acc[k]);
     }
 #pragma unroll
-    for (int o = 8; o < 32; o <<= 1)
-#pragma unroll
-        for (int hf = 0; hf < 2; hf++) {
-            bs[hf] += __shfl_xor_sync(0xffffffffu, bs[hf], o);
-            g2[hf][0] += __shfl_xor_sync(0xffffffffu, g2[hf][0], o);
-            g2[hf][1] += __shfl_xor_sync(0xffffffffu, g2[hf][1], o);
-        }
-    if (lane < 8)
-#pragma unroll
-        for (int hf = 0; hf < 2; hf++) {
-            atomicAdd(dc1 + ch + 64 * hf, bs[hf]);
-            atomicAdd(dW2 + ch + 64 * hf, g2[hf][0]);
-            atomicAdd(dW2 + kProj + ch + 64 * hf, g2[hf][1]);
-        }
-    for (int o = 16; o > 0; o >>= 1) dsum += __shfl_xor_sync(0xffffffffu, dsum, o);
-    if (lane == 0) atomicAdd(dc2 + tid / kG, dsum);
+    for (int k = 0; k < kQSums; k++) {
+        double v = pair_value(sums[k * kBT]);
+        if (k == 6)  // dout: a plane's 256 threads
+            for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        v += __shfl_xor_sync(0xffffffffu, v, 8);
+        v += __shfl_xor_sync(0xffffffffu, v, 16);
+        const int o = ch + 64 * (k / 3);
+        if (k == 6 ? lane == 0 : lane < 8)
+            atomicAdd(k == 6 ? dc2 + tid / kG : k % 3 == 0 ? dc1 + o : dW2 + (k % 3 - 1) * kProj + o, v);
+    }
     tmem_free(tmem, 256, warp);
 }
 
@@ -1067,17 +1102,18 @@ cudaError_t fourier_bwd_fused(const __nv_bfloat16* W, const __nv_bfloat16* Fx, c
                                                              true, st);
 }
 
-// u NULL: no activation (du is dh and is not written).  dW and db accumulate.
+// u NULL: no activation (du is dh and is not written).  dW and db accumulate;
+// db, and dc1, dW2 and dc2 below, are FP64 sums that the caller clears.
 cudaError_t layer_bwd_fused(const __nv_bfloat16* Gx, const float* dh, const float* u, const float* h, float* du, float* dbb,
-                            float* dW, float* db, int B, unsigned* status, cudaStream_t st)
+                            float* dW, double* db, int B, unsigned* status, cudaStream_t st)
 {
     using namespace umma;
     const int lines = B * kG, grid = lines < sm_count() ? lines : sm_count();
     const long Nc = (long)B * kW * kModes;
     auto go = [&](auto kern) {
-        const cudaError_t e = allow_smem(kern, 3 * kXBytes);
+        const cudaError_t e = allow_smem(kern, kLBytes);
         if (e != cudaSuccess) return e;
-        kern<<<grid, kBT, 3 * kXBytes, st>>>(Gx, dh, u, h, du, dbb, dW, db, lines, Nc, status);
+        kern<<<grid, kBT, kLBytes, st>>>(Gx, dh, u, h, du, dbb, dW, db, lines, Nc, status);
         return cudaGetLastError();
     };
     return u ? go(k_layer_bwd<true, true, kW>) : go(k_layer_bwd<false, true, kW>);
@@ -1086,19 +1122,19 @@ cudaError_t layer_bwd_fused(const __nv_bfloat16* Gx, const float* dh, const floa
 // The lift's gradients: dW (64 x nin) += dh x^T, db += sum dh.
 bool lift_bwd_supported(int nin) { return nin == 8; }
 
-cudaError_t lift_bwd_fused(const float* dh, const float* x, float* dW, float* db, int B, unsigned* status, cudaStream_t st)
+cudaError_t lift_bwd_fused(const float* dh, const float* x, float* dW, double* db, int B, unsigned* status, cudaStream_t st)
 {
     using namespace umma;
-    const cudaError_t e = allow_smem(k_layer_bwd<false, false, 8>, 3 * kXBytes);
+    const cudaError_t e = allow_smem(k_layer_bwd<false, false, 8>, kLBytes);
     if (e != cudaSuccess) return e;
     const int lines = B * kG, grid = lines < sm_count() ? lines : sm_count();
-    k_layer_bwd<false, false, 8><<<grid, kBT, 3 * kXBytes, st>>>(nullptr, dh, nullptr, x, nullptr, nullptr, dW, db, lines,
-                                                                 (long)B * kW * kModes, status);
+    k_layer_bwd<false, false, 8><<<grid, kBT, kLBytes, st>>>(nullptr, dh, nullptr, x, nullptr, nullptr, dW, db, lines,
+                                                             (long)B * kW * kModes, status);
     return cudaGetLastError();
 }
 
 cudaError_t project_bwd_fused(const __nv_bfloat16* W1, const __nv_bfloat16* W2, const float* dout, const float* qpre,
-                              const float* u, float* dh, float* dW1, float* dc1, float* dW2, float* dc2, int B,
+                              const float* u, float* dh, float* dW1, double* dc1, double* dW2, double* dc2, int B,
                               unsigned* status, cudaStream_t st)
 {
     using namespace umma;
