@@ -218,13 +218,49 @@ __global__ void k_mse(const float* __restrict__ out, const float* __restrict__ t
     }
 }
 
-// Mode mixing y[b][o][k] = sum_c R[k][o][c] z[b][c][k] (complex) for KX
-// neighbouring kx of one ky (blockIdx.x = ky (m / KX) + kx / KX).  z / y: row ky
-// holds the real parts, row m + ky the imaginary parts; in a row mode kx of
-// (sample, channel) bc is at kx sk + bc sc: [B w][m] (sk = 1, sc = m) or, at the
-// shape of the fused kernels, [m][B w] (sk = B w, sc = 1), whose loads and
-// stores are whole runs (the scattered 4-byte stores of the first took most of
-// 75 us).
+// Mode mixing y[b][o][k] = sum_c R[k][o][c] z[b][c][k] (complex), one CTA per
+// mode k = (ky, kx).  z / y layout [2m][B w][m]: row ky holds the real parts,
+// row m + ky the imaginary parts, then (sample, channel), then kx.
+__global__ void k_modemix(const __nv_bfloat16* __restrict__ R, const float* __restrict__ z, float* __restrict__ y,
+                          int B, int w, int m)
+{
+    const int k = blockIdx.x, ky = k / m, kx = k % m;
+    const long Nc = (long)B * w * m;
+    const long ore = (long)ky * Nc + kx, oim = (long)(m + ky) * Nc + kx;
+    extern __shared__ float4 mix_smem[];
+    float* zs = reinterpret_cast<float*>(mix_smem);          // [B][w][2]
+    float2* rs = reinterpret_cast<float2*>(zs + 2 * B * w);  // [w][w + 1]: R[o][c], padded rows
+    const __nv_bfloat162* Rk = reinterpret_cast<const __nv_bfloat162*>(R) + (size_t)k * w * w;
+    for (int i = threadIdx.x; i < w * w; i += blockDim.x)  // coalesced (re, im) pairs
+        rs[(i / w) * (w + 1) + i % w] = make_float2(__low2float(Rk[i]), __high2float(Rk[i]));
+    for (int i = threadIdx.x; i < B * w; i += blockDim.x) {
+        zs[2 * i] = z[(long)i * m + ore];
+        zs[2 * i + 1] = z[(long)i * m + oim];
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < B * w; i += blockDim.x) {
+        const int o = i % w;
+        const float2* r = rs + o * (w + 1);
+        const float* zb = zs + 2 * (i - o);
+        float sr = 0.0f, si = 0.0f;
+        for (int c = 0; c < w; c++) {
+            const float2 rc = r[c];
+            const float zr = zb[2 * c], zi = zb[2 * c + 1];
+            sr += rc.x * zr - rc.y * zi;
+            si += rc.x * zi + rc.y * zr;
+        }
+        y[(long)i * m + ore] = sr;
+        y[(long)i * m + oim] = si;
+    }
+}
+
+size_t modemix_smem(int B, int w) { return sizeof(float) * (2 * (size_t)B * w + 2 * (size_t)w * (w + 1)); }
+
+// The same for KX neighbouring kx of one ky (blockIdx.x = ky (m / KX) + kx / KX),
+// kMixB samples at a time.  Mode kx of (sample, channel) bc is at kx sk + bc sc
+// of its row: [B w][m] as above (sk = 1, sc = m) or, at the shape of the fused
+// kernels, [m][B w] (sk = B w, sc = 1), whose loads and stores are whole runs
+// (the scattered 4-byte stores of the first took most of 75 us).
 // FP32 FMAs bound it: 8 w^2 B m^2 operations, 7 us for a batch of 16 at the
 // default shape.  A thread owns one (mode, output channel) and kMixB samples:
 // a weight is read from shared memory once for all of them and the samples'
@@ -236,8 +272,8 @@ __global__ void k_mse(const float* __restrict__ out, const float* __restrict__ t
 constexpr int kMixB = 8;
 // WC: the width as a constant (0: the argument); the staging loops divide by it.
 template <int KX, int WC>
-__global__ void __launch_bounds__(256, WC ? 4 : 1) k_modemix(const __nv_bfloat16* __restrict__ R, const float* __restrict__ z,
-                                                 float* __restrict__ y, int B, int width, int m, long sk, long sc)
+__global__ void __launch_bounds__(256, WC ? 4 : 1) k_modemix_samples(const __nv_bfloat16* __restrict__ R, const float* __restrict__ z,
+                                                                    float* __restrict__ y, int B, int width, int m, long sk, long sc)
 {
     const int w = WC ? WC : width;
     const int groups = m / KX, ky = blockIdx.x / groups, kx0 = blockIdx.x % groups * KX;
@@ -329,24 +365,32 @@ __global__ void __launch_bounds__(256, WC ? 4 : 1) k_modemix(const __nv_bfloat16
 }
 
 template <int KX>
-constexpr size_t modemix_smem(int w) { return (size_t)KX * ((size_t)kMixB * w * 8 + (size_t)w * (w + 1) * 4); }
+constexpr size_t modemix_samples_smem(int w) { return (size_t)KX * ((size_t)kMixB * w * 8 + (size_t)w * (w + 1) * 4); }
 
-// Four neighbouring modes per CTA where they fit twice into an SM, else two or one.
-cudaError_t modemix(const __nv_bfloat16* R, const float* z, float* y, int B, int w, int m, long sk, long sc, cudaStream_t st)
+// planes: the fused kernels' layout.  Else one thread per output value where
+// two of its CTAs fit an SM (its weights are FP32): products of kMixB samples
+// whatever the batch cost more there than its shared reads (layers of width 64
+// and 32 modes: 575 against 658 us for a network's single frame, 702 against
+// 786 for two, equal at 16; width 96: 537 against 609).  Above, its one CTA
+// waits for every load and the BF16 weights of the other form fit three times
+// (width 128: 685 against 552 us for one frame, 2160 against 1875 for 16).
+cudaError_t modemix(const __nv_bfloat16* R, const float* z, float* y, int B, int w, int m, bool planes, cudaStream_t st)
 {
-    auto go = [&](auto kern, size_t sm, int kx) -> cudaError_t {
-        if (sm > 48 * 1024) {
-            const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-            if (e != cudaSuccess) return e;
-        }
-        kern<<<m * m / kx, 256, sm, st>>>(R, z, y, B, w, m, sk, sc);
-        return cudaGetLastError();
+    auto allow = [](auto kern, size_t sm) {
+        return sm > 48 * 1024 ? cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm) : cudaSuccess;
     };
-    // (whole runs per mode need no neighbours: two modes make twice the CTAs)
-    if (sc == 1 && w == 64) return go(k_modemix<2, 64>, modemix_smem<2>(w), 2);
-    if (m % 4 == 0 && modemix_smem<4>(w) <= 113 * 1024) return go(k_modemix<4, 0>, modemix_smem<4>(w), 4);
-    if (modemix_smem<2>(w) <= 113 * 1024) return go(k_modemix<2, 0>, modemix_smem<2>(w), 2);  // m is even
-    return go(k_modemix<1, 0>, modemix_smem<1>(w), 1);
+    if (planes) {  // width 64; whole runs per mode need no neighbours: two modes make twice the CTAs
+        k_modemix_samples<2, 64><<<m * m / 2, 256, modemix_samples_smem<2>(w), st>>>(R, z, y, B, w, m, (long)B * w, 1);
+    } else if (modemix_smem(B, w) <= 113 * 1024) {
+        const size_t sm = modemix_smem(B, w);
+        if (const cudaError_t e = allow(k_modemix, sm)) return e;
+        k_modemix<<<m * m, 256, sm, st>>>(R, z, y, B, w, m);
+    } else {
+        const size_t sm = modemix_samples_smem<1>(w);
+        if (const cudaError_t e = allow(k_modemix_samples<1, 0>, sm)) return e;
+        k_modemix_samples<1, 0><<<m * m, 256, sm, st>>>(R, z, y, B, w, m, 1, m);
+    }
+    return cudaGetLastError();
 }
 
 // Backward of the mode mixing: dz = R^H dy per mode, and dR += sum_b dy z^H.
@@ -770,9 +814,8 @@ atmwfs_status spectral_fwd(atmwfs_fno* f, int l, const void* h, int h_bf16, floa
     else
         FN_CUDA(gemm(2 * m, (int)Nc, 2 * G, f->FyAB, 2 * G, 0, 0, a, Nc, 0, 0, z, Nc, 0.0f, 1, 0, 0, 0, nullptr, 0, st));
     // y = R z per mode
-    const size_t smf = sizeof(float) * (2 * B * w + 2 * w * (w + 1));
-    if (smf > 227 * 1024) return err(ATMWFS_ERR_INVALID, "batch %d x width %d exceeds the mode-mixing shared memory", B, w);
-    FN_CUDA(modemix(f->pbf + f->L.R[l], z, f->y, B, w, m, spec ? 1 : BW, spec ? m : 1, st));
+    if (modemix_smem(B, w) > 227 * 1024) return err(ATMWFS_ERR_INVALID, "batch %d x width %d exceeds the mode-mixing shared memory", B, w);
+    FN_CUDA(modemix(f->pbf + f->L.R[l], z, f->y, B, w, m, !spec, st));
     // bb = GyBig y: [2G, 2m] x [2m, Nc], on tcgen05 where compiled
     if (!spec)
         FN_CUDA(yinv_fused(f->GyBig_bf, f->y, f->bb, B, umma_status_ptr(), st));
