@@ -315,6 +315,7 @@ struct Class {
     std::vector<int> pslots;
     PhaseJob* d_pjobs = nullptr;
     int* d_pslots = nullptr;
+    bool phase_small = false;
 };
 
 }  // namespace atmwfs
@@ -570,7 +571,8 @@ atmwfs_status launch_phases(atmwfs_ctx* c, Class& cl, double* bytes, cudaStream_
     a.pjobs = cl.d_pjobs;
     a.pslots = cl.d_pslots;
     a.pdl_ctas = step_pdl_ctas(c);
-    const int RR = phase_rows(cl.N);
+    a.phase_small = cl.phase_small;
+    const int RR = phase_rows(cl.N, cl.phase_small);
     if (bytes) {
         *bytes = 4.0 * (RR + 3) / RR * c->L * (double)cl.N * cl.N * cl.pjobs.size();
         for (int q : cl.pslots) *bytes += 8.0 * c->hinst[q].Nout * c->hinst[q].Nout;
@@ -877,6 +879,22 @@ atmwfs_status phase_jobs(atmwfs_ctx* c, Class& cl)
         if (f) cl.pjobs.push_back(PhaseJob{c->group_leader[g], first, (int)cl.pslots.size() - first, 1});
     }
     if (cl.pjobs.empty()) return ATMWFS_OK;
+    cl.phase_small = phase_small(cl.N, (long)cl.pjobs.size());
+    // a group's members are written one after the other: where SMs are left
+    // idle, jobs of their own (the interpolation repeated there)
+    const long idle = cl.phase_small ? sm_count() / (cl.N / phase_rows(cl.N, true) * (long)cl.pjobs.size()) : 1;
+    if (idle > 1) {
+        std::vector<PhaseJob> whole;
+        whole.swap(cl.pjobs);
+        for (const PhaseJob& j : whole) {
+            const int parts = (int)std::min<long>(idle, j.count);
+            for (int p = 0, m0 = 0; p < parts; p++) {
+                const int m1 = (int)((long)j.count * (p + 1) / parts);
+                cl.pjobs.push_back(PhaseJob{j.gidx, j.first + m0, m1 - m0, j.factored});
+                m0 = m1;
+            }
+        }
+    }
     if (!cl.d_pjobs) {
         AW_TRY(dalloc(c, (void**)&cl.d_pjobs, sizeof(PhaseJob) * cl.pslots.size()));  // at most one job per member
         AW_TRY(dalloc(c, (void**)&cl.d_pslots, sizeof(int) * cl.pslots.size()));
@@ -980,7 +998,7 @@ atmwfs_status commit(atmwfs_ctx* c)
     AW_CUDA(cudaMemcpyAsync(c->d_inst, c->hinst.data(), sizeof(InstDev) * c->hinst.size(), cudaMemcpyHostToDevice, c->st));
     for (Class& cl : c->classes) {
         memset(&cl.maps, 0, sizeof cl.maps);
-        const int rows = (c->amplitude ? win_rows(cl.N) : phase_rows(cl.N)) + 3;
+        const int rows = (c->amplitude ? win_rows(cl.N) : phase_rows(cl.N, cl.phase_small)) + 3;
         for (int o = 0; o < 2; o++)
             for (int l = 0; l < c->L; l++)
                 if (c->d_pad[o][l]) AW_TRY(make_tma_map(&cl.maps.m[o][l], c->d_pad[o][l], c->Wp, c->Hp, rows));

@@ -31,6 +31,18 @@ __device__ __forceinline__ void pdl_gate()
 }
 #endif
 
+inline int sm_count()
+{
+    static const int n = [] {
+        int dev = 0, sms = 0;
+        if (cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess)
+            return sms;
+        cudaGetLastError();
+        return 1;
+    }();
+    return n;
+}
+
 // Grids of at most this many CTAs get the attribute: one CTA per SM.
 // Such launches are bound by launch latency, which the early scheduling
 // hides (a 256^2 single-frame step: 29.1 -> 25.0 us).  Larger grids are
@@ -44,13 +56,7 @@ inline int pdl_max_ctas()
     static const int n = [] {
         const char* e = getenv("ATMWFS_PDL");
         if (e && atoi(e) == 0) return 0;
-        int dev = 0, sms = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess ||
-            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
-            cudaGetLastError();
-            return 0;
-        }
-        return sms;
+        return sm_count();
     }();
     return n;
 }
@@ -211,6 +217,7 @@ struct PassArgs {
     // phase-only frames: their jobs (blockIdx.y) and the jobs' instance slots
     const PhaseJob* pjobs;
     const int* pslots;
+    int phase_small;           // their shape (phase_small)
     long pdl_ctas;             // host: largest grid launched with programmatic dependent launch
 };
 
@@ -271,11 +278,22 @@ constexpr TileCfg tile_cfg(int N, int c)
 // Window kernel and phase-only frames: rows per CTA and threads (four columns
 // each; a warp at least).  Eight rows cost 11 / 8 of the horizontal sums.  At
 // 2048 the phase-only frames take four, so that their two tiles leave room for
-// a second CTA per SM.
+// a second CTA per SM.  Where these shapes give an SM two warps at most, a CTA's
+// own chain through the layers is the time of the step: two rows per CTA then (5 / 2
+// of the sums, on SMs that idle; more tiles in flight changed nothing).  us per
+// step through 1 / 7 / 16 layers, eight rows against two: one 256^2 frame 8.5 /
+// 15.2 / 25.2, 6.5 / 10.6 / 16.8; four directions (1.7 warps per SM) 8.5 / 15.4 /
+// 25.8, 6.5 / 12.8 / 19.1; eight (3.4) 8.5 / 16.8 / 27.2, 10.3 / 19.4 / 34.5; the
+// line lies between the same at 64, 128 and 512.
 constexpr int win_rows(int) { return 8; }
 constexpr int win_threads(int N) { return N < 128 ? 32 : N / 4; }
-constexpr int phase_rows(int N) { return N <= 1024 ? 8 : 4; }
+constexpr int phase_rows(int N, bool small) { return small ? 2 : N <= 1024 ? 8 : 4; }
 constexpr int phase_threads(int N) { return N < 128 ? 32 : N < 1024 ? N / 4 : 256; }
+constexpr int kPhaseSmallMax = 512;
+inline bool phase_small(int N, long jobs)
+{
+    return N <= kPhaseSmallMax && N / phase_rows(N, false) * jobs * (phase_threads(N) / 32) <= 2L * sm_count();
+}
 
 // Threads of a phase-sum CTA and CTAs per instance of its launch.
 constexpr int kPhasumThreads = 256;

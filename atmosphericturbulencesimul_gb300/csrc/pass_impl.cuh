@@ -82,10 +82,12 @@ __device__ __forceinline__ void cp_async_wait_group1() { asm volatile("cp.async.
 __device__ __forceinline__ bool cta_wait_tile(uint64_t* bar, int parity, unsigned* status)
 {
     const uint64_t limit = 1000000000ull;  // 1 s
-    const uint64_t t0 = gtimer_ns();
     int timed_out = 0;
-    while (!mbar_try_wait(bar, parity)) {
-        if (gtimer_ns() - t0 > limit) { timed_out = 1; break; }
+    if (!mbar_try_wait(bar, parity)) {
+        const uint64_t t0 = gtimer_ns();
+        while (!mbar_try_wait(bar, parity)) {
+            if (gtimer_ns() - t0 > limit) { timed_out = 1; break; }
+        }
     }
     if (__syncthreads_or(timed_out)) {
         if (threadIdx.x == 0 && status) atomicOr(status, kStatTmaTimeout);
@@ -673,6 +675,10 @@ __global__ void __launch_bounds__(NT)
 // k_phasum where Scoeff depends on the layer) and an output pass, bit for bit.
 // Issue bounds it: about 16 instructions per pixel and layer.  16 directions
 // of 512^2 through 10 layers: windows 60 + sums 45 + output pass 46 us before.
+// With few CTAs latency does, since layers and instances follow one another:
+// what a layer or an instance needs is in shared memory before the first tile
+// lands (instances read where they were used: 0.7 us each), and CTAs of two rows
+// take over (phase_small).
 // ---------------------------------------------------------------------------
 template <int N, int RR, int NT>
 __global__ void __launch_bounds__(NT) k_phase_frames(const __grid_constant__ PassArgs a, const __grid_constant__ TmaSet maps)
@@ -683,24 +689,39 @@ __global__ void __launch_bounds__(NT) k_phase_frames(const __grid_constant__ Pas
     extern __shared__ __align__(1024) unsigned char sm[];
     float* tiles = reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(sm) + 127) & ~uintptr_t(127));
     constexpr int TILE = (int)(G::TILE_BYTES / 4);
+    struct Member {
+        float *pha, *amp;  // the step's frames
+        int off, Nout;
+        float sg;
+    };
+    constexpr int NM = 32;  // instances in shared memory at a time
     __shared__ __align__(8) uint64_t bar[2];
+    __shared__ LayerPos s_pos[kMaxLayers];  // from the top layer down, as s_sc
+    __shared__ float s_sc[kMaxLayers];
+    __shared__ Member s_mem[NM];
     pdl_gate();
     const PhaseJob J = a.pjobs[blockIdx.y];
     const int tid = threadIdx.x, y0 = blockIdx.x * RR, L = a.L;
     const int step = *a.d_step;
-    const LayerPos* pos = a.pos + ((size_t)(step % a.poscap) * a.ninst_total + J.gidx) * L;
-    if (tid == 0) {
-        mbar_init(&bar[0], 1);
-        mbar_init(&bar[1], 1);
+    if (tid < L) {
+        s_pos[tid] = a.pos[((size_t)(step % a.poscap) * a.ninst_total + J.gidx) * L + L - 1 - tid];
+        s_sc[tid] = J.factored ? 1.0f : a.inst[a.pslots[J.first]].scoeff[L - 1 - tid];
     }
+    if (tid < 2) mbar_init(&bar[tid], 1);
+    auto load_members = [&](int m0) {
+        if (tid < NM && m0 + tid < J.count) {
+            const InstDev& I = a.inst[a.pslots[J.first + m0 + tid]];
+            const size_t slot = (size_t)(step % I.ring) * I.ostride;
+            s_mem[tid] = Member{I.out_pha + slot, I.out_amp + slot, I.off, I.Nout, I.scoeff[0]};
+        }
+    };
     __syncthreads();
     auto issue = [&](int i) {
-        const TileGeom g = tile_geom(pos[L - 1 - i], 0, y0);
-        tma_issue_layer<N, RR>(maps, 0, L - 1 - i, g, tiles + (i & 1) * TILE, &bar[i & 1], tid, NT);
+        tma_issue_layer<N, RR>(maps, 0, L - 1 - i, tile_geom(s_pos[i], 0, y0), tiles + (i & 1) * TILE, &bar[i & 1], tid, NT);
     };
     issue(0);
     if (L > 1) issue(1);
-    const InstDev* I0 = a.inst + a.pslots[J.first];
+    load_members(0);  // read after the layers' barriers
     float hi[QPT][RR][4], lo[QPT][RR][4];
 #pragma unroll
     for (int q = 0; q < QPT; q++)
@@ -715,8 +736,8 @@ __global__ void __launch_bounds__(NT) k_phase_frames(const __grid_constant__ Pas
             if (i + 1 < L) cta_wait_tile(&bar[(i + 1) & 1], ((i + 1) >> 1) & 1, a.d_status);
             return;
         }
-        const TileGeom g = tile_geom(pos[L - 1 - i], 0, y0);
-        const float sc = J.factored ? 1.0f : I0->scoeff[L - 1 - i];
+        const TileGeom g = tile_geom(s_pos[i], 0, y0);
+        const float sc = s_sc[i];
         float wx[4], wy[4];
         keys_weights(g.fx, wx);
         keys_weights(g.fy, wy);
@@ -740,12 +761,16 @@ __global__ void __launch_bounds__(NT) k_phase_frames(const __grid_constant__ Pas
         if (i + 2 < L) issue(i + 2);
     }
     for (int m = 0; m < J.count; m++) {
-        const InstDev* I = a.inst + a.pslots[J.first + m];
-        const int off = I->off, Nout = I->Nout;
-        const size_t slot = (size_t)(step % I->ring) * I->ostride;
-        float* __restrict__ opha = I->out_pha + slot;
-        float* __restrict__ oamp = I->out_amp + slot;
-        const float sg = I->scoeff[0];
+        if (m > 0 && m % NM == 0) {
+            __syncthreads();
+            load_members(m);
+            __syncthreads();
+        }
+        const Member& M = s_mem[m % NM];
+        const int off = M.off, Nout = M.Nout;
+        float* __restrict__ opha = M.pha;
+        float* __restrict__ oamp = M.amp;
+        const float sg = M.sg;
         const bool v4 = (off % 4) == 0 && (Nout % 4) == 0 && (reinterpret_cast<uintptr_t>(opha) & 15) == 0 &&
                         (reinterpret_cast<uintptr_t>(oamp) & 15) == 0;
 #pragma unroll
@@ -897,15 +922,19 @@ cudaError_t launch_pass_t(int var, dim3 grid, const PassArgs& a, const TmaSet* m
             return launch_gated_up_to(a.pdl_ctas, k_layer_windows<N, WR, WT>, grid, dim3(WT), sm, st, a, *maps);
         }
         case kVarPhases: {
-            constexpr int PR = phase_rows(N), PT = phase_threads(N);
-            constexpr size_t sm = 2 * PassGeom<N, PR>::TILE_BYTES + 128;
-            static bool attr = false;
-            if (!attr) {
-                cudaError_t e = cudaFuncSetAttribute(k_phase_frames<N, PR, PT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-                if (e != cudaSuccess) return e;
-                attr = true;
+            constexpr int PT = phase_threads(N);
+            auto go = [&](auto kern, size_t tile) -> cudaError_t {
+                const size_t sm = 2 * tile + 128;
+                const cudaError_t e = sm > 40 * 1024 ? cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm)
+                                                     : cudaSuccess;
+                return e != cudaSuccess ? e : launch_gated_up_to(a.pdl_ctas, kern, grid, dim3(PT), sm, st, a, *maps);
+            };
+            if constexpr (N <= kPhaseSmallMax) {
+                constexpr int SR = phase_rows(N, true);
+                if (a.phase_small) return go(k_phase_frames<N, SR, PT>, PassGeom<N, SR>::TILE_BYTES);
             }
-            return launch_gated_up_to(a.pdl_ctas, k_phase_frames<N, PR, PT>, grid, dim3(PT), sm, st, a, *maps);
+            constexpr int PR = phase_rows(N, false);
+            return go(k_phase_frames<N, PR, PT>, PassGeom<N, PR>::TILE_BYTES);
         }
         default: return cudaErrorInvalidValue;
     }
