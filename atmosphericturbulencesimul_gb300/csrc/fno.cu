@@ -906,7 +906,8 @@ cudaError_t pointwise_fwd(const __nv_bfloat16* W, int o, int c, const void* X, i
                           float beta, const float* bias, cudaStream_t st, void* act = nullptr, int a_bf16 = 0,
                           bool keep_c = true)
 {
-    if (umma_enabled() && pointwise_umma_supported(o, c) && P % 8 == 0) {
+    // (a caller's input may lie on any element)
+    if (umma_enabled() && pointwise_umma_supported(o, c) && P % 8 == 0 && (reinterpret_cast<uintptr_t>(X) & 15) == 0) {
         unsigned* status = umma_status_ptr();
         if (!status) return cudaErrorUnknown;
         return pointwise_umma(W, o, c, X, x_bf16, C, B, P, beta, bias, act, a_bf16, status, 0, keep_c || !act, st);

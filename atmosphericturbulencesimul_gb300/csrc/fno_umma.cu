@@ -219,7 +219,7 @@ template <int O, int C, typename TX, typename TA, int CR = C>
 cudaError_t launch(const __nv_bfloat16* W, const TX* X, float* Cm, TA* act, const float* bias, float beta, int B, long P,
                    unsigned* status, int swap, int write_c, cudaStream_t st)
 {
-    if (P % 8 != 0) return cudaErrorNotSupported;  // 16-byte copies of the channel rows
+    if (P % 8 != 0 || (reinterpret_cast<uintptr_t>(X) & 15)) return cudaErrorNotSupported;  // 16-byte copies of the channel rows
     // shared memory: the staging buffer, A and B; at most three CTAs per SM
     // (registers), whose TMEM allocations (at most 128 columns) fit the 512
     constexpr size_t smem = (size_t)C * kM * sizeof(TX) + (size_t)kM * C * 2 + (size_t)O * C * 2;
@@ -732,8 +732,9 @@ extern "C" atmwfs_status atmwfs_fno_pointwise_dev(const void* W, int o, int c, c
     }
     const cudaError_t e = pointwise_umma(w, o, c, X, 0, C, batch, P, beta, bias, act, 0, status, engine == 2, true, st);
     if (e != cudaSuccess) {
-        set_error_message(cudaGetErrorString(e));
-        return ATMWFS_ERR_CUDA;
+        set_error_message(e == cudaErrorNotSupported ? "atmwfs_fno_pointwise_dev: X is read in 16-byte pieces"
+                                                     : cudaGetErrorString(e));
+        return e == cudaErrorNotSupported ? ATMWFS_ERR_INVALID : ATMWFS_ERR_CUDA;
     }
     return ATMWFS_OK;
 }
@@ -746,8 +747,8 @@ extern "C" atmwfs_status atmwfs_fno_spectral_dev(const void* W, int o, int c, co
         set_error_message("atmwfs_fno_spectral_dev: bad arguments");
         return ATMWFS_ERR_INVALID;
     }
-    if (!spectral_umma_supported(o, c) || P % 8 != 0) {
-        set_error_message("atmwfs_fno_spectral_dev: shape not compiled for the tcgen05 product");
+    if (!spectral_umma_supported(o, c) || P % 8 != 0 || (reinterpret_cast<uintptr_t>(X) & 15)) {
+        set_error_message("atmwfs_fno_spectral_dev: shape not compiled for the tcgen05 product, or X not on 16 bytes");
         return ATMWFS_ERR_INVALID;
     }
     unsigned* status = umma_status_ptr();
