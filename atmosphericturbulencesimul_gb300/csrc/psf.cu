@@ -17,7 +17,6 @@
 // frame (amplitude + phase) read, 2 x 16 W^2 B of intermediate written and
 // read, and 8 (2W)^2 / batch B of accumulator update.
 #include <algorithm>
-#include <cfloat>
 #include <cmath>
 #include <cstdio>
 #include <vector>
@@ -25,7 +24,7 @@
 #include "atmwfs_psf.h"
 #include "aux_kernels.cuh"
 #include "pass_impl.cuh"
-#include "atan_ff.cuh"
+#include "chromat_ff.cuh"
 #include "workspace.cuh"
 
 namespace atmwfs {
@@ -169,37 +168,13 @@ __global__ void k_expo_layout(const float* __restrict__ src, float* __restrict__
 // accumulation is in float.  I_s is centred on read: I(j, i) =
 // I_s[(i + h) % n][(j + h) % n].
 //
-// The reference's double expressions, (1 - u)(1 - t) v00 and two more, each
-// rounded to float, are evaluated in float-float: 1 - u as an exact pair, the
-// products as exact two-products, one rounding at the end -- the float of the
-// double expression except when that lies within about 2^-46 of a midpoint.
+// The taps are added in FP32 arithmetic with the reference's result (chromat_ff.cuh).
 // In doubles the FP64 pipe bounded the sum, and with the lanes along ii every
 // tap was a gather over 32 rows of I_s (lanes now run along jj): 365 us for 40
-// steps of 512^2.
-__device__ __forceinline__ void ff_mul_f(float ah, float al, float b, float& h, float& l)
+// steps of 512^2, now 66 (60 without the rounding test).
+__device__ __noinline__ float chromat_taps_slow(float u, float t, float v00, float v01, float v10, float v11)
 {
-    h = ff_mul(ah, b);
-    l = ff_fma(ah, b, -h);
-    l = ff_fma(al, b, l);
-}
-
-// (ah + al) (bh + bl) v as a pair: the weight is exact to 2^-48, v a float.  An
-// infinite or undefined product keeps its value (its error term has none).
-__device__ __forceinline__ void tap(float ah, float al, float bh, float bl, float v, float& h, float& l)
-{
-    float wh = ff_mul(ah, bh);
-    float wl = ff_fma(ah, bh, -wh);
-    wl = ff_fma(ah, bl, ff_fma(al, bh, wl));
-    ff_mul_f(wh, wl, v, h, l);
-    if (!(fabsf(h) <= FLT_MAX)) l = 0.0f;
-}
-
-// float(t + (h + l))
-__device__ __forceinline__ float add_pair(float t, float h, float l)
-{
-    float s, e;
-    ff_two_sum(t, h, s, e);
-    return fabsf(s) <= FLT_MAX ? ff_add(s, ff_add(e, l)) : s;
+    return chromat_taps_f64(u, t, v00, v01, v10, v11);
 }
 
 __global__ void __launch_bounds__(256) k_chromat_sum(const float* __restrict__ I, int S, int n, const float* __restrict__ coeff,
@@ -221,16 +196,8 @@ __global__ void __launch_bounds__(256) k_chromat_sum(const float* __restrict__ I
             const float* r1 = I + (size_t)s * np + (size_t)((i + 1 + h) & mk) * n;
             const int j0 = (j + h) & mk, j1 = (j + 1 + h) & mk;
             const float v00 = r0[j0], v01 = r0[j1], v10 = r1[j0], v11 = r1[j1];
-            float duh, dul, dth, dtl, a, b;
-            ff_two_sum(1.0f, -u, duh, dul);
-            ff_two_sum(1.0f, -t, dth, dtl);
-            tap(duh, dul, dth, dtl, v00, a, b);
-            float tmp = ff_add(a, b);
-            tap(duh, dul, t, 0.0f, v01, a, b);
-            tmp = add_pair(tmp, a, b);
-            tap(u, 0.0f, dth, dtl, v10, a, b);
-            tmp = add_pair(tmp, a, b);
-            tmp = __fadd_rn(tmp, __fmul_rn(__fmul_rn(u, t), v11));   // u * t * F: float arithmetic
+            float tmp;
+            if (!chromat_taps(u, t, v00, v01, v10, v11, tmp)) tmp = chromat_taps_slow(u, t, v00, v01, v10, v11);
             acc = __fadd_rn(acc, __fdiv_rn(__fdiv_rn(__fmul_rn(mcoeff[s], tmp), c), c));
         }
     }
