@@ -3,15 +3,16 @@
 // each sum to float (psf.c:54-136):
 //   s = (1-u)(1-t) v00,  s = s + (1-u) t v01,  s = s + u (1-t) v10.
 // The FP64 pipe bounded the zoom, so the sums are formed in float-float (pairs
-// hi + lo): 1 - u as an exact pair, the products as exact two-products.  A sum
-// of non-negative terms is within 2^-43.5 of the exact one this way and the
-// reference's own within 2^-50; where all values within 2^-42 of the pair round
-// to one float, that float is the reference's (Ziv's rounding test, "Fast
-// evaluation of elementary mathematical functions with correctly rounded last
-// bit", ACM TOMS 17, 1991).  The rest -- a sum beside a midpoint, about one pixel
-// in 60,000, a first tap below 2^-80, after which error terms may underflow,
-// infinities and NaN -- is left to the double expressions.  Host-compilable, checked against
-// them on the CPU.
+// hi + lo): 1 - u as an exact pair, the products as exact two-products.  A sum is
+// within 2^-43.5 of the exact one this way and the reference's own within 2^-50,
+// both relative to the size of its terms (a position between -1 and 0 belongs to
+// pixel 0, where u < 0 and taps are subtracted); where all values within 2^-42 of
+// that size around the pair round to one float, that float is the reference's
+// (Ziv's rounding test, "Fast evaluation of elementary mathematical functions with
+// correctly rounded last bit", ACM TOMS 17, 1991).  The rest -- a sum beside a
+// midpoint, about one pixel in 50,000, terms below 2^-80, whose errors may
+// underflow, infinities and NaN -- is left to the double expressions.
+// Host-compilable, checked against them on the CPU.
 #pragma once
 #include "atan_ff.cuh"
 
@@ -27,21 +28,24 @@ AW_HD float chromat_taps_f64(float u, float t, float v00, float v01, float v10, 
     return ff_add(s, ff_mul(ff_mul(u, t), v11));
 }
 
-// s = float(r + e), |e| <= 2^-22 r; false: values within 2^-42 of it round otherwise.
-AW_HD bool chromat_round(float r, float e, float& s)
+// s = float(r + e), m the size of what was added; false: values within 2^-42 m
+// of r + e round otherwise.
+AW_HD bool chromat_round(float r, float e, float m, float& s)
 {
-    const float d = ff_mul(r, 0x1p-42f);
+    const float d = ff_mul(m, 0x1p-42f);
     s = ff_add(r, ff_sub(e, d));
     return s == ff_add(r, ff_add(e, d));
 }
 
-// s = float(s + (wh + wl) v)
-AW_HD bool chromat_add(float wh, float wl, float v, float& s)
+// s = float(s + (wh + wl) v); m: the smaller of m and the size of the terms.
+AW_HD bool chromat_add(float wh, float wl, float v, float& s, float& m)
 {
     const float h = ff_mul(wh, v), l = ff_fma(wl, v, ff_fma(wh, v, -h));
     float r, e;
     ff_two_sum(s, h, r, e);
-    return chromat_round(r, ff_add(e, l), s);
+    const float n = ff_add(fabsf(r), fabsf(h));
+    m = fminf(m, n);
+    return chromat_round(r, ff_add(e, l), n, s);
 }
 
 // The bilinear value; false: chromat_taps_f64 has to say.
@@ -54,11 +58,11 @@ AW_HD bool chromat_taps(float u, float t, float v00, float v01, float v10, float
     const float w0l = ff_fma(duh, dtl, ff_fma(dul, dth, ff_fma(duh, dth, -w0)));
     const float w1l = ff_fma(dul, t, ff_fma(duh, t, -w1)), w2l = ff_fma(u, dtl, ff_fma(u, dth, -w2));
     const float h = ff_mul(w0, v00);
-    bool sure = chromat_round(h, ff_fma(w0l, v00, ff_fma(w0, v00, -h)), s);
-    sure = chromat_add(w1, w1l, v01, s) && sure;
-    sure = chromat_add(w2, w2l, v10, s) && sure;
-    // the sums grow from the first tap's h, whose weight is not 0
-    sure = sure && (h >= 0x1p-80f || (v00 == 0.0f && v01 == 0.0f && v10 == 0.0f));
+    float m = fabsf(h);
+    bool sure = chromat_round(h, ff_fma(w0l, v00, ff_fma(w0, v00, -h)), m, s);
+    sure = chromat_add(w1, w1l, v01, s, m) && sure;
+    sure = chromat_add(w2, w2l, v10, s, m) && sure;
+    sure = sure && (m >= 0x1p-80f || (v00 == 0.0f && v01 == 0.0f && v10 == 0.0f));
     out = ff_add(s, ff_mul(ff_mul(u, t), v11));
     return sure;
 }

@@ -30,7 +30,8 @@ static bool same(float a, float b)
     return x == y;
 }
 
-// f() in [0, 1) for the fractions, v() for the four values
+// f() in (-1, 1) for the fractions (a position between -1 and 0 belongs to pixel
+// 0, so that its weights exceed 1 and two taps are subtracted), v() for the values
 template <typename Fn, typename Vn>
 static void check(const char* name, long n, Fn f, Vn v)
 {
@@ -59,7 +60,14 @@ int main()
         return r < 0.2 ? std::numeric_limits<float>::infinity() : r < 0.4 ? std::numeric_limits<float>::quiet_NaN()
                                                                 : r < 0.6 ? 3.4e38f : r < 0.8 ? 0.0f : (float)urand();
     };
+    auto either = [] { return (float)(1.9999999 * urand() - 0.9999999); };
+    auto few_either = [] { return (float)((int)(urand() * 31) - 15) / 16.0f; };
+    auto close = [] { return (float)(1.0 + 1e-3 * urand()); };                            // the taps nearly cancel
     check("psf", 20000000, frac, psf);
+    check("outside", 10000000, either, psf);
+    check("outside_few", 5000000, few_either, ints);
+    check("outside_close", 5000000, either, close);
+    check("outside_wide", 5000000, either, wide);
     check("psf_tiny_fractions", 5000000, tiny, psf);
     check("psf_few_fractions", 5000000, few, psf);
     check("ties", 5000000, few, ints);

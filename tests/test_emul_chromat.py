@@ -25,7 +25,7 @@ def chromat(tmp_path_factory):
     return {l.split()[0]: tuple(map(float, l.split()[1:])) for l in out.strip().splitlines()}
 
 
-@pytest.mark.parametrize("name", ["psf", "psf_tiny_fractions", "psf_few_fractions", "ties", "dark", "dark_few", "zero",
+@pytest.mark.parametrize("name", ["psf", "outside", "outside_few", "outside_close", "outside_wide", "psf_tiny_fractions", "psf_few_fractions", "ties", "dark", "dark_few", "zero",
                                   "wide", "wide_tiny", "faint", "nonfinite"])
 def test_the_doubles_result(chromat, name):
     count, differ, _ = chromat[name]
@@ -33,5 +33,5 @@ def test_the_doubles_result(chromat, name):
 
 
 def test_the_doubles_are_rare_on_psfs(chromat):
-    assert chromat["psf"][2] < 1e-4
+    assert chromat["psf"][2] < 1e-4 and chromat["outside"][2] < 1e-4
     assert chromat["zero"][2] == 0
