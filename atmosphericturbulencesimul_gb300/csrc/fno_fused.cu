@@ -12,10 +12,11 @@
 //   k_layer_bwd  a layer's GELU gradient, its weight and bias gradients and
 //              the transposed inverse DFT along x, from one read of the line;
 //   k_project_bwd  every gradient of the head, without storing dq.
-// The products keep the operands' BF16 rounding, the K order and the FP32
-// accumulation of the separate products (k_pointwise, k_rowprod, the mma.sync
-// GEMM), so a layer's activations and gradients are the same bits (sums over
-// pixels, which were atomic before, are not).
+// The products keep the operands' BF16 rounding and the FP32 accumulation of the
+// separate products (k_pointwise, k_rowprod, the mma.sync GEMM).  The order of
+// the additions is not the same everywhere (the head's two outputs, sums over
+// pixels), so results agree to FP32 rounding, not in every bit: outputs to 2e-7 of
+// their scale with the tcgen05 products.
 //
 // Spectral images here are planar with the channels fastest, so that a
 // mode's values of every channel are one run (the mode mixing) and a
