@@ -5,6 +5,7 @@
 #include "atmwfs.h"
 #include "atmwfs_fno.h"
 #include "fno_gemm.cuh"
+#include "smem_limit.cuh"
 
 namespace atmwfs {
 
@@ -28,12 +29,8 @@ template <int BM, int BN>
 cudaError_t launch_tile(dim3 grid, const GemmArgs& g, cudaStream_t st)
 {
     constexpr size_t sm = gemm::stage_bytes(BM, BN);
-    static bool attr = false;
-    if (!attr) {
-        const cudaError_t e = cudaFuncSetAttribute(gemm::k_gemm<BM, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-        if (e != cudaSuccess) return e;
-        attr = true;
-    }
+    static SmemLimit limit;
+    if (const cudaError_t e = limit.raise(gemm::k_gemm<BM, BN>, sm)) return e;
     gemm::k_gemm<BM, BN><<<grid, 256, sm, st>>>(g);
     return cudaGetLastError();
 }

@@ -24,6 +24,7 @@
 
 #include "atmwfs_fno.h"
 #include "fno_gemm.cuh"
+#include "smem_limit.cuh"
 #include "umma_core.cuh"
 
 namespace atmwfs {
@@ -223,13 +224,8 @@ cudaError_t launch(const __nv_bfloat16* W, const TX* X, float* Cm, TA* act, cons
     // shared memory: the staging buffer, A and B; at most three CTAs per SM
     // (registers), whose TMEM allocations (at most 128 columns) fit the 512
     constexpr size_t smem = (size_t)C * kM * sizeof(TX) + (size_t)kM * C * 2 + (size_t)O * C * 2;
-    static bool attr = false;
-    if (!attr) {
-        cudaError_t e = cudaFuncSetAttribute(k_pointwise<O, C, TX, TA, CR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)smem);
-        if (e != cudaSuccess) return e;
-        attr = true;
-    }
+    static SmemLimit limit;
+    if (const cudaError_t e = limit.raise(k_pointwise<O, C, TX, TA, CR>, smem)) return e;
     const long tiles = (long)B * ((P + kM - 1) / kM);
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
@@ -426,12 +422,8 @@ cudaError_t launch_chunked(const __nv_bfloat16* W, const float* X, float* Cm, lo
 {
     if (P % 8 != 0) return cudaErrorNotSupported;
     constexpr size_t smem = (size_t)kKch * kM * 4 + (size_t)kM * kKch * 2 + (size_t)O * C * 2;
-    static bool attr = false;
-    if (!attr) {
-        cudaError_t e = cudaFuncSetAttribute(k_chunked<O, C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-        attr = true;
-    }
+    static SmemLimit limit;
+    if (const cudaError_t e = limit.raise(k_chunked<O, C>, smem)) return e;
     const long tiles = (P + kM - 1) / kM;
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
@@ -629,12 +621,8 @@ cudaError_t launch_rowprod(const __nv_bfloat16* Bt, const RowMaps& g, unsigned* 
         g.c_nhi % 4 || (reinterpret_cast<uintptr_t>(g.A) & 15) || (reinterpret_cast<uintptr_t>(g.C) & 15))
         return cudaErrorNotSupported;  // 16-byte pieces of A rows and C rows
     constexpr size_t smem = (size_t)kM * kKch * 4 + (size_t)kM * kKch * 2 + (size_t)N * K * 2;
-    static bool attr = false;
-    if (!attr) {
-        cudaError_t e = cudaFuncSetAttribute(k_rowprod<N, K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-        attr = true;
-    }
+    static SmemLimit limit;
+    if (const cudaError_t e = limit.raise(k_rowprod<N, K>, smem)) return e;
     const long tiles = (g.M + kM - 1) / kM;
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);

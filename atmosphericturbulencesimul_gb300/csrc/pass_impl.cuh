@@ -12,6 +12,7 @@
 #include "epi_math.cuh"
 #include "fft_half.cuh"
 #include "gather_core.cuh"
+#include "smem_limit.cuh"
 
 namespace atmwfs {
 
@@ -876,12 +877,9 @@ cudaError_t launch_pass_t(int var, dim3 grid, const PassArgs& a, const TmaSet* m
 #define AW_CASE(VAR)                                                                                   \
     case VAR: {                                                                                        \
         constexpr size_t sm = G::smem(VAR, HS);                                                        \
-        static bool attr = false;                                                                      \
-        if (!attr) {                                                                                   \
-            cudaError_t e = cudaFuncSetAttribute(k_pass<N, RR, MINB, VAR, ALIAS, HP, V, HS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm); \
-            if (e != cudaSuccess) return e;                                                            \
-            attr = true;                                                                               \
-        }                                                                                              \
+        static SmemLimit limit;                                                                        \
+        const cudaError_t e = limit.raise(k_pass<N, RR, MINB, VAR, ALIAS, HP, V, HS>, sm);             \
+        if (e != cudaSuccess) return e;                                                                \
         return launch_gated_up_to(I_SERIES(VAR) ? a.pdl_ctas : kUnitPdlWaves * pdl_max_ctas(), k_pass<N, RR, MINB, VAR, ALIAS, HP, V, HS>, grid, block, sm, st, a, tw); \
     }
     if constexpr (UNIT) {
@@ -913,28 +911,25 @@ cudaError_t launch_pass_t(int var, dim3 grid, const PassArgs& a, const TmaSet* m
         case kVarWindows: {
             constexpr int WR = win_rows(N), WT = win_threads(N);
             constexpr size_t sm = PassGeom<N, WR>::TILE_BYTES + 128;
-            static bool attr = false;
-            if (!attr) {
-                cudaError_t e = cudaFuncSetAttribute(k_layer_windows<N, WR, WT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-                if (e != cudaSuccess) return e;
-                attr = true;
-            }
+            static SmemLimit limit;
+            const cudaError_t e = limit.raise(k_layer_windows<N, WR, WT>, sm);
+            if (e != cudaSuccess) return e;
             return launch_gated_up_to(a.pdl_ctas, k_layer_windows<N, WR, WT>, grid, dim3(WT), sm, st, a, *maps);
         }
         case kVarPhases: {
             constexpr int PT = phase_threads(N);
-            auto go = [&](auto kern, size_t tile) -> cudaError_t {
+            auto go = [&](auto kern, SmemLimit& limit, size_t tile) -> cudaError_t {
                 const size_t sm = 2 * tile + 128;
-                const cudaError_t e = sm > 40 * 1024 ? cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm)
-                                                     : cudaSuccess;
+                const cudaError_t e = limit.raise(kern, sm);
                 return e != cudaSuccess ? e : launch_gated_up_to(a.pdl_ctas, kern, grid, dim3(PT), sm, st, a, *maps);
             };
+            static SmemLimit large, small;
             if constexpr (N <= kPhaseSmallMax) {
                 constexpr int SR = phase_rows(N, true);
-                if (a.phase_small) return go(k_phase_frames<N, SR, PT>, PassGeom<N, SR>::TILE_BYTES);
+                if (a.phase_small) return go(k_phase_frames<N, SR, PT>, small, PassGeom<N, SR>::TILE_BYTES);
             }
             constexpr int PR = phase_rows(N, false);
-            return go(k_phase_frames<N, PR, PT>, PassGeom<N, PR>::TILE_BYTES);
+            return go(k_phase_frames<N, PR, PT>, large, PassGeom<N, PR>::TILE_BYTES);
         }
         default: return cudaErrorInvalidValue;
     }
