@@ -163,6 +163,7 @@ SIGNATURES = [
     ("atmwfs_fft2d", C.c_int, [_fp, _fp, C.c_long, C.c_int]),
     ("atmwfs_fft2d_dev", C.c_int, [C.c_void_p, C.c_void_p, C.c_long, C.c_int, C.c_void_p]),
     ("atmwfs_master_screen", C.c_int, [C.c_uint64, C.c_uint32, C.c_long, C.c_double, C.c_double, _fp, _fp, _dp]),
+    ("atmwfs_release_workspaces", None, []),
     ("atmwfs_last_error", C.c_char_p, []),
     # include/atmwfs_mkwfs.h
     ("atmwfs_conf_read", C.c_int, [C.c_char_p, C.c_char_p, C.c_char_p, C.c_long]),

@@ -175,7 +175,7 @@ static const float2* twiddles(int N, int V = 0)
     const std::vector<float2> h = host_twiddles(N, V);
     if (h.empty()) return nullptr;
     float2* d = nullptr;
-    if (cudaMalloc(&d, sizeof(float2) * h.size()) != cudaSuccess) return nullptr;
+    if (device_malloc((void**)&d, sizeof(float2) * h.size()) != cudaSuccess) return nullptr;
     if (cudaMemcpy(d, h.data(), sizeof(float2) * h.size(), cudaMemcpyHostToDevice) != cudaSuccess) return nullptr;
     cache[key] = d;
     return d;
@@ -201,7 +201,7 @@ static const __half2* twiddles_half(int N)
     std::vector<__half2> hh(h.size());
     for (size_t i = 0; i < h.size(); i++) hh[i] = __floats2half2_rn(h[i].x, h[i].y);
     __half2* d = nullptr;
-    if (cudaMalloc(&d, sizeof(__half2) * hh.size()) != cudaSuccess) return nullptr;
+    if (device_malloc((void**)&d, sizeof(__half2) * hh.size()) != cudaSuccess) return nullptr;
     if (cudaMemcpy(d, hh.data(), sizeof(__half2) * hh.size(), cudaMemcpyHostToDevice) != cudaSuccess) return nullptr;
     cache[key] = d;
     return d;
@@ -398,7 +398,7 @@ namespace {
 
 atmwfs_status dalloc(atmwfs_ctx* c, void** p, size_t bytes)
 {
-    cudaError_t e = cudaMalloc(p, bytes);
+    cudaError_t e = device_malloc(p, bytes);
     if (e != cudaSuccess) return fail(ATMWFS_ERR_NOMEM, "cudaMalloc(%zu) failed: %s", bytes, cudaGetErrorString(e));
     c->allocs.push_back(*p);
     return ATMWFS_OK;
@@ -1381,8 +1381,8 @@ atmwfs_status atmwfs_normalize_screens_ext(atmwfs_ctx* c, float lambda_ref, floa
     double* acc = nullptr;
     float* ext = nullptr;
     atmwfs_status s = ATMWFS_OK;
-    if (cudaMalloc(&acc, sizeof(double) * nm) != cudaSuccess ||
-        (nextra > 0 && cudaMalloc(&ext, sizeof(float) * M2 * nextra) != cudaSuccess))
+    if (device_malloc((void**)&acc, sizeof(double) * nm) != cudaSuccess ||
+        (nextra > 0 && device_malloc((void**)&ext, sizeof(float) * M2 * nextra) != cudaSuccess))
         s = fail(ATMWFS_ERR_NOMEM, "cudaMalloc failed");
     for (long e = 0; e < nextra && s == ATMWFS_OK; e++) {
         scr.push_back(ext + M2 * e);

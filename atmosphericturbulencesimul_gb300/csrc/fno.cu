@@ -154,7 +154,7 @@ atmwfs_status err(atmwfs_status s, const char* fmt, ...)
 
 atmwfs_status dalloc(atmwfs_fno* f, void** p, size_t bytes)
 {
-    if (cudaMalloc(p, bytes) != cudaSuccess) return err(ATMWFS_ERR_NOMEM, "cudaMalloc(%zu) failed", bytes);
+    if (device_malloc(p, bytes) != cudaSuccess) return err(ATMWFS_ERR_NOMEM, "cudaMalloc(%zu) failed", bytes);
     f->allocs.push_back(*p);
     return ATMWFS_OK;
 }

@@ -9,13 +9,16 @@ namespace atmwfs {
 // device.  The pool keeps up to kWorkspaceKeep bytes of what calls have freed,
 // so that a call need not map and unmap its buffers (cudaMalloc / cudaFree, or
 // the default pool, which returns everything at the next synchronisation: an
-// 8192^2 transform waited 1.3 of 2.2 ms for that); it is emptied when an
-// engine context or a surrogate is destroyed.  Any thread and stream may
-// allocate and free; a buffer is used on the stream it was allocated on.
+// 8192^2 transform waited 1.3 of 2.2 ms for that); what it keeps is given back
+// when an engine context or a surrogate is destroyed, when an allocation of the
+// library finds too little memory, and by atmwfs_release_workspaces.  Any thread
+// and stream may allocate and free; a buffer is used on the stream it was
+// allocated on.
 constexpr size_t kWorkspaceKeep = size_t(1) << 30;
 cudaError_t workspace_alloc(void** p, size_t bytes, cudaStream_t st);
-void workspace_free(void* p, cudaStream_t st);   // p may be null
-void workspace_release();                        // give back what the pool keeps
+void workspace_free(void* p, cudaStream_t st);          // p may be null
+cudaError_t device_malloc(void** p, size_t bytes);      // cudaMalloc of what outlives a call
+void workspace_release();                               // give back what the pools of all devices keep
 
 // A workspace of one scope.
 class Workspace {

@@ -274,6 +274,11 @@ def fft2d(a: np.ndarray, sign: int = -1) -> np.ndarray:
     return out
 
 
+def release_workspaces() -> None:
+    """Give back the device memory (at most 1 GiB per device) that single calls keep for the next one."""
+    _lib.load().atmwfs_release_workspaces()
+
+
 def master_screen(seed: int, M: int, outer_pix: float, inner_pix: float, stream: int = 0):
     """Seeded von Karman master screen pair and the structure-function constants."""
     lib = _lib.load()

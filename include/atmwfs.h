@@ -250,6 +250,15 @@ atmwfs_status atmwfs_fft2d_dev(const void* in, void* out, long n, int sign, void
 atmwfs_status atmwfs_master_screen(uint64_t seed, uint32_t stream, long M, double outer_pix, double inner_pix,
                                    float* out1, float* out2, double* cfit);
 
+/* Calls that keep no context (transforms, hops, master screens and the PSFs of
+ * atmwfs_psf.h; not atmwfs_fresnel_noalloc) take their device buffers from a
+ * memory pool of the library, one per device, which keeps up to 1 GiB of what
+ * they have freed for the next call.  It is given back when an engine context or
+ * a surrogate is destroyed, when an allocation of the library finds too little
+ * device memory, and by this call (all devices; buffers still in use by work on a
+ * stream stay). */
+void atmwfs_release_workspaces(void);
+
 /* Last error message of this thread. */
 const char* atmwfs_last_error(void);
 
