@@ -738,6 +738,7 @@ atmwfs_status ensure_batch(atmwfs_fno* f, int B)
     for (float** p : {&f->y, &f->bb, &f->qpre, &f->q, &f->dh, &f->dh2, &f->du, &f->dq, &f->dz, &f->dy,
                       &f->da, &f->dbb, &f->dout})
         drop(*p);
+    f->cap = 0;  // until all of the new set is there
     const atmwfs_fno_cfg& c = f->cfg;
     const size_t P = (size_t)c.grid * c.grid;
     const size_t act = (size_t)B * c.width * P * 4, spa = (size_t)B * c.width * c.grid * 2 * c.modes * 4,
