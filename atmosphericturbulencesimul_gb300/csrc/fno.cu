@@ -921,9 +921,11 @@ cudaError_t pointwise_fwd(const __nv_bfloat16* W, int o, int c, const void* X, i
 // reads are not stored.  With ATMWFS_FNO_BF16_ACT=1 (tcgen05 path) the
 // activations between the Fourier layers (h[1..]) and of the projection (q)
 // are also stored as BF16, which changes no value (every product that reads
-// them rounds its operands to BF16) but measured slower (4,180 against
-// 4,460 frames/s at 256^2: the spectral product reads its BF16 operand in
-// 8-byte pieces), so FP32 storage is the default.
+// them rounds its operands to BF16) but is slower: 4,180 against 4,460 frames/s
+// on the separate products (the spectral product reads its BF16 operand in
+// 8-byte pieces), and the fused kernels of the default shape, which read FP32,
+// are left for these products (3,150 against 1,121 us for 16 frames).  FP32
+// storage is the default.
 atmwfs_status forward(atmwfs_fno* f, const float* x, float* out, int B, cudaStream_t st, bool training)
 {
     const atmwfs_fno_cfg& c = f->cfg;

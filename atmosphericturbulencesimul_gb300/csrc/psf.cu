@@ -171,7 +171,7 @@ __global__ void k_expo_layout(const float* __restrict__ src, float* __restrict__
 // The taps are added in FP32 arithmetic with the reference's result (chromat_ff.cuh).
 // In doubles the FP64 pipe bounded the sum, and with the lanes along ii every
 // tap was a gather over 32 rows of I_s (lanes now run along jj): 365 us for 40
-// steps of 512^2, now 66 (60 without the rounding test).
+// steps of 512^2, now 68 (59 without the rounding test).
 __device__ __noinline__ float chromat_taps_slow(float u, float t, float v00, float v01, float v10, float v11)
 {
     return chromat_taps_f64(u, t, v00, v01, v10, v11);

@@ -86,7 +86,8 @@ atmwfs_status atmwfs_gemm_bf16(int M, int N, int K, const void* A, long lda, int
  * C[b] (o x P) = W (o x c, BF16) X[b] (c x P, FP32) + bias[o] + beta C[b],
  * act[b] = gelu(C[b]) if act is not NULL, on the tcgen05 tensor cores
  * (accumulator in tensor memory), compiled for o x c = 64 x 64 and 128 x 64, and
- * 64 x 8 without act (the lift: K padded to 16 with zero channels).
+ * 64 x 8 without act (the lift: K padded to 16 with zero channels).  X on a
+ * 16-byte boundary, P a multiple of 8, else ATMWFS_ERR_INVALID.
  * engine 1: the product the network uses; 2: the same with the two
  * core-matrix strides of its shared-memory descriptors exchanged (a check
  * that only engine 1 matches the FP32 product). */
@@ -96,7 +97,8 @@ atmwfs_status atmwfs_fno_pointwise_dev(const void* W, int o, int c, const float*
  * (no counterpart in the reference): C (o x P) = W (o x c, BF16) X (c x P,
  * FP32, rounded to BF16), K taken in chunks of 64 accumulated in tensor
  * memory; compiled for o x c = 64 x 512 (the forward DFT of a 256 grid with
- * 32 modes) and 512 x 64 (its inverse); P a multiple of 8.  engine as for
+ * 32 modes) and 512 x 64 (its inverse); P a multiple of 8 and X on a 16-byte
+ * boundary.  engine as for
  * atmwfs_fno_pointwise_dev. */
 atmwfs_status atmwfs_fno_spectral_dev(const void* W, int o, int c, const float* X, float* C, long P, int engine,
                                       void* stream);
